@@ -687,6 +687,30 @@ BehlerFn make_fn(double Rc, double p1, double p2, double p3, int kind, int out) 
   return b;
 }
 
+// The evaluation order of a grid's powers (BehlerGrid::chain, general).
+void grid_powers(BehlerGrid& gr) {
+  int count[2] = {0, 0};
+  std::fill(&gr.general[0][0], &gr.general[0][0] + 2 * (AE_BG_NL + AE_BG_NZ), -1);
+  std::fill(&gr.slot[0][0], &gr.slot[0][0] + 2 * AE_BG_NZ, -1);
+  std::vector<int> zs;
+  bool powers = true;
+  for (int l = 0; l < gr.nl; ++l) {
+    const int s = gr.lam[l] > 0.0 ? 0 : 1, z = gr.izeta[l];
+    gr.general[s][count[s]++] = l;
+    if (z <= 0 || (z & (z - 1))) powers = false;
+    if (std::find(zs.begin(), zs.end(), z) == zs.end()) zs.push_back(z);
+  }
+  gr.ngeneral = std::max(count[0], count[1]);
+  std::sort(zs.begin(), zs.end());
+  gr.chain = powers && (int)zs.size() <= AE_BG_NZ ? (int)zs.size() : 0;
+  int at = 1;
+  for (int i = 0; i < gr.chain; ++i) {
+    for (gr.sq[i] = 0; at < zs[i]; at *= 2) ++gr.sq[i];
+    for (int l = 0; l < gr.nl; ++l)
+      if (gr.izeta[l] == zs[i]) gr.slot[gr.lam[l] > 0.0 ? 0 : 1][i] = l;
+  }
+}
+
 // Whether the angular functions fns[f0, f1) form a product grid (one kind,
 // one Rc, lambda = +-1, every (lambda, zeta) x eta combination once); fills
 // `gr` when they do.
@@ -732,6 +756,7 @@ bool angular_grid(const std::vector<BehlerFn>& fns, int f0, int f1, BehlerGrid& 
     gr.eta[e] = et[e];
     gr.feta[e] = (float)et[e];
   }
+  grid_powers(gr);
   return true;
 }
 

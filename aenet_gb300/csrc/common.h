@@ -71,6 +71,7 @@ struct BehlerFn {     // one radial (G1..G3) or angular (G4, G5) function
 // one power per (lambda, zeta) instead of one of each per function.
 #define AE_BG_NL 16
 #define AE_BG_NE 8
+#define AE_BG_NZ 4      // zetas per sign that one pass of the kernels evaluates
 struct BehlerGrid {
   int kind;                           // 4 or 5
   int nl, ne;
@@ -81,6 +82,15 @@ struct BehlerGrid {
   float flam[AE_BG_NL], fzeta[AE_BG_NL], feta[AE_BG_NE];
   int izeta[AE_BG_NL];                // zeta as an integer in [1, 64], else 0
   int out[AE_BG_NL * AE_BG_NE];       // feature index of (l, e): out[l * AE_BG_NE + e]
+  // entries by sign (0: lambda = +1, 1: -1), -1 where a sign has none.
+  // chain > 0: the grid's chain <= AE_BG_NZ zetas are powers of two; the i-th
+  // power is reached from the one before it (the first from u) by sq[i]
+  // squarings, slot[s][i] is its entry.  general: each sign's entries in
+  // order, ngeneral of the longer sign (grids without a chain).
+  int chain, ngeneral;
+  int sq[AE_BG_NZ];
+  int slot[2][AE_BG_NZ];
+  int general[2][AE_BG_NL + AE_BG_NZ];
 };
 
 // Per central species: functions grouped by neighbour species (radial) and

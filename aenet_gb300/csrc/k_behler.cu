@@ -8,15 +8,22 @@
 // or neighbour pairs, of a single kind:
 //   radial  : lanes over the neighbours of a bucket, the list's functions
 //             accumulated in registers (chunks of 16), warp reduction;
-//   angular : lanes over the pairs of a bucket (triangle, circulant order)
-//             or of two buckets (rectangle), p = lane, lane + 32, ..., so
-//             every lane gets the same number of pairs.
+//   angular : the pairs of a bucket or of two buckets, offset by offset,
+//             compacted through a queue so that 32 live pairs are evaluated
+//             at a time (run_pairs).
 // Angular lists that form a product grid (one kind and Rc, lambda = +-1,
 // every (lambda, zeta) x eta combination; BehlerGrid) are evaluated per
 // pair with one exponential per eta and one power per (lambda, zeta), the
-// functions being their products; other lists function by function.
-// G4 pairs with r_jk >= Rc contribute nothing (fc(r_jk) = 0) and are
-// skipped after the distance test.
+// functions being their products; the factors of one neighbour alone,
+// exp(-eta r^2) fc(r), are staged with it.  Other lists go function by
+// function.
+//
+// What bounds them: instruction issue in FP32 and the FP64 pipe (two lanes
+// per clock and SM, 75-80 % busy) in FP64; the neighbour rows fit L2.
+// Measured on rutile Ti/O with 64 functions, before (an exponential of the
+// whole sum per eta and pair, sin/cos of r_jk, shared-memory atomics in the
+// adjoint) and now: 9,000 atoms mixed, forward 324 -> 243 us, adjoint 717 ->
+// 431 us; 763 atoms FP64, forward 1160 -> 515 us, adjoint 1733 -> 897 us.
 // The tables come from build_behler (capi.cpp): they already encode the
 // reference's indexing (functions registered under the global species
 // index, evaluated with the central atom's local one) and the feature
@@ -41,6 +48,15 @@ namespace {
 
 constexpr double SF_PI = 3.14159265358979;   // symmfunc.f90:38
 constexpr int FCH = 16;                      // functions per register chunk
+// resident one-warp blocks per SM asked of the register allocator (FP32);
+// 9,000 rutile atoms: forward 243 us at 24, 270 at 20, 251 at 28; adjoint
+// 431 us at 16, 464 at 20, 440 at 24
+#ifndef BEH_FWD_BLOCKS
+#define BEH_FWD_BLOCKS 24
+#endif
+#ifndef BEH_ADJ_BLOCKS
+#define BEH_ADJ_BLOCKS 16
+#endif
 
 template <typename T>
 struct V4;
@@ -123,10 +139,12 @@ __device__ __forceinline__ T ipow(T a, int n) {
 }
 
 // radial value and d/dr (sf_G1_ij, sf_G2_ij, sf_G3_ij)
+// A: the staged (1/r, fc, dfc), used when the function's cut-off is theirs
 template <typename T>
-__device__ __forceinline__ void radial_fn(const Fn<T>& f, T r, T& v, T& dv) {
-  T fc, dfc;
-  cutfn(r, f.Rc, fc, dfc);
+__device__ __forceinline__ void radial_fn(const Fn<T>& f, T r, bool cached,
+                                          const typename V4<T>::type& A, T& v, T& dv) {
+  T fc = A.y, dfc = A.z;
+  if (!cached) cutfn(r, f.Rc, fc, dfc);
   if (f.kind == 2) {
     const T a = r - f.p1;
     const T e = exp_t(-f.p2 * a * a);
@@ -172,20 +190,6 @@ __device__ __forceinline__ double normalise(double g, const PotDevice& pd, size_
 __device__ __forceinline__ float normalise(float g, const PotDevice& pd, size_t k) {
   const float2 sh = pd.shift2[k];
   return ((g - sh.x) - sh.y) * pd.scale32[k];
-}
-
-// Shared memory of one warp: the staged neighbours sR (x, y, z, r), their
-// per-neighbour terms sA (1/r, fc, dfc at the table's largest Rc), in the
-// adjoint the per-neighbour gradient accumulators sF (x, y, z) and the
-// scaled dE/dG row sg, then the table slot of each staged neighbour and a
-// queue of QCAP packed pairs (the surviving G4 pairs, see run_pairs).
-constexpr int QCAP = 64;
-template <typename T>
-__host__ __device__ inline size_t behler_smem_per_warp(int cap, int nsf_pad, bool adjoint) {
-  using T4 = typename V4<T>::type;
-  size_t per = 2 * sizeof(T4) * (size_t)cap + 4 * (size_t)cap + 4 * QCAP +
-               (adjoint ? sizeof(T) * (3 * (size_t)cap + nsf_pad) : 0);
-  return (per + 31) & ~size_t(31);
 }
 
 // Stage the neighbours inside rc into shared memory grouped by species.
@@ -238,73 +242,90 @@ __device__ __forceinline__ const BehlerGrid* grids_of(const BehlerTable* tab) {
                                              tab->grid_off);
 }
 
-// ---- pair schedules: lanes take pairs p = lane, lane + 32, ... of a list.
-// Unordered pairs of one bucket of m neighbours on a circulant schedule:
-// p = q m + r -> (r, (r + q + 1) mod m); with q < (m - 1)/2, plus the pairs
-// at distance m/2 from r < m/2 when m is even, every pair occurs once.
-// Pairs of bucket A (ma) x bucket C (mc): p = q ma + r -> (r, (q + r) mod mc).
-// Each lane keeps (q, r) and r mod mc and advances them by 32 with integer
-// adds and compares only (int <-> float conversions are slow on this GPU).
+// ---- pairs of staged neighbours, walked by the offset q between the row r
+// of one bucket and its partner:
+//   unordered pairs of one bucket of m : (r, (r + q) mod m), q = 1 .. m/2
+//     (q = m/2 from the lower half only when m is even)
+//   pairs of two buckets (mr >= mc)    : (r, (r + q) mod mc), q = 0 .. mc - 1
+// so that every pair occurs once and the rows of one offset have distinct
+// partners (in runs of mc rows).  Such a run is a pair's key.
+//
+// G4 pairs with r_jk >= Rc contribute nothing (fc(r_jk) = 0): an FP32 test
+// drops them (with a margin when the pair itself is evaluated in FP64, which
+// then decides), and the survivors go through a per-warp queue in shared
+// memory, so that the body runs on 32 live pairs instead of the ~45 % that
+// the loop leaves.  A queue entry carries its key: pairs with the same key
+// touch distinct rows and distinct partners, which lets the adjoint add to
+// the neighbours' accumulators without atomics.
 struct PairList {
-  int a0, ma, c0, mc, P;
-  int s32, mam;     // 32 mod mc, ma mod mc (rectangle)
+  int r0, mr, c0, mc;   // rows and partners (bucket start and size)
+  int rs, cs;           // their buckets
   bool tri;
 };
 
 __device__ __forceinline__ PairList pair_list(const int* bstart, int a, int c) {
   PairList L;
-  L.a0 = bstart[a];
-  L.ma = bstart[a + 1] - bstart[a];
-  L.c0 = bstart[c];
-  L.mc = bstart[c + 1] - bstart[c];
   L.tri = a == c;
-  L.P = L.tri ? L.ma * (L.ma - 1) / 2 : L.ma * L.mc;
-  L.s32 = L.mc > 0 ? 32 % L.mc : 0;
-  L.mam = L.mc > 0 ? L.ma % L.mc : 0;
+  const int na = bstart[a + 1] - bstart[a], nc = bstart[c + 1] - bstart[c];
+  const int rows = na >= nc ? a : c, part = na >= nc ? c : a;
+  L.rs = rows;
+  L.cs = part;
+  L.r0 = bstart[rows];
+  L.mr = bstart[rows + 1] - bstart[rows];
+  L.c0 = bstart[part];
+  L.mc = bstart[part + 1] - bstart[part];
   return L;
 }
+__device__ __forceinline__ bool empty(const PairList& L) {
+  return L.tri ? L.mr < 2 : L.mr < 1 || L.mc < 1;
+}
 
-struct PairWalk {
-  int p, q, r, rm;
-  __device__ __forceinline__ void init(const PairList& L, int lane) {
-    p = lane;
-    if (L.P == 0) return;
-    q = lane / L.ma;
-    r = lane - q * L.ma;
-    rm = L.tri ? 0 : r % L.mc;
-  }
-  __device__ __forceinline__ void get(const PairList& L, int& j, int& k) const {
-    if (L.tri) {
-      int kk = r + q + 1;
-      if (kk >= L.ma) kk -= L.ma;
-      j = L.a0 + r;
-      k = L.a0 + kk;
-    } else {
-      int kk = q + rm;
-      if (kk >= L.mc) kk -= L.mc;
-      j = L.a0 + r;
-      k = L.c0 + kk;
-    }
-  }
-  __device__ __forceinline__ void advance(const PairList& L) {
-    p += 32;
-    r += 32;
-    if (!L.tri) {
-      rm += L.s32;
-      if (rm >= L.mc) rm -= L.mc;
-    }
-    while (r >= L.ma) {
-      r -= L.ma;
-      ++q;
-      if (!L.tri) {
-        rm -= L.mam;
-        if (rm < 0) rm += L.mc;
+// body(live, j, k, key): called by the whole warp; lanes without a pair get
+// live = false and the indices of some staged pair.  The rows are cut into
+// blocks of equal width, so that no block leaves steps of a few lanes (each
+// step of a batch costs the adjoint one pass of add_pair).
+template <typename Body>
+__device__ __forceinline__ void run_pairs(const PairList& L, const float4* sP, bool filter,
+                                          float Rc2, int2* queue, int lane, Body body) {
+  const unsigned lt = (1u << lane) - 1u;
+  const int sub = !L.tri && L.mc < 32 ? lane / L.mc : 0;
+  const int qfirst = L.tri ? 1 : 0, qlast = L.tri ? L.mr / 2 : L.mc - 1;
+  const int nb = (L.mr + 31) / 32, width = (L.mr + nb - 1) / nb;
+  if (!filter) Rc2 = 3e38f;
+  int head = 0, key = sub;
+  for (int rb = 0; rb < L.mr; rb += width) {
+    const int r = rb + lane;
+    const bool row = lane < width && r < L.mr;
+    const float4 P = sP[L.r0 + (row ? r : rb)];
+    const int k0 = row ? (L.tri ? r + 1 : r % L.mc) : 0;
+    // the last offset of an even bucket pairs its lower half only
+    const int qend = !row ? 0 : (L.tri && !(L.mr & 1) && r >= L.mr / 2 ? qlast : qlast + 1);
+    const int jr = L.r0 + r;
+    int kc = L.c0 + (k0 < L.mc ? k0 : 0);
+    const int kend = L.c0 + L.mc;
+    for (int q = qfirst; q <= qlast; ++q, key += 32) {
+      const float4 O = sP[kc];
+      const float dx = O.x - P.x, dy = O.y - P.y, dz = O.z - P.z;
+      const bool ok = q < qend && dx * dx + dy * dy + dz * dz < Rc2;
+      const unsigned m = __ballot_sync(0xffffffffu, ok);
+      if (ok) queue[head + __popc(m & lt)] = make_int2(jr | (kc << 16), key);
+      head += __popc(m);
+      if (++kc == kend) kc = L.c0;
+      const bool last = q == qlast && rb + width >= L.mr;
+      while (head >= 32 || (last && head > 0)) {
+        __syncwarp();
+        const int n = min(head, 32);
+        head -= n;
+        const bool live = lane < n;
+        const int2 e = queue[head + (live ? lane : 0)];
+        __syncwarp();
+        body(live, e.x & 0xffff, e.x >> 16, e.y);
       }
     }
   }
-};
+}
 
-// ---- powers of the grid path: F = u^zeta (and dF/du = zeta u^(zeta-1))
+// ---- powers of the grid path: F = u^zeta, D = dF/du, u = (1 +- cos)/2
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -315,234 +336,425 @@ __device__ __forceinline__ float lg2_approx(float x) {
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
-// Per-pair terms of the angular factor ((1 + lambda cos)/2)^zeta for
-// lambda = +1 and -1.  FP32: u^zeta = 2^(zeta log2 u) (one log per sign,
-// one power per (lambda, zeta)); FP64: repeated squaring for integer zeta.
+__device__ __forceinline__ float rsq_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// e^(-eta x) from rate = -eta (FP64) or -eta log2 e (FP32)
+__device__ __forceinline__ float decay_rate(float eta) { return -1.4426950408889634f * eta; }
+__device__ __forceinline__ double decay_rate(double eta) { return -eta; }
+__device__ __forceinline__ float decay(float rate, float x) { return ex2_approx(rate * x); }
+__device__ __forceinline__ double decay(double rate, double x) { return exp(rate * x); }
 template <typename T>
-struct Ang;
+__device__ __forceinline__ T gval(const double* d, const float* f, int i);
 template <>
-struct Ang<float> {
-  float up, um, lp, lm, ip, im;
-  __device__ __forceinline__ void init(float c) {
-    up = 0.5f + 0.5f * c;
-    um = 0.5f - 0.5f * c;
-    lp = lg2_approx(up);
-    lm = lg2_approx(um);
-    ip = up > 0.f ? __frcp_rn(up) : 0.f;
-    im = um > 0.f ? __frcp_rn(um) : 0.f;
-  }
-  __device__ __forceinline__ float F(bool pos, float zeta, int) const {
-    return ex2_approx(zeta * (pos ? lp : lm));
-  }
-  // dF/dcos = zeta lambda u^(zeta - 1) / 2
-  __device__ __forceinline__ void FdF(bool pos, float zeta, int iz, float& F, float& dF) const {
-    F = ex2_approx(zeta * (pos ? lp : lm));
-    const float pz1 = iz == 1 ? 1.f : F * (pos ? ip : im);
-    dF = (pos ? 0.5f : -0.5f) * zeta * pz1;
-  }
-};
-template <>
-struct Ang<double> {
-  double up, um;
-  __device__ __forceinline__ void init(double c) {
-    up = 0.5 + 0.5 * c;
-    um = 0.5 - 0.5 * c;
-  }
-  __device__ __forceinline__ double F(bool pos, double zeta, int iz) const {
-    const double u = pos ? up : um;
-    return iz > 0 ? ipow(u, iz) : pow(u, zeta);
-  }
-  __device__ __forceinline__ void FdF(bool pos, double zeta, int iz, double& F, double& dF) const {
-    const double u = pos ? up : um;
-    double pz1;
-    if (iz > 0) {
-      pz1 = ipow(u, iz - 1);
-      F = pz1 * u;
-    } else {
-      F = pow(u, zeta);
-      pz1 = pow(u, zeta - 1.0);
-    }
-    dF = (pos ? 0.5 : -0.5) * zeta * pz1;
-  }
-};
-
-template <typename T>
-__device__ __forceinline__ T gval(const BehlerGrid* g, const double* d, const float* f, int i);
-template <>
-__device__ __forceinline__ float gval<float>(const BehlerGrid*, const double*, const float* f, int i) {
+__device__ __forceinline__ float gval<float>(const double*, const float* f, int i) {
   return f[i];
 }
 template <>
-__device__ __forceinline__ double gval<double>(const BehlerGrid*, const double* d, const float*, int i) {
+__device__ __forceinline__ double gval<double>(const double* d, const float*, int i) {
   return d[i];
 }
 
-// Run body(j, k) over the pairs of a list.  For G4 (kind 4) pairs with
-// r_jk >= Rc contribute nothing; they are filtered first and the
-// survivors go through a per-warp queue in shared memory, so that every
-// call of the body has 32 live pairs (one per lane) instead of the ~45 %
-// that a plain strided loop leaves active.  The queue holds j | k << 16
-// (staged indices < cap <= 65535).
-template <typename T, typename Body>
-__device__ __forceinline__ void run_pairs(const PairList& L, const typename V4<T>::type* sR,
-                                          bool filter, T Rc2, int* queue, int lane, Body body) {
+constexpr int BE = 2;   // eta values per grid block
+
+// fc and its derivative as functions of x = r^2: fc = (1 + cos sqrt(y))/2
+// with y = (pi/Rc)^2 x.  FP64: cos sqrt(y) is an entire function of y; its
+// Taylor series about pi^2/2 to degree 13 leaves less than 1e-18 on
+// [0, pi^2] and needs no square root, no sine and no division (the FP64
+// pipe, two lanes per clock and SM, bounds these kernels; 14 or 27
+// multiply-adds instead of ~60).
+constexpr double FC_Y0 = 4.9348022005446793094;   // pi^2 / 2
+__device__ __forceinline__ double fc_series(double z) {
+  double p = -1.1311932861159658242e-27;
+  p = fma(p, z, 7.2986588589149819688e-25);
+  p = fma(p, z, -3.9940266677874554912e-22);
+  p = fma(p, z, 1.8262231133604611914e-19);
+  p = fma(p, z, -6.8529250117771331873e-17);
+  p = fma(p, z, 2.0645516741852144221e-14);
+  p = fma(p, z, -4.8575286692910524617e-12);
+  p = fma(p, z, 8.612487525263789767e-10);
+  p = fma(p, z, -1.0965771688152239754e-7);
+  p = fma(p, z, 9.3591834506349915894e-6);
+  p = fma(p, z, -0.00048082314182966815651);
+  p = fma(p, z, 0.012207779738690289425);
+  p = fma(p, z, -0.089546946503311004436);
+  return fma(p, z, 0.1971500664605932856);
+}
+__device__ __forceinline__ double fc_series_d(double z) {
+  double p = -13.0 * 1.1311932861159658242e-27;
+  p = fma(p, z, 12.0 * 7.2986588589149819688e-25);
+  p = fma(p, z, -11.0 * 3.9940266677874554912e-22);
+  p = fma(p, z, 10.0 * 1.8262231133604611914e-19);
+  p = fma(p, z, -9.0 * 6.8529250117771331873e-17);
+  p = fma(p, z, 8.0 * 2.0645516741852144221e-14);
+  p = fma(p, z, -7.0 * 4.8575286692910524617e-12);
+  p = fma(p, z, 6.0 * 8.612487525263789767e-10);
+  p = fma(p, z, -5.0 * 1.0965771688152239754e-7);
+  p = fma(p, z, 4.0 * 9.3591834506349915894e-6);
+  p = fma(p, z, -3.0 * 0.00048082314182966815651);
+  p = fma(p, z, 2.0 * 0.012207779738690289425);
+  return fma(p, z, -0.089546946503311004436);
+}
+// fc(sqrt(x)) and d fc / dx; beyond Rc zero (FP64) or at the value of Rc,
+// which rounds to zero (FP32, whose pairs are inside).  a2 = (pi/Rc)^2,
+// a = pi/Rc
+template <bool DERIV>
+__device__ __forceinline__ void cut_x(double x, double Rc2, double a2, double, double& fc,
+                                      double& dfc) {
+  const double z = fma(a2, x, -FC_Y0);
+  fc = x < Rc2 ? fc_series(z) : 0.0;
+  if (DERIV) dfc = x < Rc2 ? a2 * fc_series_d(z) : 0.0;
+}
+template <bool DERIV>
+__device__ __forceinline__ void cut_x(float x, float Rc2, float, float a, float& fc, float& dfc) {
+  const float ri = rsq_approx(fmaxf(x, 1e-16f));
+  float s, c;
+  __sincosf(a * (fminf(x, Rc2) * ri), &s, &c);
+  fc = fmaf(0.5f, c, 0.5f);
+  if (DERIV) dfc = -0.25f * a * s * ri;
+}
+
+// Per-neighbour factors of a grid block: h_e = exp(-eta_e r^2) fc(r), 1/r
+// and fc'/fc (whose products with h_e and -2 eta_e r h_e give dh_e/dr; fc is
+// kept away from zero so that h_e fc'/fc stays exp(-eta_e r^2) fc' up to the
+// cut-off).  Filled per bucket and kept while the etas and Rc stay the same.
+template <typename T>
+struct FactorKey {
+  T eta0, eta1, Rc;
+  unsigned filled;   // buckets whose factors are in place
+};
+__device__ __forceinline__ double fc_floor(double fc) { return fmax(fc, 1e-30); }
+__device__ __forceinline__ float fc_floor(float fc) { return fmaxf(fc, 1e-12f); }
+template <typename T>
+__device__ __forceinline__ void fill_factors(const typename V4<T>::type* sR, T Rc, T a, T a2,
+                                             const T (&eta)[BE], int j0, int j1,
+                                             typename V4<T>::type* sH, int lane) {
   using T4 = typename V4<T>::type;
-  PairWalk w;
-  w.init(L, lane);
-  if (!filter) {
-    for (; w.p < L.P; w.advance(L)) {
-      int j, k;
-      w.get(L, j, k);
-      body(j, k);
-    }
-    return;
+  for (int j = j0 + lane; j < j1; j += 32) {
+    const T r = sR[j].w, x = r * r;
+    T fc, dfc;
+    cut_x<true>(x, Rc * Rc, a2, a, fc, dfc);
+    fc = fc_floor(fc);
+    T4 h;
+    h.x = exp_t(-eta[0] * x) * fc;
+    h.y = exp_t(-eta[1] * x) * fc;
+    h.z = T(1) / r;
+    h.w = T(2) * r * dfc / fc;
+    if (!(x < Rc * Rc)) h.x = h.y = T(0);
+    sH[j] = h;
   }
-  const unsigned lt = (1u << lane) - 1u;
-  int head = 0;
-  for (int p0 = 0; p0 < L.P; p0 += 32, w.advance(L)) {
-    int j = 0, k = 0;
-    bool ok = false;
-    if (w.p < L.P) {
-      w.get(L, j, k);
-      const T4 Rj = sR[j], Rk = sR[k];
-      const T dx = Rk.x - Rj.x, dy = Rk.y - Rj.y, dz = Rk.z - Rj.z;
-      ok = dx * dx + dy * dy + dz * dz < Rc2;
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (ok) queue[head + __popc(m & lt)] = j | (k << 16);
-    head += __popc(m);
-    __syncwarp();
-    if (head >= 32) {
-      head -= 32;
-      const int e = queue[head + lane];
-      __syncwarp();
-      body(e & 0xffff, e >> 16);
-    }
+}
+// the factors of a list's two buckets
+template <typename T>
+__device__ __forceinline__ void need_factors(FactorKey<T>& key, const PairList& L,
+                                             const typename V4<T>::type* sR, T Rc, T a, T a2,
+                                             const T (&eta)[BE], typename V4<T>::type* sH,
+                                             int lane) {
+  if (key.eta0 != eta[0] || key.eta1 != eta[1] || key.Rc != Rc) {
+    key.eta0 = eta[0];
+    key.eta1 = eta[1];
+    key.Rc = Rc;
+    key.filled = 0u;
   }
-  __syncwarp();
-  if (lane < head) {
-    const int e = queue[lane];
-    body(e & 0xffff, e >> 16);
-  }
+  __syncwarp();   // the previous list's readers are done
+  if (!(key.filled >> L.rs & 1u)) fill_factors<T>(sR, Rc, a, a2, eta, L.r0, L.r0 + L.mr, sH, lane);
+  if (!L.tri && !(key.filled >> L.cs & 1u))
+    fill_factors<T>(sR, Rc, a, a2, eta, L.c0, L.c0 + L.mc, sH, lane);
+  key.filled |= (1u << L.rs) | (1u << L.cs);
   __syncwarp();
 }
 
-constexpr int BL = 8;   // (lambda, zeta) pairs per grid block
-constexpr int BE = 2;   // eta values per grid block
-
-// Geometry of one pair (j, k) of staged neighbours for the grid path.
+// sum over the warp of 16 values per lane: lane l returns the sum of value
+// l >> 1 (each step hands half of the values to the partner: 16 additions
+// instead of the 80 of 16 butterflies)
 template <typename T>
-struct PairGeo {
-  typename V4<T>::type Rj, Rk;
-  T dx, dy, dz, rjk2, cosv, fcj, dfcj, fck, dfck, S;
-  __device__ __forceinline__ void load(const typename V4<T>::type* sR,
-                                       const typename V4<T>::type* sA, int j, int k, int kind,
-                                       T Rc, bool cached) {
-    Rj = sR[j];
-    Rk = sR[k];
-    dx = Rk.x - Rj.x;
-    dy = Rk.y - Rj.y;
-    dz = Rk.z - Rj.z;
-    rjk2 = dx * dx + dy * dy + dz * dz;
-    const typename V4<T>::type Aj = sA[j], Ak = sA[k];
-    cosv = (Rj.x * Rk.x + Rj.y * Rk.y + Rj.z * Rk.z) * Aj.x * Ak.x;
-    cosv = fmax(T(-1), fmin(T(1), cosv));
-    if (cached) {
-      fcj = Aj.y;
-      dfcj = Aj.z;
-      fck = Ak.y;
-      dfck = Ak.z;
-    } else {
-      cutfn(Rj.w, Rc, fcj, dfcj);
-      cutfn(Rk.w, Rc, fck, dfck);
+__device__ __forceinline__ T reduce16(T (&v)[16], int lane) {
+#pragma unroll
+  for (int h = 8, d = 16; h > 0; h >>= 1, d >>= 1) {
+    const bool up = lane & d;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const T give = up ? v[q] : v[q + h];
+      const T keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, give, d);
     }
-    S = Rj.w * Rj.w + Rk.w * Rk.w + (kind == 4 ? rjk2 : T(0));
   }
-};
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// The (lambda, zeta) entries of a grid handled together: slot [s][i] is sign
+// s (0: lambda = +1, 1: -1) and the i-th zeta.  CHAIN: the zetas of the grid
+// are z_0 = 2^s_0, z_i = z_{i-1} 2^{s_i} (BehlerGrid::chain), so that a
+// sign's powers are a run of squarings; otherwise up to four entries of any
+// zeta per pass, in list order.
+constexpr int NZ = AE_BG_NZ;
 
 // ----------------------------------------------------------------------
 // forward
 // ----------------------------------------------------------------------
 template <typename T>
-__device__ void forward_grid(const BehlerGrid* gr, const PairList& L, const typename V4<T>::type* sR,
-                             const typename V4<T>::type* sA, bool cached, int* queue, T* G,
-                             const PotDevice& pd, size_t nrow, int lane) {
-  const int kind = gr->kind, nl = gr->nl, ne = gr->ne;
-  const T Rc = gval<T>(gr, &gr->Rc, &gr->fRc, 0);
-  for (int l0 = 0; l0 < nl; l0 += BL)
-    for (int e0 = 0; e0 < ne; e0 += BE) {
-      T eta[BE], zeta[BL];
-      int iz[BL];
-      bool pos[BL];
+struct WarpMem {
+  typename V4<T>::type *sR, *sH, *sF;   // neighbours, factors, accumulators
+  float4* sP;                                // FP32 positions (aliases sR in the FP32 kernels)
+  T* sg;
+  T* sB;                                     // [2][NZ] (g_0, g_1) of a grid block
+  int* sslot;
+  int2* queue;
+};
+
+// Shared memory of one warp: the staged neighbours (x, y, z, r), their
+// factors (first 1/r, fc, dfc at the table's largest Rc for the radial
+// functions, then those of the grids), FP32 positions for the pair test (FP64
+// kernels), in the adjoint the accumulators and the scaled dE/dG row, the
+// table slot of each staged neighbour and the pair queue.
+constexpr int QCAP = 64;
+template <typename T>
+__host__ __device__ inline size_t behler_smem_per_warp(int cap, int nsf_pad, bool adjoint) {
+  using T4 = typename V4<T>::type;
+  size_t per = (adjoint ? 3 : 2) * sizeof(T4) * (size_t)cap + 4 * (size_t)cap + 8 * QCAP +
+               (sizeof(T) == 8 ? sizeof(float4) * (size_t)cap : 0) +
+               (adjoint ? sizeof(T) * ((size_t)nsf_pad + 2 * NZ * BE) : 0);
+  return (per + 31) & ~size_t(31);
+}
+template <typename T>
+__device__ __forceinline__ WarpMem<T> warp_mem(unsigned char* base, int cap, int nsf_pad,
+                                               bool adjoint) {
+  using T4 = typename V4<T>::type;
+  WarpMem<T> w;
+  w.sR = reinterpret_cast<T4*>(base);
+  w.sH = w.sR + cap;
+  w.sF = w.sH + cap;
+  T4* next = adjoint ? w.sF + cap : w.sF;
+  if (sizeof(T) == 8) {
+    w.sP = reinterpret_cast<float4*>(next);
+    w.sg = reinterpret_cast<T*>(w.sP + cap);
+  } else {
+    w.sP = reinterpret_cast<float4*>(w.sR);
+    w.sg = reinterpret_cast<T*>(next);
+  }
+  w.sB = w.sg;
+  if (adjoint) w.sg += 2 * NZ * BE;
+  w.queue = reinterpret_cast<int2*>(w.sg + (adjoint ? nsf_pad : 0));
+  w.sslot = reinterpret_cast<int*>(w.queue + QCAP);
+  return w;
+}
+__device__ __forceinline__ void fill_positions(const double4_32a* sR, float4* sP, int n, int lane) {
+  for (int j = lane; j < n; j += 32) {
+    const double4_32a R = sR[j];
+    sP[j] = make_float4((float)R.x, (float)R.y, (float)R.z, 0.f);
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void fill_positions(const float4*, float4*, int, int) {}
+
+// squared cut-off of the FP32 pair test: exact for FP32 pairs, wider than any
+// rounding of the FP32 positions for FP64 ones
+__device__ __forceinline__ float filter_rc2(float Rc) { return Rc * Rc; }
+__device__ __forceinline__ float filter_rc2(double Rc) {
+  return (float)(Rc * Rc) * 1.0001f + 1e-4f;
+}
+
+// Block of a grid: the etas e0, e0 + 1 and the zeta entries of pass l0.
+template <typename T>
+struct GridBlock {
+  T eta[BE], rate[BE];
+  int iz[2][NZ];
+  T zeta[2][NZ];
+  int sq[NZ];
+  // the grid entry of slot (s, i), or -1
+  static __device__ __forceinline__ int entry(const BehlerGrid* gr, bool chain, int l0, int s,
+                                              int i) {
+    return chain ? gr->slot[s][i] : gr->general[s][l0 + i];
+  }
+  // the feature of slot (s, i) and eta e, or -1
+  static __device__ __forceinline__ int feature(const BehlerGrid* gr, bool chain, int l0, int e0,
+                                                int s, int i, int e) {
+    const int l = entry(gr, chain, l0, s, i);
+    return l >= 0 && e0 + e < gr->ne ? gr->out[l * AE_BG_NE + e0 + e] : -1;
+  }
+  __device__ __forceinline__ void load(const BehlerGrid* gr, bool chain, int l0, int e0) {
 #pragma unroll
-      for (int e = 0; e < BE; ++e) eta[e] = e0 + e < ne ? gval<T>(gr, gr->eta, gr->feta, e0 + e) : T(0);
+    for (int e = 0; e < BE; ++e)
+      eta[e] = e0 + e < gr->ne ? gval<T>(gr->eta, gr->feta, e0 + e) : T(0);
 #pragma unroll
-      for (int l = 0; l < BL; ++l) {
-        const int ll = min(l0 + l, nl - 1);
-        zeta[l] = gval<T>(gr, gr->zeta, gr->fzeta, ll);
-        iz[l] = gr->izeta[ll];
-        pos[l] = gr->flam[ll] > 0.f;
+    for (int e = 0; e < BE; ++e) rate[e] = decay_rate(eta[e]);
+#pragma unroll
+    for (int i = 0; i < NZ; ++i) sq[i] = gr->sq[i];
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int i = 0; i < NZ; ++i) {
+        const int l = entry(gr, chain, l0, s, i);
+        iz[s][i] = l >= 0 ? gr->izeta[l] : 1;
+        zeta[s][i] = l >= 0 ? gval<T>(gr->zeta, gr->fzeta, l) : T(1);
       }
-      T acc[BL][BE];
+  }
+};
+
+// F (and D = dF/du) of one sign's entries at u: squarings along the chain
+// (FP64: 8 multiplications for the zetas 1, 2, 4, 16 of both signs), or one
+// power per entry (FP32: u^zeta = 2^(zeta log2 u) on the special-function
+// unit, which the pair's work leaves idle, costs fewer instructions than the
+// uniform loops of a chain)
+template <bool CHAIN, bool DERIV>
+__device__ __forceinline__ void powers(double u, const GridBlock<double>& B, int s, int nz,
+                                       double (&F)[NZ], double (&D)[NZ]) {
+  if (CHAIN) {
+    double f = u, d = 1.0;
 #pragma unroll
-      for (int l = 0; l < BL; ++l)
-#pragma unroll
-        for (int e = 0; e < BE; ++e) acc[l][e] = T(0);
-      run_pairs<T>(L, sR, kind == 4, Rc * Rc, queue, lane, [&](int j, int k) {
-        PairGeo<T> q;
-        q.load(sR, sA, j, k, kind, Rc, cached);
-        T FC = T(2) * q.fcj * q.fck;
-        if (kind == 4) {
-          T fjk, dum;
-          cutfn(sqrt(q.rjk2), Rc, fjk, dum);
-          FC *= fjk;
+    for (int i = 0; i < NZ; ++i) {
+      if (i < nz) {
+        for (int t = B.sq[i]; t > 0; --t) {
+          if (DERIV) d *= f + f;
+          f *= f;
         }
-        T E[BE];
+      }
+      F[i] = f;
+      if (DERIV) D[i] = d;
+    }
+  } else {
 #pragma unroll
-        for (int e = 0; e < BE; ++e) E[e] = exp_t(-eta[e] * q.S) * FC;
-        Ang<T> ang;
-        ang.init(q.cosv);
+    for (int i = 0; i < NZ; ++i)
+      if (i < nz) {
+        if (B.iz[s][i] > 0) {
+          const double p = ipow(u, B.iz[s][i] - 1);
+          F[i] = p * u;
+          D[i] = B.zeta[s][i] * p;
+        } else {
+          F[i] = pow(u, B.zeta[s][i]);
+          if (DERIV) D[i] = B.zeta[s][i] * pow(u, B.zeta[s][i] - 1.0);
+        }
+      }
+  }
+}
+template <bool CHAIN>
+__device__ __forceinline__ void powers(float u, const GridBlock<float>& B, int s, int nz,
+                                       float (&F)[NZ]) {
+  const float l = lg2_approx(u);
 #pragma unroll
-        for (int l = 0; l < BL; ++l) {
-          if (l0 + l < nl) {
-            const T F = ang.F(pos[l], zeta[l], iz[l]);
+  for (int i = 0; i < NZ; ++i) F[i] = ex2_approx(B.zeta[s][i] * l);   // absent entries too
+}
+
+// A_e += sum_i g_ie F_i and d_e = sum_i g_ie D_i of one sign
+template <bool CHAIN>
+__device__ __forceinline__ void power_sums(double u, const GridBlock<double>& B, int s, int nz,
+                                           const double* g, double (&A)[BE], double (&d)[BE]) {
+  double F[NZ], D[NZ];
+  powers<CHAIN, true>(u, B, s, nz, F, D);
 #pragma unroll
-            for (int e = 0; e < BE; ++e) acc[l][e] += F * E[e];
-          }
+  for (int e = 0; e < BE; ++e) d[e] = 0.0;
+#pragma unroll
+  for (int i = 0; i < NZ; ++i)
+    if (i < nz) {
+#pragma unroll
+      for (int e = 0; e < BE; ++e) {
+        const double ge = g[(s * NZ + i) * BE + e];
+        A[e] = fma(ge, F[i], A[e]);
+        d[e] = fma(ge, D[i], d[e]);
+      }
+    }
+}
+// FP32: D = zeta F / u (zero at u = 0, where the gradient of the cosine that
+// it multiplies vanishes)
+template <bool CHAIN>
+__device__ __forceinline__ void power_sums(float u, const GridBlock<float>& B, int s, int nz,
+                                           const float* g, float (&A)[BE], float (&d)[BE]) {
+  float F[NZ];
+  powers<CHAIN>(u, B, s, nz, F);
+#pragma unroll
+  for (int e = 0; e < BE; ++e) d[e] = 0.f;
+  const float4* g4 = reinterpret_cast<const float4*>(g + s * NZ * BE);
+#pragma unroll
+  for (int i = 0; i < NZ; i += 2) {
+    const float4 q = g4[i / 2];
+    const float z0 = B.zeta[s][i] * F[i], z1 = B.zeta[s][i + 1] * F[i + 1];
+    A[0] = fmaf(q.z, F[i + 1], fmaf(q.x, F[i], A[0]));
+    A[1] = fmaf(q.w, F[i + 1], fmaf(q.y, F[i], A[1]));
+    d[0] = fmaf(q.z, z1, fmaf(q.x, z0, d[0]));
+    d[1] = fmaf(q.w, z1, fmaf(q.y, z0, d[1]));
+  }
+  const float inv = rcp_approx(fmaxf(u, 1e-30f));   // F is zero at u = 0
+#pragma unroll
+  for (int e = 0; e < BE; ++e) d[e] *= inv;
+}
+
+template <bool CHAIN>
+__device__ __forceinline__ void powers(double u, const GridBlock<double>& B, int s, int nz,
+                                       double (&F)[NZ]) {
+  double D[NZ];
+  powers<CHAIN, false>(u, B, s, nz, F, D);
+}
+
+template <typename T, bool CHAIN>
+__device__ void forward_grid(const BehlerGrid* gr, const PairList& L, const WarpMem<T>& w,
+                             FactorKey<T>& key, T* G, const PotDevice& pd, size_t nrow, int lane) {
+  using T4 = typename V4<T>::type;
+  const bool g4 = gr->kind == 4;
+  const T Rc = gval<T>(&gr->Rc, &gr->fRc, 0);
+  const T a = T(SF_PI) / Rc, a2 = a * a, Rc2 = Rc * Rc;
+  const int npass = CHAIN ? 1 : (gr->ngeneral + NZ - 1) / NZ;
+  for (int e0 = 0; e0 < gr->ne; e0 += BE)
+    for (int pass = 0; pass < npass; ++pass) {
+      GridBlock<T> B;
+      B.load(gr, CHAIN, NZ * pass, e0);
+      const int nz = CHAIN ? gr->chain : min(NZ, gr->ngeneral - NZ * pass);
+      need_factors<T>(key, L, w.sR, Rc, a, a2, B.eta, w.sH, lane);
+      T acc[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) acc[q] = T(0);
+      run_pairs(L, w.sP, g4, filter_rc2(Rc), w.queue, lane, [&](bool live, int j, int k, int) {
+        const T4 Rj = w.sR[j], Rk = w.sR[k], Hj = w.sH[j], Hk = w.sH[k];
+        T E[BE] = {Hj.x * Hk.x, Hj.y * Hk.y};
+        if (g4) {
+          const T dx = Rk.x - Rj.x, dy = Rk.y - Rj.y, dz = Rk.z - Rj.z;
+          const T x = dx * dx + dy * dy + dz * dz;
+          T fc, dum;
+          cut_x<false>(x, Rc2, a2, a, fc, dum);
+#pragma unroll
+          for (int e = 0; e < BE; ++e) E[e] *= decay(B.rate[e], x) * fc;
+        }
+        if (!live) E[0] = E[1] = T(0);
+        const T c = (Rj.x * Rk.x + Rj.y * Rk.y + Rj.z * Rk.z) * (Hj.z * Hk.z);
+        const T ch = fmax(T(-0.5), fmin(T(0.5), T(0.5) * c));
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          T F[NZ];
+          powers<CHAIN>(s ? T(0.5) - ch : T(0.5) + ch, B, s, nz, F);
+#pragma unroll
+          for (int i = 0; i < NZ; ++i)
+            if (sizeof(T) == 4 || i < nz) {
+#pragma unroll
+              for (int e = 0; e < BE; ++e)
+                acc[(s * NZ + i) * BE + e] = fma(F[i], E[e], acc[(s * NZ + i) * BE + e]);
+            }
         }
       });
-#pragma unroll
-      for (int l = 0; l < BL; ++l)
-#pragma unroll
-        for (int e = 0; e < BE; ++e) {
-          if (l0 + l < nl && e0 + e < ne) {
-            const T v = warp_sum(acc[l][e]);
-            if (lane == 0) {
-              const int out = gr->out[(l0 + l) * AE_BG_NE + e0 + e];
-              G[out] = normalise(v, pd, nrow + out);
-            }
-          }
-        }
+      const T v = T(2) * reduce16(acc, lane);   // the factor 2 of symmfunc.f90:724
+      const int out = GridBlock<T>::feature(gr, CHAIN, NZ * pass, e0, lane >> 4, (lane >> 2) & 3,
+                                            (lane >> 1) & 1);
+      if (!(lane & 1) && out >= 0) G[out] = normalise(v, pd, nrow + out);
     }
 }
 
 template <typename T>
 __device__ void forward_generic(const BehlerTable* tab, int f0, int f1e, const PairList& L,
-                                const typename V4<T>::type* sR, T* G, const PotDevice& pd,
-                                size_t nrow, int lane) {
+                                const WarpMem<T>& w, T* G, const PotDevice& pd, size_t nrow,
+                                int lane) {
   using T4 = typename V4<T>::type;
   for (int c0 = f0; c0 < f1e; c0 += FCH) {
     const int nf = min(FCH, f1e - c0);
     T acc[FCH];
 #pragma unroll
     for (int q = 0; q < FCH; ++q) acc[q] = T(0);
-    PairWalk w;
-    w.init(L, lane);
-    for (; w.p < L.P; w.advance(L)) {
-      int j, k;
-      w.get(L, j, k);
-      const T4 Rj = sR[j], Rk = sR[k];
+    run_pairs(L, w.sP, false, 0.f, w.queue, lane, [&](bool live, int j, int k, int) {
+      const T4 Rj = w.sR[j], Rk = w.sR[k];
       const T dxx = Rk.x - Rj.x, dyy = Rk.y - Rj.y, dzz = Rk.z - Rj.z;
       const T rjk2 = dxx * dxx + dyy * dyy + dzz * dzz;
       const T rjk = sqrt(rjk2);
@@ -562,13 +774,14 @@ __device__ void forward_generic(const BehlerTable* tab, int f0, int f1e, const P
           }
           T F, dF;
           f1(f, cosv, F, dF);
+          if (!live) F = T(0);
           if (f.kind == 4)
             acc[q] += T(2) * F * exp_t(-f.p3 * (rij2 + rik2 + rjk2)) * fij * fik * fjk;
           else
             acc[q] += T(2) * F * exp_t(-f.p3 * (rij2 + rik2)) * fij * fik;
         }
       }
-    }
+    });
 #pragma unroll
     for (int q = 0; q < FCH; ++q) {
       if (q < nf) {
@@ -583,20 +796,15 @@ __device__ void forward_generic(const BehlerTable* tab, int f0, int f1e, const P
 }
 
 // GRID: every angular list is a BehlerGrid (the generic path is left out,
-// which frees its registers)
+// which frees its registers).  One warp per block: the warps of a block
+// share nothing, and small blocks spread a few hundred atoms evenly.
 template <typename T, bool GRID>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) k_behler_forward(PotDevice pd, DescBuffers b) {
+__global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_behler_forward(PotDevice pd, DescBuffers b) {
   using T4 = typename V4<T>::type;
   extern __shared__ __align__(32) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int i = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (i >= b.natoms) return;
-  unsigned char* base = smem_raw + behler_smem_per_warp<T>(b.cap, pd.nsf_pad, false) * warp;
-  T4* sR = reinterpret_cast<T4*>(base);
-  T4* sA = sR + b.cap;
-  int* sslot = reinterpret_cast<int*>(sA + b.cap);
-  int* queue = sslot + b.cap;
+  const int lane = threadIdx.x;
+  const int i = blockIdx.x;
+  const WarpMem<T> w = warp_mem<T>(smem_raw, b.cap, pd.nsf_pad, false);
   const int ti = b.types[i];
   const BehlerTable* tab = table_of<T>(pd, ti);
   const int nt = pd.ntypes;
@@ -604,7 +812,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) k_behler_forward(
   const T4* __restrict__ vec = reinterpret_cast<const T4*>(b.nb_vec) + (size_t)i * b.cap;
   const int* __restrict__ jt = b.nb_jt + (size_t)i * b.cap;
   int bstart[AE_MAXT + 1];
-  stage_buckets<T>(vec, jt, n, nt, T(tab->rc_max), sR, sA, sslot, bstart, lane);
+  const int nst = stage_buckets<T>(vec, jt, n, nt, T(tab->rc_max), w.sR, w.sH, w.sslot, bstart,
+                                   lane);
+  fill_positions(w.sR, w.sP, nst, lane);
   const size_t nrow = (size_t)ti * pd.nsf_pad;
   T* G = reinterpret_cast<T*>(b.G) + (size_t)i * pd.nsf_pad;
   const int nsf = pd.sp[ti].nsf;
@@ -618,10 +828,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) k_behler_forward(
     const int f0 = tab->rad_off[s], f1e = tab->rad_off[s + 1];
     for (int q = f0; q < f1e; ++q) {
       const Fn<T> f = load_fn<T>(&tab->fn[q]);
+      const bool cached = f.Rc == T(tab->rc_max);
       T acc = T(0);
       for (int j = bstart[s] + lane; j < bstart[s + 1]; j += 32) {
         T v, dv;
-        radial_fn(f, sR[j].w, v, dv);
+        radial_fn(f, w.sR[j].w, cached, w.sH[j], v, dv);
         acc += v;
       }
       acc = warp_sum(acc);
@@ -630,19 +841,23 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1) k_behler_forward(
   }
 
   // ---- angular lists (one per unordered pair of neighbour species)
+  FactorKey<T> key{T(-1), T(-1), T(-1), 0u};
   const BehlerGrid* grids = grids_of(tab);
   for (int a = 0; a < nt; ++a) {
     for (int c = a; c < nt; ++c) {
       const int f0 = tab->ang_off[a * nt + c], f1e = tab->ang_off[a * nt + c + 1];
       if (f0 == f1e) continue;
       const PairList L = pair_list(bstart, a, c);
-      if (L.P == 0) continue;
+      if (empty(L)) continue;
       const int gi = tab->grid_of[a * nt + c];
       if (GRID || gi >= 0) {
         const BehlerGrid* gr = grids + gi;
-        forward_grid<T>(gr, L, sR, sA, gr->Rc == tab->rc_max, queue, G, pd, nrow, lane);
+        if (sizeof(T) == 8 && gr->chain)
+          forward_grid<T, sizeof(T) == 8>(gr, L, w, key, G, pd, nrow, lane);
+        else
+          forward_grid<T, false>(gr, L, w, key, G, pd, nrow, lane);
       } else {
-        if constexpr (!GRID) forward_generic<T>(tab, f0, f1e, L, sR, G, pd, nrow, lane);
+        if constexpr (!GRID) forward_generic<T>(tab, f0, f1e, L, w, G, pd, nrow, lane);
       }
     }
   }
@@ -665,109 +880,163 @@ __device__ __forceinline__ void atomic_add3<double>(double* F, int atom, double 
   atomicAdd(F + 4 * atom + 2, fz);
 }
 
-// Gradient of one pair's terms with respect to R_j and R_k from the
-// partials of the pair's function sum: Sc (cos theta_jik), Sij (r_ij),
-// Sik (r_ik), Sjk (r_jk); added to the staged neighbours' accumulators.
+// The gradient of one pair's terms with respect to R_j and R_k from the
+// partials Sc (cos), Sj and Sk (r_ij, r_ik) and Sx (twice that in r_jk^2),
+// added to the neighbours' accumulators in shared memory.  Step by step of
+// the pair schedule the lanes hold distinct rows and distinct partners, so
+// plain adds are enough (shared-memory atomics, six per pair, are loops).
+//   FP32: the vector gradients, as
+//     Sc/r_j (v - cos u) + Sj u - Sx (R_k - R_j)
+//   FP64: their coefficients of the two position vectors, alpha R_k + beta_j
+//     R_j and alpha R_j + beta_k R_k, with beta summed per neighbour (10
+//     multiply-adds less per pair; the sums cancel to the vectors, which
+//     costs FP32 a digit and FP64 nothing that its results show)
 template <typename T>
-__device__ __forceinline__ void scatter_pair(const typename V4<T>::type& Rj,
-                                             const typename V4<T>::type& Rk, T invj, T invk,
-                                             T cosv, T dx, T dy, T dz, T rjk, T Sc, T Sij, T Sik,
-                                             T Sjk, T* sF, int j, int k) {
-  const T ux = Rj.x * invj, uy = Rj.y * invj, uz = Rj.z * invj;
-  const T vx = Rk.x * invk, vy = Rk.y * invk, vz = Rk.z * invk;
-  const T cj = Sc * invj, ck = Sc * invk;
-  const T ijk = rjk > T(1e-8) ? Sjk / rjk : T(0);
-  atomicAdd(sF + 3 * j, cj * (vx - cosv * ux) + Sij * ux - ijk * dx);
-  atomicAdd(sF + 3 * j + 1, cj * (vy - cosv * uy) + Sij * uy - ijk * dy);
-  atomicAdd(sF + 3 * j + 2, cj * (vz - cosv * uz) + Sij * uz - ijk * dz);
-  atomicAdd(sF + 3 * k, ck * (ux - cosv * vx) + Sik * vx + ijk * dx);
-  atomicAdd(sF + 3 * k + 1, ck * (uy - cosv * vy) + Sik * vy + ijk * dy);
-  atomicAdd(sF + 3 * k + 2, ck * (uz - cosv * vz) + Sik * vz + ijk * dz);
-}
+struct PairGrad;
+template <>
+struct PairGrad<float> {
+  float gx, gy, gz, hx, hy, hz;
+  __device__ __forceinline__ PairGrad(const float4& Rj, const float4& Rk, float invj, float invk,
+                                      float c, float Sc, float Sj, float Sk, float Sx) {
+    const float ux = Rj.x * invj, uy = Rj.y * invj, uz = Rj.z * invj;
+    const float vx = Rk.x * invk, vy = Rk.y * invk, vz = Rk.z * invk;
+    const float dx = Sx * (Rk.x - Rj.x), dy = Sx * (Rk.y - Rj.y), dz = Sx * (Rk.z - Rj.z);
+    const float cj = Sc * invj, ck = Sc * invk;
+    const float bj = fmaf(-cj, c, Sj), bk = fmaf(-ck, c, Sk);
+    gx = fmaf(cj, vx, fmaf(bj, ux, -dx));
+    gy = fmaf(cj, vy, fmaf(bj, uy, -dy));
+    gz = fmaf(cj, vz, fmaf(bj, uz, -dz));
+    hx = fmaf(ck, ux, fmaf(bk, vx, dx));
+    hy = fmaf(ck, uy, fmaf(bk, vy, dy));
+    hz = fmaf(ck, uz, fmaf(bk, vz, dz));
+  }
+  __device__ __forceinline__ void add_j(float4& f, const float4&) const {
+    f.x += gx;
+    f.y += gy;
+    f.z += gz;
+  }
+  __device__ __forceinline__ void add_k(float4& f, const float4&) const {
+    f.x += hx;
+    f.y += hy;
+    f.z += hz;
+  }
+};
+template <>
+struct PairGrad<double> {
+  double alpha, bj, bk;
+  __device__ __forceinline__ PairGrad(const double4_32a&, const double4_32a&, double invj,
+                                      double invk, double c, double Sc, double Sj, double Sk,
+                                      double Sx) {
+    alpha = fma(Sc, invj * invk, -Sx);
+    const double scc = Sc * c;
+    bj = fma(invj, fma(-scc, invj, Sj), Sx);
+    bk = fma(invk, fma(-scc, invk, Sk), Sx);
+  }
+  __device__ __forceinline__ void add_j(double4_32a& f, const double4_32a& Rk) const {
+    f.x = fma(alpha, Rk.x, f.x);
+    f.y = fma(alpha, Rk.y, f.y);
+    f.z = fma(alpha, Rk.z, f.z);
+    f.w += bj;
+  }
+  __device__ __forceinline__ void add_k(double4_32a& f, const double4_32a& Rj) const {
+    f.x = fma(alpha, Rj.x, f.x);
+    f.y = fma(alpha, Rj.y, f.y);
+    f.z = fma(alpha, Rj.z, f.z);
+    f.w += bk;
+  }
+};
 
 template <typename T>
-__device__ void adjoint_grid(const BehlerGrid* gr, const PairList& L, const typename V4<T>::type* sR,
-                             const typename V4<T>::type* sA, bool cached, const T* sg, T* sF,
-                             int* queue, int lane) {
-  const int kind = gr->kind, nl = gr->nl, ne = gr->ne;
-  const T Rc = gval<T>(gr, &gr->Rc, &gr->fRc, 0);
-  for (int l0 = 0; l0 < nl; l0 += BL)
-    for (int e0 = 0; e0 < ne; e0 += BE) {
-      T eta[BE], zeta[BL], g[BL][BE];
-      int iz[BL];
-      bool pos[BL];
-#pragma unroll
-      for (int e = 0; e < BE; ++e) eta[e] = e0 + e < ne ? gval<T>(gr, gr->eta, gr->feta, e0 + e) : T(0);
-#pragma unroll
-      for (int l = 0; l < BL; ++l) {
-        const int ll = min(l0 + l, nl - 1);
-        zeta[l] = gval<T>(gr, gr->zeta, gr->fzeta, ll);
-        iz[l] = gr->izeta[ll];
-        pos[l] = gr->flam[ll] > 0.f;
-#pragma unroll
-        for (int e = 0; e < BE; ++e)
-          g[l][e] = (l0 + l < nl && e0 + e < ne) ? T(2) * sg[gr->out[(l0 + l) * AE_BG_NE + e0 + e]]
-                                                 : T(0);
+__device__ __forceinline__ void add_pair(typename V4<T>::type* sF, bool live, int j, int k, int key,
+                                         const typename V4<T>::type& Rj,
+                                         const typename V4<T>::type& Rk, const PairGrad<T>& p) {
+  using T4 = typename V4<T>::type;
+  // runs of equal keys, in lane order
+  const int lane = threadIdx.x;
+  const int before = __shfl_up_sync(0xffffffffu, key, 1);
+  const unsigned first = __ballot_sync(0xffffffffu, live && (lane == 0 || key != before));
+  const int run = live ? __popc(first & (0xffffffffu >> (31 - lane))) : 0;
+  const int nrun = __popc(first);
+  for (int q = 1; q <= nrun; ++q) {
+    if (run == q) {
+      T4 f = sF[j];
+      p.add_j(f, Rk);
+      sF[j] = f;
+    }
+    __syncwarp();
+    if (run == q) {
+      T4 f = sF[k];
+      p.add_k(f, Rj);
+      sF[k] = f;
+    }
+    __syncwarp();
+  }
+}
+
+template <typename T, bool CHAIN>
+__device__ void adjoint_grid(const BehlerGrid* gr, const PairList& L, const WarpMem<T>& w,
+                             FactorKey<T>& key, int lane) {
+  using T4 = typename V4<T>::type;
+  const bool g4 = gr->kind == 4;
+  const T Rc = gval<T>(&gr->Rc, &gr->fRc, 0);
+  const T a = T(SF_PI) / Rc, a2 = a * a, Rc2 = Rc * Rc;
+  const int npass = CHAIN ? 1 : (gr->ngeneral + NZ - 1) / NZ;
+  for (int e0 = 0; e0 < gr->ne; e0 += BE)
+    for (int pass = 0; pass < npass; ++pass) {
+      GridBlock<T> B;
+      B.load(gr, CHAIN, NZ * pass, e0);
+      const int nz = CHAIN ? gr->chain : min(NZ, gr->ngeneral - NZ * pass);
+      __syncwarp();
+      if (lane < 2 * NZ * BE) {
+        const int f = GridBlock<T>::feature(gr, CHAIN, NZ * pass, e0, lane / (NZ * BE),
+                                            lane / BE % NZ, lane % BE);
+        w.sB[lane] = f >= 0 ? T(2) * w.sg[f] : T(0);
       }
-      run_pairs<T>(L, sR, kind == 4, Rc * Rc, queue, lane, [&](int j, int k) {
-        PairGeo<T> q;
-        q.load(sR, sA, j, k, kind, Rc, cached);
-        T rjk = T(0), fjk = T(1), dfjk = T(0);
-        if (kind == 4) {
-          rjk = sqrt(q.rjk2);
-          cutfn(rjk, Rc, fjk, dfjk);
+      need_factors<T>(key, L, w.sR, Rc, a, a2, B.eta, w.sH, lane);
+      run_pairs(L, w.sP, g4, filter_rc2(Rc), w.queue, lane, [&](bool live, int j, int k, int step) {
+        const T4 Rj = w.sR[j], Rk = w.sR[k], Hj = w.sH[j], Hk = w.sH[k];
+        const T invj = Hj.z, invk = Hk.z;
+        const T c = (Rj.x * Rk.x + Rj.y * Rk.y + Rj.z * Rk.z) * (invj * invk);
+        const T ch = fmax(T(-0.5), fmin(T(0.5), T(0.5) * c));
+        T A[BE] = {T(0), T(0)}, C[BE] = {T(0), T(0)};   // sum of g F, twice its d/dcos
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          T d[BE];
+          power_sums<CHAIN>(s ? T(0.5) - ch : T(0.5) + ch, B, s, nz, w.sB, A, d);
+#pragma unroll
+          for (int e = 0; e < BE; ++e) C[e] = s ? C[e] - d[e] : d[e];
         }
-        T Es[BE];
+        T h[BE] = {Hj.x * Hk.x, Hj.y * Hk.y};
+        T fc = T(1), dfc = T(0);
+        if (g4) {
+          const T dx = Rk.x - Rj.x, dy = Rk.y - Rj.y, dz = Rk.z - Rj.z;
+          const T x = dx * dx + dy * dy + dz * dz;
+          cut_x<true>(x, Rc2, a2, a, fc, dfc);
 #pragma unroll
-        for (int e = 0; e < BE; ++e) Es[e] = exp_t(-eta[e] * q.S);
-        Ang<T> ang;
-        ang.init(q.cosv);
-        T A[BE], B[BE];
-#pragma unroll
-        for (int e = 0; e < BE; ++e) A[e] = B[e] = T(0);
-#pragma unroll
-        for (int l = 0; l < BL; ++l) {
-          if (l0 + l < nl) {
-            T F, dF;
-            ang.FdF(pos[l], zeta[l], iz[l], F, dF);
-#pragma unroll
-            for (int e = 0; e < BE; ++e) {
-              A[e] += g[l][e] * F;
-              B[e] += g[l][e] * dF;
-            }
-          }
+          for (int e = 0; e < BE; ++e) h[e] *= decay(B.rate[e], x);
         }
-        T SE = T(0), Seta = T(0), SB = T(0);
-#pragma unroll
-        for (int e = 0; e < BE; ++e) {
-          SE += A[e] * Es[e];
-          Seta += A[e] * Es[e] * eta[e];
-          SB += B[e] * Es[e];
-        }
-        const T FC = q.fcj * q.fck * fjk;
-        const T t2 = T(2) * FC * Seta;
-        const T Sc = SB * FC;
-        const T Sij = SE * q.dfcj * q.fck * fjk - t2 * q.Rj.w;
-        const T Sik = SE * q.fcj * q.dfck * fjk - t2 * q.Rk.w;
-        const T Sjk = kind == 4 ? SE * q.fcj * q.fck * dfjk - t2 * rjk : T(0);
-        scatter_pair<T>(q.Rj, q.Rk, sA[j].x, sA[k].x, q.cosv, q.dx, q.dy, q.dz, rjk, Sc, Sij,
-                        Sik, Sjk, sF, j, k);
+        // with s_e = A_e h_e fc(r_jk): the partials in r_ij, r_ik and r_jk^2
+        // from the sums of s_e and eta_e s_e
+        const T s0 = A[0] * h[0], s1 = A[1] * h[1];
+        const T sum = s0 + s1;
+        const T S = sum * fc, Se = fma(B.eta[0], s0, B.eta[1] * s1) * fc;
+        const T Sc = T(0.5) * fc * fma(C[0], h[0], C[1] * h[1]);
+        const T e2 = Se + Se;
+        const T Sj = fma(S, Hj.w, -e2 * Rj.w), Sk = fma(S, Hk.w, -e2 * Rk.w);
+        const T Sx = g4 ? T(2) * fma(sum, dfc, -Se) : T(0);
+        const PairGrad<T> p(Rj, Rk, invj, invk, ch + ch, Sc, Sj, Sk, Sx);
+        add_pair<T>(w.sF, live, j, k, step, Rj, Rk, p);
       });
     }
 }
 
 template <typename T>
 __device__ void adjoint_generic(const BehlerTable* tab, int f0, int f1e, const PairList& L,
-                                const typename V4<T>::type* sR, const typename V4<T>::type* sA,
-                                const T* sg, T* sF, int lane) {
+                                const WarpMem<T>& w, int lane) {
   using T4 = typename V4<T>::type;
-  PairWalk w;
-  w.init(L, lane);
-  for (; w.p < L.P; w.advance(L)) {
-    int j, k;
-    w.get(L, j, k);
-    const T4 Rj = sR[j], Rk = sR[k];
-    const T invj = sA[j].x, invk = sA[k].x;
+  run_pairs(L, w.sP, false, 0.f, w.queue, lane, [&](bool live, int j, int k, int key) {
+    const T4 Rj = w.sR[j], Rk = w.sR[k];
+    const T invj = T(1) / Rj.w, invk = T(1) / Rk.w;
     const T dx = Rk.x - Rj.x, dy = Rk.y - Rj.y, dz = Rk.z - Rj.z;
     const T rjk2 = dx * dx + dy * dy + dz * dz;
     const T rjk = sqrt(rjk2);
@@ -784,7 +1053,7 @@ __device__ void adjoint_generic(const BehlerTable* tab, int f0, int f1e, const P
         cutfn(Rk.w, rc_cur, fik, dfik);
         cutfn(rjk, rc_cur, fjk, dfjk);
       }
-      const T g2 = T(2) * sg[f.out];
+      const T g2 = T(2) * w.sg[f.out];
       T F1v, dF1v;
       f1(f, cosv, F1v, dF1v);
       if (f.kind == 4) {
@@ -800,31 +1069,24 @@ __device__ void adjoint_generic(const BehlerTable* tab, int f0, int f1e, const P
         Sik += base3 * F1v * fij * (dfik - T(2) * f.p3 * Rk.w * fik);
       }
     }
-    scatter_pair<T>(Rj, Rk, invj, invk, cosv, dx, dy, dz, rjk, Sc, Sij, Sik, Sjk, sF, j, k);
-  }
+    const T Sx = rjk > T(1e-8) ? Sjk / rjk : T(0);   // 2 dE/d(r_jk^2)
+    const PairGrad<T> p(Rj, Rk, invj, invk, cosv, Sc, Sij, Sik, Sx);
+    add_pair<T>(w.sF, live, j, k, key, Rj, Rk, p);
+  });
 }
 
 // One-sided adjoint: every pair (j, k) is evaluated once, by one lane, and
 // its gradient goes to both staged neighbours' accumulators in shared
-// memory (shared-memory atomics; the pair schedules keep the 32 addresses
-// of a step mostly distinct).  The central atom's gradient is minus the
+// memory (add_pair).  The central atom's gradient is minus the
 // sum over its neighbours (the energy depends on R_j - R_i only), and the
 // atom's virial contribution is -sum_j R_ij (x) dE_i/dR_j.
 template <typename T, bool GRID>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_behler_adjoint(PotDevice pd, DescBuffers b) {
+__global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_behler_adjoint(PotDevice pd, DescBuffers b) {
   using T4 = typename V4<T>::type;
   extern __shared__ __align__(32) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int i = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (i >= b.natoms) return;
-  unsigned char* base = smem_raw + behler_smem_per_warp<T>(b.cap, pd.nsf_pad, true) * warp;
-  T4* sR = reinterpret_cast<T4*>(base);
-  T4* sA = sR + b.cap;
-  T* sF = reinterpret_cast<T*>(sA + b.cap);
-  T* sg = sF + 3 * b.cap;
-  int* sslot = reinterpret_cast<int*>(sg + pd.nsf_pad);
-  int* queue = sslot + b.cap;
+  const int lane = threadIdx.x;
+  const int i = blockIdx.x;
+  const WarpMem<T> w = warp_mem<T>(smem_raw, b.cap, pd.nsf_pad, true);
   const int ti = b.types[i];
   const BehlerTable* tab = table_of<T>(pd, ti);
   const int nt = pd.ntypes;
@@ -835,9 +1097,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_behler_adjoint(
   const T gs = b.grad_scale ? T(b.grad_scale[sid]) : T(1);
   const T* gsrc = reinterpret_cast<const T*>(b.dEdG) + (size_t)i * pd.nsf_pad;
   const int nsf = pd.sp[ti].nsf;
-  for (int k = lane; k < nsf; k += 32) sg[k] = gs * gsrc[k];
+  for (int k = lane; k < nsf; k += 32) w.sg[k] = gs * gsrc[k];
   int bstart[AE_MAXT + 1];
-  const int nst = stage_buckets<T>(vec, jt, n, nt, T(tab->rc_max), sR, sA, sslot, bstart, lane);
+  const int nst = stage_buckets<T>(vec, jt, n, nt, T(tab->rc_max), w.sR, w.sH, w.sslot, bstart,
+                                   lane);
+  fill_positions(w.sR, w.sP, nst, lane);
 
   // radial terms: d/dr_ij of sum_f g_f G_f(r_ij) along Rhat_ij (initialises
   // each staged neighbour's accumulator)
@@ -845,36 +1109,46 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_behler_adjoint(
     int tj = 0;
     for (int s = 0; s < nt; ++s)
       if (j >= bstart[s + 1]) tj = s + 1;
-    const T4 Rj = sR[j];
-    const T inv = sA[j].x;
+    const T r = w.sR[j].w;
+    const T4 A = w.sH[j];
     const int f0 = tab->rad_off[tj], f1e = tab->rad_off[tj + 1];
     T c = T(0);
     for (int q = f0; q < f1e; ++q) {
       const Fn<T> f = load_fn<T>(&tab->fn[q]);
       T v, dv;
-      radial_fn(f, Rj.w, v, dv);
-      c += sg[f.out] * dv;
+      radial_fn(f, r, f.Rc == T(tab->rc_max), A, v, dv);
+      c += w.sg[f.out] * dv;
     }
-    sF[3 * j] = c * Rj.x * inv;
-    sF[3 * j + 1] = c * Rj.y * inv;
-    sF[3 * j + 2] = c * Rj.z * inv;
+    // FP64 sums coefficients of R_j, FP32 the vector
+    T4 acc = w.sR[j];
+    c *= A.x;
+    const T cv = sizeof(T) == 8 ? T(0) : c;
+    acc.x *= cv;
+    acc.y *= cv;
+    acc.z *= cv;
+    acc.w = sizeof(T) == 8 ? c : T(0);
+    w.sF[j] = acc;
   }
   __syncwarp();
 
   // angular terms, each pair once
+  FactorKey<T> key{T(-1), T(-1), T(-1), 0u};
   const BehlerGrid* grids = grids_of(tab);
   for (int a = 0; a < nt; ++a) {
     for (int c = a; c < nt; ++c) {
       const int f0 = tab->ang_off[a * nt + c], f1e = tab->ang_off[a * nt + c + 1];
       if (f0 == f1e) continue;
       const PairList L = pair_list(bstart, a, c);
-      if (L.P == 0) continue;
+      if (empty(L)) continue;
       const int gi = tab->grid_of[a * nt + c];
       if (GRID || gi >= 0) {
         const BehlerGrid* gr = grids + gi;
-        adjoint_grid<T>(gr, L, sR, sA, gr->Rc == tab->rc_max, sg, sF, queue, lane);
+        if (sizeof(T) == 8 && gr->chain)
+          adjoint_grid<T, sizeof(T) == 8>(gr, L, w, key, lane);
+        else
+          adjoint_grid<T, false>(gr, L, w, key, lane);
       } else {
-        if constexpr (!GRID) adjoint_generic<T>(tab, f0, f1e, L, sR, sA, sg, sF, lane);
+        if constexpr (!GRID) adjoint_generic<T>(tab, f0, f1e, L, w, lane);
       }
     }
   }
@@ -886,10 +1160,10 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_behler_adjoint(
   T fix = T(0), fiy = T(0), fiz = T(0);
   T w00 = 0, w01 = 0, w02 = 0, w10 = 0, w11 = 0, w12 = 0, w20 = 0, w21 = 0, w22 = 0;
   for (int j = lane; j < nst; j += 32) {
-    const T gx = sF[3 * j], gy = sF[3 * j + 1], gz = sF[3 * j + 2];
-    atomic_add3<T>(F, jt[sslot[j]] & AE_INDEX_MASK, -gx, -gy, -gz);
+    const T4 Rj = w.sR[j], f = w.sF[j];
+    const T gx = fma(f.w, Rj.x, f.x), gy = fma(f.w, Rj.y, f.y), gz = fma(f.w, Rj.z, f.z);
+    atomic_add3<T>(F, jt[w.sslot[j]] & AE_INDEX_MASK, -gx, -gy, -gz);
     if (want_virial) {
-      const T4 Rj = sR[j];
       w00 -= Rj.x * gx; w01 -= Rj.x * gy; w02 -= Rj.x * gz;
       w10 -= Rj.y * gx; w11 -= Rj.y * gy; w12 -= Rj.y * gz;
       w20 -= Rj.z * gx; w21 -= Rj.z * gy; w22 -= Rj.z * gz;
@@ -916,15 +1190,13 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_behler_adjoint(
 
 template <typename T>
 int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
-  const int warps = 4;
-  const size_t smem = behler_smem_per_warp<T>(b.cap, pd.nsf_pad, adjoint) * warps;
+  const size_t smem = behler_smem_per_warp<T>(b.cap, pd.nsf_pad, adjoint);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  const int blocks = (b.natoms + warps - 1) / warps;
   auto kern = adjoint ? (pd.behler_grid_only ? k_behler_adjoint<T, true> : k_behler_adjoint<T, false>)
                       : (pd.behler_grid_only ? k_behler_forward<T, true> : k_behler_forward<T, false>);
   if (smem + AE_STATIC_SMEM > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kern<<<blocks, warps * 32, smem, s>>>(pd, b);
+  kern<<<b.natoms, 32, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }
 
@@ -983,7 +1255,7 @@ __global__ void __launch_bounds__(128) k_behler_jacobian(PotDevice pd, DescBuffe
     for (int q = tab->rad_off[tj]; q < tab->rad_off[tj + 1]; ++q) {
       const Fn<T> f = load_fn<T>(&tab->fn[q]);
       T v, dv;
-      radial_fn(f, Rj.w, v, dv);
+      radial_fn(f, Rj.w, false, T4{}, v, dv);
       Ja[f.out * 3] += dv * ux;
       Ja[f.out * 3 + 1] += dv * uy;
       Ja[f.out * 3 + 2] += dv * uz;
