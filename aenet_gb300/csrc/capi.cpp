@@ -958,6 +958,7 @@ struct aenet_gpu_plan {
   double* E_struct = nullptr;
   double* virial = nullptr;
   unsigned* status = nullptr;
+  unsigned* ticket = nullptr;   // of the energy reduction's last block
   int nchunks = 0;            // energy-reduction chunks over all structures
   int one_chunk_each = 0;     // every structure has 1 .. AE_ECHUNK atoms
   double2* e_part = nullptr;
@@ -1292,6 +1293,7 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   P->E_struct = (double*)(b + o_Es);
   P->virial = (double*)(b + o_V);
   P->status = (unsigned*)(b + o_st);
+  P->ticket = P->status + 2;
   P->e_part = (double2*)(b + o_ep);
   P->chunk_struct = (int*)(b + o_chs);
   P->order = (int*)(b + o_ord);
@@ -1416,38 +1418,43 @@ NbBuffers nb_buffers(aenet_gpu_plan* P) {
 
 int ck(int e) { return e ? AENET_ERR_CUDA : 0; }
 
-// The types the neighbour search reads: the per-structure searches take
-// the caller's 1-based ids and write the checked 0-based ones themselves;
-// the other searches read the 0-based ids of the type kernel, launched
-// here.  Null on a launch error.
-const int* search_types(aenet_gpu_plan* P, NbBuffers& nb, const int* d_types, cudaStream_t s) {
-  if ((nb.cell_kernel == 4 || nb.cell_kernel == 5) && nb.struct_order) {
-    nb.types0_out = P->types0;
-    nb.ntypes = P->pd->ntypes;
-    return d_types;
+// Buffers of a plan's own search: it reads the caller's 1-based type ids and
+// writes the checked 0-based ones itself; small plans' searches also group
+// the atoms by species (`grouped`).
+NbBuffers search_buffers(aenet_gpu_plan* P, bool* grouped) {
+  NbBuffers nb = nb_buffers(P);
+  nb.types0_out = P->types0;
+  nb.ntypes = P->pd->ntypes;
+  const bool per_struct = (nb.cell_kernel == 4 || nb.cell_kernel == 5) && nb.struct_order;
+  *grouped = !per_struct && P->natoms > 0 && ae_cells_one(P->natoms, P->ncells);
+  if (*grouped) {
+    nb.order_out = P->order;
+    nb.spec_off_out = P->spec_off;
   }
-  if (ae_launch_types(P->natoms, d_types, P->types0, P->pd->ntypes, P->status, s)) return nullptr;
-  return P->types0;
+  return nb;
 }
 
-int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s);
+int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s,
+              bool zero_F = false, bool grouped = false);
 
 // neighbours + descriptors + networks + energies
+// (zero_F: an adjoint follows in the same call; the descriptor kernel clears
+// its force accumulator, one memset less)
 int plan_forward(aenet_gpu_plan* P, const double* d_coords, const int* d_types, double* d_E,
-                 double* d_E_atoms, cudaStream_t s) {
-  NbBuffers nb = nb_buffers(P);
-  const int* t_in = search_types(P, nb, d_types, s);
-  if (!t_in) return AENET_ERR_CUDA;
-  if (ck(ae_launch_neighbors(P->natoms, d_coords, t_in, nb, P->fp64, s))) return AENET_ERR_CUDA;
-  return plan_eval(P, d_E, d_E_atoms, s);
+                 double* d_E_atoms, cudaStream_t s, bool zero_F = false) {
+  bool grouped;
+  const NbBuffers nb = search_buffers(P, &grouped);
+  if (ck(ae_launch_neighbors(P->natoms, d_coords, d_types, nb, P->fp64, s))) return AENET_ERR_CUDA;
+  return plan_eval(P, d_E, d_E_atoms, s, zero_F, grouped);
 }
 
 // networks: tensor-core kernel on the mixed path when the networks fit it
-// (atoms grouped by species first), the SIMT kernel otherwise
-int plan_networks(aenet_gpu_plan* P, const DescBuffers& d, cudaStream_t s) {
+// (atoms grouped by species first, unless the search did), the SIMT kernel
+// otherwise
+int plan_networks(aenet_gpu_plan* P, const DescBuffers& d, cudaStream_t s, bool grouped = false) {
   const PotDevice& pd = *P->pd;
   if (!P->fp64 && pd.tc_ok && g.networks_tc) {
-    if (ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
+    if (!grouped && ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
                                P->spec_off, s)))
       return AENET_ERR_CUDA;
     return ck(ae_launch_mlp_tc(pd, d, P->order, P->spec_off, s));
@@ -1456,9 +1463,11 @@ int plan_networks(aenet_gpu_plan* P, const DescBuffers& d, cudaStream_t s) {
 }
 
 // descriptors + networks + energies on the current neighbour table
-int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s) {
+int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s, bool zero_F,
+              bool grouped) {
   const PotDevice& pd = *P->pd;
   DescBuffers d = desc_buffers(P, nullptr, false);
+  d.zero_F = zero_F ? 1 : 0;
   if (d.nb_rank &&
       ck(ae_launch_stale_order(P->natoms, P->geom_d, P->atom_struct, P->r_wrap, pd, d, P->fp64,
                                P->stale_caller_order, P->nb_rank, P->nb_seff, s)))
@@ -1466,11 +1475,10 @@ int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s)
   int e = (pd.sp[0].sftype == AE_SF_BEHLER) ? ae_launch_behler_forward(pd, d, P->fp64, s)
                                              : ae_launch_chebyshev_forward(pd, d, P->fp64, s);
   if (ck(e)) return AENET_ERR_CUDA;
-  if (plan_networks(P, d, s)) return AENET_ERR_CUDA;
+  if (plan_networks(P, d, s, grouped)) return AENET_ERR_CUDA;
   if (ck(ae_launch_energy_reduce_chunked(P->nstruc, P->nchunks, P->geom_d, P->chunk_struct,
-                                         P->E_atom, P->e_part, P->E_struct, P->one_chunk_each, s)))
-    return AENET_ERR_CUDA;
-  if (d_E && cudaMemcpyAsync(d_E, P->E_struct, 8 * (size_t)P->nstruc, cudaMemcpyDeviceToDevice, s))
+                                         P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
+                                         P->ticket, d_E, s)))
     return AENET_ERR_CUDA;
   if (d_E_atoms &&
       cudaMemcpyAsync(d_E_atoms, P->E_atom, 8 * (size_t)P->natoms, cudaMemcpyDeviceToDevice, s))
@@ -1479,10 +1487,10 @@ int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s)
 }
 
 int plan_adjoint(aenet_gpu_plan* P, const double* grad_scale, double* d_out, double out_sign,
-                 double* d_virial, cudaStream_t s) {
+                 double* d_virial, cudaStream_t s, bool F_zeroed = false) {
   const PotDevice& pd = *P->pd;
   const size_t tsz = P->fp64 ? 8 : 4;
-  if (cudaMemsetAsync(P->Facc, 0, 4 * tsz * (size_t)P->natoms, s)) return AENET_ERR_CUDA;
+  if (!F_zeroed && cudaMemsetAsync(P->Facc, 0, 4 * tsz * (size_t)P->natoms, s)) return AENET_ERR_CUDA;
   if (d_virial && cudaMemsetAsync(P->virial, 0, 72 * (size_t)P->nstruc, s)) return AENET_ERR_CUDA;
   DescBuffers d = desc_buffers(P, grad_scale, d_virial != nullptr);
   if (g.lpa_adjoint) d.lpa = g.lpa_adjoint;
@@ -2413,11 +2421,11 @@ EXPORT int aenet_gpu_plan_run(aenet_gpu_plan* P, const double* d_coords, const i
                               unsigned flags, void* stream) {
   if (!P) return AENET_ERR_INPUT;
   cudaStream_t s = (cudaStream_t)stream;
-  int st = plan_forward(P, d_coords, d_types, d_E, d_E_atoms, s);
-  if (st) return st;
-  if ((flags & (AENET_GPU_FORCES | AENET_GPU_VIRIAL)) || d_F || d_virial)
-    return plan_adjoint(P, nullptr, d_F, 1.0, (flags & AENET_GPU_VIRIAL) ? d_virial : nullptr, s);
-  return 0;
+  const bool adjoint = (flags & (AENET_GPU_FORCES | AENET_GPU_VIRIAL)) || d_F || d_virial;
+  int st = plan_forward(P, d_coords, d_types, d_E, d_E_atoms, s, adjoint);
+  if (st || !adjoint) return st;
+  return plan_adjoint(P, nullptr, d_F, 1.0, (flags & AENET_GPU_VIRIAL) ? d_virial : nullptr, s,
+                      true);
 }
 
 EXPORT int aenet_gpu_plan_forward(aenet_gpu_plan* P, const double* d_coords, const int* d_types,
@@ -2484,10 +2492,10 @@ EXPORT int aenet_gpu_plan_loss_gradient(aenet_gpu_plan* P, const double* d_coord
   int st = plan_train_alloc(P);
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  st = plan_forward(P, d_coords, d_types, d_E, nullptr, s);
+  st = plan_forward(P, d_coords, d_types, d_E, nullptr, s, force_term || d_F);
   if (st) return st;
   if (force_term || d_F) {
-    st = plan_adjoint(P, nullptr, d_F, 1.0, nullptr, s);
+    st = plan_adjoint(P, nullptr, d_F, 1.0, nullptr, s, true);
     if (st) return st;
   }
   if (ck(ae_launch_loss(P->nstruc, P->geom_d, P->E_struct, d_E_target, P->Facc,
@@ -3015,9 +3023,8 @@ EXPORT int aenet_gpu_plan_descriptor_loss_gradient(aenet_gpu_plan* P, const int*
   DescBuffers d = desc_buffers(P, nullptr, false);
   if (plan_networks(P, d, s)) return AENET_ERR_CUDA;
   if (ck(ae_launch_energy_reduce_chunked(P->nstruc, P->nchunks, P->geom_d, P->chunk_struct,
-                                         P->E_atom, P->e_part, P->E_struct, P->one_chunk_each, s)))
-    return AENET_ERR_CUDA;
-  if (d_E && cudaMemcpyAsync(d_E, P->E_struct, 8 * (size_t)P->nstruc, cudaMemcpyDeviceToDevice, s))
+                                         P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
+                                         P->ticket, d_E, s)))
     return AENET_ERR_CUDA;
   if (ck(ae_launch_loss(P->nstruc, P->geom_d, P->E_struct, d_E_target, P->Facc, nullptr, 0, 1.0, 0.0,
                         pd.sp[0].E_scale, P->cE, P->U, P->loss_s, d_loss, P->fp64, s)) ||
@@ -3112,12 +3119,11 @@ EXPORT int aenet_gpu_plan_profile(aenet_gpu_plan* P, const double* d_coords, con
   for (int q = 0; q < 9; ++q) cudaEventCreate(&ev[q]);
   int e = 0;
   cudaEventRecord(ev[0], s);
-  NbBuffers nb = nb_buffers(P);
-  const int* t_in = search_types(P, nb, d_types, s);
-  if (!t_in) e = 1;
+  bool grouped;
+  NbBuffers nb = search_buffers(P, &grouped);   // the searches check the types themselves
   cudaEventRecord(ev[1], s);
   nb.ev_search = ev[8];
-  if (t_in) e |= ae_launch_neighbors(P->natoms, d_coords, t_in, nb, P->fp64, s);
+  e |= ae_launch_neighbors(P->natoms, d_coords, d_types, nb, P->fp64, s);
   cudaEventRecord(ev[2], s);
   DescBuffers d = desc_buffers(P, nullptr, false);
   if (d.nb_rank)
@@ -3126,11 +3132,11 @@ EXPORT int aenet_gpu_plan_profile(aenet_gpu_plan* P, const double* d_coords, con
   e |= (pd.sp[0].sftype == AE_SF_BEHLER) ? ae_launch_behler_forward(pd, d, P->fp64, s)
                                           : ae_launch_chebyshev_forward(pd, d, P->fp64, s);
   cudaEventRecord(ev[3], s);
-  e |= plan_networks(P, d, s);
+  e |= plan_networks(P, d, s, grouped);
   cudaEventRecord(ev[4], s);
   e |= ae_launch_energy_reduce_chunked(P->nstruc, P->nchunks, P->geom_d, P->chunk_struct,
-                                       P->E_atom, P->e_part, P->E_struct, P->one_chunk_each, s);
-  if (d_E) cudaMemcpyAsync(d_E, P->E_struct, 8 * (size_t)P->nstruc, cudaMemcpyDeviceToDevice, s);
+                                       P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
+                                       P->ticket, d_E, s);
   cudaEventRecord(ev[5], s);
   const size_t tsz = P->fp64 ? 8 : 4;
   cudaMemsetAsync(P->Facc, 0, 4 * tsz * (size_t)P->natoms, s);

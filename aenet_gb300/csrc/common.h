@@ -225,7 +225,7 @@ struct NbBuffers {
   double* r_wrap;             // [N][3] Cartesian of the wrapped coordinates
   float4* r_f32;              // [N] (x, y, z, species as int bits)
   int* cell_of;               // [N] packed cell coordinates cx|cy<<10|cz<<20
-  int* slot_of;               // [N] rank of the atom inside its cell
+  int* slot_of;               // [N] rank of the atom inside its cell (or its cell's index)
   int* cell_count;            // [ncells_total]
   int* cell_start;            // [ncells_total + 1] exclusive prefix of counts
   int* scan_tmp;              // [scan blocks + 1]
@@ -244,17 +244,23 @@ struct NbBuffers {
   // shared-memory capacity of one block (atoms, cells); null = unavailable
   const int* struct_order;
   int smem_atoms, smem_cells;
-  // optional, per-structure search only: the search reads the caller's
-  // 1-based type ids and writes the checked 0-based ones here (no separate
-  // type kernel)
+  // optional: the search reads the caller's 1-based type ids and writes the
+  // checked 0-based ones here (no separate type kernel)
   int* types0_out;
   int ntypes;
+  // optional, plans that ae_cells_one() takes: the atoms grouped by species
+  int* order_out;
+  int* spec_off_out;
   int cell_kernel;            // 0: warp per atom; warp per home cell with a lane per
                               // home atom (1) or a lane per candidate (2); 3: warp per
                               // atom over the half stencil, each pair written to both rows;
                               // 4: block per structure, cell lists in shared memory
 };
 
+// plans whose cell lists one block builds (with the grouping by species)
+#define AE_ONE_ATOMS 12288
+#define AE_ONE_CELLS 16384
+bool ae_cells_one(int natoms, int ncells);
 int ae_launch_neighbors(int natoms, const double* pos, const int* types,
                         const NbBuffers& nb, int fp64, cudaStream_t s);
 // ELL table from a caller's CSR neighbour list (local atoms, indices into
@@ -276,6 +282,7 @@ struct DescBuffers {
   void* dEdG;                  // [N][nsf_pad] (T)
   double* E_atom;              // [N]
   void* F;                     // [N][4] (T) force accumulator (T=float: float4)
+  int zero_F;                  // the forward kernels clear it
   double* virial;             // [nstruc][9] or null
   const int* atom_struct;
   const double* grad_scale;    // per structure factor on dE (or null = 1)
@@ -359,11 +366,14 @@ int ae_launch_types(int natoms, const int* types1, int* types0, int ntypes,
 // per-structure energies: FP64 sums over chunks of AE_ECHUNK atoms (one
 // warp each; chunk_struct[c] = structure of chunk c), then over each
 // structure's chunks, in pairwise order
-// one_chunk_each: every structure has 1 .. AE_ECHUNK atoms (the chunk pass
-// then writes every total and the combining pass is skipped)
+// one_chunk_each: every structure has 1 .. AE_ECHUNK atoms (a warp per
+// structure); otherwise a block per chunk, and the last block to finish adds
+// the chunks (ticket: a zeroed word, zero again afterwards).  E_out: optional
+// second copy of the totals.
 int ae_launch_energy_reduce_chunked(int nstruc, int nchunks, const StructGeom* geom,
                                     const int* chunk_struct, const double* E_atom, double2* part,
-                                    double* E_struct, int one_chunk_each, cudaStream_t s);
+                                    double* E_struct, int one_chunk_each, unsigned* ticket,
+                                    double* E_out, cudaStream_t s);
 int ae_launch_energy_reduce(int nstruc, const StructGeom* geom,
                             const double* E_atom, double* E_struct,
                             cudaStream_t s);

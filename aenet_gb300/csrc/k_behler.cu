@@ -815,6 +815,11 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_beh
   const int nst = stage_buckets<T>(vec, jt, n, nt, T(tab->rc_max), w.sR, w.sH, w.sslot, bstart,
                                    lane);
   fill_positions(w.sR, w.sP, nst, lane);
+  if (b.zero_F && lane == 0) {
+    T4 z;
+    z.x = z.y = z.z = z.w = T(0);
+    reinterpret_cast<T4*>(b.F)[i] = z;
+  }
   const size_t nrow = (size_t)ti * pd.nsf_pad;
   T* G = reinterpret_cast<T*>(b.G) + (size_t)i * pd.nsf_pad;
   const int nsf = pd.sp[ti].nsf;

@@ -362,6 +362,11 @@ __global__ void __launch_bounds__(128, MOM ? (A <= 5 ? AE_MOM_FWD_BLOCKS : 3) : 
   const T4* __restrict__ vec = reinterpret_cast<const T4*>(b.nb_vec) + (size_t)i * b.cap;
   const int* __restrict__ jt = b.nb_jt + (size_t)i * b.cap;
   if (sl == 0) prefetch_rows(vec, jt, n);
+  if (b.zero_F && active && sl == 0) {
+    T4 z;
+    z.x = z.y = z.z = z.w = T(0);
+    reinterpret_cast<T4*>(b.F)[i] = z;
+  }
   const int nloop = warp_max(n);
   const T r_Rc = T(ct.r_Rc), a_Rc = T(ct.a_Rc);
   const T two_over_rc = T(2) / r_Rc;

@@ -155,48 +155,98 @@ __global__ void k_energy_reduce(int nstruc, const StructGeom* geom, const double
   if (lane == 0) E_struct[sidx] = s + c;
 }
 
-// chunk c of the structure whose chunk range contains it
-__global__ void k_energy_chunks(int nstruc, int nchunks, const StructGeom* __restrict__ geom,
-                                const int* __restrict__ chunk_struct,
-                                const double* __restrict__ E_atom, double2* __restrict__ part,
-                                double* __restrict__ E_struct) {
-  const int lane = threadIdx.x & 31;
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (c >= nchunks) return;
-  const int sidx = chunk_struct[c];
-  const StructGeom& g = geom[sidx];
-  const int a0 = (c - g.chunk_off) * AE_ECHUNK;
-  const int a1 = min(g.natoms, a0 + AE_ECHUNK);
-  // pairwise order (a lane's run, then a tree over the lanes): the rounding
-  // error stays within (AE_ECHUNK/32 + 5) ulp of sum |E_i|
-  double s = 0.0;
-  for (int a = a0 + lane; a < a1; a += 32) s += E_atom[g.atom_off + a];
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-  if (lane == 0) {
-    part[c] = make_double2(s, 0.0);
-    if (g.natoms <= AE_ECHUNK) E_struct[sidx] = s;   // single chunk: final already
-  }
-}
-
-// one warp per structure over its chunks
-__global__ void k_energy_struct(int nstruc, int nchunks, const StructGeom* __restrict__ geom,
-                                const double2* __restrict__ part, double* __restrict__ E_struct) {
+// structures of one chunk: a warp each.  Pairwise order (a lane's run, then a
+// tree over the lanes): the rounding error stays within (AE_ECHUNK/32 + 5) ulp
+// of sum |E_i|
+__global__ void k_energy_warp(int nstruc, const StructGeom* __restrict__ geom,
+                              const double* __restrict__ E_atom, double* __restrict__ E_struct,
+                              double* __restrict__ E_out) {
   const int lane = threadIdx.x & 31;
   const int sidx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (sidx >= nstruc) return;
-  const int c0 = geom[sidx].chunk_off;
-  const int c1 = sidx + 1 < nstruc ? geom[sidx + 1].chunk_off : nchunks;
-  if (c1 - c0 == 1) return;   // written by k_energy_chunks
-  if (c1 == c0) {
-    if (lane == 0) E_struct[sidx] = 0.0;
-    return;
-  }
+  const int n = geom[sidx].natoms;
+  const double* E = E_atom + geom[sidx].atom_off;
   double s = 0.0;
-  for (int c = c0 + lane; c < c1; c += 32) s += part[c].x;
+  for (int a = lane; a < n; a += 32) s += E[a];
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-  if (lane == 0) E_struct[sidx] = s;
+  if (lane == 0) {
+    E_struct[sidx] = s;
+    if (E_out) E_out[sidx] = s;
+  }
+}
+
+// a block of 256 threads per chunk of AE_ECHUNK atoms (eight atoms a thread,
+// then a tree), and the last block to finish adds each structure's chunks in
+// the same way: one launch, the same order every time.  (One warp per chunk
+// and a second kernel took 13 us at 4,000 atoms, a chain of 64 loads and FP64
+// additions.)
+__device__ __forceinline__ double block_sum256(double s, double* ws) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = 0.0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) s += ws[w];
+  return s;
+}
+__global__ void __launch_bounds__(256) k_energy_blocks(int nstruc, int nchunks,
+                                                       const StructGeom* __restrict__ geom,
+                                                       const int* __restrict__ chunk_struct,
+                                                       const double* __restrict__ E_atom,
+                                                       double2* part, double* __restrict__ E_struct,
+                                                       double* __restrict__ E_out,
+                                                       unsigned* ticket) {
+  __shared__ double ws[8];
+  __shared__ bool s_last;
+  const int c = blockIdx.x;
+  if (c < nchunks) {
+    const StructGeom& g = geom[chunk_struct[c]];
+    const int a0 = (c - g.chunk_off) * AE_ECHUNK, a1 = min(g.natoms, a0 + AE_ECHUNK);
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < AE_ECHUNK / 256; ++q) {
+      const int a = a0 + q * 256 + threadIdx.x;
+      if (a < a1) s += E_atom[g.atom_off + a];
+    }
+    s = block_sum256(s, ws);
+    if (threadIdx.x == 0) part[c] = make_double2(s, 0.0);
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const volatile double2* vp = part;
+  // a warp per structure for many, the whole block for one
+  if (nstruc == 1) {
+    double s = 0.0;
+    for (int k = threadIdx.x; k < nchunks; k += 256) s += vp[k].x;
+    s = block_sum256(s, ws);
+    if (threadIdx.x == 0) {
+      E_struct[0] = s;
+      if (E_out) E_out[0] = s;
+    }
+  } else {
+    const int lane = threadIdx.x & 31;
+    for (int sidx = threadIdx.x >> 5; sidx < nstruc; sidx += 8) {
+      const int c0 = geom[sidx].chunk_off;
+      const int c1 = sidx + 1 < nstruc ? geom[sidx + 1].chunk_off : nchunks;
+      double s = 0.0;
+      for (int k = c0 + lane; k < c1; k += 32) s += vp[k].x;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      if (lane == 0) {
+        E_struct[sidx] = s;
+        if (E_out) E_out[sidx] = s;
+      }
+    }
+  }
+  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 template <typename T>
@@ -304,13 +354,16 @@ int ae_launch_mlp(const PotDevice& pd, const DescBuffers& b, int fp64, cudaStrea
 
 int ae_launch_energy_reduce_chunked(int nstruc, int nchunks, const StructGeom* geom,
                                     const int* chunk_struct, const double* E_atom, double2* part,
-                                    double* E_struct, int one_chunk_each, cudaStream_t s) {
+                                    double* E_struct, int one_chunk_each, unsigned* ticket,
+                                    double* E_out, cudaStream_t s) {
   if (nstruc <= 0) return 0;
-  if (nchunks > 0)
-    k_energy_chunks<<<(nchunks + 7) / 8, 256, 0, s>>>(nstruc, nchunks, geom, chunk_struct, E_atom,
-                                                      part, E_struct);
-  if (!one_chunk_each)
-    k_energy_struct<<<(nstruc + 7) / 8, 256, 0, s>>>(nstruc, nchunks, geom, part, E_struct);
+  // one structure takes the blocks at any size (a block sums 256 atoms at a
+  // time, a warp 32)
+  if (one_chunk_each && nstruc > 1)
+    k_energy_warp<<<(nstruc + 7) / 8, 256, 0, s>>>(nstruc, geom, E_atom, E_struct, E_out);
+  else
+    k_energy_blocks<<<nchunks > 0 ? nchunks : 1, 256, 0, s>>>(nstruc, nchunks, geom, chunk_struct,
+                                                             E_atom, part, E_struct, E_out, ticket);
   return (int)cudaGetLastError();
 }
 

@@ -16,6 +16,8 @@
 //                  coordinates, cell, rank inside the cell (atomic count)
 //   k_scan_*       exclusive prefix sum of the cell counts (CSR offsets)
 //   k_scatter      atoms and their FP32 positions in cell order
+//   k_cells_one    the last two and the grouping of the atoms by species for
+//                  up to AE_ONE_ATOMS atoms, in one block
 //   k_neighbors    one warp per atom.  The stencil of cells around the
 //                  atom's cell is walked as units (row d0, d1; image t2 along
 //                  the third axis): each unit is one contiguous run of cells
@@ -34,6 +36,18 @@
 namespace {
 
 constexpr double TWO_PI = 6.283185307179586;  // 2 * 3.141592653589793
+
+// x / (2 pi), correctly rounded: Markstein's division by a divisor whose
+// correctly rounded reciprocal is at hand (P. Markstein, IBM J. Res. Dev. 34,
+// 1990): a faithful quotient, its exact remainder by a fused multiply-add,
+// one correction.  Five FP64 instructions on the pipe that bounds k_wrap_bin;
+// same bits as the division.
+constexpr double INV_TWO_PI = 1.0 / TWO_PI;
+__host__ __device__ __forceinline__ double over_two_pi(double x) {
+  double q = x * INV_TWO_PI;
+  q = fma(fma(-q, TWO_PI, x), INV_TWO_PI, q);
+  return fma(fma(-q, TWO_PI, x), INV_TWO_PI, q);
+}
 
 __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double da(double a, double b) { return __dadd_rn(a, b); }
@@ -63,25 +77,35 @@ __device__ __forceinline__ int wrap_bin_atom(int i, const StructGeom* g, const d
   double r[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
   double s[3], rw[3];
   const int nc[3] = {g->nc[0], g->nc[1], g->nc[2]};
+  const bool ortho = g->ortho;
   if (g->pbc) {
     for (int v = 0; v < 3; ++v) {
       double t;
       if (g->frac_mode == 2) {
         t = r[v];
       } else {
-        // (B r) summed in column order (geometry.f90:708)
-        t = dm(g->B[3 * v], r[0]);
-        t = da(t, dm(g->B[3 * v + 1], r[1]));
-        t = da(t, dm(g->B[3 * v + 2], r[2]));
-        if (g->frac_mode == 0) t = __ddiv_rn(t, TWO_PI);
+        // (B r) summed in column order (geometry.f90:708); the terms that
+        // are zero in an orthogonal cell change no bit of the sum
+        if (ortho) {
+          t = dm(g->B[4 * v], r[v]);
+        } else {
+          t = dm(g->B[3 * v], r[0]);
+          t = da(t, dm(g->B[3 * v + 1], r[1]));
+          t = da(t, dm(g->B[3 * v + 2], r[2]));
+        }
+        if (g->frac_mode == 0) t = over_two_pi(t);
       }
       s[v] = wrap_coordinate(t, nb.status);
     }
     for (int c = 0; c < 3; ++c) {
-      double t = dm(g->L[c], s[0]);
-      t = da(t, dm(g->L[3 + c], s[1]));
-      t = da(t, dm(g->L[6 + c], s[2]));
-      rw[c] = t;
+      if (ortho) {
+        rw[c] = dm(g->L[4 * c], s[c]);
+      } else {
+        double t = dm(g->L[c], s[0]);
+        t = da(t, dm(g->L[3 + c], s[1]));
+        t = da(t, dm(g->L[6 + c], s[2]));
+        rw[c] = t;
+      }
     }
   } else {
     for (int v = 0; v < 3; ++v) {
@@ -117,15 +141,19 @@ __device__ __forceinline__ int wrap_bin_atom(int i, const StructGeom* g, const d
   return (cc[0] * nc[1] + cc[1]) * nc[2] + cc[2];
 }
 
-// one thread per atom; the rank inside the cell from an atomic count
+// one thread per atom; the rank inside the cell from an atomic count, or
+// (one: k_cells_one follows, which counts) the cell's index alone
 __global__ void k_wrap_bin(int natoms, const double* __restrict__ pos,
-                           const int* __restrict__ types, NbBuffers nb) {
+                           const int* __restrict__ types, NbBuffers nb, int one) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= natoms) return;
   const StructGeom* g = nb.geom + nb.atom_struct[i];
-  const int lin = wrap_bin_atom(i, g, pos, types, nb);
-  nb.slot_of[i] = atomicAdd(&nb.cell_count[g->cell_off + lin], 1);
+  const int lin = g->cell_off + wrap_bin_atom(i, g, pos, types, nb);
+  nb.slot_of[i] = one ? lin : atomicAdd(&nb.cell_count[lin], 1);
 }
+// Its threads per block: the FP64 pipe bounds it, so that a few hundred
+// atoms are spread over the SMs (256 atoms: 11.5 us in one block of 256).
+constexpr int WRAP_B = 64;
 
 // ---- exclusive scan of the cell counts (three phases, 1024 per block)
 constexpr int SCAN_B = 1024;
@@ -200,6 +228,84 @@ __global__ void k_scatter(int natoms, NbBuffers nb) {
   const int p = nb.cell_start[g->cell_off + lin] + nb.slot_of[i];
   nb.cell_atoms[p] = i;
   nb.cell_pos[p] = nb.r_f32[i];
+}
+
+// Cell offsets, the atoms in cell order (ascending index inside a cell, so
+// that rows come out the same every time) and, when asked, the atoms grouped
+// by species, for small plans in one block: one launch instead of a memset,
+// three scans, a scatter and the three kernels of the general partition, none
+// of which does more than launch at these sizes (whole pass, with the energy
+// sum in one launch: 256 copper atoms 112 -> 79 us, 4,000 Au/Cu 152 -> 109).
+constexpr int ONE_B = 1024;
+constexpr int ONE_PER = AE_ONE_ATOMS / ONE_B;
+__global__ void __launch_bounds__(ONE_B) k_cells_one(int natoms, NbBuffers nb) {
+  extern __shared__ int sm_one[];
+  __shared__ int wt[33], sp_cnt[AE_MAXT], sp_off[AE_MAXT];
+  const int nc = nb.ncells_total;
+  int* start = sm_one;            // [nc + 1] counts, then offsets
+  int* list = sm_one + nc + 1;    // [natoms] atoms by cell, unordered
+  for (int c = threadIdx.x; c < nc; c += ONE_B) start[c] = 0;
+  if (threadIdx.x < AE_MAXT) sp_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  int cell[ONE_PER], rank[ONE_PER], spec[ONE_PER], srank[ONE_PER];
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < ONE_PER; ++q) {
+    const int i = q * ONE_B + threadIdx.x;
+    cell[q] = -1;
+    spec[q] = -1;
+    if (i < natoms) {
+      cell[q] = nb.slot_of[i];
+      rank[q] = atomicAdd(&start[cell[q]], 1);
+      spec[q] = __float_as_int(nb.r_f32[i].w);
+    }
+    if (nb.order_out && __any_sync(0xffffffffu, i < natoms)) {
+      const unsigned m = __match_any_sync(0xffffffffu, spec[q]);
+      const int lead = __ffs(m) - 1;
+      int b = 0;
+      if (lane == lead && spec[q] >= 0) b = atomicAdd(&sp_cnt[spec[q]], __popc(m));
+      srank[q] = __shfl_sync(0xffffffffu, b, lead) + __popc(m & ((1u << lane) - 1u));
+    }
+  }
+  __syncthreads();
+  // offsets: a run of cells per thread
+  const int per = (nc + ONE_B - 1) / ONE_B, c0 = threadIdx.x * per;
+  int sum = 0;
+  for (int c = c0; c < min(nc, c0 + per); ++c) sum += start[c];
+  int total, run = block_excl_scan(sum, wt, total);
+  for (int c = c0; c < min(nc, c0 + per); ++c) {
+    const int v = start[c];
+    start[c] = run;
+    nb.cell_start[c] = run;
+    run += v;
+  }
+  if (threadIdx.x == 0) {
+    start[nc] = total;
+    nb.cell_start[nc] = total;
+    int o = 0;
+    for (int t = 0; t < nb.ntypes; ++t) {
+      sp_off[t] = o;
+      if (nb.order_out) nb.spec_off_out[t] = o;
+      o += sp_cnt[t];
+    }
+    if (nb.order_out) nb.spec_off_out[nb.ntypes] = o;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < ONE_PER; ++q)
+    if (cell[q] >= 0) list[start[cell[q]] + rank[q]] = q * ONE_B + threadIdx.x;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < ONE_PER; ++q)
+    if (cell[q] >= 0) {
+      const int i = q * ONE_B + threadIdx.x;
+      const int b = start[cell[q]], e = start[cell[q] + 1];
+      int p = b;
+      for (int k = b; k < e; ++k) p += list[k] < i;
+      nb.cell_atoms[p] = i;
+      nb.cell_pos[p] = nb.r_f32[i];
+      if (nb.order_out) nb.order_out[sp_off[spec[q]] + srank[q]] = i;
+    }
 }
 
 __device__ __forceinline__ int sext10i(int v) { return (v ^ 512) - 512; }
@@ -1594,6 +1700,14 @@ int ae_launch_ell_from_csr(int nlocal, int nall, const double* x, const int* typ
   return (int)cudaGetLastError();
 }
 
+// Up to 12,288 atoms and 16,384 cells (115 KB of shared memory).  Mixed
+// passes with the one block and with the general kernels: 2,048 Au/Cu atoms
+// 83 and 97 us, 4,000 108 and 125, 8,192 138 and 156, 9,000 rutile atoms 738
+// and 750, 16,384 Au/Cu atoms 205 both ways.
+bool ae_cells_one(int natoms, int ncells) {
+  return natoms <= AE_ONE_ATOMS && ncells <= AE_ONE_CELLS;
+}
+
 int ae_launch_neighbors(int natoms, const double* pos, const int* types, const NbBuffers& nb,
                         int fp64, cudaStream_t s) {
   if (natoms <= 0) return 0;
@@ -1632,15 +1746,25 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
     return (int)cudaGetLastError();
   }
   const int nc = nb.ncells_total;
-  cudaError_t e = cudaMemsetAsync(nb.cell_count, 0, sizeof(int) * (size_t)nc, s);
-  if (e != cudaSuccess) return (int)e;
-  k_wrap_bin<<<(natoms + 255) / 256, 256, 0, s>>>(natoms, pos, types, nb);
-  // CSR offsets: cell_start[c] = sum of the counts before c, cell_start[nc] = natoms
-  const int nblk = (nc + SCAN_B - 1) / SCAN_B;
-  k_scan_blocks<<<nblk, SCAN_B, 0, s>>>(nc, nb.cell_count, nb.cell_start, nb.scan_tmp);
-  k_scan_sums<<<1, SCAN_B, 0, s>>>(nblk, nb.scan_tmp, nb.cell_start + nc);
-  k_scan_add<<<nblk, SCAN_B, 0, s>>>(nc, nb.cell_start, nb.scan_tmp);
-  k_scatter<<<(natoms + 255) / 256, 256, 0, s>>>(natoms, nb);
+  cudaError_t e = cudaSuccess;
+  const int wrap_blocks = (natoms + WRAP_B - 1) / WRAP_B;
+  if (ae_cells_one(natoms, nc)) {
+    k_wrap_bin<<<wrap_blocks, WRAP_B, 0, s>>>(natoms, pos, types, nb, 1);
+    const size_t smem = sizeof(int) * ((size_t)nc + 1 + natoms);
+    if (smem + AE_STATIC_SMEM > 48 * 1024)
+      cudaFuncSetAttribute(k_cells_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_cells_one<<<1, ONE_B, smem, s>>>(natoms, nb);
+  } else {
+    e = cudaMemsetAsync(nb.cell_count, 0, sizeof(int) * (size_t)nc, s);
+    if (e != cudaSuccess) return (int)e;
+    k_wrap_bin<<<wrap_blocks, WRAP_B, 0, s>>>(natoms, pos, types, nb, 0);
+    // CSR offsets: cell_start[c] = sum of the counts before c, cell_start[nc] = natoms
+    const int nblk = (nc + SCAN_B - 1) / SCAN_B;
+    k_scan_blocks<<<nblk, SCAN_B, 0, s>>>(nc, nb.cell_count, nb.cell_start, nb.scan_tmp);
+    k_scan_sums<<<1, SCAN_B, 0, s>>>(nblk, nb.scan_tmp, nb.cell_start + nc);
+    k_scan_add<<<nblk, SCAN_B, 0, s>>>(nc, nb.cell_start, nb.scan_tmp);
+    k_scatter<<<(natoms + 255) / 256, 256, 0, s>>>(natoms, nb);
+  }
   if (nb.ev_search) cudaEventRecord(nb.ev_search, s);
   if (nb.cell_kernel == 3) {
     e = cudaMemsetAsync(nb.nb_cnt, 0, sizeof(int) * (size_t)natoms, s);
