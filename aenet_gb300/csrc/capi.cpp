@@ -328,9 +328,9 @@ float typespin(int num_types, int l) {
 // Legendre expansion of the angular basis: T_n(x(c)) = sum_l q[n][l] P_l(c)
 // for n < a_N <= AE_MOMA, x(c) = c or the legacy (2c - pi)/pi of
 // sfbasis.f90's PI.  Monomial coefficients in c, peeled from the top degree.
-std::vector<float> legendre_table(int a_N, int legacy) {
+std::vector<double> legendre_table(int a_N, int legacy) {
   const int D = AE_MOMA;
-  std::vector<float> q(D * D, 0.f);
+  std::vector<double> q(D * D, 0.0);
   if (a_N > D) return q;
   const double pi = 3.14159265358979;
   const double al = legacy ? 2.0 / pi : 1.0, be = legacy ? -1.0 : 0.0;
@@ -358,7 +358,7 @@ std::vector<float> legendre_table(int a_N, int legacy) {
     std::vector<double> rem = Tn[n];
     for (int l = n; l >= 0; --l) {
       const double c = rem[l] / Pl[l][l];
-      q[n * D + l] = (float)c;
+      q[n * D + l] = c;
       for (int e = 0; e <= l; ++e) rem[e] -= c * Pl[l][e];
     }
   }
@@ -588,12 +588,13 @@ int build_device_tables() {
   // split-BF16 images for the tensor-core networks
   std::vector<unsigned char> tc_img = make_tc_image(pd, scale);
   // Legendre tables of the moment form (Chebyshev species)
-  std::vector<float> qleg((size_t)g.ntypes * AE_MOMA * AE_MOMA, 0.f);
+  std::vector<double> qleg64((size_t)g.ntypes * AE_MOMA * AE_MOMA, 0.0);
   for (int t = 0; t < g.ntypes; ++t)
     if (pd.sp[t].sftype == AE_SF_CHEBYSHEV) {
-      std::vector<float> qt = legendre_table(pd.sp[t].cheb.a_N, pd.sp[t].cheb.angular_legacy);
-      std::copy(qt.begin(), qt.end(), qleg.begin() + (size_t)t * AE_MOMA * AE_MOMA);
+      std::vector<double> qt = legendre_table(pd.sp[t].cheb.a_N, pd.sp[t].cheb.angular_legacy);
+      std::copy(qt.begin(), qt.end(), qleg64.begin() + (size_t)t * AE_MOMA * AE_MOMA);
     }
+  std::vector<float> qleg(qleg64.begin(), qleg64.end());
   g.scale_host = scale;
   // Behler tables
   std::vector<std::vector<unsigned char>> bt;
@@ -620,6 +621,8 @@ int build_device_tables() {
   blob_bytes = align(blob_bytes + tc_img.size());
   size_t off_q = blob_bytes;
   blob_bytes = align(blob_bytes + qleg.size() * 4);
+  size_t off_q64 = blob_bytes;
+  blob_bytes = align(blob_bytes + qleg64.size() * 8);
   size_t off_beh = blob_bytes;
   std::vector<size_t> beh_off;
   for (auto& b : bt) {
@@ -639,6 +642,7 @@ int build_device_tables() {
     cudaMemcpy(base + off_beh + beh_off[q], bt[q].data(), bt[q].size(), cudaMemcpyHostToDevice);
   if (!tc_img.empty()) cudaMemcpy(base + off_tc, tc_img.data(), tc_img.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(base + off_q, qleg.data(), qleg.size() * 4, cudaMemcpyHostToDevice);
+  cudaMemcpy(base + off_q64, qleg64.data(), qleg64.size() * 8, cudaMemcpyHostToDevice);
   if (cudaDeviceSynchronize() != cudaSuccess) return AENET_ERR_CUDA;
   pd.shift = (const double*)(base + off_shift);
   pd.scale = (const double*)(base + off_scale);
@@ -649,6 +653,7 @@ int build_device_tables() {
   pd.behler_blob = (const unsigned char*)(base + off_beh);
   pd.tc_img = tc_img.empty() ? nullptr : (const unsigned char*)(base + off_tc);
   pd.qleg = (const float*)(base + off_q);
+  pd.qleg64 = (const double*)(base + off_q64);
   for (size_t q = 0; q < bt.size(); ++q) pd.sp[q].behler_off = (int)beh_off[q];
   g.pd = pd;
   g.blob = std::move(blob);
@@ -945,6 +950,7 @@ struct aenet_gpu_plan {
   void* nb_vec = nullptr;
   int* nb_img = nullptr;
   float* M = nullptr;         // angular moments of the FP32 moment form
+  double* M64 = nullptr;      // the same of the FP64 kernels
   int mom_pad = 0;
   int* nb_rank = nullptr;     // stale-spin order of the table slots (option angular_spin)
   float* nb_seff = nullptr;
@@ -1223,14 +1229,14 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   size_t o_jt = take(4 * npairs);
   size_t o_vec = take((P->fp64 ? 32 : 16) * npairs);
   size_t o_img = P->keep_images ? take(4 * npairs) : 0;
-  // moment buffer of the FP32 path: both blocks' moments per atom
+  // moment buffer: both blocks' moments per atom
   P->mom_pad = 0;
-  if (!P->fp64 && P->pd && P->pd->qleg) {
+  if (P->pd && P->pd->qleg) {
     int aN = 0;
     for (int t = 0; t < P->pd->ntypes; ++t) aN = std::max(aN, P->pd->sp[t].cheb.a_N);
-    if (aN <= AE_MOMA) P->mom_pad = (2 * aN * aN + 3) & ~3;
+    if (aN <= (P->fp64 ? AE_MOMA64 : AE_MOMA)) P->mom_pad = (2 * aN * aN + 3) & ~3;
   }
-  size_t o_M = P->mom_pad ? take(4 * (size_t)P->mom_pad * N) : 0;
+  size_t o_M = P->mom_pad ? take(tsz * (size_t)P->mom_pad * N) : 0;
   const bool stale = stale_spin_wanted();
   size_t o_rk = stale ? take(4 * npairs) : 0;
   size_t o_se = stale ? take(4 * npairs) : 0;
@@ -1283,7 +1289,8 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   P->nb_jt = (int*)(b + o_jt);
   P->nb_vec = (void*)(b + o_vec);
   P->nb_img = P->keep_images ? (int*)(b + o_img) : nullptr;
-  P->M = P->mom_pad ? (float*)(b + o_M) : nullptr;
+  P->M = P->mom_pad && !P->fp64 ? (float*)(b + o_M) : nullptr;
+  P->M64 = P->mom_pad && P->fp64 ? (double*)(b + o_M) : nullptr;
   P->nb_rank = stale ? (int*)(b + o_rk) : nullptr;
   P->nb_seff = stale ? (float*)(b + o_se) : nullptr;
   P->G = (void*)(b + o_G);
@@ -1375,14 +1382,16 @@ DescBuffers desc_buffers(aenet_gpu_plan* P, const double* grad_scale, bool viria
   d.atom_struct = P->atom_struct;
   d.grad_scale = grad_scale;
   d.status = P->status;
-  if (g.angular_moments && P->M) {
+  if (g.angular_moments) {
     d.M = P->M;
+    d.M64 = P->M64;
     d.mom_pad = P->mom_pad;
   }
   if (P->nb_rank) {
     d.nb_rank = P->nb_rank;
     d.nb_seff = P->nb_seff;
     d.M = nullptr;    // ordered spin weights need the pair form
+    d.M64 = nullptr;
   }
   return d;
 }

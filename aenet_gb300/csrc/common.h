@@ -28,6 +28,7 @@
 #define AE_MAXG4 64          // Behler angular functions per triple type
 #define AE_MAXG2 64          // Behler radial functions per pair type
 #define AE_MOMA 7            // angular functions (order + 1) of the moment form
+#define AE_MOMA64 5          // the same of the FP64 kernels (registers)
 // static shared memory a kernel may add to its dynamic allocation; the
 // launchers opt in to large dynamic shared memory once the sum passes 48 KB
 #define AE_STATIC_SMEM 1024
@@ -151,6 +152,7 @@ struct PotDevice {
   // expansion T_n(x(c)) = sum_l q[n][l] P_l(c) of the angular basis in
   // c = cos(theta), [ntypes][AE_MOMA][AE_MOMA]; null when unavailable
   const float* qleg;
+  const double* qleg64;               // the same in FP64
 };
 
 // Per-species image for the tensor-core networks.  Operand tiles are
@@ -290,6 +292,7 @@ struct DescBuffers {
   const void* U;               // [N] T4 per-atom directions of the tangent pass
   void* V;                     // [N][nsf_pad] (T) normalised descriptor tangents
   float* M;                    // [N][mom_pad] angular moments (FP32 moment form) or null
+  double* M64;                 // the same of the FP64 kernels, or null
   int mom_pad;
   // angular spin weights as sfb_eval forms them (sfbasis.f90:514, 556):
   // the pair (j, k) of a row, j first in the reference's neighbour order,

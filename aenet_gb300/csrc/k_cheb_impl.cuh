@@ -1,4 +1,6 @@
-// Chebyshev descriptor (replaces sfb_eval / sfb_radial / sfb_angular of
+// FP32 kernels of the Chebyshev descriptor (the FP64 ones: k_cheb64.cuh;
+// helpers of both precisions serve the tangent and Jacobian kernels)
+// (replaces sfb_eval / sfb_radial / sfb_angular of
 // src/ext/sfbasis.f90:440-571, 762-858 and chebyshev.f90:41-128) and its
 // adjoint (the force chain rule of src/aenet.f90:471-477, without ever
 // materialising the descriptor Jacobian).

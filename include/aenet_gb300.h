@@ -44,8 +44,9 @@ extern "C" {
  *   "z_refine" = "1" .. "4"   the search cells are that many times narrower
  *       along the third lattice axis: the same stencil rows, each cut more
  *       finely to the cut-off sphere (performance only).
- *   "lanes_per_atom" = "8" | "16" | "32"   descriptor kernels' lanes per
- *       atom (performance only).
+ *   "lanes_per_atom" = "8" | "16" | "32"   the mixed path's descriptor
+ *       kernels' lanes per atom (performance only; the FP64 kernels choose by
+ *       the number of atoms).
  *   "adjoint_lanes_per_atom" = "0" | "8" | "16" | "32"   the same for the
  *       adjoint kernels; 0 follows lanes_per_atom (performance only).
  *   "neighbour_kernel" = "atom" | "cell" | "stream" | "half" | "struct" |
@@ -67,11 +68,11 @@ extern "C" {
  *   "networks" = "tensor" | "simt"   mixed-path networks on the tcgen05
  *       tensor cores (split BF16, FP32 accumulation; networks with two
  *       hidden layers and widths up to 64) or on FP32 SIMT.
- *   "angular_terms" = "moments" | "pairs"   mixed-path angular Chebyshev
- *       terms from per-atom moments of real spherical harmonics (the pair
- *       sum rewritten by the addition theorem; cost linear in the angular
- *       neighbours, angular orders up to 6) or from the pair sum itself.
- *       Same values up to FP32 rounding; the FP64 path always sums pairs.
+ *   "angular_terms" = "moments" | "pairs"   angular Chebyshev terms from
+ *       per-atom moments of real spherical harmonics (the pair sum rewritten
+ *       by the addition theorem; cost linear in the angular neighbours;
+ *       angular orders up to 6 on the mixed path, up to 4 in FP64) or from
+ *       the pair sum itself.  Same values up to rounding.
  *   "angular_spin" = "own" | "stale"   spin weights of the Chebyshev
  *       angular pairs (species-weighted bases).  own: s_j s_k.  stale: as
  *       sfb_eval forms them (src/ext/sfbasis.f90:514, 556), where s_j is
