@@ -373,6 +373,50 @@ __device__ __noinline__ bool band_fp64(const NbBuffers& nb, const StructGeom* g,
   return e2 <= rc2;
 }
 
+// sqrt of an FP64 squared length: one Newton step of the reciprocal square
+// root from an FP32 seed (relative error 2^-23, then 2^-45) and one correction
+// of the root by its exact residual, which leaves the rounding of the last
+// operation; eight FP64 instructions.  Lengths too small for the seed take the
+// library's root.
+__device__ __forceinline__ double root(double x) {
+  if (!(x > 1e-30)) return sqrt(x);
+  const float f = rsqrtf((float)x);
+  const double y = (double)f, h = (double)(0.5f * f);
+  const double g = x * y;
+  const double e = fma(-g, y, 1.0);              // 1 - x y^2
+  const double r = fma(0.5 * g, e, g);           // sqrt(x) to 2^-45
+  return fma(fma(-r, r, x), h, r);
+}
+
+// R_ij = L (s_j + T) - L s_i in FP64 and its length (the vectors the
+// reference's descriptor sees), the reference's unfused operations.  At T = 0
+// L s_j is the wrapped position itself, and in an orthogonal cell the terms
+// that are zero change no bit of the sums.
+__device__ __forceinline__ double4_32a pair_vector64(const StructGeom* g, const NbBuffers& nb,
+                                                     int pbc, int i, int j, int T0, int T1,
+                                                     int T2) {
+  const double *ri = nb.r_wrap + 3 * (size_t)i, *rj = nb.r_wrap + 3 * (size_t)j;
+  double R[3] = {rj[0], rj[1], rj[2]};
+  if (pbc && (T0 | T1 | T2)) {
+    const double* sj = nb.s_wrap + 3 * (size_t)j;
+    const double u0 = da(sj[0], (double)T0), u1 = da(sj[1], (double)T1), u2 = da(sj[2], (double)T2);
+    if (g->ortho) {
+      R[0] = dm(g->L[0], u0);
+      R[1] = dm(g->L[4], u1);
+      R[2] = dm(g->L[8], u2);
+    } else {
+      for (int c = 0; c < 3; ++c) {
+        double t = dm(g->L[c], u0);
+        t = da(t, dm(g->L[3 + c], u1));
+        R[c] = da(t, dm(g->L[6 + c], u2));
+      }
+    }
+  }
+  for (int c = 0; c < 3; ++c) R[c] = da(R[c], -ri[c]);
+  const double dist = root(da(da(dm(R[0], R[0]), dm(R[1], R[1])), dm(R[2], R[2])));
+  return make_double4_32a(R[0], R[1], R[2], dist);
+}
+
 // stencil units per lane in one round of the search (a round holds
 // 32 NB_UPL units; the stencils of the batch workloads need at most 125)
 constexpr int NB_UPL = 1;
@@ -576,27 +620,8 @@ __device__ __forceinline__ void search_atom(int i, const NbBuffers& nb, const St
           nb.nb_jt[row + k] = j | (tj << AE_TYPE_SHIFT);
           if (nb.nb_img) nb.nb_img[row + k] = img;
           if (VecOut<T4>::fp64) {
-            // R_ij = L (s_j + T) - L s_i in FP64 (the vectors the reference's
-            // descriptor sees)
-            const int oT0 = sext10i(img & 1023), oT1 = sext10i((img >> 10) & 1023),
-                      oT2 = sext10i((img >> 20) & 1023);
-            double R[3];
-            if (pbc) {
-              const double* sj = nb.s_wrap + 3 * j;
-              double u0 = da(sj[0], (double)oT0), u1 = da(sj[1], (double)oT1),
-                     u2 = da(sj[2], (double)oT2);
-              for (int c = 0; c < 3; ++c) {
-                double t = dm(g->L[c], u0);
-                t = da(t, dm(g->L[3 + c], u1));
-                t = da(t, dm(g->L[6 + c], u2));
-                R[c] = da(t, -nb.r_wrap[3 * i + c]);
-              }
-            } else {
-              for (int c = 0; c < 3; ++c) R[c] = da(nb.r_wrap[3 * j + c], -nb.r_wrap[3 * i + c]);
-            }
-            double dist = sqrt(da(da(dm(R[0], R[0]), dm(R[1], R[1])), dm(R[2], R[2])));
-            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] =
-                make_double4_32a(R[0], R[1], R[2], dist);
+            // the vector follows below, for whole warps of accepted pairs
+            *reinterpret_cast<int*>(reinterpret_cast<double4_32a*>(nb.nb_vec) + row + k) = img;
           } else {
             reinterpret_cast<float4*>(nb.nb_vec)[row + k] =
                 make_float4(dx, dy, dz, pair_length(dd2));
@@ -604,6 +629,19 @@ __device__ __forceinline__ void search_atom(int i, const NbBuffers& nb, const St
         }
       }
       cnt += __popc(mask);
+    }
+  }
+  if (VecOut<T4>::fp64) {
+    // the FP64 vectors of the finished row: the FP64 pipe bounds this kernel,
+    // and 32 accepted pairs at a time use all of its lanes (a batch of
+    // candidates leaves most idle).  512 Li/Si/O cells: 1082 -> 354 us, with
+    // pair_vector64's shortcuts; 2,765 Au/Cu atoms 65 -> 27 us.
+    __syncwarp();
+    for (int k = lane; k < min(cnt, cap); k += 32) {
+      double4_32a* v = reinterpret_cast<double4_32a*>(nb.nb_vec) + row + k;
+      const int img = *reinterpret_cast<const volatile int*>(v);
+      *v = pair_vector64(g, nb, pbc, i, nb.nb_jt[row + k] & AE_INDEX_MASK, sext10i(img & 1023),
+                         sext10i((img >> 10) & 1023), sext10i((img >> 20) & 1023));
     }
   }
   if (lane == 0) {
@@ -894,24 +932,8 @@ __global__ void __launch_bounds__(256) k_neighbors_cell(int ncells, NbBuffers nb
               nb.nb_jt[row + cnt] = j | (__float_as_int(rj.w) << AE_TYPE_SHIFT);
               if (nb.nb_img) nb.nb_img[row + cnt] = img;
               if (VecOut<T4>::fp64) {
-                double R[3];
-                if (pbc) {
-                  const double* sj = nb.s_wrap + 3 * j;
-                  const double u0 = da(sj[0], (double)t0), u1 = da(sj[1], (double)t1),
-                               u2 = da(sj[2], (double)t2);
-                  for (int cc = 0; cc < 3; ++cc) {
-                    double t = dm(g->L[cc], u0);
-                    t = da(t, dm(g->L[3 + cc], u1));
-                    t = da(t, dm(g->L[6 + cc], u2));
-                    R[cc] = da(t, -nb.r_wrap[3 * ih + cc]);
-                  }
-                } else {
-                  for (int cc = 0; cc < 3; ++cc)
-                    R[cc] = da(nb.r_wrap[3 * j + cc], -nb.r_wrap[3 * ih + cc]);
-                }
-                const double dist = sqrt(da(da(dm(R[0], R[0]), dm(R[1], R[1])), dm(R[2], R[2])));
                 reinterpret_cast<double4_32a*>(nb.nb_vec)[row + cnt] =
-                    make_double4_32a(R[0], R[1], R[2], dist);
+                    pair_vector64(g, nb, pbc, ih, j, t0, t1, t2);
               } else {
                 reinterpret_cast<float4*>(nb.nb_vec)[row + cnt] =
                     make_float4(dx, dy, dz, sqrtf(dd2));
@@ -973,28 +995,6 @@ __device__ __forceinline__ bool band_accept(const StructGeom* g, const NbBuffers
     e2 = da(da(dm(c0d, c0d), dm(c1d, c1d)), dm(c2d, c2d));
   }
   return e2 <= rc2;
-}
-
-// R_ij = L (s_j + T) - L s_i in FP64 and its length
-__device__ __forceinline__ double4_32a fp64_pair_vector(const StructGeom* g, const NbBuffers& nb,
-                                                        int pbc, int ih, int j, int t0, int t1,
-                                                        int t2) {
-  double R[3];
-  if (pbc) {
-    const double* sj = nb.s_wrap + 3 * j;
-    const double u0 = da(sj[0], (double)t0), u1 = da(sj[1], (double)t1),
-                 u2 = da(sj[2], (double)t2);
-    for (int cc = 0; cc < 3; ++cc) {
-      double t = dm(g->L[cc], u0);
-      t = da(t, dm(g->L[3 + cc], u1));
-      t = da(t, dm(g->L[6 + cc], u2));
-      R[cc] = da(t, -nb.r_wrap[3 * ih + cc]);
-    }
-  } else {
-    for (int cc = 0; cc < 3; ++cc) R[cc] = da(nb.r_wrap[3 * j + cc], -nb.r_wrap[3 * ih + cc]);
-  }
-  const double dist = sqrt(da(da(dm(R[0], R[0]), dm(R[1], R[1])), dm(R[2], R[2])));
-  return make_double4_32a(R[0], R[1], R[2], dist);
 }
 
 template <typename T4>
@@ -1155,7 +1155,7 @@ __global__ void __launch_bounds__(32 * NBS_WARPS) k_neighbors_stream(int ncells,
             nb.nb_jt[row + k] = jt;
             if (nb.nb_img) nb.nb_img[row + k] = img;
             if (VecOut<T4>::fp64) {
-              reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = fp64_pair_vector(
+              reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = pair_vector64(
                   g, nb, pbc, ih, cj, sext10i(img & 1023), sext10i((img >> 10) & 1023),
                   sext10i((img >> 20) & 1023));
             } else {
@@ -1354,7 +1354,7 @@ __global__ void __launch_bounds__(256, 4) k_neighbors_half(int natoms, NbBuffers
           nb.nb_jt[row + k] = j | (tj << AE_TYPE_SHIFT);
           if (nb.nb_img) nb.nb_img[row + k] = img;
           if (VecOut<T4>::fp64) {
-            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = fp64_pair_vector(
+            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = pair_vector64(
                 g, nb, pbc, i, j, sext10i(img & 1023), sext10i((img >> 10) & 1023),
                 sext10i((img >> 20) & 1023));
           } else {
@@ -1371,7 +1371,7 @@ __global__ void __launch_bounds__(256, 4) k_neighbors_half(int natoms, NbBuffers
           nb.nb_jt[row + k] = iti;
           if (nb.nb_img) nb.nb_img[row + k] = nimg;
           if (VecOut<T4>::fp64) {
-            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = fp64_pair_vector(
+            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = pair_vector64(
                 g, nb, pbc, j, i, -sext10i(img & 1023), -sext10i((img >> 10) & 1023),
                 -sext10i((img >> 20) & 1023));
           } else {
@@ -1552,7 +1552,7 @@ __device__ __forceinline__ void search_atom_half(int i, int a0, const NbBuffers&
           nb.nb_jt[row + k] = j | (tj << AE_TYPE_SHIFT);
           if (nb.nb_img) nb.nb_img[row + k] = img;
           if (VecOut<T4>::fp64) {
-            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = fp64_pair_vector(
+            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = pair_vector64(
                 g, nb, pbc, i, j, sext10i(img & 1023), sext10i((img >> 10) & 1023),
                 sext10i((img >> 20) & 1023));
           } else {
@@ -1569,7 +1569,7 @@ __device__ __forceinline__ void search_atom_half(int i, int a0, const NbBuffers&
           nb.nb_jt[row + k] = iti;
           if (nb.nb_img) nb.nb_img[row + k] = nimg;
           if (VecOut<T4>::fp64) {
-            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = fp64_pair_vector(
+            reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] = pair_vector64(
                 g, nb, pbc, j, i, -sext10i(img & 1023), -sext10i((img >> 10) & 1023),
                 -sext10i((img >> 20) & 1023));
           } else {
