@@ -1,6 +1,6 @@
-// FP32 instantiations of the Chebyshev descriptor and adjoint kernels with
-// the angular terms as pair sums (mixed-precision path) and the launch entry
-// points of both precisions.
+// FP32 instantiations of the Chebyshev descriptor and adjoint kernels (the
+// mixed-precision path; the adjoint in moment form is k_cheb_mom.cu's) and the
+// launch entry points of both precisions.
 #include "k_cheb_impl.cuh"
 #include "k_cheb_rows.cuh"
 
@@ -8,13 +8,9 @@ int ae_cheb_f64(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStr
 
 namespace {
 int cheb_f32(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
-  // the moment form where it is instantiated and asked for, pair sums
-  // otherwise
-  if (b.M && pd.qleg && !b.nb_rank) {
-    const int e = cheb::dispatch_moments(pd, b, adjoint, s);
-    if (e != cheb::AE_MOM_NA) return e;
-  }
-  return chebr::dispatch_rows<float>(pd, b, adjoint, true, s);
+  // the adjoint in moment form where the forward left moments
+  if (adjoint && chebr::moment_form<float>(pd, b)) return cheb::dispatch_adjoint_mom(pd, b, s);
+  return chebr::dispatch_rows<float>(pd, b, adjoint, s);
 }
 }  // namespace
 

@@ -3,5 +3,5 @@
 #include "k_cheb_rows.cuh"
 
 int ae_cheb_f64(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
-  return chebr::dispatch_rows<double>(pd, b, adjoint, true, s);
+  return chebr::dispatch_rows<double>(pd, b, adjoint, s);
 }

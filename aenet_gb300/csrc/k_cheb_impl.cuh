@@ -1,36 +1,15 @@
-// FP32 kernels of the Chebyshev descriptor (the FP64 ones: k_cheb64.cuh;
-// helpers of both precisions serve the tangent and Jacobian kernels)
-// (replaces sfb_eval / sfb_radial / sfb_angular of
-// src/ext/sfbasis.f90:440-571, 762-858 and chebyshev.f90:41-128) and its
-// adjoint (the force chain rule of src/aenet.f90:471-477, without ever
-// materialising the descriptor Jacobian).
-//
-// One group of LPA lanes (8, 16 or 32) per central atom.  Radial terms:
-// lanes over neighbours, each lane runs the T_n recurrence for its
-// neighbour and accumulates all orders in registers; a group reduction
-// follows.  In the same pass the neighbours inside the angular cut-off are
-// compacted into shared memory (unit vector, distance, cut-off value and
-// slope, spin, table slot).  Angular terms: the pairs j < k of those are
-// spread over the group's lanes in row-major order of the upper triangle.
+// Chebyshev descriptor: the FP32 adjoint with the angular terms in moment form
+// (k_cheb_mom.cuh), and helpers of both precisions for the tangent and
+// Jacobian kernels.  k_cheb_rows.cuh has the forward of both precisions, the
+// FP64 adjoint and the pair sums.  The descriptor replaces sfb_eval /
+// sfb_radial / sfb_angular of src/ext/sfbasis.f90:440-571, 762-858 and
+// chebyshev.f90:41-128, the adjoint is the force chain rule of
+// src/aenet.f90:471-477 without ever materialising the descriptor Jacobian.
 //
 // Feature layout per atom (sfbasis.f90:114-131):
 //   [radial R][angular A][radial x spin R][angular x spin A]
 // The spin block exists when the setup has more than one species;
-// typespin follows sfbasis.f90:142-147.  R and A are compile-time in the
-// exact instantiations (no predicated padding); GUARD instantiations take
-// them at run time up to their template bounds.
-//
-// The adjoint contracts dE/dG (already multiplied by E_scale and the
-// normalisation scale) with the analytic derivatives:
-//   radial:  dE/dd_ij = sum_n g_n (fc' T_n + fc T_n')       along R_ij/d_ij
-//   angular: E_jk = w A(cos), w = fc_j fc_k, A = sum_n g_n T_n
-//            grad_j E_jk = fc_j' fc_k A Rhat_j + w A' (Rhat_k - cos Rhat_j)/d_j
-// In the adjoint every angular pair is evaluated once, on a circulant
-// schedule (the owner of staged neighbour a takes partners a + t mod na,
-// t = 1 .. na/2): the lanes of a group always touch distinct partners, so
-// partner forces accumulate in shared memory without atomics and the
-// owner's in registers; each neighbour's force is scattered to global
-// memory once; the central atom receives minus the sum.
+// typespin follows sfbasis.f90:142-147.
 #pragma once
 #include "common.h"
 #include "k_cheb_mom.cuh"
@@ -121,54 +100,6 @@ __device__ __forceinline__ float normalise(float g, const PotDevice& pd, size_t 
   return ((g - sh.x) - sh.y) * pd.scale32[k];
 }
 
-template <typename T>
-struct GroupSmem {
-  typename Vec4<T>::type* au;   // angular neighbours: unit vector, distance
-  typename Vec4<T>::type* af;   // fc, fc', spin, table slot
-  T* fbuf;                      // [cap_a][3] forces on angular neighbours
-  T* g;                         // [nsf_pad] dE/dG
-};
-
-// the staging area of the forward doubles as the moment reduction scratch
-// (`scratch` bytes at least)
-template <typename T>
-__host__ __device__ inline size_t group_smem_bytes(int cap_a, int nsf_pad, bool adjoint,
-                                                   size_t scratch = 0) {
-  using T4 = typename Vec4<T>::type;
-  size_t stage = 2 * sizeof(T4) * cap_a;
-  if (stage < scratch) stage = scratch;
-  size_t per = stage + (adjoint ? (3 * sizeof(T) * cap_a + sizeof(T) * nsf_pad) : 0);
-  return (per + 31) & ~size_t(31);
-}
-
-template <typename T>
-__device__ __forceinline__ GroupSmem<T> group_smem(unsigned char* base, int cap_a, int nsf_pad,
-                                                   int group, bool adjoint, size_t scratch = 0) {
-  using T4 = typename Vec4<T>::type;
-  unsigned char* p = base + group_smem_bytes<T>(cap_a, nsf_pad, adjoint, scratch) * group;
-  GroupSmem<T> w;
-  w.au = reinterpret_cast<T4*>(p);
-  w.af = w.au + cap_a;
-  w.fbuf = reinterpret_cast<T*>(w.af + cap_a);
-  w.g = w.fbuf + 3 * cap_a;
-  return w;
-}
-
-// moment form: values per lane in the reduction (both blocks' moments, then
-// the two weight sums), padded to whole float4
-template <int A>
-__host__ __device__ constexpr int mom_nv() {
-  return 2 * A * A + 2;
-}
-template <int A>
-__host__ __device__ constexpr int mom_nvp() {
-  return (mom_nv<A>() + 3) & ~3;
-}
-template <int A, int LPA>
-__host__ __device__ constexpr size_t mom_scratch_bytes() {
-  return sizeof(float) * (size_t)(LPA + 1) * mom_nvp<A>();
-}
-
 // row-major walk of the upper triangle a < b < na with a fixed stride
 struct PairWalk {
   int a, b;
@@ -207,356 +138,28 @@ __device__ __forceinline__ void prefetch_rows(const T4* vec, const int* jt, int 
                : "memory");
 }
 
-template <typename T>
-__device__ __forceinline__ void atomic_add3(T* F, int atom, T fx, T fy, T fz);
-template <>
-__device__ __forceinline__ void atomic_add3<float>(float* F, int atom, float fx, float fy, float fz) {
-  atomicAdd(reinterpret_cast<float4*>(F) + atom, make_float4(fx, fy, fz, 0.f));
-}
-template <>
-__device__ __forceinline__ void atomic_add3<double>(double* F, int atom, double fx, double fy,
-                                                    double fz) {
-  atomicAdd(F + 4 * atom, fx);
-  atomicAdd(F + 4 * atom + 1, fy);
-  atomicAdd(F + 4 * atom + 2, fz);
-}
-
-// Angular block of the forward in moment form (FP32): the group's lanes
-// accumulate moments over the staged neighbours, the partial sums are
-// reduced through the (then free) staging area, the moments are stored for
-// the adjoint and each output lane assembles its G_n from the power spectra.
-template <int A, int LPA>
-__device__ __forceinline__ void forward_moments(const PotDevice& pd, const DescBuffers& b,
-                                                const GroupSmem<float>& sm, const ChebTable& ct,
-                                                int na, int sl, unsigned gmask, bool active, int i,
-                                                int ti, bool multi, float* G, size_t nrow) {
-  constexpr int L = A - 1;
-  constexpr int K = A * A;
-  constexpr int NV = mom_nv<A>(), NVP = mom_nvp<A>();
-  float M0[K], M1[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    M0[k] = 0.f;
-    M1[k] = 0.f;
-  }
-  float W0 = 0.f, W1 = 0.f;
-  for (int a = sl; a < na; a += LPA) {
-    const float4 u = sm.au[a], f = sm.af[a];
-    const float w1 = f.x * f.z;   // fc x spin (zero for a single species)
-    mom_accumulate<L, true>(u.x, u.y, u.z, f.x, w1, M0, M1);
-    W0 = fmaf(f.x, f.x, W0);
-    W1 = fmaf(w1, w1, W1);
-  }
-  __syncwarp(gmask);   // the staged neighbours are consumed: reuse the area
-  float* scr = reinterpret_cast<float*>(sm.au);
-  float4* dst = reinterpret_cast<float4*>(scr + sl * NVP);
-#pragma unroll
-  for (int c4 = 0; c4 < NVP / 4; ++c4) {
-    float v[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int c = 4 * c4 + e;
-      v[e] = c < K ? M0[c] : (c < 2 * K ? M1[c - K] : (c == 2 * K ? W0 : (c == 2 * K + 1 ? W1 : 0.f)));
-    }
-    dst[c4] = make_float4(v[0], v[1], v[2], v[3]);
-  }
-  __syncwarp(gmask);
-  float* sq = scr + LPA * NVP;
-  float* Mg = b.M + (size_t)i * b.mom_pad;
-  for (int c = sl; c < NV; c += LPA) {
-    float t = 0.f;
-#pragma unroll
-    for (int r = 0; r < LPA; ++r) t += scr[r * NVP + c];
-    if (c < 2 * K) {
-      if (active) Mg[c] = t;
-      sq[c] = t * t;
-    } else {
-      sq[c] = t;
-    }
-  }
-  __syncwarp(gmask);
-  if (!active || sl >= A) return;
-  float p0[A], p1[A];
-#pragma unroll
-  for (int l = 0; l < A; ++l) {
-    float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-    for (int k = l * l; k < (l + 1) * (l + 1); ++k) {
-      s0 += sq[k];
-      s1 += sq[K + k];
-    }
-    p0[l] = s0;
-    p1[l] = s1;
-  }
-  W0 = sq[2 * K];
-  W1 = sq[2 * K + 1];
-  const float* q = pd.qleg + (size_t)ti * AE_MOMA * AE_MOMA;
-#pragma unroll
-  for (int n = 0; n < A; ++n) {
-    if (n % LPA == sl) {
-      float g0 = 0.f, g1 = 0.f, t1 = 0.f;
-#pragma unroll
-      for (int l = 0; l <= n; ++l) {
-        const float ql = q[n * AE_MOMA + l];
-        g0 = fmaf(ql, p0[l], g0);
-        g1 = fmaf(ql, p1[l], g1);
-        t1 += ql;
-      }
-      G[ct.a_i1 + n] = normalise(0.5f * (g0 - t1 * W0), pd, nrow + ct.a_i1 + n);
-      if (multi) G[ct.a_i2 + n] = normalise(0.5f * (g1 - t1 * W1), pd, nrow + ct.a_i2 + n);
-    }
-  }
-}
-
-// Spin weight of the staged angular pair (a, k) with the reference's
-// stale s_j (sfbasis.f90:514, 556): the member first in the reference's
-// neighbour order contributes s_eff, the other its own spin.  f.z is the
-// neighbour's own spin, f.w its slot in the atom's table row.
-template <typename T>
-__device__ __forceinline__ T ordered_spin(const DescBuffers& b, int i,
-                                          const typename Vec4<T>::type& fa,
-                                          const typename Vec4<T>::type& fk) {
-  const size_t rb = (size_t)i * b.cap;
-  const int sa = (int)fa.w, sk = (int)fk.w;
-  return b.nb_rank[rb + sa] < b.nb_rank[rb + sk] ? T(b.nb_seff[rb + sa]) * fk.z
-                                                 : T(b.nb_seff[rb + sk]) * fa.z;
-}
-
-// ----------------------------------------------------------------------
-// forward
-// ----------------------------------------------------------------------
-// resident blocks per SM asked of the register allocator (moment form)
-#ifndef AE_MOM_FWD_BLOCKS
-#define AE_MOM_FWD_BLOCKS 6
-#endif
+// Adjoint, one group of LPA lanes (8, 16 or 32) per central atom: contracts
+// dE/dG (already multiplied by E_scale and the normalisation scale) with
+//   radial:  dE/dd_ij = sum_n g_n (fc' T_n + fc T_n')       along R_ij/d_ij
+//   angular: k_cheb_mom.cuh
+// Bound by instruction issue and by the latency of the table rows.  The
+// angular neighbours are compacted in the radial pass and prepared (unit
+// vector, fc, fc') densely in the angular one, where each scatters its whole
+// force once; the moments' coefficients stay in registers.  4,096 Li/Si/O
+// cells (597,000 atoms): 576 us with both done in the radial pass, 528 us now
+// (580 and 549 us at four and six resident blocks).
 #ifndef AE_MOM_ADJ_BLOCKS
 #define AE_MOM_ADJ_BLOCKS 5
 #endif
-#ifndef AE_PAIR_ADJ_BLOCKS
-#define AE_PAIR_ADJ_BLOCKS 5
-#endif
-
-template <typename T, int R, int A, int LPA, bool GUARD, bool MOM>
-__global__ void __launch_bounds__(128, MOM ? (A <= 5 ? AE_MOM_FWD_BLOCKS : 3) : 1)
-    k_forward(PotDevice pd, DescBuffers b) {
-  using T4 = typename Vec4<T>::type;
-  constexpr int GPW = 32 / LPA;
-  extern __shared__ __align__(32) unsigned char smem_raw[];
-  // typespin of (central species, neighbour species): a shared table, as
-  // the per-neighbour lookups in the parameter bank would serialise
-  __shared__ float s_spin[AE_MAXT * AE_MAXT];
-  for (int q = threadIdx.x; q < pd.ntypes * AE_MAXT; q += blockDim.x)
-    s_spin[q] = pd.sp[q / AE_MAXT].cheb.spin[q % AE_MAXT];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int grp = lane / LPA, sl = lane % LPA;
-  const int wglobal = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (wglobal * GPW >= b.natoms) return;   // whole warp idle
-  const int gid = wglobal * GPW + grp;
-  const bool active = gid < b.natoms;
-  const int i = active ? gid : b.natoms - 1;
-  GroupSmem<T> sm = group_smem<T>(smem_raw, b.cap_a, pd.nsf_pad, warp * GPW + grp, false,
-                                  MOM ? mom_scratch_bytes<A, LPA>() : 0);
-  const int ti = b.types[i];
-  const ChebTable& ct = pd.sp[ti].cheb;
-  const int n = active ? b.nb_cnt[i] : 0;
-  const T4* __restrict__ vec = reinterpret_cast<const T4*>(b.nb_vec) + (size_t)i * b.cap;
-  const int* __restrict__ jt = b.nb_jt + (size_t)i * b.cap;
-  if (sl == 0) prefetch_rows(vec, jt, n);
-  if (b.zero_F && active && sl == 0) {
-    T4 z;
-    z.x = z.y = z.z = z.w = T(0);
-    reinterpret_cast<T4*>(b.F)[i] = z;
-  }
-  const int nloop = warp_max(n);
-  const T r_Rc = T(ct.r_Rc), a_Rc = T(ct.a_Rc);
-  const T two_over_rc = T(2) / r_Rc;
-  const T r_a = T(SFB_PI) / r_Rc, a_a = T(SFB_PI) / a_Rc;
-  const int rN = GUARD ? ct.r_N : R;
-  const int aN = GUARD ? ct.a_N : A;
-  const bool multi = ct.multi;
-  const unsigned gmask = (LPA == 32) ? 0xffffffffu : (((1u << LPA) - 1u) << (grp * LPA));
-
-  // ---- radial terms and angular staging
-  T acc[R], accs[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    acc[q] = T(0);
-    accs[q] = T(0);
-  }
-  int na = 0;
-  // the table row is read one iteration ahead (its load latency overlaps
-  // the previous neighbour's work)
-  T4 vn;
-  int qn = 0;
-  if (sl < n) {
-    vn = vec[sl];
-    qn = jt[sl];
-  }
-  for (int base = 0; base < nloop; base += LPA) {
-    const int j = base + sl;
-    const bool valid = j < n;
-    T4 v = vn;
-    const int t = valid ? (qn >> AE_TYPE_SHIFT) : 0;
-    if (!valid) {
-      v.x = v.y = v.z = T(0);
-      v.w = T(1e30);
-    }
-    if (j + LPA < n) {
-      vn = vec[j + LPA];
-      qn = jt[j + LPA];
-    }
-    const T d = v.w;
-    const T s = multi ? T(s_spin[ti * AE_MAXT + t]) : T(0);
-    if (d <= r_Rc && d > T(SFB_EPS)) {
-      T fc, dfc;
-      cutoff_a(d, r_Rc, r_a, fc, dfc);
-      const T x = radial_x(d, r_Rc, two_over_rc);
-      const T x2 = x + x;
-      const T sfc = s * fc;
-      T tm1 = T(1), t0 = x;
-      acc[0] += fc;
-      accs[0] += sfc;
-#pragma unroll
-      for (int q = 1; q < R; ++q) {
-        if (!GUARD || q < rN) {
-          acc[q] = fma(fc, t0, acc[q]);
-          accs[q] = fma(sfc, t0, accs[q]);
-          const T tn = fma(x2, t0, -tm1);
-          tm1 = t0;
-          t0 = tn;
-        }
-      }
-    }
-    const bool inA = d <= a_Rc && d >= T(SFB_EPS);
-    const unsigned m = __ballot_sync(0xffffffffu, inA) & gmask;
-    if (inA) {
-      const int k = na + __popc(m & ((1u << lane) - 1u));
-      if (k < b.cap_a) {
-        const T inv = div_t(T(1), d);
-        T fc, dfc;
-        cutoff_a(d, a_Rc, a_a, fc, dfc);
-        T4 u, f;
-        u.x = v.x * inv;
-        u.y = v.y * inv;
-        u.z = v.z * inv;
-        u.w = d;
-        f.x = fc;
-        f.y = dfc;
-        f.z = s;
-        f.w = T(j);
-        sm.au[k] = u;
-        sm.af[k] = f;
-      }
-    }
-    na += __popc(m);
-  }
-  if (na > b.cap_a) {
-    if (sl == 0 && active) atomicOr(b.status, AE_ST_NB_OVERFLOW);
-    na = b.cap_a;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    acc[q] = gsum<T, LPA>(acc[q]);
-    if (multi) accs[q] = gsum<T, LPA>(accs[q]);
-  }
-  const size_t nrow = (size_t)ti * pd.nsf_pad;
-  T* G = reinterpret_cast<T*>(b.G) + (size_t)i * pd.nsf_pad;
-  if (active) {
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      if (q % LPA == sl && q < rN) {
-        G[ct.r_i1 + q] = normalise(acc[q], pd, nrow + ct.r_i1 + q);
-        if (multi) G[ct.r_i2 + q] = normalise(accs[q], pd, nrow + ct.r_i2 + q);
-      }
-    }
-  }
-
-  // ---- angular terms
-  if constexpr (MOM) {
-    forward_moments<A, LPA>(pd, b, sm, ct, na, sl, gmask, active, i, ti, multi, G, nrow);
-  } else {
-    T ang[A], angs[A];
-#pragma unroll
-    for (int q = 0; q < A; ++q) {
-      ang[q] = T(0);
-      angs[q] = T(0);
-    }
-    // pairs (a, k = a + t mod na), t = 1 .. na/2, as in the adjoint: the
-    // owner of a keeps it in registers and every pair is visited once
-    const int tmax = na / 2;
-    for (int a0 = 0; a0 < na; a0 += LPA) {
-      const int a = a0 + sl;
-      const bool own = active && a < na;
-      T4 uj, fj;
-      if (own) {
-        uj = sm.au[a];
-        fj = sm.af[a];
-      } else {
-        uj.x = uj.y = uj.z = uj.w = T(0);
-        fj.x = fj.y = fj.z = fj.w = T(0);
-      }
-      for (int t = 1; t <= tmax; ++t) {
-        int k = a + t;
-        if (k >= na) k -= na;
-        if (own && !(2 * t == na && a >= tmax)) {
-          const T4 uk = sm.au[k];
-          const T4 fk = sm.af[k];
-          const T cosv = uj.x * uk.x + uj.y * uk.y + uj.z * uk.z;
-          const T w = fj.x * fk.x;
-          T sw = fj.z * fk.z * w;
-          if constexpr (GUARD) {
-            if (b.nb_rank) sw = w * ordered_spin<T>(b, i, fj, fk);
-          }
-          T x, dxdc;
-          angular_arg(cosv, ct.angular_legacy, x, dxdc);
-          const T x2 = x + x;
-          T tm1 = T(1), t0 = x;
-          ang[0] += w;
-          angs[0] += sw;
-#pragma unroll
-          for (int q = 1; q < A; ++q) {
-            if (!GUARD || q < aN) {
-              ang[q] = fma(w, t0, ang[q]);
-              angs[q] = fma(sw, t0, angs[q]);
-              const T tn = fma(x2, t0, -tm1);
-              tm1 = t0;
-              t0 = tn;
-            }
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < A; ++q) {
-      ang[q] = gsum<T, LPA>(ang[q]);
-      if (multi) angs[q] = gsum<T, LPA>(angs[q]);
-    }
-    if (active) {
-#pragma unroll
-      for (int q = 0; q < A; ++q) {
-        if (q % LPA == sl && q < aN) {
-          G[ct.a_i1 + q] = normalise(ang[q], pd, nrow + ct.a_i1 + q);
-          if (multi) G[ct.a_i2 + q] = normalise(angs[q], pd, nrow + ct.a_i2 + q);
-        }
-      }
-    }
-  }
+// shared memory of a group: staged rows (vector, distance), radial terms,
+// table slot and species, and the dE/dG row; groups 16 bytes apart in banks
+__host__ __device__ inline size_t adjoint_mom_smem(int cap_a, int nsf_pad) {
+  const size_t per = 24 * (size_t)cap_a + 4 * (size_t)nsf_pad;
+  return ((per + 111) & ~size_t(127)) + 16;
 }
-
-// ----------------------------------------------------------------------
-// adjoint
-// ----------------------------------------------------------------------
-// FP32 pair form of the exact-size instances: five blocks as well; the
-// moment form of degree 6 keeps three (its sums would spill under more)
-template <typename T, int R, int A, int LPA, bool GUARD, bool MOM>
-__global__ void __launch_bounds__(128, MOM ? (A <= 5 ? AE_MOM_ADJ_BLOCKS : 3)
-                                           : (sizeof(T) == 4 && !GUARD ? AE_PAIR_ADJ_BLOCKS : 1))
-    k_adjoint(PotDevice pd,
-                                                                             DescBuffers b) {
-  using T4 = typename Vec4<T>::type;
+template <int R, int A, int LPA>
+__global__ void __launch_bounds__(128, A <= 5 ? AE_MOM_ADJ_BLOCKS : 3)
+    k_adjoint_mom(PotDevice pd, DescBuffers b) {
   constexpr int GPW = 32 / LPA;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   // typespin of (central species, neighbour species): a shared table, as
@@ -566,133 +169,109 @@ __global__ void __launch_bounds__(128, MOM ? (A <= 5 ? AE_MOM_ADJ_BLOCKS : 3)
     s_spin[q] = pd.sp[q / AE_MAXT].cheb.spin[q % AE_MAXT];
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
   const int grp = lane / LPA, sl = lane % LPA;
-  const int wglobal = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (wglobal * GPW >= b.natoms) return;
-  const int gid = wglobal * GPW + grp;
+  const int first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * GPW;
+  if (first >= b.natoms) return;
+  const int gid = first + grp;
   const bool active = gid < b.natoms;
   const int i = active ? gid : b.natoms - 1;
-  GroupSmem<T> sm = group_smem<T>(smem_raw, b.cap_a, pd.nsf_pad, warp * GPW + grp, true);
+  unsigned char* base = smem_raw + adjoint_mom_smem(b.cap_a, pd.nsf_pad) * (threadIdx.x / LPA);
+  float4* au = reinterpret_cast<float4*>(base);
+  float* rad = reinterpret_cast<float*>(au + b.cap_a);
+  int* info = reinterpret_cast<int*>(rad + b.cap_a);
+  float* sg = reinterpret_cast<float*>(info + b.cap_a);
   const int ti = b.types[i];
   const ChebTable& ct = pd.sp[ti].cheb;
   const int n = active ? b.nb_cnt[i] : 0;
-  const T4* __restrict__ vec = reinterpret_cast<const T4*>(b.nb_vec) + (size_t)i * b.cap;
+  const float4* __restrict__ vec = reinterpret_cast<const float4*>(b.nb_vec) + (size_t)i * b.cap;
   const int* __restrict__ jt = b.nb_jt + (size_t)i * b.cap;
   if (sl == 0) prefetch_rows(vec, jt, n);
   const int nloop = warp_max(n);
-  const T r_Rc = T(ct.r_Rc), a_Rc = T(ct.a_Rc);
-  const T two_over_rc = T(2) / r_Rc;
-  const T r_a = T(SFB_PI) / r_Rc, a_a = T(SFB_PI) / a_Rc;
-  const int rN = GUARD ? ct.r_N : R;
-  const int aN = GUARD ? ct.a_N : A;
+  const float r_Rc = float(ct.r_Rc), a_Rc = float(ct.a_Rc);
+  const float two_over_rc = 2.f / r_Rc;
+  const float r_a = float(SFB_PI) / r_Rc, a_a = float(SFB_PI) / a_Rc;
   const bool multi = ct.multi;
   const unsigned gmask = (LPA == 32) ? 0xffffffffu : (((1u << LPA) - 1u) << (grp * LPA));
   const int sid = b.atom_struct[i];
-  const T gs = b.grad_scale ? T(b.grad_scale[sid]) : T(1);
+  const float gs = b.grad_scale ? float(b.grad_scale[sid]) : 1.f;
   const bool want_virial = b.virial != nullptr;
-  T* F = reinterpret_cast<T*>(b.F);
+  float* F = reinterpret_cast<float*>(b.F);
 
-  const T* gsrc = reinterpret_cast<const T*>(b.dEdG) + (size_t)i * pd.nsf_pad;
-  for (int k = sl; k < ct.nsf; k += LPA) sm.g[k] = gs * gsrc[k];
+  const float* gsrc = reinterpret_cast<const float*>(b.dEdG) + (size_t)i * pd.nsf_pad;
+  for (int k = sl; k < ct.nsf; k += LPA) sg[k] = gs * gsrc[k];
   __syncwarp();
   // radial coefficients in registers
-  T gr[R], grs[R];
+  float gr[R], grs[R];
 #pragma unroll
   for (int q = 0; q < R; ++q) {
-    gr[q] = (!GUARD || q < rN) ? sm.g[ct.r_i1 + q] : T(0);
-    grs[q] = (multi && (!GUARD || q < rN)) ? sm.g[ct.r_i2 + q] : T(0);
+    gr[q] = sg[ct.r_i1 + q];
+    grs[q] = multi ? sg[ct.r_i2 + q] : 0.f;
   }
 
-  T fix = T(0), fiy = T(0), fiz = T(0);
-  T w00 = 0, w01 = 0, w02 = 0, w10 = 0, w11 = 0, w12 = 0, w20 = 0, w21 = 0, w22 = 0;
+  float fix = 0.f, fiy = 0.f, fiz = 0.f;
+  float w00 = 0, w01 = 0, w02 = 0, w10 = 0, w11 = 0, w12 = 0, w20 = 0, w21 = 0, w22 = 0;
   int na = 0;
-  // the table row is read one iteration ahead, as in the forward
-  T4 vn;
+  // the table row is read one iteration ahead (its load latency overlaps the
+  // previous neighbour's work)
+  float4 vn = make_float4(0.f, 0.f, 0.f, 1e30f);
   int qn = 0;
   if (sl < n) {
     vn = vec[sl];
     qn = jt[sl];
   }
-  for (int base = 0; base < nloop; base += LPA) {
-    const int j = base + sl;
-    const bool valid = j < n;
-    T4 v = vn;
-    int t = 0, jatom = 0;
-    if (valid) {
-      t = qn >> AE_TYPE_SHIFT;
-      jatom = qn & AE_INDEX_MASK;
-    } else {
-      v.x = v.y = v.z = T(0);
-      v.w = T(1e30);
-    }
+  for (int base_j = 0; base_j < nloop; base_j += LPA) {
+    const int j = base_j + sl;
+    const float4 v = vn;
+    const int t = qn >> AE_TYPE_SHIFT, jatom = qn & AE_INDEX_MASK;
+    vn = make_float4(0.f, 0.f, 0.f, 1e30f);
+    qn = 0;
     if (j + LPA < n) {
       vn = vec[j + LPA];
       qn = jt[j + LPA];
     }
-    const T d = v.w;
-    const T s = multi ? T(s_spin[ti * AE_MAXT + t]) : T(0);
-    T c = T(0);
-    if (d <= r_Rc && d > T(SFB_EPS)) {
-      T fc, dfc;
+    const float d = v.w;
+    float c = 0.f;   // (dE/dd) / d
+    if (d <= r_Rc && d > float(SFB_EPS)) {
+      const float s = multi ? s_spin[ti * AE_MAXT + t] : 0.f;
+      float fc, dfc;
       cutoff_a(d, r_Rc, r_a, fc, dfc);
-      const T x = radial_x(d, r_Rc, two_over_rc);
-      const T x2 = x + x;
-      // T_q and T_q' = q U_{q-1} (chebyshev_polynomial_d1), times dx/dd
-      T tm1 = T(1), t0 = x, um1 = T(1), u0 = x2;
-      c = (gr[0] + s * grs[0]) * dfc;
+      const float x = fmaf(d, two_over_rc, -1.f), x2 = x + x;
+      // sum g_q T_q and sum g_q q U_{q-1} (chebyshev_polynomial_d1)
+      float tm1 = 1.f, t0 = x, um1 = 1.f, u0 = x2;
+      float Av = fmaf(s, grs[0], gr[0]), Bv = 0.f;
 #pragma unroll
       for (int q = 1; q < R; ++q) {
-        if (!GUARD || q < rN) {
-          const T gq = gr[q] + s * grs[q];
-          const T dT = T(q) * um1 * two_over_rc;
-          c = fma(gq, fma(dfc, t0, fc * dT), c);
-          const T tn = fma(x2, t0, -tm1);
-          tm1 = t0;
-          t0 = tn;
-          const T un = fma(x2, u0, -um1);
-          um1 = u0;
-          u0 = un;
-        }
+        const float gq = fmaf(s, grs[q], gr[q]);
+        Av = fmaf(gq, t0, Av);
+        Bv = fmaf(q == 1 ? gq : float(q) * gq, um1, Bv);
+        const float tn = fmaf(x2, t0, -tm1);
+        tm1 = t0;
+        t0 = tn;
+        const float un = fmaf(x2, u0, -um1);
+        um1 = u0;
+        u0 = un;
       }
+      c = __fdividef(fmaf(dfc, Av, fc * two_over_rc * Bv), d);
     }
-    // grad_j E = c R_ij / d; the force on j is minus that
-    const T inv = (d > T(SFB_EPS) && d < T(1e29)) ? div_t(c, d) : T(0);
-    const T gx = inv * v.x, gy = inv * v.y, gz = inv * v.z;
-    const bool inA = d <= a_Rc && d >= T(SFB_EPS);
+    const bool inA = d <= a_Rc && d >= float(SFB_EPS);
     const unsigned m = __ballot_sync(0xffffffffu, inA) & gmask;
     bool staged = false;
     if (inA) {
       const int k = na + __popc(m & ((1u << lane) - 1u));
       if (k < b.cap_a) {
-        const T invd = div_t(T(1), d);
-        T fc, dfc;
-        cutoff_a(d, a_Rc, a_a, fc, dfc);
-        T4 u, f;
-        u.x = v.x * invd;
-        u.y = v.y * invd;
-        u.z = v.z * invd;
-        u.w = invd;   // the angular loop needs 1/d only
-        f.x = fc;
-        f.y = dfc;
-        f.z = s;
-        f.w = T(j);
-        sm.au[k] = u;
-        sm.af[k] = f;
-        sm.fbuf[3 * k] = -gx;
-        sm.fbuf[3 * k + 1] = -gy;
-        sm.fbuf[3 * k + 2] = -gz;
+        au[k] = v;
+        rad[k] = c * d;
+        info[k] = (j << 3) | t;
         staged = true;
       }
     }
-    if (!staged) {
-      // staged neighbours hand their force to the central atom at the end
+    if (!staged && c != 0.f) {
+      // dE/dR_j = c R_ij: the force on j is minus that
+      const float gx = c * v.x, gy = c * v.y, gz = c * v.z;
       fix += gx;
       fiy += gy;
       fiz += gz;
-    }
-    if (valid && !staged && c != T(0)) {
-      atomic_add3<T>(F, jatom, -gx, -gy, -gz);
+      atomicAdd(reinterpret_cast<float4*>(F) + jatom, make_float4(-gx, -gy, -gz, 0.f));
       if (want_virial) {
         w00 -= v.x * gx; w01 -= v.x * gy; w02 -= v.x * gz;
         w10 -= v.y * gx; w11 -= v.y * gy; w12 -= v.y * gz;
@@ -707,231 +286,130 @@ __global__ void __launch_bounds__(128, MOM ? (A <= 5 ? AE_MOM_ADJ_BLOCKS : 3)
   }
   __syncwarp();
 
-  // ---- angular terms, one-sided on a circulant schedule: the lane that
-  // owns staged neighbour a evaluates the pairs (a, k = a + t mod na) for
-  // t = 1 .. na/2 (t = na/2 only from the lower half when na is even), so
-  // every pair is evaluated once.  At each step the lanes of a group touch
-  // distinct partners k, so the partner's force is added to shared memory
-  // without atomics; a's own gradient stays in registers until the end of
-  // its round.
-  const T* ga = sm.g + ct.a_i1;
-  const T* gas = sm.g + ct.a_i2;
-  T gav[A], gasv[A];
+  // ---- angular terms: D = B_l M (plain and spin blocks), then one pass over
+  // the staged neighbours, each adding its angular gradient to its radial
+  // force and scattering the total once
+  constexpr int L = A - 1;
+  constexpr int K = A * A;
+  const float* q = pd.qleg + (size_t)ti * AE_MOMA * AE_MOMA;
+  float B0[A], B1[A];
 #pragma unroll
-  for (int q = 0; q < A; ++q) {
-    gav[q] = (!GUARD || q < aN) ? ga[q] : T(0);
-    gasv[q] = (multi && (!GUARD || q < aN)) ? gas[q] : T(0);
+  for (int l = 0; l < A; ++l) {
+    B0[l] = 0.f;
+    B1[l] = 0.f;
   }
-  if constexpr (MOM) {
-    // moment form: D = B_l M (plain and spin blocks), then one pass over
-    // the staged neighbours, each adding its angular gradient to its
-    // radial force and scattering the total once
-    constexpr int L = A - 1;
-    constexpr int K = A * A;
-    const float* q = pd.qleg + (size_t)ti * AE_MOMA * AE_MOMA;
-    float B0[A], B1[A];
 #pragma unroll
-    for (int l = 0; l < A; ++l) {
-      B0[l] = 0.f;
-      B1[l] = 0.f;
-    }
+  for (int nn = 0; nn < A; ++nn) {
+    const float g0 = sg[ct.a_i1 + nn], g1 = multi ? sg[ct.a_i2 + nn] : 0.f;
 #pragma unroll
-    for (int nn = 0; nn < A; ++nn) {
-#pragma unroll
-      for (int l = 0; l <= nn; ++l) {
-        const float ql = q[nn * AE_MOMA + l];
-        B0[l] = fmaf(gav[nn], ql, B0[l]);
-        B1[l] = fmaf(gasv[nn], ql, B1[l]);
-      }
-    }
-    float tau0 = 0.f, tau1 = 0.f;
-#pragma unroll
-    for (int l = 0; l < A; ++l) {
-      tau0 += B0[l];
-      tau1 += B1[l];
-    }
-    float Mv[4 * ((2 * K + 3) / 4)];
-    const float4* M4 = reinterpret_cast<const float4*>(b.M + (size_t)i * b.mom_pad);
-#pragma unroll
-    for (int c4 = 0; c4 < (2 * K + 3) / 4; ++c4) {
-      const float4 t4 = M4[c4];
-      Mv[4 * c4] = t4.x;
-      Mv[4 * c4 + 1] = t4.y;
-      Mv[4 * c4 + 2] = t4.z;
-      Mv[4 * c4 + 3] = t4.w;
-    }
-    float D0[K], D1[K];
-#pragma unroll
-    for (int l = 0; l < A; ++l) {
-#pragma unroll
-      for (int k = l * l; k < (l + 1) * (l + 1); ++k) {
-        D0[k] = B0[l] * Mv[k];
-        D1[k] = B1[l] * Mv[K + k];
-      }
-    }
-    for (int a = sl; a < na; a += LPA) {
-      if (!active) break;
-      const float4 u = sm.au[a], f = sm.af[a];   // unit vector, 1/d; fc, fc', spin, slot
-      float Fv, px, py, pz;
-      mom_gradient<L, true>(u.x, u.y, u.z, f.z, D0, D1, Fv, px, py, pz);
-      const float up = u.x * px + u.y * py + u.z * pz;
-      const float wd = f.x * u.w;
-      const float cu = f.y * (Fv - (tau0 + tau1 * f.z * f.z) * f.x) - wd * up;
-      const int slot = (int)f.w;
-      const float fx = sm.fbuf[3 * a] - fmaf(cu, u.x, wd * px);
-      const float fy = sm.fbuf[3 * a + 1] - fmaf(cu, u.y, wd * py);
-      const float fz = sm.fbuf[3 * a + 2] - fmaf(cu, u.z, wd * pz);
-      atomic_add3<T>(F, jt[slot] & AE_INDEX_MASK, fx, fy, fz);
-      fix -= fx;
-      fiy -= fy;
-      fiz -= fz;
-      if (want_virial) {
-        const T4 v = vec[slot];
-        w00 += v.x * fx; w01 += v.x * fy; w02 += v.x * fz;
-        w10 += v.y * fx; w11 += v.y * fy; w12 += v.y * fz;
-        w20 += v.z * fx; w21 += v.z * fy; w22 += v.z * fz;
-      }
-    }
-  } else {
-    const int tmax = na / 2;
-    for (int a0 = 0; a0 < na; a0 += LPA) {
-      const int a = a0 + sl;
-      const bool own = active && a < na;
-      T4 ua, fa;
-      if (own) {
-        ua = sm.au[a];
-        fa = sm.af[a];
-      } else {
-        ua.x = ua.y = ua.z = T(0);
-        ua.w = T(1);
-        fa.x = fa.y = fa.z = fa.w = T(0);
-      }
-      const T inva = ua.w;
-      T gax = T(0), gay = T(0), gaz = T(0);
-      for (int t = 1; t <= tmax; ++t) {
-        int k = a + t;
-        if (k >= na) k -= na;
-        if (own && !(2 * t == na && a >= tmax)) {
-          const T4 uk = sm.au[k];
-          const T4 fk = sm.af[k];
-          const T cosv = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
-          const T w = fa.x * fk.x;
-          T ss = fa.z * fk.z;
-          if constexpr (GUARD) {
-            if (b.nb_rank) ss = ordered_spin<T>(b, i, fa, fk);
-          }
-          T x, dxdc;
-          angular_arg(cosv, ct.angular_legacy, x, dxdc);
-          const T x2 = x + x;
-          T tm1 = T(1), t0 = x, um1 = T(1), u0 = x2;
-          T Av = fma(ss, gasv[0], gav[0]), Bv = T(0);
-#pragma unroll
-          for (int q = 1; q < A; ++q) {
-            if (!GUARD || q < aN) {
-              const T cq = fma(ss, gasv[q], gav[q]);
-              Av = fma(cq, t0, Av);
-              Bv = fma(cq * T(q), um1, Bv);
-              const T tn = fma(x2, t0, -tm1);
-              tm1 = t0;
-              t0 = tn;
-              const T un = fma(x2, u0, -um1);
-              um1 = u0;
-              u0 = un;
-            }
-          }
-          const T invk = uk.w;
-          const T Bc = w * Bv * dxdc;
-          const T dEda = fa.y * fk.x * Av, ca = Bc * inva;   // d/dd_a of w A, (dE/dcos)/d_a
-          const T dEdk = fa.x * fk.y * Av, ck = Bc * invk;
-          const T gx = dEda * ua.x + ca * (uk.x - cosv * ua.x);
-          const T gy = dEda * ua.y + ca * (uk.y - cosv * ua.y);
-          const T gz = dEda * ua.z + ca * (uk.z - cosv * ua.z);
-          const T hx = dEdk * uk.x + ck * (ua.x - cosv * uk.x);
-          const T hy = dEdk * uk.y + ck * (ua.y - cosv * uk.y);
-          const T hz = dEdk * uk.z + ck * (ua.z - cosv * uk.z);
-          gax += gx;
-          gay += gy;
-          gaz += gz;
-          sm.fbuf[3 * k] -= hx;
-          sm.fbuf[3 * k + 1] -= hy;
-          sm.fbuf[3 * k + 2] -= hz;
-        }
-        __syncwarp(gmask);
-      }
-      if (own) {
-        sm.fbuf[3 * a] -= gax;
-        sm.fbuf[3 * a + 1] -= gay;
-        sm.fbuf[3 * a + 2] -= gaz;
-      }
-      __syncwarp(gmask);
-    }
-    // forces on the staged neighbours (radial + angular), one scatter each
-    for (int a = sl; a < na; a += LPA) {
-      if (!active) break;
-      const int slot = (int)sm.af[a].w;
-      const T fx = sm.fbuf[3 * a], fy = sm.fbuf[3 * a + 1], fz = sm.fbuf[3 * a + 2];
-      atomic_add3<T>(F, jt[slot] & AE_INDEX_MASK, fx, fy, fz);
-      fix -= fx;   // the central atom takes minus the neighbour's force
-      fiy -= fy;
-      fiz -= fz;
-      if (want_virial) {
-        const T4 v = vec[slot];
-        w00 += v.x * fx; w01 += v.x * fy; w02 += v.x * fz;
-        w10 += v.y * fx; w11 += v.y * fy; w12 += v.y * fz;
-        w20 += v.z * fx; w21 += v.z * fy; w22 += v.z * fz;
-      }
+    for (int l = 0; l <= nn; ++l) {
+      const float ql = q[nn * AE_MOMA + l];
+      B0[l] = fmaf(g0, ql, B0[l]);
+      B1[l] = fmaf(g1, ql, B1[l]);
     }
   }
-  fix = gsum<T, LPA>(fix);
-  fiy = gsum<T, LPA>(fiy);
-  fiz = gsum<T, LPA>(fiz);
-  if (active && sl == 0) atomic_add3<T>(F, i, fix, fiy, fiz);
+  float tau0 = 0.f, tau1 = 0.f;
+#pragma unroll
+  for (int l = 0; l < A; ++l) {
+    tau0 += B0[l];
+    tau1 += B1[l];
+  }
+  float Mv[4 * ((2 * K + 3) / 4)];
+  const float4* M4 = reinterpret_cast<const float4*>(b.M + (size_t)i * b.mom_pad);
+#pragma unroll
+  for (int c4 = 0; c4 < (2 * K + 3) / 4; ++c4) {
+    const float4 t4 = M4[c4];
+    Mv[4 * c4] = t4.x;
+    Mv[4 * c4 + 1] = t4.y;
+    Mv[4 * c4 + 2] = t4.z;
+    Mv[4 * c4 + 3] = t4.w;
+  }
+  float D0[K], D1[K];
+#pragma unroll
+  for (int l = 0; l < A; ++l) {
+#pragma unroll
+    for (int k = l * l; k < (l + 1) * (l + 1); ++k) {
+      D0[k] = B0[l] * Mv[k];
+      D1[k] = multi ? B1[l] * Mv[K + k] : 0.f;
+    }
+  }
+  for (int a = sl; a < na; a += LPA) {
+    if (!active) break;
+    const float4 v = au[a];
+    const int slot = info[a] >> 3;
+    const float s = multi ? s_spin[ti * AE_MAXT + (info[a] & 7)] : 0.f;
+    const float inv = __fdividef(1.f, v.w);
+    const float ux = v.x * inv, uy = v.y * inv, uz = v.z * inv;
+    float fc, dfc;
+    cutoff_a(v.w, a_Rc, a_a, fc, dfc);
+    float Fv, px, py, pz;
+    mom_gradient<L, true>(ux, uy, uz, s, D0, D1, Fv, px, py, pz);
+    const float up = ux * px + uy * py + uz * pz;
+    const float wd = fc * inv;
+    const float cu = fmaf(dfc, fmaf(-fmaf(tau1 * s, s, tau0), fc, Fv), fmaf(-wd, up, rad[a]));
+    const float fx = -fmaf(cu, ux, wd * px), fy = -fmaf(cu, uy, wd * py),
+                fz = -fmaf(cu, uz, wd * pz);
+    atomicAdd(reinterpret_cast<float4*>(F) + (jt[slot] & AE_INDEX_MASK),
+              make_float4(fx, fy, fz, 0.f));
+    fix -= fx;
+    fiy -= fy;
+    fiz -= fz;
+    if (want_virial) {
+      w00 += v.x * fx; w01 += v.x * fy; w02 += v.x * fz;
+      w10 += v.y * fx; w11 += v.y * fy; w12 += v.y * fz;
+      w20 += v.z * fx; w21 += v.z * fy; w22 += v.z * fz;
+    }
+  }
+  fix = gsum<float, LPA>(fix);
+  fiy = gsum<float, LPA>(fiy);
+  fiz = gsum<float, LPA>(fiz);
+  if (active && sl == 0)
+    atomicAdd(reinterpret_cast<float4*>(F) + i, make_float4(fix, fiy, fiz, 0.f));
   if (want_virial) {
-    T wv[9] = {w00, w01, w02, w10, w11, w12, w20, w21, w22};
+    float wv[9] = {w00, w01, w02, w10, w11, w12, w20, w21, w22};
 #pragma unroll
-    for (int q = 0; q < 9; ++q) wv[q] = gsum<T, LPA>(wv[q]);
+    for (int k = 0; k < 9; ++k) wv[k] = gsum<float, LPA>(wv[k]);
     if (active && sl == 0) {
-      double* V = b.virial + 9 * sid;
+      double* V = b.virial + 9 * (size_t)sid;
 #pragma unroll
-      for (int q = 0; q < 9; ++q) atomicAdd(V + q, (double)wv[q]);
+      for (int k = 0; k < 9; ++k) atomicAdd(V + k, (double)wv[k]);
     }
   }
 }
 
-template <typename T, int R, int A, int LPA, bool GUARD, bool MOM>
-int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
+template <int R, int A, int LPA>
+int launch_adjoint_mom(const PotDevice& pd, const DescBuffers& b, cudaStream_t s) {
   // four warps per block, fewer when the atoms do not fill them (the
   // per-atom calls: one group, so long rows still fit shared memory)
   const int gpw = 32 / LPA;
   const int warps = b.natoms >= 4 * gpw ? 4 : (b.natoms + gpw - 1) / gpw;
   const int groups = warps * gpw;
-  size_t scratch = 0;
-  if constexpr (MOM) scratch = adjoint ? 0 : mom_scratch_bytes<A, LPA>();
-  size_t smem = group_smem_bytes<T>(b.cap_a, pd.nsf_pad, adjoint, scratch) * groups;
+  const size_t smem = adjoint_mom_smem(b.cap_a, pd.nsf_pad) * groups;
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  const int atoms_per_block = groups;
-  const int blocks = (b.natoms + atoms_per_block - 1) / atoms_per_block;
-  if (adjoint) {
-    auto kern = k_adjoint<T, R, A, LPA, GUARD, MOM>;
-    if (smem + AE_STATIC_SMEM > 48 * 1024)
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<blocks, warps * 32, smem, s>>>(pd, b);
-  } else {
-    auto kern = k_forward<T, R, A, LPA, GUARD, MOM>;
-    if (smem + AE_STATIC_SMEM > 48 * 1024)
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<blocks, warps * 32, smem, s>>>(pd, b);
-  }
+  const int blocks = (b.natoms + groups - 1) / groups;
+  auto kern = k_adjoint_mom<R, A, LPA>;
+  if (smem + AE_STATIC_SMEM > 48 * 1024)
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kern<<<blocks, warps * 32, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }
-
-template <typename T, int R, int A, bool MOM>
-int launch_lpa(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
-  switch (b.lpa) {
-    case 8: return launch<T, R, A, 8, false, MOM>(pd, b, adjoint, s);
-    case 32: return launch<T, R, A, 32, false, MOM>(pd, b, adjoint, s);
-    default: return launch<T, R, A, 16, false, MOM>(pd, b, adjoint, s);
-  }
+// Lanes per atom: as asked (8 or 32), else 8 from 20 atoms per SM on and 16
+// below.  Whole mixed passes with 8, 16 and 32 lanes: 864 Au/Cu atoms 74, 72
+// and 72 us, 4,000 90, 94 and 97, 32,000 246, 261 and 290; 512 Li/Si/O cells
+// (72,513 atoms) 359, 380 and 418 us.  More lanes where a block's rows would
+// not fit its shared memory.
+template <int R, int A>
+int adjoint_mom(const PotDevice& pd, const DescBuffers& b, cudaStream_t s) {
+  int dev = 0, nsm = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  int lanes = b.lpa == 8 || b.lpa == 32 ? b.lpa : b.natoms >= 20 * nsm ? 8 : 16;
+  while (lanes < 32 &&
+         adjoint_mom_smem(b.cap_a, pd.nsf_pad) * (size_t)(4 * 32 / lanes) > 200 * 1024)
+    lanes *= 2;
+  return lanes == 8    ? launch_adjoint_mom<R, A, 8>(pd, b, s)
+         : lanes == 16 ? launch_adjoint_mom<R, A, 16>(pd, b, s)
+                       : launch_adjoint_mom<R, A, 32>(pd, b, s);
 }
 
 // common (radial, angular) sizes of every species, or false
@@ -946,39 +424,9 @@ inline bool uniform_sizes(const PotDevice& pd, int& rN, int& aN) {
   return same;
 }
 
-// FP32 moment form of the angular terms (k_cheb_mom.cu); returns
-// AE_MOM_NA when the sizes have no moment instantiation
+// FP32 adjoint in moment form (k_cheb_mom.cu); AE_MOM_NA when the sizes have
+// no moment instantiation
 constexpr int AE_MOM_NA = -1;
-int dispatch_moments(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s);
-
-// Exact instantiations for the common (radial, angular) sizes, guarded
-// ones for everything else.  FP32 evaluations with a moment buffer take
-// the moment form where it is instantiated.
-template <typename T>
-int dispatch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
-  int rN, aN;
-  const bool same = uniform_sizes(pd, rN, aN);
-  if (b.nb_rank) {
-    // ordered spin weights: pair form of the guarded instances
-    if (rN <= 24 && aN <= 16) return launch<T, 24, 16, 16, true, false>(pd, b, adjoint, s);
-    if (rN <= 32 && aN <= 32) return launch<T, 32, 32, 16, true, false>(pd, b, adjoint, s);
-    return (int)cudaErrorInvalidValue;
-  }
-  if constexpr (sizeof(T) == 4) {
-    if (b.M && pd.qleg) {
-      const int e = dispatch_moments(pd, b, adjoint, s);
-      if (e != AE_MOM_NA) return e;
-    }
-  }
-  if (same) {
-    if (rN == 11 && aN == 5) return launch_lpa<T, 11, 5, false>(pd, b, adjoint, s);
-    if (rN == 13 && aN == 7) return launch_lpa<T, 13, 7, false>(pd, b, adjoint, s);
-    if (rN == 17 && aN == 9) return launch_lpa<T, 17, 9, false>(pd, b, adjoint, s);
-    if (rN == 17 && aN == 5) return launch_lpa<T, 17, 5, false>(pd, b, adjoint, s);
-  }
-  if (rN <= 24 && aN <= 16) return launch<T, 24, 16, 16, true, false>(pd, b, adjoint, s);
-  if (rN <= 32 && aN <= 32) return launch<T, 32, 32, 16, true, false>(pd, b, adjoint, s);
-  return (int)cudaErrorInvalidValue;
-}
+int dispatch_adjoint_mom(const PotDevice& pd, const DescBuffers& b, cudaStream_t s);
 
 }  // namespace cheb

@@ -74,45 +74,6 @@ __host__ __device__ constexpr MomConsts mom_consts() {
 
 static __constant__ MomConsts c_mom = mom_consts();
 
-// M0 += w0 Y(u), M1 += w1 Y(u) for all components up to degree L
-template <int L, bool MULTI>
-__device__ __forceinline__ void mom_accumulate(float x, float y, float z, float w0, float w1,
-                                               float (&M0)[(L + 1) * (L + 1)],
-                                               float (&M1)[(L + 1) * (L + 1)]) {
-  float cm = 1.f, sm = 0.f;
-#pragma unroll
-  for (int m = 0; m <= L; ++m) {
-    if (m > 0) {
-      const float cn = fmaf(x, cm, -y * sm);
-      sm = fmaf(x, sm, y * cm);
-      cm = cn;
-    }
-    const float c0 = w0 * cm, s0 = w0 * sm, c1 = w1 * cm, s1 = w1 * sm;
-    float q1 = 0.f, q2 = 0.f;
-#pragma unroll
-    for (int l = m; l <= L; ++l) {
-      float q;
-      if (l == m) q = c_mom.qmm[m];
-      else if (l == m + 1) q = c_mom.a1[m] * z * q1;
-      else q = fmaf(c_mom.a[l][m] * z, q1, -c_mom.b[l][m] * q2);
-      q2 = q1;
-      q1 = q;
-      const int k = l * l + (m ? 2 * m - 1 : 0);
-      if (m == 0) {
-        M0[k] = fmaf(q, w0, M0[k]);
-        if (MULTI) M1[k] = fmaf(q, w1, M1[k]);
-      } else {
-        M0[k] = fmaf(q, c0, M0[k]);
-        M0[k + 1] = fmaf(q, s0, M0[k + 1]);
-        if (MULTI) {
-          M1[k] = fmaf(q, c1, M1[k]);
-          M1[k + 1] = fmaf(q, s1, M1[k + 1]);
-        }
-      }
-    }
-  }
-}
-
 // F = sum_k C_k Y_k(u) with C = D0 + s D1, and the gradient (px, py, pz) of
 // its polynomial extension at u
 template <int L, bool MULTI>

@@ -29,7 +29,9 @@
 // neighbours, 21 angular) forward 2481 -> 1138 us, adjoint 4527 -> 1516 us;
 // 2,765 Au/Cu atoms forward 144 -> 80 us, adjoint 323 -> 109 us.  The error
 // against 64-bit automatic differentiation is that of the pair sums (1.6e-14
-// of the forces of the batch, 1.7e-14 before).
+// of the forces of the batch, 1.7e-14 before).  FP32: 256,000 Cu/Au atoms (78
+// neighbours, 18 angular, pair sums) forward 645 -> 235 us, adjoint 614 -> 444
+// us; 4,096 Li/Si/O cells (597,000 atoms, moments) forward 569 -> 460 us.
 #pragma once
 #include "common.h"
 #include "cutoff64.cuh"
@@ -163,7 +165,7 @@ __device__ __forceinline__ void series(const typename Num<T>::v2* tab, T x, int 
 // vector and 1/d; fc and fc'; table slot and species), in the adjoint their
 // sums (V, S) and radial term and the coefficient tables; in the moment form
 // the moments and, in the adjoint, their tables.
-// info: table slot << 5 | spin + 1 (unit spins) << 3 | species
+// info: table slot << 5 | spin + 1 (adjoint, unit spins) << 3 | species
 struct Layout {
   int sf, info, acc, rad, g, tab_r, tab_a, mom, bytes;
 };
@@ -434,23 +436,42 @@ __device__ __forceinline__ void monic_gradient(T x, T y, T z, const typename Num
   }
 }
 
+// Bulk prefetch of an atom's neighbour rows into L2 (one instruction per row,
+// issued by the group's first lane): the radial rounds then wait on L2 instead
+// of DRAM.  Rows start 16-byte aligned (the ELL capacity is a multiple of 32)
+// and the sizes are rounded up to 16 bytes inside the row.  FP32 only: the
+// FP64 kernels wait on their pipe.
+__device__ __forceinline__ void prefetch_rows(const float4* vec, const int* jt, int n) {
+  if (n <= 0) return;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(vec)),
+               "r"(16 * n)
+               : "memory");
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(jt)),
+               "r"((4 * n + 15) & ~15)
+               : "memory");
+}
+__device__ __forceinline__ void prefetch_rows(const double4_32a*, const int*, int) {}
+
 // the moment rows and the Legendre tables of a precision
 template <typename T>
 struct MomRows;
 template <>
 struct MomRows<float> {
-  static __device__ __forceinline__ float* rows(const DescBuffers& b) { return b.M; }
-  static __device__ __forceinline__ const float* q(const PotDevice& pd) { return pd.qleg; }
+  static __host__ __device__ __forceinline__ float* rows(const DescBuffers& b) { return b.M; }
+  static __host__ __device__ __forceinline__ const float* q(const PotDevice& pd) { return pd.qleg; }
 };
 template <>
 struct MomRows<double> {
-  static __device__ __forceinline__ double* rows(const DescBuffers& b) { return b.M64; }
-  static __device__ __forceinline__ const double* q(const PotDevice& pd) { return pd.qleg64; }
+  static __host__ __device__ __forceinline__ double* rows(const DescBuffers& b) { return b.M64; }
+  static __host__ __device__ __forceinline__ const double* q(const PotDevice& pd) { return pd.qleg64; }
 };
 
 // warps per block (they share only the spin table) and the resident blocks
 // asked of the register allocator: FP64 leaves it to one-warp blocks, which
 // spread few atoms evenly; FP32 asks for the occupancy that its latencies need
+// (256,000 Cu/Au atoms: forward 279, 250, 239 and 241 us at 5, 6, 7 and 8
+// blocks, adjoint 477 and 487 us at 6 and 7; 4,096 Li/Si/O cells: forward 494,
+// 480 and 501 us at 6, 7 and 8)
 template <typename T>
 constexpr int max_threads() {
   return sizeof(T) == 8 ? 32 : 128;
@@ -461,9 +482,12 @@ constexpr int max_threads() {
 #ifndef AE_ROWS_ADJ
 #define AE_ROWS_ADJ 6
 #endif
-template <typename T, int A, int SPIN, bool MOM>
+#ifndef AE_MROWS_FWD
+#define AE_MROWS_FWD 7
+#endif
+template <typename T, int R, int A, int SPIN, bool MOM>
 constexpr int fwd_blocks() {
-  return sizeof(T) == 8 ? 1 : AE_ROWS_FWD;
+  return sizeof(T) == 8 ? 1 : MOM ? (A <= 5 ? AE_MROWS_FWD : 3) : R <= 17 ? AE_ROWS_FWD : 4;
 }
 template <typename T, int A, int SPIN, bool MOM>
 constexpr int adj_blocks() {
@@ -474,7 +498,7 @@ constexpr int adj_blocks() {
 // forward
 // ----------------------------------------------------------------------
 template <typename T, int R, int A, int LPA, bool GUARD, int SPIN, bool MOM>
-__global__ void __launch_bounds__(max_threads<T>(), fwd_blocks<T, A, SPIN, MOM>())
+__global__ void __launch_bounds__(max_threads<T>(), fwd_blocks<T, R, A, SPIN, MOM>())
     k_forward_rows(PotDevice pd, DescBuffers b) {
   using T4 = typename Num<T>::v4;
   using T2 = typename Num<T>::v2;
@@ -501,6 +525,7 @@ __global__ void __launch_bounds__(max_threads<T>(), fwd_blocks<T, A, SPIN, MOM>(
   const T4* __restrict__ vec =
       reinterpret_cast<const T4*>(b.nb_vec) + (size_t)i * b.cap;
   const int* __restrict__ jt = b.nb_jt + (size_t)i * b.cap;
+  if (sl == 0) prefetch_rows(vec, jt, n);
   const int nloop = warp_max(n);
   const T r_Rc = T(ct.r_Rc), a_Rc = T(ct.a_Rc);
   const T two_over_rc = T(2) / r_Rc, r_a = T(SFB_PI) / r_Rc;
@@ -567,7 +592,7 @@ __global__ void __launch_bounds__(max_threads<T>(), fwd_blocks<T, A, SPIN, MOM>(
       const int k = na + __popc(m & ((1u << lane) - 1u));
       if (k < b.cap_a) {
         w.su[k] = v;
-        w.info[k] = (j << 5) | (SPIN == SPIN_UNIT ? ((int)s + 1) << 3 : 0) | t;
+        w.info[k] = (j << 5) | t;
       }
     }
     na += __popc(m);
@@ -730,6 +755,7 @@ __global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>(
   const T4* __restrict__ vec =
       reinterpret_cast<const T4*>(b.nb_vec) + (size_t)i * b.cap;
   const int* __restrict__ jt = b.nb_jt + (size_t)i * b.cap;
+  if (sl == 0) prefetch_rows(vec, jt, n);
   const int nloop = warp_max(n);
   const T r_Rc = T(ct.r_Rc), a_Rc = T(ct.a_Rc);
   const T two_over_rc = T(2) / r_Rc, r_a = T(SFB_PI) / r_Rc;
@@ -1021,6 +1047,11 @@ size_t group_smem(const PotDevice& pd, const DescBuffers& b, bool adjoint) {
 }
 
 constexpr size_t SMEM_MAX = 226 * 1024;
+// the FP32 adjoint in moment form is k_cheb_impl.cuh's, which keeps its
+// coefficients in registers: 576 us for 4,096 Li/Si/O cells against 625 us
+// with the tables of this file's and 620 us with registers in it
+template <typename T, bool MOM>
+constexpr bool HAS_ADJOINT = sizeof(T) == 8 || !MOM;
 
 template <typename T, int R, int A, int LPA, bool GUARD, int SPIN, bool MOM>
 int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int warps,
@@ -1029,8 +1060,10 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
   const size_t smem = group_smem<T, R, A, SPIN, MOM>(pd, b, adjoint) * atoms;
   if (smem > SMEM_MAX) return (int)cudaErrorInvalidValue;
   const int blocks = (b.natoms + atoms - 1) / atoms;
-  auto kern = adjoint ? k_adjoint_rows<T, R, A, LPA, GUARD, SPIN, MOM>
-                      : k_forward_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
+  void (*kern)(PotDevice, DescBuffers) = k_forward_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
+  if constexpr (HAS_ADJOINT<T, MOM>) {
+    if (adjoint) kern = k_adjoint_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
+  }
   if (smem + AE_STATIC_SMEM > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   kern<<<blocks, 32 * warps, smem, s>>>(pd, b);
@@ -1042,7 +1075,8 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
 // each) and take rows too long for several groups' shared memory.  Whole FP64
 // passes with 32, 16 and 8 lanes: 864 Au/Cu atoms 148, 158 and 217 us; 1,176
 // 168, 165 and 224; 1,792 239, 222 and 253; 2,772 361, 331 and 337; 4,840
-// Cu/Au atoms 541, 464 and 442.  Hence below 8 atoms per SM 32, below 20 16.
+// Cu/Au atoms 541, 464 and 442.  Hence below 8 atoms per SM 32, below 20 16
+// (the FP32 kernels follow the same line).
 template <typename T, int R, int A, bool GUARD, int SPIN, bool MOM>
 int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
   int dev = 0, nsm = 152;
@@ -1059,44 +1093,74 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
   return launch_lanes<T, R, A, 32, GUARD, SPIN, MOM>(pd, b, adjoint, 1, s);
 }
 
+// (the forward takes any spins in its SPIN_UNIT instance)
 template <typename T, int R, int A, bool MOM>
 int launch_spin(const PotDevice& pd, const DescBuffers& b, int spin, bool adjoint, cudaStream_t s) {
-  return spin == SPIN_NONE ? launch<T, R, A, false, SPIN_NONE, MOM>(pd, b, adjoint, s)
-                           : launch<T, R, A, false, SPIN_UNIT, MOM>(pd, b, adjoint, s);
+  if (spin == SPIN_NONE) return launch<T, R, A, false, SPIN_NONE, MOM>(pd, b, adjoint, s);
+  if constexpr (!MOM) {
+    if (adjoint && spin == SPIN_ANY)
+      return launch<T, R, A, false, SPIN_ANY, false>(pd, b, adjoint, s);
+  }
+  return launch<T, R, A, false, SPIN_UNIT, MOM>(pd, b, adjoint, s);
+}
+
+// common sizes and spin range of a set of potentials
+struct Sizes {
+  int rN = 0, aN = 0, spin = SPIN_NONE;
+  bool same = true;
+};
+inline Sizes sizes(const PotDevice& pd) {
+  Sizes z;
+  for (int t = 0; t < pd.ntypes; ++t) {
+    const ChebTable& ct = pd.sp[t].cheb;
+    if (t > 0 && (ct.r_N != z.rN || ct.a_N != z.aN)) z.same = false;
+    z.rN = max(z.rN, ct.r_N);
+    z.aN = max(z.aN, ct.a_N);
+    if (!ct.multi) continue;
+    z.spin = max(z.spin, (int)SPIN_UNIT);
+    for (int q = 0; q < pd.ntypes; ++q)
+      if (ct.spin[q] < -1.f || ct.spin[q] > 1.f) z.spin = SPIN_ANY;
+  }
+  return z;
+}
+inline bool exact(const Sizes& z, const DescBuffers& b) {
+  return z.same && !b.nb_rank;
+}
+// whether the angular terms take the moment form: a moment buffer, an
+// instantiated size, and in FP64 spins that the adjoint's tables cover
+template <typename T>
+bool moment_form(const PotDevice& pd, const DescBuffers& b) {
+  const Sizes z = sizes(pd);
+  if (!exact(z, b) || !MomRows<T>::rows(b) || !MomRows<T>::q(pd) ||
+      b.mom_pad < 2 * z.aN * z.aN || (sizeof(T) == 8 && z.spin == SPIN_ANY))
+    return false;
+  return (z.rN == 11 && z.aN == 5) || (z.rN == 17 && z.aN == 5) ||
+         (sizeof(T) == 4 && z.rN == 13 && z.aN == 7);
 }
 
 // The instances for a set of potentials: exact ones for the common (radial,
-// angular) sizes and spins within -1 .. 1 (up to three species), guarded ones
-// for everything else; -1 where `guarded` is false and only those would do.
+// angular) sizes, guarded ones for everything else.
 template <typename T>
-int dispatch_rows(const PotDevice& pd, const DescBuffers& b, bool adjoint, bool guarded,
-                  cudaStream_t s) {
-  int rN = 0, aN = 0, spin = SPIN_NONE;
-  bool same = true;
-  for (int t = 0; t < pd.ntypes; ++t) {
-    const ChebTable& ct = pd.sp[t].cheb;
-    if (t > 0 && (ct.r_N != rN || ct.a_N != aN)) same = false;
-    rN = max(rN, ct.r_N);
-    aN = max(aN, ct.a_N);
-    if (!ct.multi) continue;
-    spin = max(spin, (int)SPIN_UNIT);
-    for (int q = 0; q < pd.ntypes; ++q)
-      if (ct.spin[q] < -1.f || ct.spin[q] > 1.f) spin = SPIN_ANY;
+int dispatch_rows(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
+  const Sizes z = sizes(pd);
+  const bool mom = moment_form<T>(pd, b);
+  if (exact(z, b)) {
+    if (z.rN == 11 && z.aN == 5)
+      return mom ? launch_spin<T, 11, 5, true>(pd, b, z.spin, adjoint, s)
+                 : launch_spin<T, 11, 5, false>(pd, b, z.spin, adjoint, s);
+    if (z.rN == 17 && z.aN == 5)
+      return mom ? launch_spin<T, 17, 5, true>(pd, b, z.spin, adjoint, s)
+                 : launch_spin<T, 17, 5, false>(pd, b, z.spin, adjoint, s);
+    if (z.rN == 13 && z.aN == 7) {
+      if constexpr (sizeof(T) == 4) {
+        if (mom) return launch_spin<T, 13, 7, true>(pd, b, z.spin, adjoint, s);
+      }
+      return launch_spin<T, 13, 7, false>(pd, b, z.spin, adjoint, s);
+    }
+    if (z.rN == 17 && z.aN == 9) return launch_spin<T, 17, 9, false>(pd, b, z.spin, adjoint, s);
   }
-  if (same && spin != SPIN_ANY && !b.nb_rank) {
-    const bool mom = sizeof(T) == 8 && b.M64 && pd.qleg64 && b.mom_pad >= 2 * aN * aN;
-    if (rN == 11 && aN == 5)
-      return mom ? launch_spin<T, 11, 5, sizeof(T) == 8>(pd, b, spin, adjoint, s)
-                 : launch_spin<T, 11, 5, false>(pd, b, spin, adjoint, s);
-    if (rN == 17 && aN == 5)
-      return mom ? launch_spin<T, 17, 5, sizeof(T) == 8>(pd, b, spin, adjoint, s)
-                 : launch_spin<T, 17, 5, false>(pd, b, spin, adjoint, s);
-    if (rN == 13 && aN == 7) return launch_spin<T, 13, 7, false>(pd, b, spin, adjoint, s);
-    if (rN == 17 && aN == 9) return launch_spin<T, 17, 9, false>(pd, b, spin, adjoint, s);
-  }
-  if (!guarded) return -1;
-  if (rN <= 24 && aN <= 16) return launch<T, 24, 16, true, SPIN_ANY, false>(pd, b, adjoint, s);
-  if (rN <= 32 && aN <= 32) return launch<T, 32, 32, true, SPIN_ANY, false>(pd, b, adjoint, s);
+  if (z.rN <= 24 && z.aN <= 16) return launch<T, 24, 16, true, SPIN_ANY, false>(pd, b, adjoint, s);
+  if (z.rN <= 32 && z.aN <= 32) return launch<T, 32, 32, true, SPIN_ANY, false>(pd, b, adjoint, s);
   return (int)cudaErrorInvalidValue;
 }
 

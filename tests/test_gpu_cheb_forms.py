@@ -1,4 +1,4 @@
-"""The FP64 Chebyshev kernels over the forms that they accept: exact and
+"""The Chebyshev kernels of both precisions over the forms that they accept: exact and
 guarded orders, one species, spins within -1 .. 1 (three species) and beyond
 (five), both angular domains, the pair and the moment form of the angular
 terms, rows with none, one, two and more angular neighbours than lanes, and
@@ -39,12 +39,12 @@ def _workload(ntypes, orders, seed):
 @pytest.mark.parametrize("domain", ["current", "legacy"])
 @pytest.mark.parametrize("ntypes", [1, 3, 5])
 @pytest.mark.parametrize("orders", [(10, 4), (16, 4), (12, 6), (16, 8), (7, 3), (25, 17)])
-def test_fp64_chebyshev_forms_match_oracle(oracle, tmp_path, orders, ntypes, domain):
+def test_chebyshev_forms_match_oracle(oracle, tmp_path, orders, ntypes, domain):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
         pytest.skip("no GPU")
     from aenet_gb300 import workloads
-    from aenet_gb300.core import ANNPotentials, FP64, set_option
+    from aenet_gb300.core import ANNPotentials, FP64, MIXED, set_option
     w = _workload(ntypes, orders, 3 + ntypes)
     s = w.structures[0]
     nsf = w.arch[0]
@@ -62,6 +62,8 @@ def test_fp64_chebyshev_forms_match_oracle(oracle, tmp_path, orders, ntypes, dom
             got[terms] = ann.structure_energy_forces(*one[:3], precision=FP64, virial=True)
             got[terms + "8"] = [ann.batch_energy_forces([one] * r, precision=FP64, virial=True)
                                 for r in many]
+            got[terms + "32"] = [ann.batch_energy_forces([one] * r, precision=MIXED, virial=True)
+                                 for r in [1] + many]
     finally:
         set_option("angular_terms", "moments")
         set_option("angular_domain", "current")
@@ -77,4 +79,10 @@ def test_fp64_chebyshev_forms_match_oracle(oracle, tmp_path, orders, ntypes, dom
             assert np.abs(r8["energy"] - et).max() / s.natoms < 1e-10 * scale
             assert np.abs(r8["forces"].reshape(-1, s.natoms, 3) - F).max() < 1e-9 * scale
             assert np.abs(r8["virial"] - r["virial"]).max() < 1e-8 * scale
+        # FP32: the mixed path's contract (1 meV/atom, 20 meV/A RMS)
+        for r32 in got[terms + "32"]:
+            assert np.abs(r32["energy"] - et).max() / s.natoms < 1e-3
+            dF = r32["forces"].reshape(-1, s.natoms, 3) - F
+            assert np.sqrt(np.mean(dF ** 2)) < 2e-2
+            assert np.abs(r32["virial"] - r["virial"]).max() < 1e-3 * scale * s.natoms
     assert np.abs(got["moments"]["virial"] - got["pairs"]["virial"]).max() < 1e-8 * scale
