@@ -957,6 +957,7 @@ struct aenet_gpu_plan {
   int stale_caller_order = 0; // table rows hold a caller's lists (rank = slot)
   int* struct_order = nullptr;  // structures by decreasing size (per-structure search)
   int smem_atoms = 0, smem_cells = 0;
+  bool all_pairs = false;     // every structure periodic, orthogonal, wide and small
   void* G = nullptr;
   void* dEdG = nullptr;
   double* E_atom = nullptr;
@@ -1138,6 +1139,19 @@ int make_geom(StructGeom& G, const double* lat, int pbc, const double* coords, i
   return 0;
 }
 
+// whether every structure suits the search over all pairs: small, periodic,
+// orthogonal and two cut-offs wide (as wide_structure in k_neighbors.cu)
+bool all_pairs_geometry(const aenet_gpu_plan* P) {
+  for (int s = 0; s < P->nstruc; ++s) {
+    const StructGeom& G = P->geom_h[s];
+    const float w = 2.002f * G.rcf + 2e-3f;
+    if (!G.pbc || !G.ortho || P->natoms_h[s] > AE_PAIRS_ATOMS || G.Lf[0] < w || G.Lf[4] < w ||
+        G.Lf[8] < w)
+      return false;
+  }
+  return true;
+}
+
 // the loaded potentials are Chebyshev bases with a spin block and the
 // stale-spin option is on
 bool stale_spin_wanted() {
@@ -1180,6 +1194,7 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
     if (!G.pbc) nbexp = std::min(nbexp, (double)P->natoms_h[s]);
     dens_max = std::max(dens_max, nbexp);
   }
+  P->all_pairs = all_pairs_geometry(P);
   P->natoms = (int)natoms;
   P->ncells = cell_off;
   P->nchunks = nchunks;
@@ -1435,7 +1450,10 @@ NbBuffers search_buffers(aenet_gpu_plan* P, bool* grouped) {
   nb.types0_out = P->types0;
   nb.ntypes = P->pd->ntypes;
   const bool per_struct = (nb.cell_kernel == 4 || nb.cell_kernel == 5) && nb.struct_order;
-  *grouped = !per_struct && P->natoms > 0 && ae_cells_one(P->natoms, P->ncells);
+  // wide small structures: the default search gives way to the one over all
+  // pairs (the per-structure ones do so by themselves)
+  nb.all_pairs = P->all_pairs && nb.cell_kernel == 0;
+  *grouped = !per_struct && !nb.all_pairs && P->natoms > 0 && ae_cells_one(P->natoms, P->ncells);
   if (*grouped) {
     nb.order_out = P->order;
     nb.spec_off_out = P->spec_off;
@@ -2420,6 +2438,7 @@ EXPORT int aenet_gpu_plan_set_lattices(aenet_gpu_plan* P, const double* lattices
     G.chunk_off = O.chunk_off;
     O = G;
   }
+  P->all_pairs = all_pairs_geometry(P);
   if (cudaMemcpy(P->geom_d, P->geom_h.data(), sizeof(StructGeom) * P->nstruc, cudaMemcpyHostToDevice))
     return AENET_ERR_CUDA;
   return 0;

@@ -253,6 +253,7 @@ struct NbBuffers {
   // optional, plans that ae_cells_one() takes: the atoms grouped by species
   int* order_out;
   int* spec_off_out;
+  int all_pairs;              // every structure fits the search over all its atoms
   int cell_kernel;            // 0: warp per atom; warp per home cell with a lane per
                               // home atom (1) or a lane per candidate (2); 3: warp per
                               // atom over the half stencil, each pair written to both rows;
@@ -263,6 +264,8 @@ struct NbBuffers {
 #define AE_ONE_ATOMS 12288
 #define AE_ONE_CELLS 16384
 bool ae_cells_one(int natoms, int ncells);
+// largest structure that the search over all pairs takes
+#define AE_PAIRS_ATOMS 768
 int ae_launch_neighbors(int natoms, const double* pos, const int* types,
                         const NbBuffers& nb, int fp64, cudaStream_t s);
 // ELL table from a caller's CSR neighbour list (local atoms, indices into

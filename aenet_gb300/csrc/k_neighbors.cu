@@ -27,6 +27,10 @@
 //                  32 units are flattened into one candidate index space
 //                  processed 32 candidates at a time; accepted neighbours are
 //                  compacted with ballots into the atom's ELL row.
+//   k_neighbors_all  one warp per atom over all atoms of its structure (small
+//                  orthogonal structures at least two cut-offs wide, which
+//                  the per-structure kernel treats so too): k_wrap_bin is
+//                  all that comes before.
 //   k_neighbors_struct  one block per structure for batches of small
 //                  structures: wrap and bin, cell counts, scan and scatter
 //                  in shared memory, then the same per-atom search (the
@@ -664,6 +668,177 @@ __global__ void __launch_bounds__(256, 4) k_neighbors(int natoms, NbBuffers nb) 
   search_atom<T4>(i, nb, g, src, su_base[warp], su_sh[warp], su_first[warp], lane);
 }
 
+// ---- all pairs of a periodic orthogonal structure whose edges are at least
+// twice the cut-off long ("wide"): of a pair's images only the nearest can be
+// a neighbour (where the nearest is ambiguous, half an edge away, none is), so
+// the structure's atoms in turn are the candidates, 32 at a time, without
+// cells: |dx| = min(|dx|, |L - |dx||) along each axis, about 22 instructions a
+// batch.  Pairs inside the cut-off go through a per-warp queue, so that the
+// sign of the image, the FP64 test near the cut-off, the FP64 vector and the
+// stores run on 32 of them at once.  A cell stencil needs 900 to 1,300
+// instructions per atom, its set-up and its partly filled batches, at any
+// size.  Rows come out in the same order every time.  Bound by the issue of
+// instructions; one pass of a whole plan, with cells -> like this (us): 256
+// atoms 68.4 -> 62.4, 864 atoms 72.2 -> 71.0, 1,372 atoms 78.5 -> 80.4, 2,048
+// atoms 78.1 -> 83.9, hence the limit AE_PAIRS_ATOMS; FP64, 256 atoms 106.6 ->
+// 93.5.  In the per-structure kernels, the search of 4,096 Li/Si/O structures
+// (three atoms in four are in wide ones): 723 -> 561 us.
+__device__ __forceinline__ bool wide_structure(const StructGeom* g) {
+  const float w = 2.002f * g->rcf + 2e-3f;
+  return g->natoms <= AE_PAIRS_ATOMS && g->pbc && g->ortho && g->Lf[0] >= w && g->Lf[4] >= w &&
+         g->Lf[8] >= w;
+}
+
+// nearest image of dx along an edge of length L: dx + T L
+__device__ __forceinline__ float nearest(float dx, float L, int& T) {
+  const float far = dx - copysignf(L, dx);
+  const bool other = fabsf(far) < fabsf(dx);
+  T = other ? (dx > 0.f ? -1 : 1) : 0;
+  return other ? far : dx;
+}
+
+// One accepted pair per lane into the row: vector e (to image img of atom j)
+// and its squared length dd2; FP64 decides near the cut-off.
+template <typename T4>
+__device__ __forceinline__ void push_pair(bool in, int i, int j, float4 rj, float ex, float ey,
+                                          float ez, float dd2, int t0, int t1, int t2,
+                                          const NbBuffers& nb, const StructGeom* g, size_t row,
+                                          int& cnt, unsigned lt) {
+  bool accept = in;
+  const int img = (t0 & 1023) | ((t1 & 1023) << 10) | ((t2 & 1023) << 20);
+  if (accept && !(dd2 < g->rc2_lo))
+    accept = dd2 <= g->rc2_hi && band_fp64(nb, g, g->pbc, false, img, i, j, g->rc2);
+  const unsigned mask = __ballot_sync(0xffffffffu, accept);
+  const int k = cnt + __popc(mask & lt);
+  if (accept && k < nb.cap) {
+    nb.nb_jt[row + k] = j | (__float_as_int(rj.w) << AE_TYPE_SHIFT);
+    if (nb.nb_img) nb.nb_img[row + k] = img;
+    if (VecOut<T4>::fp64)
+      reinterpret_cast<double4_32a*>(nb.nb_vec)[row + k] =
+          pair_vector64(g, nb, g->pbc, i, j, t0, t1, t2);
+    else
+      reinterpret_cast<float4*>(nb.nb_vec)[row + k] = make_float4(ex, ey, ez, pair_length(dd2));
+  }
+  cnt += __popc(mask);
+}
+
+template <typename T4>
+__device__ __forceinline__ void search_all(int i, const NbBuffers& nb, const StructGeom* g,
+                                           const float4* pos, int* queue, int lane) {
+  const int n = g->natoms, a0 = g->atom_off, self = i - a0;
+  const float L0 = g->Lf[0], L1 = g->Lf[4], L2 = g->Lf[8];
+  const float rc2_hi = g->rc2_hi;
+  const float4 ri = pos[self];
+  const int cap = nb.cap;
+  const size_t row = (size_t)i * cap;
+  const unsigned lt = (1u << lane) - 1u;
+  int cnt = 0, head = 0;
+  float4 rn = pos[min(lane, n - 1)];
+  for (int jb = 0; jb < n; jb += 32) {
+    const int j = jb + lane;
+    const float4 rj = rn;
+    rn = pos[min(j + 32, n - 1)];   // the next batch
+    float dx = fabsf(rj.x - ri.x), dy = fabsf(rj.y - ri.y), dz = fabsf(rj.z - ri.z);
+    dx = fminf(dx, fabsf(dx - L0));
+    dy = fminf(dy, fabsf(dy - L1));
+    dz = fminf(dz, fabsf(dz - L2));
+    const bool ok = dx * dx + dy * dy + dz * dz <= rc2_hi && j < n && j != self;
+    const unsigned m = __ballot_sync(0xffffffffu, ok);
+    if (ok) queue[head + __popc(m & lt)] = j;
+    head += __popc(m);
+    while (head >= 32 || (head > 0 && jb + 32 >= n)) {
+      __syncwarp();
+      const int c = min(head, 32);
+      // oldest entries first (the row keeps the atoms' order)
+      const int e = lane < c ? queue[lane] : 0;
+      const int rest = lane + 32 < head ? queue[lane + 32] : 0;
+      __syncwarp();
+      head -= c;
+      if (lane < head) queue[lane] = rest;
+      const float4 rq = pos[e];
+      int t0, t1, t2;
+      const float ex = nearest(rq.x - ri.x, L0, t0), ey = nearest(rq.y - ri.y, L1, t1),
+                  ez = nearest(rq.z - ri.z, L2, t2);
+      const float dd2 = ex * ex + ey * ey + ez * ez;
+      push_pair<T4>(lane < c, i, a0 + e, rq, ex, ey, ez, dd2, t0, t1, t2, nb, g, row, cnt, lt);
+      __syncwarp();
+    }
+  }
+  if (lane == 0) {
+    nb.nb_cnt[i] = min(cnt, cap);
+    if (cnt > cap) atomicOr(nb.status, AE_ST_NB_OVERFLOW);
+  }
+}
+
+// The same for any periodic cell, over all images that the cells' stencil
+// reaches: for a plan whose lattices have become narrow or oblique since its
+// launches were recorded in a graph.
+template <typename T4>
+__device__ __noinline__ void search_images(int i, const NbBuffers& nb, const StructGeom* g,
+                                           int lane) {
+  const int n = g->natoms, a0 = g->atom_off;
+  const int m0 = (g->nc[0] - 1 + g->kr[0]) / g->nc[0], m1 = (g->nc[1] - 1 + g->kr[1]) / g->nc[1],
+            m2 = (g->nc[2] - 1 + g->kr[2]) / g->nc[2];
+  const float4 ri = nb.r_f32[i];
+  const size_t row = (size_t)i * nb.cap;
+  int cnt = 0;
+  for (int t0 = -m0; t0 <= m0; ++t0)
+    for (int t1 = -m1; t1 <= m1; ++t1)
+      for (int t2 = -m2; t2 <= m2; ++t2) {
+        const float sx = t0 * g->Lf[0] + t1 * g->Lf[3] + t2 * g->Lf[6] - ri.x;
+        const float sy = t0 * g->Lf[1] + t1 * g->Lf[4] + t2 * g->Lf[7] - ri.y;
+        const float sz = t0 * g->Lf[2] + t1 * g->Lf[5] + t2 * g->Lf[8] - ri.z;
+        for (int jb = 0; jb < n; jb += 32) {
+          const int j = a0 + min(jb + lane, n - 1);
+          const float4 rj = nb.r_f32[j];
+          const float ex = rj.x + sx, ey = rj.y + sy, ez = rj.z + sz;
+          const float dd2 = ex * ex + ey * ey + ez * ez;
+          const bool in = jb + lane < n && dd2 <= g->rc2_hi && (j != i || t0 || t1 || t2);
+          if (__any_sync(0xffffffffu, in))
+            push_pair<T4>(in, i, j, rj, ex, ey, ez, dd2, t0, t1, t2, nb, g, row, cnt,
+                          (1u << lane) - 1u);
+        }
+      }
+  if (lane == 0) {
+    nb.nb_cnt[i] = min(cnt, nb.cap);
+    if (cnt > nb.cap) atomicOr(nb.status, AE_ST_NB_OVERFLOW);
+  }
+}
+
+// plans of wide structures only: a warp per atom
+template <typename T4>
+__global__ void __launch_bounds__(256) k_neighbors_all(int natoms, NbBuffers nb) {
+  __shared__ int s_queue[8][64];
+  const int lane = threadIdx.x & 31;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= natoms) return;
+  const StructGeom* g = nb.geom + nb.atom_struct[i];
+  if (!wide_structure(g)) {
+    search_images<T4>(i, nb, g, lane);
+    return;
+  }
+  search_all<T4>(i, nb, g, nb.r_f32 + g->atom_off, s_queue[threadIdx.x >> 5], lane);
+}
+
+// The block's structure, when it is wide: wrapped, its positions in shared
+// memory, and every atom's row by search_all.  (su_sh: scratch of the other
+// search, here the warps' queues.)
+template <typename T4>
+__device__ __forceinline__ bool struct_all(const StructGeom* g, const double* __restrict__ pos,
+                                           const int* __restrict__ types, const NbBuffers& nb,
+                                           float4* spos, float4* su_sh_w) {
+  if (!wide_structure(g)) return false;
+  const int n = g->natoms, a0 = g->atom_off;
+  for (int q = threadIdx.x; q < n; q += blockDim.x) {
+    wrap_bin_atom(a0 + q, g, pos, types, nb);
+    spos[q] = nb.r_f32[a0 + q];
+  }
+  __syncthreads();
+  for (int a = threadIdx.x >> 5; a < n; a += (blockDim.x >> 5))
+    search_all<T4>(a0 + a, nb, g, spos, reinterpret_cast<int*>(su_sh_w), threadIdx.x & 31);
+  return true;
+}
+
 // The cell lists of one structure in shared memory (block-wide): atoms
 // wrapped and binned (wrap_bin_atom), counted per cell with shared-memory
 // atomics, the counts scanned (scs[c] = first entry of cell c, scs[ncell] =
@@ -740,6 +915,7 @@ __global__ void __launch_bounds__(256, NB_STRUCT_BLOCKS)
   int* satoms = reinterpret_cast<int*>(spos + nb.smem_atoms);
   int* scs = satoms + nb.smem_atoms;      // [ncell + 1]: counts, then offsets
   int* sbin = scs + nb.smem_cells + 1;    // per atom: cell | rank << 16
+  if (struct_all<T4>(g, pos, types, nb, spos, su_sh[warp])) return;
   struct_cells(g, pos, types, nb, spos, satoms, scs, sbin, s_wt);
   const CellSrc src{scs, spos, satoms, 0};
   for (int a = warp; a < n; a += (blockDim.x >> 5))
@@ -1600,6 +1776,7 @@ __global__ void __launch_bounds__(256, NB_STRUCT_HALF_BLOCKS)
   int* scs = satoms + nb.smem_atoms;
   int* sbin = scs + nb.smem_cells + 1;
   int* scnt = sbin + nb.smem_atoms;       // row counters
+  if (struct_all<T4>(g, pos, types, nb, spos, su_sh[warp])) return;
   for (int q = threadIdx.x; q < n; q += blockDim.x) scnt[q] = 0;
   struct_cells(g, pos, types, nb, spos, satoms, scs, sbin, s_wt);
   for (int a = warp; a < n; a += (blockDim.x >> 5))
@@ -1711,6 +1888,15 @@ bool ae_cells_one(int natoms, int ncells) {
 int ae_launch_neighbors(int natoms, const double* pos, const int* types, const NbBuffers& nb,
                         int fp64, cudaStream_t s) {
   if (natoms <= 0) return 0;
+  if (nb.all_pairs) {
+    k_wrap_bin<<<(natoms + WRAP_B - 1) / WRAP_B, WRAP_B, 0, s>>>(natoms, pos, types, nb, 1);
+    if (nb.ev_search) cudaEventRecord(nb.ev_search, s);
+    if (fp64)
+      k_neighbors_all<double4_32a><<<(natoms + 7) / 8, 256, 0, s>>>(natoms, nb);
+    else
+      k_neighbors_all<float4><<<(natoms + 7) / 8, 256, 0, s>>>(natoms, nb);
+    return (int)cudaGetLastError();
+  }
   if (nb.cell_kernel == 5 && nb.struct_order) {
     // half stencil, cell lists and row counters inside the search blocks
     if (nb.ev_search) cudaEventRecord(nb.ev_search, s);
