@@ -976,7 +976,7 @@ struct aenet_gpu_plan {
   // training workspace, allocated by the first loss/gradient call
   void* tmem = nullptr;
   double* cE = nullptr;       // [nstruc] dL/dE coefficients
-  double* loss_s = nullptr;   // [nstruc]
+  double* loss_part = nullptr;   // [AE_LOSS_BLOCKS]
   void* U = nullptr;          // [N] T4 dL/dF
   double* partial = nullptr;  // per-block weight-gradient rows
   ~aenet_gpu_plan() {
@@ -1464,14 +1464,21 @@ NbBuffers search_buffers(aenet_gpu_plan* P, bool* grouped) {
 int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s,
               bool zero_F = false, bool grouped = false);
 
+// the networks' kernel takes the atoms grouped by species (plan_networks sees
+// to it)
+bool networks_order(const aenet_gpu_plan* P) { return !P->fp64 && P->pd->tc_ok && g.networks_tc; }
+
 // neighbours + descriptors + networks + energies
-// (zero_F: an adjoint follows in the same call; the descriptor kernel clears
+// (ordered: whether P->order and P->spec_off are the atoms grouped by species
+// afterwards;
+// zero_F: an adjoint follows in the same call; the descriptor kernel clears
 // its force accumulator, one memset less)
 int plan_forward(aenet_gpu_plan* P, const double* d_coords, const int* d_types, double* d_E,
-                 double* d_E_atoms, cudaStream_t s, bool zero_F = false) {
+                 double* d_E_atoms, cudaStream_t s, bool zero_F = false, bool* ordered = nullptr) {
   bool grouped;
   const NbBuffers nb = search_buffers(P, &grouped);
   if (ck(ae_launch_neighbors(P->natoms, d_coords, d_types, nb, P->fp64, s))) return AENET_ERR_CUDA;
+  if (ordered) *ordered = grouped || networks_order(P);
   return plan_eval(P, d_E, d_E_atoms, s, zero_F, grouped);
 }
 
@@ -1480,7 +1487,7 @@ int plan_forward(aenet_gpu_plan* P, const double* d_coords, const int* d_types, 
 // otherwise
 int plan_networks(aenet_gpu_plan* P, const DescBuffers& d, cudaStream_t s, bool grouped = false) {
   const PotDevice& pd = *P->pd;
-  if (!P->fp64 && pd.tc_ok && g.networks_tc) {
+  if (networks_order(P)) {
     if (!grouped && ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
                                P->spec_off, s)))
       return AENET_ERR_CUDA;
@@ -2481,7 +2488,7 @@ int plan_train_alloc(aenet_gpu_plan* P) {
     return o;
   };
   size_t o_ce = take(8 * (size_t)P->nstruc);
-  size_t o_ls = take(8 * (size_t)P->nstruc);
+  size_t o_ls = take(8 * (size_t)AE_LOSS_BLOCKS);
   size_t o_u = take(4 * tsz * N);
   size_t o_p = take(8 * (size_t)pd.ntypes * ae_wgrad_nblk(pd.ntypes) * ae_wgrad_wcap(pd));
   if (cudaMalloc(&P->tmem, off) != cudaSuccess) {
@@ -2490,7 +2497,7 @@ int plan_train_alloc(aenet_gpu_plan* P) {
   }
   char* b = (char*)P->tmem;
   P->cE = (double*)(b + o_ce);
-  P->loss_s = (double*)(b + o_ls);
+  P->loss_part = (double*)(b + o_ls);
   P->U = (void*)(b + o_u);
   P->partial = (double*)(b + o_p);
   if (cudaMemset(P->tmem, 0, off) != cudaSuccess) return AENET_ERR_CUDA;
@@ -2520,15 +2527,16 @@ EXPORT int aenet_gpu_plan_loss_gradient(aenet_gpu_plan* P, const double* d_coord
   int st = plan_train_alloc(P);
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  st = plan_forward(P, d_coords, d_types, d_E, nullptr, s, force_term || d_F);
+  bool ordered = false;
+  st = plan_forward(P, d_coords, d_types, d_E, nullptr, s, force_term || d_F, &ordered);
   if (st) return st;
   if (force_term || d_F) {
     st = plan_adjoint(P, nullptr, d_F, 1.0, nullptr, s, true);
     if (st) return st;
   }
-  if (ck(ae_launch_loss(P->nstruc, P->geom_d, P->E_struct, d_E_target, P->Facc,
+  if (ck(ae_launch_loss(P->nstruc, P->natoms, P->geom_d, P->E_struct, d_E_target, P->Facc,
                         force_term ? d_F_target : nullptr, mode == AENET_GPU_LOSS_ENERGY ? 0 : 1, w_E, w_F, pd.sp[0].E_scale, P->cE,
-                        P->U, P->loss_s, d_loss, P->fp64, s)))
+                        P->U, P->loss_part, d_loss, P->ticket, P->fp64, s)))
     return AENET_ERR_CUDA;
   if (force_term) {
     DescBuffers d = desc_buffers(P, nullptr, false);
@@ -2536,8 +2544,8 @@ EXPORT int aenet_gpu_plan_loss_gradient(aenet_gpu_plan* P, const double* d_coord
     d.V = P->dEdG;   // dE/dG is not needed any more in this pass
     if (ck(ae_launch_chebyshev_tangent(pd, d, P->fp64, s))) return AENET_ERR_CUDA;
   }
-  if (ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
-                             P->spec_off, s)))
+  if (!ordered && ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
+                                         P->spec_off, s)))
     return AENET_ERR_CUDA;
   if (ck(ae_launch_mlp_wgrad(pd, P->order, P->spec_off, P->G, force_term ? P->dEdG : nullptr,
                              P->atom_struct, P->cE, force_term ? -1.0 : 0.0,
@@ -3054,10 +3062,11 @@ EXPORT int aenet_gpu_plan_descriptor_loss_gradient(aenet_gpu_plan* P, const int*
                                          P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
                                          P->ticket, d_E, s)))
     return AENET_ERR_CUDA;
-  if (ck(ae_launch_loss(P->nstruc, P->geom_d, P->E_struct, d_E_target, P->Facc, nullptr, 0, 1.0, 0.0,
-                        pd.sp[0].E_scale, P->cE, P->U, P->loss_s, d_loss, P->fp64, s)) ||
-      ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
-                             P->spec_off, s)) ||
+  if (ck(ae_launch_loss(P->nstruc, P->natoms, P->geom_d, P->E_struct, d_E_target, P->Facc, nullptr, 0, 1.0, 0.0,
+                        pd.sp[0].E_scale, P->cE, P->U, P->loss_part, d_loss, P->ticket, P->fp64, s)) ||
+      (!networks_order(P) &&
+       ck(ae_launch_partition(P->natoms, pd.ntypes, P->types0, P->part_scratch, P->order,
+                              P->spec_off, s))) ||
       ck(ae_launch_mlp_wgrad(pd, P->order, P->spec_off, P->G, nullptr, P->atom_struct, P->cE, 0.0, 0,
                              P->partial, d_grad, P->fp64, s)))
     return AENET_ERR_CUDA;

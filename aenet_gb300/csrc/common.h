@@ -390,10 +390,12 @@ int ae_launch_forces_out(int natoms, const void* Facc, int fp64, double* F,
 int ae_part_scratch_ints(int natoms);
 int ae_launch_partition(int natoms, int ntypes, const int* types0, int* scratch, int* order,
                         int* spec_off, cudaStream_t s);
-int ae_launch_loss(int nstruc, const StructGeom* geom, const double* E_struct, const double* E_tgt,
+// loss_part: [AE_LOSS_BLOCKS] scratch; ticket as above
+#define AE_LOSS_BLOCKS 152
+int ae_launch_loss(int nstruc, int natoms, const StructGeom* geom, const double* E_struct, const double* E_tgt,
                    const void* Facc, const double* F_tgt, int mode, double wE, double wF,
-                   double E_scale, double* cE, void* U, double* loss_s, double* loss, int fp64,
-                   cudaStream_t s);
+                   double E_scale, double* cE, void* U, double* loss_part, double* loss,
+                   unsigned* ticket, int fp64, cudaStream_t s);
 int ae_wgrad_wcap(const PotDevice& pd);
 int ae_wgrad_nblk(int ntypes);
 int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_off, const void* G,

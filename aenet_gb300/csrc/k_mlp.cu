@@ -299,7 +299,14 @@ __global__ void k_energy_warp(int nstruc, const StructGeom* __restrict__ geom,
   const int n = geom[sidx].natoms;
   const double* E = E_atom + geom[sidx].atom_off;
   double s = 0.0;
-  for (int a = lane; a < n; a += 32) s += E[a];
+  for (int a = lane; a < n; a += 256) {
+    double e[8];   // eight loads in flight
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e[q] = a + 32 * q < n ? E[a + 32 * q] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (a + 32 * q < n) s += e[q];
+  }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
   if (lane == 0) {
@@ -512,7 +519,7 @@ int ae_launch_energy_reduce_chunked(int nstruc, int nchunks, const StructGeom* g
   // one structure takes the blocks at any size (a block sums 256 atoms at a
   // time, a warp 32)
   if (one_chunk_each && nstruc > 1)
-    k_energy_warp<<<(nstruc + 7) / 8, 256, 0, s>>>(nstruc, geom, E_atom, E_struct, E_out);
+    k_energy_warp<<<(nstruc + 1) / 2, 64, 0, s>>>(nstruc, geom, E_atom, E_struct, E_out);
   else
     k_energy_blocks<<<nchunks > 0 ? nchunks : 1, 256, 0, s>>>(nstruc, nchunks, geom, chunk_struct,
                                                              E_atom, part, E_struct, E_out, ticket);

@@ -171,48 +171,18 @@ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e
   e = (a - (s - bb)) + (b - bb);
 }
 
-// one warp per structure
-template <typename T>
-__global__ void k_loss(int nstruc, const StructGeom* __restrict__ geom,
-                       const double* __restrict__ E_struct, const double* __restrict__ E_tgt,
-                       const void* __restrict__ Facc, const double* __restrict__ F_tgt, int mode,
-                       double wE, double wF, double E_scale, double* __restrict__ cE,
-                       void* __restrict__ U, double* __restrict__ loss_s) {
-  using T4 = typename Vec4<T>::type;
-  const int lane = threadIdx.x & 31;
-  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (s >= nstruc) return;
-  const int n = geom[s].natoms, off = geom[s].atom_off;
-  const double dn = (double)n;
-  double lossE, ce;
-  if (mode == 0) {
-    const double dE = (E_tgt[s] - E_struct[s]) / (E_scale * dn);
-    lossE = 0.5 * dE * dE;
-    ce = -dE / dn;
-  } else {
-    const double r = E_struct[s] - E_tgt[s];
-    lossE = wE * r * r / (dn * dn);
-    ce = 2.0 * wE * r / (dn * dn);
-  }
-  double acc = 0.0, comp = 0.0;
-  if (mode == 1 && F_tgt) {
-    const T4* F = reinterpret_cast<const T4*>(Facc);
-    T4* Uo = reinterpret_cast<T4*>(U);
-    for (int a = lane; a < n; a += 32) {
-      const T4 f = F[off + a];
-      const double* ft = F_tgt + 3 * (size_t)(off + a);
-      const double rx = (double)f.x - ft[0], ry = (double)f.y - ft[1], rz = (double)f.z - ft[2];
-      double t, e;
-      two_sum(acc, wF * (rx * rx + ry * ry + rz * rz), t, e);
-      acc = t;
-      comp += e;
-      T4 u;
-      u.x = T(2.0 * wF * rx);
-      u.y = T(2.0 * wF * ry);
-      u.z = T(2.0 * wF * rz);
-      u.w = T(0);
-      Uo[off + a] = u;
-    }
+// compensated sum of the block's (acc, comp) pairs, in lane 0 of warp 0
+constexpr int LOSS_B = 256;
+__device__ __forceinline__ double loss_total(double acc, double comp, double* sh, double* sc) {
+  sh[threadIdx.x] = acc;
+  sc[threadIdx.x] = comp;
+  __syncthreads();
+  if (threadIdx.x >= 32) return 0.0;
+  for (int q = threadIdx.x + 32; q < LOSS_B; q += 32) {
+    double t, e;
+    two_sum(acc, sh[q], t, e);
+    acc = t;
+    comp += sc[q] + e;
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
@@ -223,35 +193,79 @@ __global__ void k_loss(int nstruc, const StructGeom* __restrict__ geom,
     acc = t;
     comp = comp + co + e;
   }
-  if (lane == 0) {
-    cE[s] = ce;
-    loss_s[s] = lossE + (acc + comp);
-  }
+  return acc + comp;
 }
 
-// deterministic sum of the structure losses (one block)
-__global__ void k_loss_sum(int nstruc, const double* __restrict__ loss_s, double* __restrict__ out) {
-  __shared__ double sh[1024], sc[1024];
-  double s = 0.0, c = 0.0;
-  for (int q = threadIdx.x; q < nstruc; q += blockDim.x) {
+// Only the total of the losses leaves the kernel, so the threads take atoms
+// and structures in turn whatever structure an atom belongs to, and the last
+// block sums the blocks.  Bound by the FP64 pipe (26 instructions an atom,
+// half of them the compensated sum) and the chains of the two folds.  512
+// Li/Si/O structures (72,500 atoms), a warp per structure and the total in a
+// launch of its own -> like this: 39.8 -> 16.8 us.
+template <typename T>
+__global__ void __launch_bounds__(LOSS_B)
+    k_loss(int nstruc, int natoms, const StructGeom* __restrict__ geom,
+           const double* __restrict__ E_struct, const double* __restrict__ E_tgt,
+           const void* __restrict__ Facc, const double* __restrict__ F_tgt, int mode, double wE,
+           double wF, double E_scale, double* __restrict__ cE, void* __restrict__ U,
+           double* loss_part, double* __restrict__ loss, unsigned* ticket) {
+  using T4 = typename Vec4<T>::type;
+  __shared__ double sh[LOSS_B], sc[LOSS_B];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, step = gridDim.x * LOSS_B;
+  double acc = 0.0, comp = 0.0;
+  auto add = [&](double x) {
     double t, e;
-    two_sum(s, loss_s[q], t, e);
-    s = t;
-    c += e;
-  }
-  sh[threadIdx.x] = s;
-  sc[threadIdx.x] = c;
-  __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) {
-      double t, e;
-      two_sum(sh[threadIdx.x], sh[threadIdx.x + h], t, e);
-      sh[threadIdx.x] = t;
-      sc[threadIdx.x] += sc[threadIdx.x + h] + e;
+    two_sum(acc, x, t, e);
+    acc = t;
+    comp += e;
+  };
+  // (a few structures in each block: their divisions are long)
+  for (int s = tid * gridDim.x + blockIdx.x; s < nstruc; s += step) {
+    const double dn = (double)geom[s].natoms;
+    if (mode == 0) {
+      const double dE = (E_tgt[s] - E_struct[s]) / (E_scale * dn);
+      add(0.5 * dE * dE);
+      cE[s] = -dE / dn;
+    } else {
+      const double r = E_struct[s] - E_tgt[s];
+      add(wE * r * r / (dn * dn));
+      cE[s] = 2.0 * wE * r / (dn * dn);
     }
-    __syncthreads();
   }
-  if (threadIdx.x == 0) out[0] = sh[0] + sc[0];
+  if (mode == 1 && F_tgt) {
+    const T4* F = reinterpret_cast<const T4*>(Facc);
+    T4* Uo = reinterpret_cast<T4*>(U);
+    for (int a = blockIdx.x * LOSS_B + tid; a < natoms; a += step) {
+      const T4 f = F[a];
+      const double* ft = F_tgt + 3 * (size_t)a;
+      const double rx = (double)f.x - ft[0], ry = (double)f.y - ft[1], rz = (double)f.z - ft[2];
+      add(wF * (rx * rx + ry * ry + rz * rz));
+      T4 u;
+      u.x = T(2.0 * wF * rx);
+      u.y = T(2.0 * wF * ry);
+      u.z = T(2.0 * wF * rz);
+      u.w = T(0);
+      Uo[a] = u;
+    }
+  }
+  const double mine = loss_total(acc, comp, sh, sc);
+  if (tid == 0) {
+    loss_part[blockIdx.x] = mine;
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const volatile double* part = loss_part;
+  acc = comp = 0.0;
+  for (int q = tid; q < (int)gridDim.x; q += LOSS_B) add(part[q]);
+  const double total = loss_total(acc, comp, sh, sc);
+  if (tid == 0) {
+    loss[0] = total;
+    *ticket = 0u;
+  }
 }
 
 // ----------------------------------------------------------------------
@@ -301,10 +315,41 @@ struct WgradArgs {
   const double* cE;        // per structure coefficient of y
   double cF;               // coefficient of ydot
   int physical;            // multiply both by the species' E_scale
-  double* partial;         // [ntypes][gridDim.x][wcap]
+  double* partial;         // [gridDim.x][wcap]
   int wcap;                // row length of partial (>= every species' layout size)
   int tile;                // atoms per tile
 };
+
+// First of the `rows` blocks (and rows of partial gradients) of species
+// t < ntypes.  One block for every species, the others in
+// proportion to the atoms: the species with the most atoms would keep its
+// blocks busy longest.
+__device__ __forceinline__ int wgrad_first(int rows, const int* spec_off, int ntypes, int t) {
+  const long long n = spec_off[ntypes];
+  return t + (n > 0 ? (int)((rows - ntypes) * (long long)spec_off[t] / n) : 0);
+}
+
+// this block's species and its atoms [a0, a1) of that species' `nt`
+struct WgradRange {
+  int t, beg, nt, a0, a1;
+};
+__device__ __forceinline__ WgradRange wgrad_range(const WgradArgs& A) {
+  WgradRange r;
+  const int rows = gridDim.x, b = blockIdx.x;
+  int t = 0, first = 0, next = 0;
+  for (;; ++t) {
+    next = t + 1 < A.ntypes ? wgrad_first(rows, A.spec_off, A.ntypes, t + 1) : rows;
+    if (b < next || t + 1 == A.ntypes) break;
+    first = next;
+  }
+  r.t = t;
+  r.beg = A.spec_off[t];
+  r.nt = A.spec_off[t + 1] - r.beg;
+  const int per = (r.nt + next - first - 1) / (next - first);
+  r.a0 = min(r.nt, (b - first) * per);
+  r.a1 = min(r.nt, r.a0 + per);
+  return r;
+}
 
 // shared-memory layout of one block (elements of T)
 struct WgLayout {
@@ -350,7 +395,8 @@ template <> __device__ __forceinline__ const double* wsrc<double>(const PotDevic
 template <typename T, bool TANG>
 __global__ void __launch_bounds__(256) k_mlp_wgrad(PotDevice pd, WgradArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int t = blockIdx.y;
+  const WgradRange range = wgrad_range(A);
+  const int t = range.t;
   const NetTable& net = pd.sp[t].net;
   const int L = net.nlayers;
   __shared__ WgLayout lay;   // indexed by layer at run time: keep it out of registers
@@ -368,9 +414,7 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad(PotDevice pd, WgradArgs A) {
     sW[q] = Wg[q];
     sdW[q] = T(0);
   }
-  const int beg = A.spec_off[t], nt = A.spec_off[t + 1] - beg;
-  const int per = (nt + gridDim.x - 1) / gridDim.x;
-  const int a0 = min(nt, blockIdx.x * per), a1 = min(nt, a0 + per);
+  const int beg = range.beg, a0 = range.a0, a1 = range.a1;
   const T kappa = A.physical ? T(pd.sp[t].E_scale) : T(1);
   const int nsf_pad = pd.nsf_pad;
   __syncthreads();
@@ -490,7 +534,7 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad(PotDevice pd, WgradArgs A) {
     }
     __syncthreads();
   }
-  double* out = A.partial + ((size_t)t * gridDim.x + blockIdx.x) * A.wcap;
+  double* out = A.partial + (size_t)blockIdx.x * A.wcap;
   for (int q = threadIdx.x; q < A.wcap; q += blockDim.x) out[q] = q < lay.wsz ? (double)sdW[q] : 0.0;
 }
 
@@ -507,11 +551,21 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad(PotDevice pd, WgradArgs A) {
 // The node adjoints of a hidden layer overwrite its f' and f'' zd rows,
 // which no other thread reads by then.  Padding atoms of the last tile
 // have zero inputs and zero coefficients, so they add nothing.
+//
+// Bound by latency at 12 warps an SM (the tile's rows fill shared memory) and,
+// behind it, by the shared-memory pipe: a 16-byte load of a warp takes four of
+// its cycles, and a 4 x 4 block needs eight of them for 64 multiply-adds.  So
+// the longest thread of each phase counts: the output layer's weights one per
+// thread (as 4 x 4 blocks nine threads did all of it), the values' and the
+// tangents' products in two lanes, biases apart (33 inputs made a second round
+// of blocks), blocks shared out to the species by their atoms.  72,500
+// Li/Si/O atoms, 32-32-32-1, with tangents: 137 -> 99.5 us, about 21 us of them
+// multiply-adds.
 constexpr int WT_TN = 32;           // atoms per tile
 constexpr int WT_P = WT_TN + 4;     // row pitch: 16-byte rows, successive rows 4 banks apart
 constexpr int WT_THREADS = 128;
 static_assert(WT_THREADS == 4 * WT_TN, "the output node takes four threads per atom");
-constexpr int WT_PF = 8;            // inputs per thread and array held for the next tile
+constexpr int WT_PF = 2;            // input quadruples per thread and array held for the next tile
 
 struct WtLayout {
   int L;
@@ -597,7 +651,8 @@ __device__ __forceinline__ void ld2(const double* p, double (&v)[2]) {
 template <typename T, bool TANG>
 __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, WgradArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int t = blockIdx.y;
+  const WgradRange range = wgrad_range(A);
+  const int t = range.t;
   const NetTable& net = pd.sp[t].net;
   __shared__ WtLayout lay;   // indexed by layer at run time: keep it out of registers
   if (threadIdx.x == 0) lay = wt_layout(net, TANG);
@@ -608,22 +663,28 @@ __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, 
   T* sdW = S + lay.wend;
   const int wbeg = net.w_off[0];
   const T* Wg = wsrc<T>(pd) + wbeg;
-  for (int q = tid; q < lay.wend + lay.wsz; q += WT_THREADS) S[q] = T(0);
+  for (int q = 4 * tid; q < lay.wend + lay.wsz; q += 4 * WT_THREADS) {
+    if (q + 4 <= lay.wend + lay.wsz) {
+      const T zero[4] = {T(0), T(0), T(0), T(0)};
+      st4(S + q, zero);
+    } else {
+      for (int e = q; e < lay.wend + lay.wsz; ++e) S[e] = T(0);
+    }
+  }
   __syncthreads();
+  const int lane = tid & 31, warp = tid >> 5;
   for (int l = 0; l + 1 < L; ++l) {
     const int nin = net.nnodes[l], nout = net.nnodes[l + 1], pitch = net.pitch[l];
     const T* Wl = Wg + (net.w_off[l] - wbeg);
-    for (int q = tid; q < nout * (nin + 1); q += WT_THREADS) {
-      const int o = q / (nin + 1), k = q - o * (nin + 1);
-      const T v = Wl[o * pitch + k];
-      S[lay.wr[l] + o * lay.pr[l] + k] = v;
-      S[lay.wt[l] + k * lay.pt[l] + o] = v;
-    }
+    for (int o = warp; o < nout; o += WT_THREADS / 32)
+      for (int k = lane; k <= nin; k += 32) {
+        const T v = Wl[o * pitch + k];
+        S[lay.wr[l] + o * lay.pr[l] + k] = v;
+        S[lay.wt[l] + k * lay.pt[l] + o] = v;
+      }
     for (int r = tid; r < WT_P; r += WT_THREADS) S[(lay.x[l] + nin) * WT_P + r] = T(1);
   }
-  const int beg = A.spec_off[t], nt = A.spec_off[t + 1] - beg;
-  const int per = (nt + gridDim.x - 1) / gridDim.x;
-  const int a0 = min(nt, blockIdx.x * per), a1 = min(nt, a0 + per);
+  const int beg = range.beg, a0 = range.a0, a1 = range.a1;
   const T kappa = A.physical ? T(pd.sp[t].E_scale) : T(1);
   const int nsf_pad = pd.nsf_pad;
   const int n0 = net.nnodes[0];
@@ -635,18 +696,23 @@ __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, 
   // inputs of a tile (zero rows past its atoms) and the energy coefficients;
   // with few enough features the next tile's are loaded into registers
   // while the current tile is processed
-  const bool pf = WT_TN * n0 <= WT_PF * WT_THREADS;
-  T pg[WT_PF], pv[WT_PF], pce = T(0);
+  const bool pf = WT_TN * n0 <= 4 * WT_PF * WT_THREADS && (nsf_pad & 3) == 0;
+  // atom and first quadruple of this thread: two neighbouring lanes read a
+  // sector, and the sixteen atoms of a warp are stored without conflicts
+  const int fr = (tid >> 1) & (WT_TN - 1), fc = (tid & 1) + 2 * (tid >> 6);
+  constexpr int FSTEP = WT_THREADS / WT_TN;
+  T pg[WT_PF][4], pv[WT_PF][4], pce = T(0);
   auto fetch = [&](int tb1) {
     const int tn1 = min(WT_TN, a1 - tb1);
+    const size_t i = fr < tn1 ? (size_t)A.order[beg + tb1 + fr] : 0;
 #pragma unroll
     for (int j = 0; j < WT_PF; ++j) {
-      const int q = tid + j * WT_THREADS, r = q / n0, k = q - r * n0;
-      pg[j] = pv[j] = T(0);
-      if (q < WT_TN * n0 && r < tn1) {
-        const size_t i = (size_t)A.order[beg + tb1 + r];
-        pg[j] = Gin[i * nsf_pad + k];
-        if (TANG) pv[j] = Vin[i * nsf_pad + k];
+      const int k = 4 * (fc + j * FSTEP);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) pg[j][e] = pv[j][e] = T(0);
+      if (fr < tn1 && k < n0) {
+        ld4(Gin + i * nsf_pad + k, pg[j]);
+        if (TANG) ld4(Vin + i * nsf_pad + k, pv[j]);
       }
     }
     if (tid < WT_TN) pce = tid < tn1 ? kappa * T(A.cE[A.atom_struct[A.order[beg + tb1 + tid]]]) : T(0);
@@ -659,11 +725,13 @@ __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, 
     if (pf) {
 #pragma unroll
       for (int j = 0; j < WT_PF; ++j) {
-        const int q = tid + j * WT_THREADS, r = q / n0, k = q - r * n0;
-        if (q < WT_TN * n0) {
-          S[(lay.x[0] + k) * WT_P + r] = pg[j];
-          if (TANG) S[(lay.xd[0] + k) * WT_P + r] = pv[j];
-        }
+        const int k = 4 * (fc + j * FSTEP);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (k + e < n0) {
+            S[(lay.x[0] + k + e) * WT_P + fr] = pg[j][e];
+            if (TANG) S[(lay.xd[0] + k + e) * WT_P + fr] = pv[j][e];
+          }
       }
       if (tid < WT_TN) CE[tid] = pce;
       if (tb + WT_TN < a1) fetch(tb + WT_TN);
@@ -774,13 +842,41 @@ __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, 
       const T* ZDB = l == L - 2 ? ZDBo : S + lay.s2[l + 1] * WT_P;
       const T* X = S + lay.x[l] * WT_P;
       const T* Xd = S + lay.xd[l] * WT_P;
-      {
-        // 4 nodes x 4 inputs per thread; the inputs of one thread are kn
-        // apart so that neighbouring lanes read neighbouring rows (banks)
-        const int kn = (nin + 1 + 3) / 4;
-        const int items = ((nout + 3) / 4) * kn;
-        T* dWl = sdW + (net.w_off[l] - wbeg);
-        for (int it = tid; it < items; it += WT_THREADS) {
+      T* dWl = sdW + (net.w_off[l] - wbeg);
+      if (nout < 4) {
+        // (the output layer) one weight per thread
+        for (int it = tid; it < nout * (nin + 1); it += WT_THREADS) {
+          const int o = it / (nin + 1), k = it - o * (nin + 1);
+          T acc = T(0);
+#pragma unroll 2
+          for (int r = 0; r < WT_TN; r += 4) {
+            T x[4], zb[4];
+            ld4(X + k * WT_P + r, x);
+            ld4(ZB + o * WT_P + r, zb);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc = fma(zb[e], x[e], acc);
+            if (TANG) {
+              ld4(Xd + k * WT_P + r, x);
+              ld4(ZDB + o * WT_P + r, zb);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) acc = fma(zb[e], x[e], acc);
+            }
+          }
+          dWl[o * net.pitch[l] + k] += acc;
+        }
+      } else {
+        // 4 nodes x 4 inputs per thread, the values' and the tangents' part
+        // in two lanes, which then take two nodes each; the inputs of one
+        // thread are kn apart so that neighbouring lanes read neighbouring
+        // rows (banks)
+        constexpr int H = TANG ? 2 : 1;
+        const int kn = (nin + 3) / 4;
+        const int items = H * ((nout + 3) / 4) * kn;
+        const int half = TANG ? lane & 1 : 0;
+        const T* Xh = half ? Xd : X;
+        const T* Zh = half ? ZDB : ZB;
+        for (int it0 = warp * 32; it0 < items; it0 += WT_THREADS) {
+          const int it = min(it0 + lane, items - H + half) / H;
           const int o0 = 4 * (it / kn), k0 = it % kn;
           int orow[4], krow[4];
 #pragma unroll
@@ -797,36 +893,41 @@ __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, 
           for (int r = 0; r < WT_TN; r += 4) {
             T x[4][4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) ld4(X + krow[c] + r, x[c]);
+            for (int c = 0; c < 4; ++c) ld4(Xh + krow[c] + r, x[c]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               T zb[4];
-              ld4(ZB + orow[j] + r, zb);
+              ld4(Zh + orow[j] + r, zb);
 #pragma unroll
               for (int c = 0; c < 4; ++c)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[j][c] = fma(zb[e], x[c][e], acc[j][c]);
             }
-            if (TANG) {
-#pragma unroll
-              for (int c = 0; c < 4; ++c) ld4(Xd + krow[c] + r, x[c]);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                T zb[4];
-                ld4(ZDB + orow[j] + r, zb);
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) acc[j][c] = fma(zb[e], x[c][e], acc[j][c]);
-              }
-            }
           }
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
+          for (int j = 0; j < 4 / H; ++j)
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (o0 + j < nout && k0 + c * kn <= nin)
-                dWl[(o0 + j) * net.pitch[l] + k0 + c * kn] += acc[j][c];
+            for (int c = 0; c < 4; ++c) {
+              T v = acc[j][c];
+              if (TANG) {
+                const T give = half ? acc[j][c] : acc[j + 2][c];
+                v = (half ? acc[j + 2][c] : acc[j][c]) + __shfl_xor_sync(0xffffffffu, give, 1);
+              }
+              const int o = o0 + j + 2 * half;
+              if (it0 + lane < items && o < nout && k0 + c * kn < nin)
+                dWl[o * net.pitch[l] + k0 + c * kn] += v;
+            }
+        }
+        // biases (the tangent of the row of ones is zero)
+        for (int o = tid; o < nout; o += WT_THREADS) {
+          T acc = T(0);
+#pragma unroll 2
+          for (int r = 0; r < WT_TN; r += 4) {
+            T zb[4];
+            ld4(ZB + o * WT_P + r, zb);
+            acc += (zb[0] + zb[1]) + (zb[2] + zb[3]);
+          }
+          dWl[o * net.pitch[l] + nin] += acc;
         }
       }
       if (l >= 1) {
@@ -884,17 +985,38 @@ __global__ void __launch_bounds__(WT_THREADS, 3) k_mlp_wgrad_tile(PotDevice pd, 
       __syncthreads();
     }
   }
-  double* out = A.partial + ((size_t)t * gridDim.x + blockIdx.x) * A.wcap;
+  double* out = A.partial + (size_t)blockIdx.x * A.wcap;
   for (int q = tid; q < A.wcap; q += WT_THREADS) out[q] = q < lay.wsz ? (double)sdW[q] : 0.0;
 }
 
 // sum the block partials (in block order) and write the gradient in the
 // reference's W order: per species, per layer, column-major (nout, nin+1)
 // with the bias in the last column (feedforward.f90:55-89)
-__global__ void k_wgrad_reduce(PotDevice pd, int nblk, int wcap, const double* __restrict__ partial,
-                               double* __restrict__ grad) {
+// A block takes WR_W weights of one species; each of its warps sums every
+// eighth row, so that the rows' loads of a weight are in flight together and
+// the FP64 sums (152 rows a weight) spread over all SMs.  Three species of
+// 2,145 weights, a thread per weight -> like this: 26.5 -> 9.8 us.
+constexpr int WR_W = 32, WR_SPLIT = 8;
+__global__ void __launch_bounds__(WR_W * WR_SPLIT) k_wgrad_reduce(
+    PotDevice pd, int rows, int wcap, const int* __restrict__ spec_off,
+    const double* __restrict__ partial, double* __restrict__ grad) {
+  __shared__ double part[WR_SPLIT][WR_W];
   const int t = blockIdx.y;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int w = threadIdx.x >> 5;
+  const int q = blockIdx.x * WR_W + (threadIdx.x & 31);
+  {
+    const int b0 = wgrad_first(rows, spec_off, pd.ntypes, t);
+    const int b1 = t + 1 < pd.ntypes ? wgrad_first(rows, spec_off, pd.ntypes, t + 1) : rows;
+    double s = 0.0;
+    const double* p = partial + q;
+    if (q < wcap) {
+#pragma unroll 4
+      for (int b = b0 + w; b < b1; b += WR_SPLIT) s += p[(size_t)b * wcap];
+    }
+    part[w][threadIdx.x & 31] = s;
+  }
+  __syncthreads();
+  if (w) return;
   const NetTable& net = pd.sp[t].net;
   const int L = net.nlayers;
   const int wbeg = net.w_off[0];
@@ -916,8 +1038,8 @@ __global__ void k_wgrad_reduce(PotDevice pd, int nblk, int wcap, const double* _
   const int nin = net.nnodes[l], nout = net.nnodes[l + 1];
   if (k > nin || o >= nout) return;   // row padding
   double s = 0.0;
-  const double* p = partial + (size_t)t * nblk * wcap + q;
-  for (int b = 0; b < nblk; ++b) s += p[(size_t)b * wcap];
+#pragma unroll
+  for (int v = 0; v < WR_SPLIT; ++v) s += part[v][threadIdx.x];
   grad[ref + o + (size_t)k * nout] = s;
 }
 
@@ -949,20 +1071,18 @@ int ae_launch_partition(int natoms, int ntypes, const int* types0, int* scratch,
   return (int)cudaGetLastError();
 }
 
-int ae_launch_loss(int nstruc, const StructGeom* geom, const double* E_struct, const double* E_tgt,
-                   const void* Facc, const double* F_tgt, int mode, double wE, double wF,
-                   double E_scale, double* cE, void* U, double* loss_s, double* loss, int fp64,
-                   cudaStream_t s) {
-  const int blocks = (nstruc * 32 + 255) / 256;
-  if (nstruc > 0) {
-    if (fp64)
-      k_loss<double><<<blocks, 256, 0, s>>>(nstruc, geom, E_struct, E_tgt, Facc, F_tgt, mode, wE, wF,
-                                            E_scale, cE, U, loss_s);
-    else
-      k_loss<float><<<blocks, 256, 0, s>>>(nstruc, geom, E_struct, E_tgt, Facc, F_tgt, mode, wE, wF,
-                                           E_scale, cE, U, loss_s);
-  }
-  k_loss_sum<<<1, 1024, 0, s>>>(nstruc, loss_s, loss);
+int ae_launch_loss(int nstruc, int natoms, const StructGeom* geom, const double* E_struct,
+                   const double* E_tgt, const void* Facc, const double* F_tgt, int mode, double wE, double wF,
+                   double E_scale, double* cE, void* U, double* loss_part, double* loss,
+                   unsigned* ticket, int fp64, cudaStream_t s) {
+  const int items = mode == 1 && F_tgt ? max(natoms, nstruc) : nstruc;
+  const int blocks = max(1, min(AE_LOSS_BLOCKS, (items + LOSS_B - 1) / LOSS_B));
+  if (fp64)
+    k_loss<double><<<blocks, LOSS_B, 0, s>>>(nstruc, natoms, geom, E_struct, E_tgt, Facc, F_tgt, mode,
+                                             wE, wF, E_scale, cE, U, loss_part, loss, ticket);
+  else
+    k_loss<float><<<blocks, LOSS_B, 0, s>>>(nstruc, natoms, geom, E_struct, E_tgt, Facc, F_tgt, mode,
+                                            wE, wF, E_scale, cE, U, loss_part, loss, ticket);
   return (int)cudaGetLastError();
 }
 
@@ -1002,8 +1122,8 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
   for (int t = 0; t < pd.ntypes; ++t)
     if (pd.sp[t].net.nnodes[pd.sp[t].net.nlayers - 1] != 1 || pd.sp[t].net.nlayers < 2)
       return (int)cudaErrorInvalidValue;
-  dim3 grid(nblk, pd.ntypes);
-  dim3 rgrid((A.wcap + 255) / 256, pd.ntypes);
+  const int rows = nblk * pd.ntypes;   // one block and one partial gradient each
+  dim3 rgrid((A.wcap + WR_W - 1) / WR_W, pd.ntypes);
   // tile kernel when its shared memory fits every species
   size_t tneed = 0;
   for (int t = 0; t < pd.ntypes; ++t) {
@@ -1015,7 +1135,7 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
     auto go_tile = [&](auto kern) {
       if (tneed + AE_STATIC_SMEM > 48 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tneed);
-      kern<<<grid, WT_THREADS, tneed, s>>>(pd, A);
+      kern<<<rows, WT_THREADS, tneed, s>>>(pd, A);
     };
     if (fp64) {
       if (tang) go_tile(k_mlp_wgrad_tile<double, true>);
@@ -1024,7 +1144,7 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
       if (tang) go_tile(k_mlp_wgrad_tile<float, true>);
       else go_tile(k_mlp_wgrad_tile<float, false>);
     }
-    k_wgrad_reduce<<<rgrid, 256, 0, s>>>(pd, nblk, A.wcap, partial, grad);
+    k_wgrad_reduce<<<rgrid, WR_W * WR_SPLIT, 0, s>>>(pd, rows, A.wcap, spec_off, partial, grad);
     return (int)cudaGetLastError();
   }
   // otherwise one warp per atom: the largest tile whose shared memory fits
@@ -1043,7 +1163,7 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
   A.tile = tile;
   auto go = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
-    kern<<<grid, warps * 32, need, s>>>(pd, A);
+    kern<<<rows, warps * 32, need, s>>>(pd, A);
   };
   if (fp64) {
     if (tang) go(k_mlp_wgrad<double, true>);
@@ -1052,6 +1172,6 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
     if (tang) go(k_mlp_wgrad<float, true>);
     else go(k_mlp_wgrad<float, false>);
   }
-  k_wgrad_reduce<<<rgrid, 256, 0, s>>>(pd, nblk, A.wcap, partial, grad);
+  k_wgrad_reduce<<<rgrid, WR_W * WR_SPLIT, 0, s>>>(pd, rows, A.wcap, spec_off, partial, grad);
   return (int)cudaGetLastError();
 }
