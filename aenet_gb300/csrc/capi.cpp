@@ -1785,11 +1785,11 @@ int atomic_eval_fused(const double* coo_i, int type_i, int n_j, const double* co
     if (vec[4 * j + 3] <= a_Rc) ++na;
   }
   const char* ho = h + in_bytes;
-  // one block is as fast for short rows whose pairs fit one round of its
-  // pair threads (a cluster's launch and barriers cost a few
-  // microseconds); the cluster is faster from there (measured on GB300:
-  // 45 vs 53 us at 78 neighbours and 250 pairs, 114 vs 552 us at 300
-  // neighbours)
+  // one block for short rows whose pairs fit one round of its pair threads (a
+  // cluster's launch and barriers cost a few microseconds), the cluster from
+  // there; block and cluster, us a call: Cu rows of 40 neighbours 43.7 and
+  // 49.0, of 78 (153 pairs) 48.9 and 52.6, of 90 (about 860 pairs) 80.1 and
+  // 55.7; Li/Si/O rows of 72 50.8 and 52.8, of 100 86.8 and 57.3
   const bool cluster =
       g.atom_fused == 3 ||
       (g.atom_fused == 2 && (n_j >= AE_ATOM_CLUSTER_ROWS || na * (na - 1) / 2 > AE_ATOM_BLOCK_PAIRS));

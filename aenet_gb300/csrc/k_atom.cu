@@ -13,15 +13,24 @@
 //   forward  warps 0-2 over the neighbours (radial T_n, chebyshev.f90:41-128),
 //            the other warps over the pairs j < k of angular neighbours;
 //            the per-thread sums are reduced column by column through
-//            shared memory, four lanes per feature;
-//   network  eight lanes per node for the sums, one lane per node for the
-//            activations, forward and back (ff_eval / ff_deriv,
-//            src/ext/feedforward.f90:586-757);
+//            shared memory, eight lanes per feature;
+//   network  a few lanes per node for its sum and activation, forward and
+//            back (ff_eval / ff_deriv, src/ext/feedforward.f90:586-757);
 //   adjoint  thread per neighbour (radial, warps 0-2) and per pair
-//            (angular, warps 3-7, at the same time); the
-//            pair gradients of each round are gathered per neighbour in a
+//            (angular, warps 3-7, at the same time); the pairs leave three
+//            numbers each, which four lanes per neighbour gather in a
 //            fixed order; the central atom takes minus the sum of the
 //            neighbour forces (aenet.f90:471-477).
+//
+// Bound by chains of FP64 instructions, of which a scheduler of the SM starts
+// one in 64 cycles: the phases of a row of 78 neighbours and 153 pairs
+// (26-20-20-1) take 7,000 cycles (the row's way from host memory among them),
+// 6,700, 14,500, 13,500 and 2,000 for the output.  Cut-offs as a series in d^2
+// (cutoff64.cuh), constants divided on the host, spin sums only where there
+// are spins, derivatives as sums over q U_(q-1) with the order multiplied
+// into the coefficients once, tanh without branches and pair gradients from
+// sums of scalars instead of two vectors a pair: the kernel 41 -> 30 us, the
+// phases before 7,600, 8,900, 19,000, 27,500 and 2,300 cycles.
 //
 // In the cluster each block stages a contiguous slice of the rows and takes
 // a contiguous slice of the pair index space; the blocks exchange their
@@ -34,18 +43,18 @@
 // one launch and one stream synchronisation.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "common.h"
 #include "activate.cuh"
+#include "cutoff64.cuh"
 #include "k_cheb_impl.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace {
 
-using cheb::angular_arg;
-using cheb::cutoff_a;
 using cheb::PairWalk;
-using cheb::radial_x;
 using cheb::SFB_EPS;
 using cheb::SFB_PI;
 
@@ -58,8 +67,8 @@ constexpr int AT_WARPS = AT_THREADS / 32;
 constexpr int AT_RAD = 96;                    // radial threads (warps 0-2)
 constexpr int AT_ANG = AT_THREADS - AT_RAD;   // pair threads (warps 3-7)
 constexpr int AT_HALF = AT_THREADS / 2;       // rows per staging pass
-constexpr int AT_LPN = 8;                     // lanes per network node
-constexpr int AT_LPF = 4;                     // lanes per feature sum
+constexpr int AT_LPF = 8;                     // lanes per feature sum
+constexpr int AT_LPA = 4;                     // lanes per angular neighbour's gradient
 constexpr int AT_NSTRIDE = AE_MAXNODES + 1;
 constexpr int AC_CTAS = 8;                    // blocks of the cluster form
 constexpr int AT_WMAX = 4096;                 // network weights staged in shared memory
@@ -96,25 +105,69 @@ __device__ __forceinline__ int tri_index(int a, int b, int na) {
   return a * (2 * na - a - 1) / 2 + (b - a - 1);
 }
 
+// constants of the central atom's basis, divided out on the host, and the
+// lanes per node of its network's layers
+struct AtomConst {
+  double two_over_rc, r_a2, a_a2;   // 2 / Rc; (pi / Rc)^2, radial and angular
+  unsigned char fwd[AE_MAXLAYERS], back[AE_MAXLAYERS];
+};
+
+// Lanes per node for sums of n terms over `nodes` nodes, `after` instructions
+// on each sum: the FP64 instructions of the busiest of the four schedulers.
+int node_lanes(int nodes, int n, int after) {
+  int best = 16, cost = 1 << 30;
+  for (int lg = 4; lg >= 1; --lg) {
+    const int k = (((nodes << lg) + 127) >> 7) * (((n + (1 << lg) - 1) >> lg) + lg + after);
+    if (k < cost) {
+      cost = k;
+      best = 1 << lg;
+    }
+  }
+  return best;
+}
+
 // per-call constants of the central atom's basis
 struct AtomCtx {
-  double r_Rc, a_Rc, two_over_rc, r_a, a_a;
+  double r_Rc, a_Rc, two_over_rc, r_a2, a_a2;
   int rN, aN, legacy;
   bool multi;
-  __device__ void init(const ChebTable& ct) {
+  __device__ void init(const ChebTable& ct, const AtomConst& k) {
     r_Rc = ct.r_Rc;
     a_Rc = ct.a_Rc;
-    two_over_rc = 2.0 / r_Rc;
-    r_a = SFB_PI / r_Rc;
-    a_a = SFB_PI / a_Rc;
+    two_over_rc = k.two_over_rc;
+    r_a2 = k.r_a2;
+    a_a2 = k.a_a2;
     rN = ct.r_N;
     aN = ct.a_N;
     legacy = ct.angular_legacy;
     multi = ct.multi;
   }
+  // angular argument, current domain [-1, 1] or legacy (2 cos - pi) / pi
+  __device__ double angular_x(double cosv) const {
+    return legacy ? fma(cosv, 2.0 / SFB_PI, -1.0) : cosv;
+  }
+  __device__ double angular_dx() const { return legacy ? 2.0 / SFB_PI : 1.0; }
 };
 
-// Rows [j0, j1) of the call: sv/sr at j - j0, the angular ones compacted in
+// cosine cut-off and its derivative over d, zero from Rc on (a2 = (pi/Rc)^2)
+__device__ __forceinline__ void cutoff_series(double d, double Rc, double a2, double& fc,
+                                              double& dfc) {
+  const double ad = a2 * d, z = fma(ad, d, -FC_Y0);
+  fc = d < Rc ? fc_series(z) : 0.0;
+  dfc = d < Rc ? 2.0 * ad * fc_series_d(z) : 0.0;
+}
+
+// 1 / d by Newton's iteration from an FP32 seed
+__device__ __forceinline__ double recip(double d) {
+  float f;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)d));
+  double y = (double)f;
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+
+// Rows [j0, j1) of the call: sv (vector and 1 / d, zero beyond the radial
+// cut-off) and sr (argument, cut-off, its derivative, spin) at j - j0, the angular ones compacted in
 // row order into au/af (slot = the row's index j), amap[j - j0] = the
 // compacted index or -1 (when amap is given).  AT_HALF rows per pass: the
 // first half of the block computes their radial records, the second half
@@ -138,14 +191,16 @@ __device__ int stage_rows(const AtomCtx& c, const ChebTable& ct, const double4_3
       s = c.multi ? (double)ct.spin[t] : 0.0;
       const double d = v.w;
       if (!ang_half) {
-        sv[j - j0] = v;
         double4_32a r;
         r.x = r.y = r.z = 0.0;
         r.w = s;
+        v.w = 0.0;
         if (d <= c.r_Rc && d > SFB_EPS) {
-          cutoff_a(d, c.r_Rc, c.r_a, r.y, r.z);
-          r.x = radial_x(d, c.r_Rc, c.two_over_rc);
+          cutoff_series(d, c.r_Rc, c.r_a2, r.y, r.z);
+          r.x = fma(d, c.two_over_rc, -1.0);
+          v.w = recip(d);
         }
+        sv[j - j0] = v;
         sr[j - j0] = r;
       } else {
         inA = d <= c.a_Rc && d >= SFB_EPS;
@@ -162,13 +217,13 @@ __device__ int stage_rows(const AtomCtx& c, const ChebTable& ct, const double4_3
     }
     const int k = off + __popc(m & ((1u << lane) - 1u));
     if (inA) {
-      const double d = v.w, invd = 1.0 / d;
+      const double d = v.w, invd = recip(d);
       double4_32a u, f;
       u.x = v.x * invd;
       u.y = v.y * invd;
       u.z = v.z * invd;
       u.w = invd;
-      cutoff_a(d, c.a_Rc, c.a_a, f.x, f.y);
+      cutoff_series(d, c.a_Rc, c.a_a2, f.x, f.y);
       f.z = s;
       f.w = (double)j;
       au[k] = u;
@@ -197,55 +252,57 @@ __device__ void forward_sums(const AtomCtx& c, const ChebTable& ct, const double
     double acc[RB], accs[RB];
 #pragma unroll
     for (int q = 0; q < RB; ++q) acc[q] = accs[q] = 0.0;
-    for (int j = tid; j < nl; j += AT_RAD) {
-      const double d = sv[j].w;
-      if (d <= c.r_Rc && d > SFB_EPS) {
+    // (rows beyond the cut-off have fc = 0)
+    auto rows = [&](auto flag) {
+      constexpr bool spin = decltype(flag)::value;
+      for (int j = tid; j < nl; j += AT_RAD) {
         const double4_32a r = sr[j];
-        const double fc = r.y, x = r.x, x2 = x + x, sfc = r.w * fc;
+        const double fc = r.y, x = r.x, x2 = x + x, sfc = spin ? r.w * fc : 0.0;
         double tm1 = 1.0, t0 = x;
         acc[0] += fc;
-        accs[0] += sfc;
+        if (spin) accs[0] += sfc;
 #pragma unroll
         for (int q = 1; q < RB; ++q) {
           if (q < rN) {
             acc[q] = fma(fc, t0, acc[q]);
-            accs[q] = fma(sfc, t0, accs[q]);
+            if (spin) accs[q] = fma(sfc, t0, accs[q]);
             const double tn = fma(x2, t0, -tm1);
             tm1 = t0;
             t0 = tn;
           }
         }
       }
-    }
+    };
+    if (c.multi) rows(std::true_type{});
+    else rows(std::false_type{});
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
       red_r[q * AT_RAD + tid] = acc[q];
-      red_r[(RB + q) * AT_RAD + tid] = accs[q];
+      if (c.multi) red_r[(RB + q) * AT_RAD + tid] = accs[q];
     }
   } else {
     const int p0 = tid - AT_RAD;
     double ang[AB], angs[AB];
 #pragma unroll
     for (int q = 0; q < AB; ++q) ang[q] = angs[q] = 0.0;
-    if (p_lo + p0 < p_hi) {
+    auto pairs = [&](auto flag) {
+      constexpr bool spin = decltype(flag)::value;
       PairWalk pw;
       pw.start(p_lo + p0, na);
       for (int p = p_lo + p0; p < p_hi; p += AT_ANG) {
         const double4_32a ua = au[pw.a], ub = au[pw.b], fa = af[pw.a], fb = af[pw.b];
         const double cosv = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
         const double w = fa.x * fb.x;
-        const double sw = fa.z * fb.z * w;
-        double x, dxdc;
-        angular_arg(cosv, c.legacy, x, dxdc);
-        const double x2 = x + x;
+        const double sw = spin ? fa.z * fb.z * w : 0.0;
+        const double x = c.angular_x(cosv), x2 = x + x;
         double tm1 = 1.0, t0 = x;
         ang[0] += w;
-        angs[0] += sw;
+        if (spin) angs[0] += sw;
 #pragma unroll
         for (int q = 1; q < AB; ++q) {
           if (q < aN) {
             ang[q] = fma(w, t0, ang[q]);
-            angs[q] = fma(sw, t0, angs[q]);
+            if (spin) angs[q] = fma(sw, t0, angs[q]);
             const double tn = fma(x2, t0, -tm1);
             tm1 = t0;
             t0 = tn;
@@ -253,11 +310,15 @@ __device__ void forward_sums(const AtomCtx& c, const ChebTable& ct, const double
         }
         pw.advance(na, AT_ANG);
       }
+    };
+    if (p_lo + p0 < p_hi) {
+      if (c.multi) pairs(std::true_type{});
+      else pairs(std::false_type{});
     }
 #pragma unroll
     for (int q = 0; q < AB; ++q) {
       red_a[q * AT_ANG + p0] = ang[q];
-      red_a[(AB + q) * AT_ANG + p0] = angs[q];
+      if (c.multi) red_a[(AB + q) * AT_ANG + p0] = angs[q];
     }
   }
   __syncthreads();
@@ -266,6 +327,7 @@ __device__ void forward_sums(const AtomCtx& c, const ChebTable& ct, const double
   const int ncol_r = min(nl, AT_RAD), ncol_a = max(0, min(p_hi - p_lo, AT_ANG));
   for (int f0 = 0; f0 < nfr + nfa; f0 += AT_THREADS / AT_LPF) {
     const int f = f0 + tid / AT_LPF, sub = tid % AT_LPF;
+    if (f0 + (tid & ~31) / AT_LPF >= nfr + nfa) continue;   // nothing for this warp
     double sum = 0.0;
     int gk = -1;
     if (f < nfr) {
@@ -280,6 +342,7 @@ __device__ void forward_sums(const AtomCtx& c, const ChebTable& ct, const double
       for (int k = sub; k < ncol_a; k += AT_LPF) sum += col[k];
       gk = (fa < aN ? ct.a_i1 : ct.a_i2) + q;
     }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     if (gk >= 0 && sub == 0) fsum[gk] = sum;
@@ -287,12 +350,42 @@ __device__ void forward_sums(const AtomCtx& c, const ChebTable& ct, const double
   __syncthreads();
 }
 
+__device__ __noinline__ void activate_other(int t, double x, double& y, double& dy) {
+  activate<double>(t, x, y, dy);
+}
+
+// activate<double> with the branch-free tanh
+__device__ __forceinline__ void activate_even(int t, double x, double& y, double& dy) {
+  if (t == 1) {
+    y = tanh_even(x);
+    dy = 1.0 - y * y;
+  } else if (t == 3 || t == 4) {
+    const double a = 1.7159, b = 0.666666666666667, c = t == 4 ? 0.1 : 0.0;
+    const double tb = tanh_even(b * x);
+    y = fma(c, x, a * tb);
+    dy = a * (1.0 - tb * tb) * b + c;
+  } else {
+    activate_other(t, x, y, dy);
+  }
+}
+
+__device__ __forceinline__ double lanes_sum(double v, int lpn) {
+  if (lpn > 8) v += __shfl_xor_sync(0xffffffffu, v, 8);
+  if (lpn > 4) v += __shfl_xor_sync(0xffffffffu, v, 4);
+  if (lpn > 2) v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v + __shfl_xor_sync(0xffffffffu, v, 1);
+}
+
 // Network of species ti on the normalised descriptor G: returns the output
 // node y and leaves dE/dG of the raw descriptor (times E_scale and the
-// normalisation scale) in D.  Block-wide.
+// normalisation scale) in D, and the same times the order of its polynomial in
+// G.  Block-wide.  A warp's FP64 instruction keeps its
+// scheduler's unit for many cycles whatever its lanes do, so the lanes of a
+// node go by node_lanes, warps without nodes take no part, and the activation
+// follows the sum on the lanes that hold it.
 __device__ double atom_network(const PotDevice& pd, const SpeciesTable& sp, int ti,
-                               const double* G, double* D, double* act, double* der,
-                               const double* wsm) {
+                               const AtomConst& kc, double* G, double* D, double* act, double* der,
+                               const double* wsm, double scale0) {
   const int tid = threadIdx.x;
   const NetTable& net = sp.net;
   const int L = net.nlayers;
@@ -309,90 +402,97 @@ __device__ double atom_network(const PotDevice& pd, const SpeciesTable& sp, int 
     double* hout = act + (l + 1) * AT_NSTRIDE;
     double* dout = der + (l + 1) * AT_NSTRIDE;
     const int fa = net.f_a[l + 1];
-    for (int ob = 0; ob < nout; ob += AT_THREADS / AT_LPN) {
-      const int o = ob + tid / AT_LPN, sub = tid % AT_LPN;
+    const int lpn = kc.fwd[l], step = AT_THREADS / lpn;
+    const int sub = tid & (lpn - 1);
+    for (int ob = 0; ob < nout; ob += step) {
+      const int o = ob + tid / lpn;
+      if (ob + (tid & ~31) / lpn >= nout) break;   // (the whole warp)
       double part = 0.0;
       if (o < nout) {
         const double* row = Wl + (size_t)o * pitch;
-        for (int k = sub; k < nin; k += AT_LPN) part = fma(row[k], hin[k], part);
+        if (sub == 0) part = row[nin];
+        for (int k = sub; k < nin; k += lpn) part = fma(row[k], hin[k], part);
       }
-      part += __shfl_xor_sync(0xffffffffu, part, 4);
-      part += __shfl_xor_sync(0xffffffffu, part, 2);
-      part += __shfl_xor_sync(0xffffffffu, part, 1);
-      if (o < nout && sub == 0) hout[o] = part + Wl[(size_t)o * pitch + nin];
-    }
-    __syncthreads();
-    // the activations on the first warp(s), one node per lane
-    for (int o = tid; o < nout; o += AT_THREADS) {
       double y, dy;
-      activate<double>(fa, hout[o], y, dy);
-      hout[o] = y;
-      dout[o] = dy;
+      activate_even(fa, lanes_sum(part, lpn), y, dy);
+      if (o < nout && sub == 0) {
+        hout[o] = y;
+        dout[o] = dy;
+      }
     }
     __syncthreads();
   }
   const double y = act[(L - 1) * AT_NSTRIDE];
   // back: delta_l = (W_l^T delta_{l+1}) f'_l, from the output node down
   const double* delta = der + (L - 1) * AT_NSTRIDE;
+  const size_t nrow = (size_t)ti * pd.nsf_pad;
   for (int l = L - 2; l >= 0; --l) {
     const int nin = net.nnodes[l], nout = net.nnodes[l + 1];
     const double* Wl = layer(l);
     const int pitch = net.pitch[l];
     double* dl = (l == 0) ? D : der + l * AT_NSTRIDE;
-    for (int kb = 0; kb < nin; kb += AT_THREADS / AT_LPN) {
-      const int k = kb + tid / AT_LPN, sub = tid % AT_LPN;
+    const int lpn = kc.back[l], step = AT_THREADS / lpn;
+    const int sub = tid & (lpn - 1);
+    for (int kb = 0; kb < nin; kb += step) {
+      const int k = kb + tid / lpn;
+      if (kb + (tid & ~31) / lpn >= nin) break;
       double part = 0.0;
       if (k < nin)
-        for (int o = sub; o < nout; o += AT_LPN) part = fma(Wl[(size_t)o * pitch + k], delta[o], part);
-      part += __shfl_xor_sync(0xffffffffu, part, 4);
-      part += __shfl_xor_sync(0xffffffffu, part, 2);
-      part += __shfl_xor_sync(0xffffffffu, part, 1);
+        for (int o = sub; o < nout; o += lpn) part = fma(Wl[(size_t)o * pitch + k], delta[o], part);
+      part = lanes_sum(part, lpn);
       if (k < nin && sub == 0) dl[k] = (l > 0) ? part * dl[k] : part;
     }
     __syncthreads();
     delta = dl;
   }
-  const size_t nrow = (size_t)ti * pd.nsf_pad;
-  for (int k = tid; k < sp.nsf; k += AT_THREADS) D[k] = sp.E_scale * D[k] * pd.scale[nrow + k];
+  const ChebTable& ct = sp.cheb;
+  for (int k = tid; k < sp.nsf; k += AT_THREADS) {
+    const double d = sp.E_scale * D[k] * (k == tid ? scale0 : pd.scale[nrow + k]);
+    // feature order: radial, angular and, with several species, both again
+    const int r = k - (k < ct.r_i2 || !ct.multi ? ct.r_i1 : ct.r_i2);
+    const int a = k - (k < ct.a_i2 || !ct.multi ? ct.a_i1 : ct.a_i2);
+    D[k] = d;
+    G[k] = (double)(r >= 0 && r < ct.r_N ? r : a) * d;
+  }
   __syncthreads();
   return y;
 }
 
 // The adjoint: radial part of the force on rows [0, nl) (-c R_ij / d into
-// sF) on warps 0-2 while warps 3-7 take the gradients of the pairs
-// [p_lo, p_hi) on both partners, in rounds of AT_ANG pairs through pbuf,
-// gathered per angular neighbour in a fixed order into aF[3 a] (zeroed
-// here).  Block-wide.
+// sF) on warps 0-2 while warps 3-7 take the pairs [p_lo, p_hi) in rounds of
+// AT_ANG (Dq: D times the order q, T_q' = q U_(q-1)).  With A = sum c_q T_q and B = sum c_q T_q' of a pair (a, b), both
+// symmetric, the gradient on neighbour a is
+//   u_a (fc'_a sum_b fc_b A - sum_b Q cos / d_a) + sum_b Q u_b / d_a,  Q = fc_a fc_b B:
+// a pair leaves three numbers (A, Q, Q cos) in pbuf, and AT_LPA lanes per
+// neighbour sum five over its partners in a fixed order, into aF[3 a] (the
+// vector) and a2[2 a].  Block-wide; aF[3 a] ends as the gradient.
 template <int RB, int AB>
 __device__ void adjoint_rows_pairs(const AtomCtx& c, const ChebTable& ct, const double* D,
-                                   const double4_32a* sv, const double4_32a* sr, int nl,
+                                   const double* Dq, const double4_32a* sv, const double4_32a* sr, int nl,
                                    double* sF, const double4_32a* au, const double4_32a* af,
                                    int na, int p_lo, int p_hi, double* pbuf, double* aF) {
   const int tid = threadIdx.x, rN = c.rN, aN = c.aN;
-  for (int a = tid; a < na; a += AT_THREADS) aF[3 * a] = aF[3 * a + 1] = aF[3 * a + 2] = 0.0;
+  double* a2 = pbuf + 3 * AT_ANG;
+  for (int a = tid; a < na; a += AT_THREADS)
+    aF[3 * a] = aF[3 * a + 1] = aF[3 * a + 2] = a2[2 * a] = a2[2 * a + 1] = 0.0;
   __syncthreads();
   if (tid < AT_RAD) {
-    double gr[RB], grs[RB];
-#pragma unroll
-    for (int q = 0; q < RB; ++q) {
-      gr[q] = q < rN ? D[ct.r_i1 + q] : 0.0;
-      grs[q] = (c.multi && q < rN) ? D[ct.r_i2 + q] : 0.0;
-    }
-    for (int j = tid; j < nl; j += AT_RAD) {
-      const double4_32a v = sv[j];
-      const double d = v.w;
-      double cc = 0.0;
-      if (d <= c.r_Rc && d > SFB_EPS) {
-        const double4_32a r = sr[j];
+    auto rows = [&](auto flag) {
+      constexpr bool spin = decltype(flag)::value;
+      for (int j = tid; j < nl; j += AT_RAD) {
+        const double4_32a v = sv[j], r = sr[j];
         const double fc = r.y, dfc = r.z, s = r.w, x = r.x, x2 = x + x;
+        const double* gr = D + ct.r_i1;
+        const double* grs = D + ct.r_i2;
+        const double* hr = Dq + ct.r_i1;
+        const double* hrs = Dq + ct.r_i2;
         double tm1 = 1.0, t0 = x, um1 = 1.0, u0 = x2;
-        cc = (gr[0] + s * grs[0]) * dfc;
+        double A = spin ? fma(s, grs[0], gr[0]) : gr[0], B = 0.0;
 #pragma unroll
         for (int q = 1; q < RB; ++q) {
           if (q < rN) {
-            const double gq = gr[q] + s * grs[q];
-            const double dT = (double)q * um1 * c.two_over_rc;
-            cc = fma(gq, fma(dfc, t0, fc * dT), cc);
+            A = fma(spin ? fma(s, grs[q], gr[q]) : gr[q], t0, A);
+            B = fma(spin ? fma(s, hrs[q], hr[q]) : hr[q], um1, B);
             const double tn = fma(x2, t0, -tm1);
             tm1 = t0;
             t0 = tn;
@@ -401,93 +501,97 @@ __device__ void adjoint_rows_pairs(const AtomCtx& c, const ChebTable& ct, const 
             u0 = un;
           }
         }
+        const bool in = __double_as_longlong(v.w) != 0;
+        const double cc = in ? fma(dfc, A, fc * c.two_over_rc * B) * v.w : 0.0;
+        sF[3 * j] = -(cc * v.x);
+        sF[3 * j + 1] = -(cc * v.y);
+        sF[3 * j + 2] = -(cc * v.z);
       }
-      const double inv = (d > SFB_EPS && d < 1e29) ? cc / d : 0.0;
-      sF[3 * j] = -(inv * v.x);
-      sF[3 * j + 1] = -(inv * v.y);
-      sF[3 * j + 2] = -(inv * v.z);
-    }
+    };
+    if (c.multi) rows(std::true_type{});
+    else rows(std::false_type{});
   }
   const int pt = tid - AT_RAD;   // pair thread
-  double gav[AB], gasv[AB];
-#pragma unroll
-  for (int q = 0; q < AB; ++q) {
-    gav[q] = q < aN ? D[ct.a_i1 + q] : 0.0;
-    gasv[q] = (c.multi && q < aN) ? D[ct.a_i2 + q] : 0.0;
-  }
   PairWalk pw;
   if (pt >= 0 && p_lo + pt < p_hi) pw.start(p_lo + pt, na);
   for (int P0 = p_lo; P0 < p_hi; P0 += AT_ANG) {
     const int p = P0 + pt;
-    if (pt >= 0) {
-      double g6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      if (p < p_hi) {
-        const double4_32a ua = au[pw.a], uk = au[pw.b], fa = af[pw.a], fk = af[pw.b];
-        const double cosv = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
-        const double w = fa.x * fk.x;
-        const double ss = fa.z * fk.z;
-        double x, dxdc;
-        angular_arg(cosv, c.legacy, x, dxdc);
-        const double x2 = x + x;
-        double tm1 = 1.0, t0 = x, um1 = 1.0, u0 = x2;
-        double Av = fma(ss, gasv[0], gav[0]), Bv = 0.0;
+    auto pair = [&](auto flag) {
+      constexpr bool spin = decltype(flag)::value;
+      const double4_32a ua = au[pw.a], uk = au[pw.b], fa = af[pw.a], fk = af[pw.b];
+      const double cosv = ua.x * uk.x + ua.y * uk.y + ua.z * uk.z;
+      const double w = fa.x * fk.x;
+      const double ss = spin ? fa.z * fk.z : 0.0;
+      const double x = c.angular_x(cosv), x2 = x + x;
+      const double* ga = D + ct.a_i1;
+      const double* gas = D + ct.a_i2;
+      const double* ha = Dq + ct.a_i1;
+      const double* has = Dq + ct.a_i2;
+      double tm1 = 1.0, t0 = x, um1 = 1.0, u0 = x2;
+      double Av = spin ? fma(ss, gas[0], ga[0]) : ga[0], Bv = 0.0;
 #pragma unroll
-        for (int q = 1; q < AB; ++q) {
-          if (q < aN) {
-            const double cq = fma(ss, gasv[q], gav[q]);
-            Av = fma(cq, t0, Av);
-            Bv = fma(cq * (double)q, um1, Bv);
-            const double tn = fma(x2, t0, -tm1);
-            tm1 = t0;
-            t0 = tn;
-            const double un = fma(x2, u0, -um1);
-            um1 = u0;
-            u0 = un;
-          }
+      for (int q = 1; q < AB; ++q) {
+        if (q < aN) {
+          Av = fma(spin ? fma(ss, gas[q], ga[q]) : ga[q], t0, Av);
+          Bv = fma(spin ? fma(ss, has[q], ha[q]) : ha[q], um1, Bv);
+          const double tn = fma(x2, t0, -tm1);
+          tm1 = t0;
+          t0 = tn;
+          const double un = fma(x2, u0, -um1);
+          um1 = u0;
+          u0 = un;
         }
-        const double inva = ua.w, invk = uk.w;
-        const double Bc = w * Bv * dxdc;
-        const double dEda = fa.y * fk.x * Av, ca = Bc * inva;
-        const double dEdk = fa.x * fk.y * Av, ck = Bc * invk;
-        g6[0] = dEda * ua.x + ca * (uk.x - cosv * ua.x);
-        g6[1] = dEda * ua.y + ca * (uk.y - cosv * ua.y);
-        g6[2] = dEda * ua.z + ca * (uk.z - cosv * ua.z);
-        g6[3] = dEdk * uk.x + ck * (ua.x - cosv * uk.x);
-        g6[4] = dEdk * uk.y + ck * (ua.y - cosv * uk.y);
-        g6[5] = dEdk * uk.z + ck * (ua.z - cosv * uk.z);
-        pw.advance(na, AT_ANG);
       }
-#pragma unroll
-      for (int q = 0; q < 6; ++q) pbuf[6 * pt + q] = g6[q];
+      const double Q = w * Bv * c.angular_dx();
+      pbuf[3 * pt] = Av;
+      pbuf[3 * pt + 1] = Q;
+      pbuf[3 * pt + 2] = Q * cosv;
+      pw.advance(na, AT_ANG);
+    };
+    if (pt >= 0 && p < p_hi) {
+      if (c.multi) pair(std::true_type{});
+      else pair(std::false_type{});
     }
     __syncthreads();
     const int P1 = min(p_hi, P0 + AT_ANG);
-    for (int a = tid; a < na; a += AT_THREADS) {
-      double gx = aF[3 * a], gy = aF[3 * a + 1], gz = aF[3 * a + 2];
-      // pairs (c, a), c < a: the gradient on their second partner
-      for (int cc = 0; cc < a; ++cc) {
-        const int q = tri_index(cc, a, na);
-        if (q >= P0 && q < P1) {
-          const double* e = pbuf + 6 * (q - P0) + 3;
-          gx += e[0];
-          gy += e[1];
-          gz += e[2];
+    for (int ab = 0; ab < na; ab += AT_THREADS / AT_LPA) {
+      const int a = ab + tid / AT_LPA, sub = tid % AT_LPA;
+      if (ab + (tid & ~31) / AT_LPA >= na) break;   // (the whole warp)
+      double s1 = 0.0, s2 = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
+      if (a < na)
+        for (int b = sub; b < na; b += AT_LPA) {
+          const int q = a < b ? tri_index(a, b, na) : tri_index(b, a, na);
+          if (b != a && q >= P0 && q < P1) {
+            const double* e = pbuf + 3 * (q - P0);
+            const double4_32a ub = au[b];
+            s1 = fma(af[b].x, e[0], s1);
+            s2 += e[2];
+            vx = fma(e[1], ub.x, vx);
+            vy = fma(e[1], ub.y, vy);
+            vz = fma(e[1], ub.z, vz);
+          }
         }
+      s1 = lanes_sum(s1, AT_LPA);
+      s2 = lanes_sum(s2, AT_LPA);
+      vx = lanes_sum(vx, AT_LPA);
+      vy = lanes_sum(vy, AT_LPA);
+      vz = lanes_sum(vz, AT_LPA);
+      if (a < na && sub == 0) {
+        aF[3 * a] += vx;
+        aF[3 * a + 1] += vy;
+        aF[3 * a + 2] += vz;
+        a2[2 * a] += s1;
+        a2[2 * a + 1] += s2;
       }
-      // pairs (a, b), b > a: consecutive indices, the first partner's
-      const int qa = tri_index(a, a + 1, na);
-      const int lo = max(qa, P0), hi = min(qa + (na - 1 - a), P1);
-      for (int q = lo; q < hi; ++q) {
-        const double* e = pbuf + 6 * (q - P0);
-        gx += e[0];
-        gy += e[1];
-        gz += e[2];
-      }
-      aF[3 * a] = gx;
-      aF[3 * a + 1] = gy;
-      aF[3 * a + 2] = gz;
     }
     __syncthreads();   // pbuf is rewritten by the next round
+  }
+  for (int a = tid; a < na; a += AT_THREADS) {
+    const double4_32a ua = au[a];
+    const double k = fma(af[a].y, a2[2 * a], -(ua.w * a2[2 * a + 1]));
+    aF[3 * a] = fma(k, ua.x, ua.w * aF[3 * a]);
+    aF[3 * a + 1] = fma(k, ua.y, ua.w * aF[3 * a + 1]);
+    aF[3 * a + 2] = fma(k, ua.z, ua.w * aF[3 * a + 2]);
   }
   __syncthreads();
 }
@@ -533,7 +637,7 @@ struct AtomSmem {
 
 template <int RB, int AB>
 __global__ void __launch_bounds__(AT_THREADS, 1)
-    k_atom(PotDevice pd, AtomCallHeader hd, int wcount, const unsigned char* __restrict__ in,
+    k_atom(PotDevice pd, AtomCallHeader hd, AtomConst kc, int wcount, const unsigned char* __restrict__ in,
            unsigned char* __restrict__ out) {
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ int s_wcnt[AT_WARPS];
@@ -545,26 +649,30 @@ __global__ void __launch_bounds__(AT_THREADS, 1)
   const SpeciesTable& sp = pd.sp[ti];
   const ChebTable& ct = sp.cheb;
   AtomCtx c;
-  c.init(ct);
+  c.init(ct, kc);
   AtomSmem sm{};
   sm.carve<RB, AB>(smem_raw, n, pd.nsf_pad, false, wcount);
   stage_weights(sp.net, pd.w64, sm.wsm);
+  // the normalisation of this thread's feature, read while the rows come
+  const size_t nrow = (size_t)ti * pd.nsf_pad;
+  const double shift0 = tid < sp.nsf ? pd.shift[nrow + tid] : 0.0;
+  const double scale0 = tid < sp.nsf ? pd.scale[nrow + tid] : 0.0;
 
   const int na = stage_rows(c, ct, vin, tin, 0, n, sm.sv, sm.sr, sm.au, sm.af, nullptr, s_wcnt);
   const int np = na * (na - 1) / 2;
   forward_sums<RB, AB>(c, ct, sm.sv, sm.sr, n, sm.au, sm.af, na, 0, np, sm.red, sm.fsum);
-  const size_t nrow = (size_t)ti * pd.nsf_pad;
   for (int k = tid; k < sp.nsf; k += AT_THREADS)
-    sm.G[k] = (sm.fsum[k] - pd.shift[nrow + k]) * pd.scale[nrow + k];
+    sm.G[k] = k == tid ? (sm.fsum[k] - shift0) * scale0
+                       : (sm.fsum[k] - pd.shift[nrow + k]) * pd.scale[nrow + k];
   __syncthreads();
-  const double y = atom_network(pd, sp, ti, sm.G, sm.D, sm.act, sm.der, sm.wsm);
+  const double y = atom_network(pd, sp, ti, kc, sm.G, sm.D, sm.act, sm.der, sm.wsm, scale0);
   if (tid == 0) {
     *reinterpret_cast<double*>(out) = sp.E_scale * y + sp.E_shift + sp.E_atom;
     *reinterpret_cast<unsigned*>(out + 8) = 0u;
   }
   if (!hd.forces) return;
 
-  adjoint_rows_pairs<RB, AB>(c, ct, sm.D, sm.sv, sm.sr, n, sm.sF, sm.au, sm.af, na, 0, np, sm.red,
+  adjoint_rows_pairs<RB, AB>(c, ct, sm.D, sm.G, sm.sv, sm.sr, n, sm.sF, sm.au, sm.af, na, 0, np, sm.red,
                              sm.aF);
   for (int a = tid; a < na; a += AT_THREADS) {
     const int slot = (int)sm.af[a].w;
@@ -589,7 +697,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1)
 
 template <int RB, int AB>
 __global__ void __cluster_dims__(AC_CTAS, 1, 1) __launch_bounds__(AT_THREADS, 1)
-    k_atom_cluster(PotDevice pd, AtomCallHeader hd, int wcount,
+    k_atom_cluster(PotDevice pd, AtomCallHeader hd, AtomConst kc, int wcount,
                    const unsigned char* __restrict__ in, unsigned char* __restrict__ out) {
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ int s_wcnt[AT_WARPS];
@@ -604,10 +712,14 @@ __global__ void __cluster_dims__(AC_CTAS, 1, 1) __launch_bounds__(AT_THREADS, 1)
   const SpeciesTable& sp = pd.sp[ti];
   const ChebTable& ct = sp.cheb;
   AtomCtx c;
-  c.init(ct);
+  c.init(ct, kc);
   AtomSmem sm{};
   sm.carve<RB, AB>(smem_raw, n, pd.nsf_pad, true, wcount);
   stage_weights(sp.net, pd.w64, sm.wsm);
+  // the normalisation of this thread's feature, read while the rows come
+  const size_t nrow = (size_t)ti * pd.nsf_pad;
+  const double shift0 = tid < sp.nsf ? pd.shift[nrow + tid] : 0.0;
+  const double scale0 = tid < sp.nsf ? pd.scale[nrow + tid] : 0.0;
   // this block's rows
   const int j0 = (int)((long long)n * rank / AC_CTAS);
   const int j1 = (int)((long long)n * (rank + 1) / AC_CTAS);
@@ -638,21 +750,20 @@ __global__ void __cluster_dims__(AC_CTAS, 1, 1) __launch_bounds__(AT_THREADS, 1)
   forward_sums<RB, AB>(c, ct, sm.sv, sm.sr, nl, sm.au, sm.af, na, p_lo, p_hi, sm.red, sm.fsum);
   cl.sync();
   // the descriptor: every block's partial sums, in block order
-  const size_t nrow = (size_t)ti * pd.nsf_pad;
   for (int k = tid; k < sp.nsf; k += AT_THREADS) {
     double s = 0.0;
     for (int r = 0; r < AC_CTAS; ++r) s += cl.map_shared_rank(sm.fsum, r)[k];
-    sm.G[k] = (s - pd.shift[nrow + k]) * pd.scale[nrow + k];
+    sm.G[k] = k == tid ? (s - shift0) * scale0 : (s - pd.shift[nrow + k]) * pd.scale[nrow + k];
   }
   cl.sync();   // no block reads another's partial sums after this
-  const double y = atom_network(pd, sp, ti, sm.G, sm.D, sm.act, sm.der, sm.wsm);
+  const double y = atom_network(pd, sp, ti, kc, sm.G, sm.D, sm.act, sm.der, sm.wsm, scale0);
   if (rank == 0 && tid == 0) {
     *reinterpret_cast<double*>(out) = sp.E_scale * y + sp.E_shift + sp.E_atom;
     *reinterpret_cast<unsigned*>(out + 8) = 0u;
   }
   if (!hd.forces) return;
 
-  adjoint_rows_pairs<RB, AB>(c, ct, sm.D, sm.sv, sm.sr, nl, sm.sF, sm.au, sm.af, na, p_lo, p_hi,
+  adjoint_rows_pairs<RB, AB>(c, ct, sm.D, sm.G, sm.sv, sm.sr, nl, sm.sF, sm.au, sm.af, na, p_lo, p_hi,
                              sm.red, sm.aF);
   cl.sync();
   // this block's rows: radial part minus every block's angular gradients
@@ -711,6 +822,14 @@ int launch_atom(const PotDevice& pd, const AtomCallHeader& hd, const void* in, v
     smem = at_smem_bytes<RB, AB>(hd.n, pd.nsf_pad, cluster, 0);
   }
   if (smem > 200 * 1024) return AE_ATOM_NA;
+  const ChebTable& ct = pd.sp[hd.ti].cheb;
+  AtomConst kc{2.0 / ct.r_Rc, (SFB_PI / ct.r_Rc) * (SFB_PI / ct.r_Rc),
+               (SFB_PI / ct.a_Rc) * (SFB_PI / ct.a_Rc), {}, {}};
+  const NetTable& net = pd.sp[hd.ti].net;
+  for (int l = 0; l + 1 < net.nlayers; ++l) {
+    kc.fwd[l] = (unsigned char)node_lanes(net.nnodes[l + 1], net.nnodes[l], net.f_a[l + 1] ? 30 : 0);
+    kc.back[l] = (unsigned char)node_lanes(net.nnodes[l], net.nnodes[l + 1], 1);
+  }
   const unsigned char* pin = static_cast<const unsigned char*>(in);
   unsigned char* pout = static_cast<unsigned char*>(out);
   // the opt-in limit is raised once per kernel (callers hold the library
@@ -723,7 +842,7 @@ int launch_atom(const PotDevice& pd, const AtomCallHeader& hd, const void* in, v
       if (e != cudaSuccess) return (int)e;
       opted = true;
     }
-    k_atom_cluster<RB, AB><<<AC_CTAS, AT_THREADS, smem, s>>>(pd, hd, wcount, pin, pout);
+    k_atom_cluster<RB, AB><<<AC_CTAS, AT_THREADS, smem, s>>>(pd, hd, kc, wcount, pin, pout);
   } else {
     static bool opted = false;
     if (!opted) {
@@ -732,7 +851,7 @@ int launch_atom(const PotDevice& pd, const AtomCallHeader& hd, const void* in, v
       if (e != cudaSuccess) return (int)e;
       opted = true;
     }
-    k_atom<RB, AB><<<1, AT_THREADS, smem, s>>>(pd, hd, wcount, pin, pout);
+    k_atom<RB, AB><<<1, AT_THREADS, smem, s>>>(pd, hd, kc, wcount, pin, pout);
   }
   return (int)cudaGetLastError();
 }
