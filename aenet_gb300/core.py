@@ -169,11 +169,12 @@ class ANNPotentials:
     def atomic_energy(self, coo_i, type_i, coo_j, type_j):
         coo_i = _f64(coo_i)
         coo_j = _f64(np.asarray(coo_j).reshape(-1, 3))
-        itype_j = _i32([self.get_type_id(str(t)) for t in type_j])
+        itype_j = self.type_ids(type_j)
         E = C.c_double(0.0)
         stat = C.c_int(0)
-        _lib.lib().aenet_atomic_energy(_ptr(coo_i), self.get_type_id(type_i), len(type_j),
-                                       _ptr(coo_j), _ptr(itype_j), C.byref(E), C.byref(stat))
+        _lib.lib().aenet_atomic_energy(coo_i.ctypes.data, self.get_type_id(type_i), len(type_j),
+                                       coo_j.ctypes.data, itype_j.ctypes.data, C.byref(E),
+                                       C.byref(stat))
         check_status(stat.value)
         return E.value
 
@@ -184,19 +185,24 @@ class ANNPotentials:
             raise TypeError("F must be a C-contiguous float64 array")
         coo_i = _f64(coo_i)
         coo_j = _f64(np.asarray(coo_j).reshape(-1, 3))
-        itype_j = _i32([self.get_type_id(str(t)) for t in type_j])
+        itype_j = self.type_ids(type_j)
         idx_j = _i32(index_j)
         E = C.c_double(0.0)
         stat = C.c_int(0)
         _lib.lib().aenet_atomic_energy_and_forces(
-            _ptr(coo_i), self.get_type_id(type_i), int(index_i), len(type_j), _ptr(coo_j),
-            _ptr(itype_j), _ptr(idx_j), F.shape[0], C.byref(E), _ptr(F), C.byref(stat))
+            coo_i.ctypes.data, self.get_type_id(type_i), int(index_i), len(type_j),
+            coo_j.ctypes.data, itype_j.ctypes.data, idx_j.ctypes.data, F.shape[0], C.byref(E),
+            F.ctypes.data, C.byref(stat))
         check_status(stat.value)
         return E.value
 
     # -------------------------------------------------- whole structures
     def type_ids(self, symbols):
-        return _i32([self.get_type_id(s) for s in symbols])
+        # each distinct symbol is looked up once (a per-atom call of 78
+        # neighbours spent a third of its time here)
+        symbols = [str(s) for s in symbols]
+        ids = {s: self.get_type_id(s) for s in dict.fromkeys(symbols)}
+        return _i32([ids[s] for s in symbols])
 
     def structure_energy_forces(self, positions, symbols_or_types, cell=None, pbc=True,
                                 precision=FP64, forces=True, virial=False):
