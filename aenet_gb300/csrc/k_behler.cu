@@ -42,6 +42,8 @@
 // Adjoint: one-sided -- each pair (j, k) once, its gradient with respect to
 // both neighbours added to per-neighbour accumulators in shared memory;
 // the central atom's force and the virial follow from those sums.
+#include <cmath>
+
 #include "common.h"
 #include "cutoff64.cuh"
 
@@ -348,10 +350,44 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 // e^(-eta x) from rate = -eta (FP64) or -eta log2 e (FP32)
+// exp in FP64 for kernels that the FP64 pipe bounds: x = k ln 2 / 32 + r, |r| <
+// ln 2 / 64, exp x = 2^(k / 32) (1 + r + r^2 (1/2 + ... + r^4 / 720)); the powers
+// of 2^(1/32) from a table (load pipe), the power of two by the exponent bits.
+// Eleven FP64 instructions, within 1 ulp; |x| beyond 700, infinities and NaN
+// go to the library.  750 rutile atoms: forward 481 -> 454 us, adjoint 846 ->
+// 815 us against exp.
+static __device__ const double EXP2_32[32] = {
+    1.0, 1.0218971486541166, 1.0442737824274138, 1.0671404006768237,
+    1.0905077326652577, 1.1143867425958924, 1.1387886347566916, 1.1637248587775775,
+    1.189207115002721, 1.215247359980469, 1.241857812073484, 1.2690509571917332,
+    1.2968395546510096, 1.3252366431597413, 1.3542555469368927, 1.383909881963832,
+    1.4142135623730951, 1.4451808069770467, 1.4768261459394993, 1.5091644275934228,
+    1.5422108254079407, 1.5759808451078865, 1.6104903319492543, 1.645755478153965,
+    1.681792830507429, 1.718619298122478, 1.7562521603732995, 1.7947090750031072,
+    1.8340080864093424, 1.8741676341103, 1.9152065613971474, 1.9571441241754002,
+};
+__device__ __forceinline__ double exp_table(double x) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x4085e000) return exp(x);
+  const double magic = 6755399441055744.0;   // 1.5 * 2^52: rounds to an integer
+  const double kd = fma(x, 46.16624130844683, magic);
+  const int k = __double2loint(kd);
+  const double kf = kd - magic;
+  double r = fma(-kf, 0.02166084937925916, x);   // ln 2 / 32 to 31 bits: exact product
+  r = fma(-kf, 1.3239129268154012e-11, r);
+  double p = fma(r, 1.0 / 720.0, 1.0 / 120.0);
+  p = fma(p, r, 1.0 / 24.0);
+  p = fma(p, r, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(p, r * r, r);
+  const double t = __ldg(EXP2_32 + (k & 31));
+  const double v = fma(t, p, t);   // in (0.98, 2)
+  return __hiloint2double(__double2hiint(v) + ((k >> 5) << 20), __double2loint(v));
+}
+
 __device__ __forceinline__ float decay_rate(float eta) { return -1.4426950408889634f * eta; }
 __device__ __forceinline__ double decay_rate(double eta) { return -eta; }
 __device__ __forceinline__ float decay(float rate, float x) { return ex2_approx(rate * x); }
-__device__ __forceinline__ double decay(double rate, double x) { return exp(rate * x); }
+__device__ __forceinline__ double decay(double rate, double x) { return exp_table(rate * x); }
 template <typename T>
 __device__ __forceinline__ T gval(const double* d, const float* f, int i);
 template <>
@@ -758,16 +794,72 @@ __device__ void forward_generic(const BehlerTable* tab, int f0, int f1e, const P
   }
 }
 
+// The pair lists of a block: all of its atom's, or (SPLIT) the one of number
+// blockIdx.y among the species pairs a <= c, the first with the radial
+// functions.
+template <bool SPLIT>
+struct ListOf {
+  int a, c;   // the one list
+  __device__ __forceinline__ explicit ListOf(int nt) {
+    if (!SPLIT) return;
+    int u = blockIdx.y;
+    a = 0;
+    while (u >= nt - a) u -= nt - a++;
+    c = a + u;
+  }
+  __device__ __forceinline__ bool first() const { return !SPLIT || blockIdx.y == 0; }
+  __device__ __forceinline__ bool list(int x, int y) const { return !SPLIT || (x == a && y == c); }
+  // whether this block sets feature k
+  __device__ __forceinline__ bool mine(const BehlerTable* tab, int nt, int k) const {
+    if (!SPLIT) return true;
+    for (int x = 0; x < nt; ++x)
+      for (int y = x; y < nt; ++y)
+        for (int q = tab->ang_off[x * nt + y]; q < tab->ang_off[x * nt + y + 1]; ++q)
+          if (tab->fn[q].out == k) return list(x, y);
+    return first();
+  }
+  // whether staged neighbour j can have a force from this block
+  __device__ __forceinline__ bool touches(const int* bstart, int j) const {
+    return first() || (j >= bstart[a] && j < bstart[a + 1]) || (j >= bstart[c] && j < bstart[c + 1]);
+  }
+};
+
+// Whether the lists of an atom go to blocks of their own.  One warp takes an
+// atom's lists in turn, as long as four to five (FP64) or many more (mixed)
+// atoms in flight on an SM take together, so a few atoms an SM, or few left
+// over after full SMs, leave it waiting; but every block stages the
+// neighbours anew.  Rutile (three lists), forward and adjoint (us), one block
+// an atom and split:
+//   FP64   72 atoms 403 + 682 and 188 + 310, 270 atoms 402 + 682 and 217 +
+//          389, 750 atoms 454 + 815 and 510 + 901, 1,512 atoms 1,212 + 2,257
+//          and 977 + 1,739, 3,072 atoms 1,837 + 3,419 and 1,857 + 3,301
+//   mixed  72 atoms 69 + 85 and 45 + 44, 750 atoms 70 + 92 and 50 + 55, 1,512
+//          atoms 75 + 102 and 88 + 98, 3,072 atoms 96 + 197 and 137 + 172
+// FP64: in units of an atom's time on a full SM (eight blocks), the last round
+// of fewer takes 4.4 at least, and splitting costs 0.65.
+template <typename T>
+bool split_lists(int natoms, int lists) {
+  if (lists < 2 || lists > 6) return false;
+  int dev = 0, nsm = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const double per = (double)natoms / nsm;
+  if (sizeof(T) == 4) return per <= 7.0;
+  const double full = 8.0 * std::floor(per / 8.0), rest = per - full;
+  return per + 0.65 < full + (rest > 0.0 ? std::fmax(4.4, rest) : 0.0);
+}
+
 // GRID: every angular list is a BehlerGrid (the generic path is left out,
 // which frees its registers).  One warp per block: the warps of a block
 // share nothing, and small blocks spread a few hundred atoms evenly.
-template <typename T, bool GRID>
+template <typename T, bool GRID, bool SPLIT>
 __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_behler_forward(PotDevice pd, DescBuffers b) {
   using T4 = typename V4<T>::type;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   const int lane = threadIdx.x;
   const int i = blockIdx.x;
   const WarpMem<T> w = warp_mem<T>(smem_raw, b.cap, pd.nsf_pad, false);
+  const ListOf<SPLIT> of(pd.ntypes);
   const int ti = b.types[i];
   const BehlerTable* tab = table_of<T>(pd, ti);
   const int nt = pd.ntypes;
@@ -778,7 +870,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_beh
   const int nst = stage_buckets<T>(vec, jt, n, nt, T(tab->rc_max), w.sR, w.sH, w.sslot, bstart,
                                    lane);
   fill_positions(w.sR, w.sP, nst, lane);
-  if (b.zero_F && lane == 0) {
+  if (b.zero_F && lane == 0 && of.first()) {
     T4 z;
     z.x = z.y = z.z = z.w = T(0);
     reinterpret_cast<T4*>(b.F)[i] = z;
@@ -786,13 +878,15 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_beh
   const size_t nrow = (size_t)ti * pd.nsf_pad;
   T* G = reinterpret_cast<T*>(b.G) + (size_t)i * pd.nsf_pad;
   const int nsf = pd.sp[ti].nsf;
-  // features that no function feeds are normalised zeros (symmfunc.f90:367)
-  for (int k = lane; k < nsf; k += 32) G[k] = normalise(T(0), pd, nrow + k);
+  // features that no function feeds are normalised zeros (symmfunc.f90:367);
+  // a block with one list of its own leaves the other lists' alone
+  for (int k = lane; k < nsf; k += 32)
+    if (of.mine(tab, nt, k)) G[k] = normalise(T(0), pd, nrow + k);
   __syncwarp();
 
   // ---- radial lists: function by function, lanes over the bucket's
   // neighbours (a few per lane), warp sum
-  for (int s = 0; s < nt; ++s) {
+  for (int s = 0; s < nt && of.first(); ++s) {
     const int f0 = tab->rad_off[s], f1e = tab->rad_off[s + 1];
     for (int q = f0; q < f1e; ++q) {
       const Fn<T> f = load_fn<T>(&tab->fn[q]);
@@ -814,7 +908,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_beh
   for (int a = 0; a < nt; ++a) {
     for (int c = a; c < nt; ++c) {
       const int f0 = tab->ang_off[a * nt + c], f1e = tab->ang_off[a * nt + c + 1];
-      if (f0 == f1e) continue;
+      if (f0 == f1e || !of.list(a, c)) continue;
       const PairList L = pair_list(bstart, a, c);
       if (empty(L)) continue;
       const int gi = tab->grid_of[a * nt + c];
@@ -1048,13 +1142,14 @@ __device__ void adjoint_generic(const BehlerTable* tab, int f0, int f1e, const P
 // memory (add_pair).  The central atom's gradient is minus the
 // sum over its neighbours (the energy depends on R_j - R_i only), and the
 // atom's virial contribution is -sum_j R_ij (x) dE_i/dR_j.
-template <typename T, bool GRID>
+template <typename T, bool GRID, bool SPLIT>
 __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_behler_adjoint(PotDevice pd, DescBuffers b) {
   using T4 = typename V4<T>::type;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   const int lane = threadIdx.x;
   const int i = blockIdx.x;
   const WarpMem<T> w = warp_mem<T>(smem_raw, b.cap, pd.nsf_pad, true);
+  const ListOf<SPLIT> of(pd.ntypes);
   const int ti = b.types[i];
   const BehlerTable* tab = table_of<T>(pd, ti);
   const int nt = pd.ntypes;
@@ -1079,7 +1174,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_beh
       if (j >= bstart[s + 1]) tj = s + 1;
     const T r = w.sR[j].w;
     const T4 A = w.sH[j];
-    const int f0 = tab->rad_off[tj], f1e = tab->rad_off[tj + 1];
+    const int f0 = tab->rad_off[tj], f1e = of.first() ? tab->rad_off[tj + 1] : f0;
     T c = T(0);
     for (int q = f0; q < f1e; ++q) {
       const Fn<T> f = load_fn<T>(&tab->fn[q]);
@@ -1105,7 +1200,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_beh
   for (int a = 0; a < nt; ++a) {
     for (int c = a; c < nt; ++c) {
       const int f0 = tab->ang_off[a * nt + c], f1e = tab->ang_off[a * nt + c + 1];
-      if (f0 == f1e) continue;
+      if (f0 == f1e || !of.list(a, c)) continue;
       const PairList L = pair_list(bstart, a, c);
       if (empty(L)) continue;
       const int gi = tab->grid_of[a * nt + c];
@@ -1128,6 +1223,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_beh
   T fix = T(0), fiy = T(0), fiz = T(0);
   T w00 = 0, w01 = 0, w02 = 0, w10 = 0, w11 = 0, w12 = 0, w20 = 0, w21 = 0, w22 = 0;
   for (int j = lane; j < nst; j += 32) {
+    if (!of.touches(bstart, j)) continue;
     const T4 Rj = w.sR[j], f = w.sF[j];
     const T gx = fma(f.w, Rj.x, f.x), gy = fma(f.w, Rj.y, f.y), gz = fma(f.w, Rj.z, f.z);
     atomic_add3<T>(F, jt[w.sslot[j]] & AE_INDEX_MASK, -gx, -gy, -gz);
@@ -1160,11 +1256,16 @@ template <typename T>
 int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
   const size_t smem = behler_smem_per_warp<T>(b.cap, pd.nsf_pad, adjoint);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  auto kern = adjoint ? (pd.behler_grid_only ? k_behler_adjoint<T, true> : k_behler_adjoint<T, false>)
-                      : (pd.behler_grid_only ? k_behler_forward<T, true> : k_behler_forward<T, false>);
+  const int lists = pd.ntypes * (pd.ntypes + 1) / 2;
+  const bool split = split_lists<T>(b.natoms, lists), grid = pd.behler_grid_only;
+  auto pick = [&](auto one, auto each) { return split ? each : one; };
+  auto kern = adjoint ? (grid ? pick(k_behler_adjoint<T, true, false>, k_behler_adjoint<T, true, true>)
+                              : pick(k_behler_adjoint<T, false, false>, k_behler_adjoint<T, false, true>))
+                      : (grid ? pick(k_behler_forward<T, true, false>, k_behler_forward<T, true, true>)
+                              : pick(k_behler_forward<T, false, false>, k_behler_forward<T, false, true>));
   if (smem + AE_STATIC_SMEM > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kern<<<b.natoms, 32, smem, s>>>(pd, b);
+  kern<<<dim3(b.natoms, split ? lists : 1), 32, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }
 
