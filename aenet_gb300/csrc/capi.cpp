@@ -1453,7 +1453,8 @@ NbBuffers search_buffers(aenet_gpu_plan* P, bool* grouped) {
   // wide small structures: the default search gives way to the one over all
   // pairs (the per-structure ones do so by themselves)
   nb.all_pairs = P->all_pairs && nb.cell_kernel == 0;
-  *grouped = !per_struct && !nb.all_pairs && P->natoms > 0 && ae_cells_one(P->natoms, P->ncells);
+  *grouped = !per_struct && P->natoms > 0 &&
+             (nb.all_pairs ? P->natoms <= AE_PART_ONE : ae_cells_one(P->natoms, P->ncells));
   if (*grouped) {
     nb.order_out = P->order;
     nb.spec_off_out = P->spec_off;
@@ -1461,8 +1462,21 @@ NbBuffers search_buffers(aenet_gpu_plan* P, bool* grouped) {
   return nb;
 }
 
+EnergySum energy_sum(const aenet_gpu_plan* P, double* d_E) {
+  return EnergySum{P->nstruc, P->nchunks, P->geom_d,   P->chunk_struct, P->E_atom,
+                   P->e_part, P->E_struct, d_E, P->ticket};
+}
+
+// what a pass hands its caller beside the forces, when one launch at its end
+// writes all of it
+struct Results {
+  double* E = nullptr;
+  double* E_atoms = nullptr;
+};
+
+// (energies: false leaves their sums and copies to the pass's last launch)
 int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s,
-              bool zero_F = false, bool grouped = false);
+              bool zero_F = false, bool grouped = false, bool energies = true);
 
 // the networks' kernel takes the atoms grouped by species (plan_networks sees
 // to it)
@@ -1474,12 +1488,13 @@ bool networks_order(const aenet_gpu_plan* P) { return !P->fp64 && P->pd->tc_ok &
 // zero_F: an adjoint follows in the same call; the descriptor kernel clears
 // its force accumulator, one memset less)
 int plan_forward(aenet_gpu_plan* P, const double* d_coords, const int* d_types, double* d_E,
-                 double* d_E_atoms, cudaStream_t s, bool zero_F = false, bool* ordered = nullptr) {
+                 double* d_E_atoms, cudaStream_t s, bool zero_F = false, bool* ordered = nullptr,
+                 bool energies = true) {
   bool grouped;
   const NbBuffers nb = search_buffers(P, &grouped);
   if (ck(ae_launch_neighbors(P->natoms, d_coords, d_types, nb, P->fp64, s))) return AENET_ERR_CUDA;
   if (ordered) *ordered = grouped || networks_order(P);
-  return plan_eval(P, d_E, d_E_atoms, s, zero_F, grouped);
+  return plan_eval(P, d_E, d_E_atoms, s, zero_F, grouped, energies);
 }
 
 // networks: tensor-core kernel on the mixed path when the networks fit it
@@ -1498,7 +1513,7 @@ int plan_networks(aenet_gpu_plan* P, const DescBuffers& d, cudaStream_t s, bool 
 
 // descriptors + networks + energies on the current neighbour table
 int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s, bool zero_F,
-              bool grouped) {
+              bool grouped, bool energies) {
   const PotDevice& pd = *P->pd;
   DescBuffers d = desc_buffers(P, nullptr, false);
   d.zero_F = zero_F ? 1 : 0;
@@ -1510,9 +1525,8 @@ int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s,
                                              : ae_launch_chebyshev_forward(pd, d, P->fp64, s);
   if (ck(e)) return AENET_ERR_CUDA;
   if (plan_networks(P, d, s, grouped)) return AENET_ERR_CUDA;
-  if (ck(ae_launch_energy_reduce_chunked(P->nstruc, P->nchunks, P->geom_d, P->chunk_struct,
-                                         P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
-                                         P->ticket, d_E, s)))
+  if (!energies) return 0;
+  if (ck(ae_launch_energy_reduce_chunked(energy_sum(P, d_E), P->one_chunk_each, s)))
     return AENET_ERR_CUDA;
   if (d_E_atoms &&
       cudaMemcpyAsync(d_E_atoms, P->E_atom, 8 * (size_t)P->natoms, cudaMemcpyDeviceToDevice, s))
@@ -1521,7 +1535,8 @@ int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s,
 }
 
 int plan_adjoint(aenet_gpu_plan* P, const double* grad_scale, double* d_out, double out_sign,
-                 double* d_virial, cudaStream_t s, bool F_zeroed = false) {
+                 double* d_virial, cudaStream_t s, bool F_zeroed = false,
+                 const Results* results = nullptr) {
   const PotDevice& pd = *P->pd;
   const size_t tsz = P->fp64 ? 8 : 4;
   if (!F_zeroed && cudaMemsetAsync(P->Facc, 0, 4 * tsz * (size_t)P->natoms, s)) return AENET_ERR_CUDA;
@@ -1531,8 +1546,13 @@ int plan_adjoint(aenet_gpu_plan* P, const double* grad_scale, double* d_out, dou
   int e = (pd.sp[0].sftype == AE_SF_BEHLER) ? ae_launch_behler_adjoint(pd, d, P->fp64, s)
                                              : ae_launch_chebyshev_adjoint(pd, d, P->fp64, s);
   if (ck(e)) return AENET_ERR_CUDA;
-  if (d_out && ck(ae_launch_forces_out(P->natoms, P->Facc, P->fp64, d_out, out_sign, s)))
+  if (results) {
+    if (ck(ae_launch_results(energy_sum(P, results->E), P->one_chunk_each, P->natoms, P->Facc, P->fp64,
+                             d_out, out_sign, results->E_atoms, s)))
+      return AENET_ERR_CUDA;
+  } else if (d_out && ck(ae_launch_forces_out(P->natoms, P->Facc, P->fp64, d_out, out_sign, s))) {
     return AENET_ERR_CUDA;
+  }
   if (d_virial &&
       cudaMemcpyAsync(d_virial, P->virial, 72 * (size_t)P->nstruc, cudaMemcpyDeviceToDevice, s))
     return AENET_ERR_CUDA;
@@ -2457,10 +2477,11 @@ EXPORT int aenet_gpu_plan_run(aenet_gpu_plan* P, const double* d_coords, const i
   if (!P) return AENET_ERR_INPUT;
   cudaStream_t s = (cudaStream_t)stream;
   const bool adjoint = (flags & (AENET_GPU_FORCES | AENET_GPU_VIRIAL)) || d_F || d_virial;
-  int st = plan_forward(P, d_coords, d_types, d_E, d_E_atoms, s, adjoint);
+  int st = plan_forward(P, d_coords, d_types, d_E, d_E_atoms, s, adjoint, nullptr, !adjoint);
   if (st || !adjoint) return st;
-  return plan_adjoint(P, nullptr, d_F, 1.0, (flags & AENET_GPU_VIRIAL) ? d_virial : nullptr, s,
-                      true);
+  const Results results{d_E, d_E_atoms};
+  return plan_adjoint(P, nullptr, d_F, 1.0, (flags & AENET_GPU_VIRIAL) ? d_virial : nullptr, s, true,
+                      &results);
 }
 
 EXPORT int aenet_gpu_plan_forward(aenet_gpu_plan* P, const double* d_coords, const int* d_types,
@@ -2848,7 +2869,6 @@ struct NlistCtx {
   void* Facc = nullptr;
   double* F = nullptr;
   double* E = nullptr;
-  double* Ea = nullptr;
   double* V = nullptr;
   cudaStream_t stream = nullptr;
   ~NlistCtx() {
@@ -2888,8 +2908,7 @@ int nlist_setup(NlistCtx& c, int nlocal, int nall, const double* x, size_t nnz, 
     };
     const size_t NA = nall, NL = nlocal;
     size_t o_x = take(24 * NA), o_t = take(4 * NA), o_o = take(4 * (NL + 1)), o_n = take(4 * nnz + 4);
-    size_t o_fa = take(4 * tsz * NA), o_f = take(24 * NA), o_e = take(8), o_ea = take(8 * NL + 8),
-           o_v = take(72);
+    size_t o_fa = take(4 * tsz * NA), o_f = take(24 * NA), o_e = take(8), o_v = take(72);
     if (cudaMalloc(&c.io, off)) {
       c.io = nullptr;
       return AENET_ERR_CUDA;
@@ -2902,7 +2921,6 @@ int nlist_setup(NlistCtx& c, int nlocal, int nall, const double* x, size_t nnz, 
     c.Facc = (void*)(b + o_fa);
     c.F = (double*)(b + o_f);
     c.E = (double*)(b + o_e);
-    c.Ea = (double*)(b + o_ea);
     c.V = (double*)(b + o_v);
     c.nall = nall;
     c.nnz_cap = nnz;
@@ -2963,7 +2981,7 @@ EXPORT int aenet_gpu_neighbor_list_energy_forces(int nlocal, int nall, const dou
         ck(ae_launch_ell_from_csr(nlocal, nall, c.x, c.types, pd.ntypes, c.offs, c.nbr, rcp * rcp,
                                   P->cap, P->nb_cnt, P->nb_jt, P->nb_vec, P->fp64, P->status, s)))
       return AENET_ERR_CUDA;
-    st = plan_eval(P, c.E, c.Ea, s);
+    st = plan_eval(P, nullptr, nullptr, s, false, false, false);
     if (st) return st;
     if (cudaMemsetAsync(c.Facc, 0, 4 * tsz * (size_t)nall, s) ||
         cudaMemsetAsync(P->virial, 0, 72, s))
@@ -2973,12 +2991,15 @@ EXPORT int aenet_gpu_neighbor_list_energy_forces(int nlocal, int nall, const dou
     if (g.lpa_adjoint) d.lpa = g.lpa_adjoint;
     int e = (pd.sp[0].sftype == AE_SF_BEHLER) ? ae_launch_behler_adjoint(pd, d, P->fp64, s)
                                                : ae_launch_chebyshev_adjoint(pd, d, P->fp64, s);
-    if (ck(e) || ck(ae_launch_forces_out(nall, c.Facc, P->fp64, c.F, 1.0, s))) return AENET_ERR_CUDA;
+    // (the atoms' energies go to the host from the plan's own array)
+    if (ck(e) || ck(ae_launch_results(energy_sum(P, c.E), P->one_chunk_each, nall, c.Facc, P->fp64, c.F,
+                                      1.0, nullptr, s)))
+      return AENET_ERR_CUDA;
     unsigned status = 0;
     double Et = 0.0;
     if (cudaMemcpyAsync(&status, P->status, 4, cudaMemcpyDeviceToHost, s) ||
         cudaMemcpyAsync(&Et, c.E, 8, cudaMemcpyDeviceToHost, s) ||
-        (E_atoms && cudaMemcpyAsync(E_atoms, c.Ea, 8 * (size_t)nlocal, cudaMemcpyDeviceToHost, s)) ||
+        (E_atoms && cudaMemcpyAsync(E_atoms, P->E_atom, 8 * (size_t)nlocal, cudaMemcpyDeviceToHost, s)) ||
         (F && cudaMemcpyAsync(F, c.F, 24 * (size_t)nall, cudaMemcpyDeviceToHost, s)) ||
         (virial && cudaMemcpyAsync(virial, P->virial, 72, cudaMemcpyDeviceToHost, s)) ||
         cudaStreamSynchronize(s))
@@ -3058,9 +3079,7 @@ EXPORT int aenet_gpu_plan_descriptor_loss_gradient(aenet_gpu_plan* P, const int*
   if (ck(ae_launch_types(P->natoms, d_types, P->types0, pd.ntypes, P->status, s))) return AENET_ERR_CUDA;
   DescBuffers d = desc_buffers(P, nullptr, false);
   if (plan_networks(P, d, s)) return AENET_ERR_CUDA;
-  if (ck(ae_launch_energy_reduce_chunked(P->nstruc, P->nchunks, P->geom_d, P->chunk_struct,
-                                         P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
-                                         P->ticket, d_E, s)))
+  if (ck(ae_launch_energy_reduce_chunked(energy_sum(P, d_E), P->one_chunk_each, s)))
     return AENET_ERR_CUDA;
   if (ck(ae_launch_loss(P->nstruc, P->natoms, P->geom_d, P->E_struct, d_E_target, P->Facc, nullptr, 0, 1.0, 0.0,
                         pd.sp[0].E_scale, P->cE, P->U, P->loss_part, d_loss, P->ticket, P->fp64, s)) ||
@@ -3171,9 +3190,7 @@ EXPORT int aenet_gpu_plan_profile(aenet_gpu_plan* P, const double* d_coords, con
   cudaEventRecord(ev[3], s);
   e |= plan_networks(P, d, s, grouped);
   cudaEventRecord(ev[4], s);
-  e |= ae_launch_energy_reduce_chunked(P->nstruc, P->nchunks, P->geom_d, P->chunk_struct,
-                                       P->E_atom, P->e_part, P->E_struct, P->one_chunk_each,
-                                       P->ticket, d_E, s);
+  e |= ae_launch_energy_reduce_chunked(energy_sum(P, d_E), P->one_chunk_each, s);
   cudaEventRecord(ev[5], s);
   const size_t tsz = P->fp64 ? 8 : 4;
   cudaMemsetAsync(P->Facc, 0, 4 * tsz * (size_t)P->natoms, s);

@@ -376,10 +376,21 @@ int ae_launch_types(int natoms, const int* types1, int* types0, int ntypes,
 // structure); otherwise a block per chunk, and the last block to finish adds
 // the chunks (ticket: a zeroed word, zero again afterwards).  E_out: optional
 // second copy of the totals.
-int ae_launch_energy_reduce_chunked(int nstruc, int nchunks, const StructGeom* geom,
-                                    const int* chunk_struct, const double* E_atom, double2* part,
-                                    double* E_struct, int one_chunk_each, unsigned* ticket,
-                                    double* E_out, cudaStream_t s);
+struct EnergySum {
+  int nstruc, nchunks;
+  const StructGeom* geom;
+  const int* chunk_struct;
+  const double* E_atom;
+  double2* part;
+  double* E_struct;
+  double* E_out;
+  unsigned* ticket;
+};
+int ae_launch_energy_reduce_chunked(const EnergySum& e, int one_chunk_each, cudaStream_t s);
+// the same with the force output (F = sign Facc, optional) and a copy of the
+// atoms' energies (optional) in one launch
+int ae_launch_results(const EnergySum& e, int one_chunk_each, int natoms, const void* Facc, int fp64,
+                      double* F, double sign, double* E_atoms, cudaStream_t s);
 int ae_launch_energy_reduce(int nstruc, const StructGeom* geom,
                             const double* E_atom, double* E_struct,
                             cudaStream_t s);
@@ -387,6 +398,9 @@ int ae_launch_forces_out(int natoms, const void* Facc, int fp64, double* F,
                          double sign, cudaStream_t s);
 
 // training: species partition, loss, weight gradients (k_train.cu)
+// (one block for at most AE_PART_ONE atoms: its tiles take about 1 us each,
+// two more launches 4)
+#define AE_PART_ONE 4096
 int ae_part_scratch_ints(int natoms);
 int ae_launch_partition(int natoms, int ntypes, const int* types0, int* scratch, int* order,
                         int* spec_off, cudaStream_t s);

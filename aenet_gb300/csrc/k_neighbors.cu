@@ -36,6 +36,7 @@
 //                  in shared memory, then the same per-atom search (the
 //                  global cell lists and the kernels above are skipped).
 #include "common.h"
+#include "partition.cuh"
 
 namespace {
 
@@ -818,11 +819,19 @@ __device__ __noinline__ void search_images(int i, const NbBuffers& nb, const Str
   }
 }
 
-// plans of wide structures only: a warp per atom
+// Plans of wide structures only: a warp per atom; one more block (when asked)
+// groups the atoms by species meanwhile, for the networks (256 Cu atoms: a
+// launch of 5 us less).
+constexpr int ALL_B = 256;
 template <typename T4>
-__global__ void __launch_bounds__(256) k_neighbors_all(int natoms, NbBuffers nb) {
-  __shared__ int s_queue[8][64];
+__global__ void __launch_bounds__(ALL_B) k_neighbors_all(int natoms, NbBuffers nb) {
+  __shared__ int s_queue[ALL_B / 32][64];
+  __shared__ PartitionScratch<ALL_B> s_part;
   const int lane = threadIdx.x & 31;
+  if (nb.order_out && blockIdx.x == gridDim.x - 1) {
+    partition_block(natoms, nb.ntypes, nb.types0_out, nb.order_out, nb.spec_off_out, s_part);
+    return;
+  }
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= natoms) return;
   const StructGeom* g = nb.geom + nb.atom_struct[i];
@@ -1904,10 +1913,11 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
   if (nb.all_pairs) {
     k_wrap_bin<<<(natoms + WRAP_B - 1) / WRAP_B, WRAP_B, 0, s>>>(natoms, pos, types, nb, 1);
     if (nb.ev_search) cudaEventRecord(nb.ev_search, s);
+    const int blocks = (natoms + 7) / 8 + (nb.order_out ? 1 : 0);
     if (fp64)
-      k_neighbors_all<double4_32a><<<(natoms + 7) / 8, 256, 0, s>>>(natoms, nb);
+      k_neighbors_all<double4_32a><<<blocks, ALL_B, 0, s>>>(natoms, nb);
     else
-      k_neighbors_all<float4><<<(natoms + 7) / 8, 256, 0, s>>>(natoms, nb);
+      k_neighbors_all<float4><<<blocks, ALL_B, 0, s>>>(natoms, nb);
     return (int)cudaGetLastError();
   }
   if (nb.cell_kernel == 5 && nb.struct_order) {

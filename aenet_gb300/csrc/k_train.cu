@@ -28,6 +28,7 @@
 // upstream do use atomics, so reruns agree to rounding, not bit for bit).
 #include "common.h"
 #include "k_cheb_impl.cuh"
+#include "partition.cuh"
 
 namespace {
 
@@ -111,55 +112,13 @@ __global__ void k_part_scatter(int n, int ntypes, const int* __restrict__ types,
   }
 }
 
-// the three phases in one block, a tile of PART_B atoms at a time
+// the three phases in one block
 __global__ void __launch_bounds__(PART_B) k_part_one(int n, int ntypes,
                                                      const int* __restrict__ types,
                                                      int* __restrict__ order,
                                                      int* __restrict__ spec_off) {
-  __shared__ int cnt[AE_MAXT], wc[PART_B / 32][AE_MAXT], tile[AE_MAXT];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < AE_MAXT) cnt[threadIdx.x] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += PART_B) atomicAdd(&cnt[types[i]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0;
-    for (int t = 0; t < ntypes; ++t) {
-      const int c = cnt[t];
-      spec_off[t] = o;
-      cnt[t] = o;
-      o += c;
-    }
-    spec_off[ntypes] = o;
-  }
-  for (int base = 0; base < n; base += PART_B) {
-    const int i = base + threadIdx.x;
-    const int t = i < n ? types[i] : -1;
-    unsigned mine = 0;
-    __syncthreads();
-    for (int q = 0; q < ntypes; ++q) {
-      const unsigned m = __ballot_sync(0xffffffffu, t == q);
-      if (q == t) mine = m;
-      if (lane == 0) wc[warp][q] = __popc(m);
-    }
-    __syncthreads();
-    // a warp per species scans the warps' counts
-    if (warp < ntypes) {
-      const int c = wc[lane][warp];
-      int x = c;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
-      }
-      wc[lane][warp] = x - c;
-      if (lane == 31) tile[warp] = x;
-    }
-    __syncthreads();
-    if (t >= 0) order[cnt[t] + wc[warp][t] + __popc(mine & ((1u << lane) - 1u))] = i;
-    __syncthreads();
-    if (threadIdx.x < ntypes) cnt[threadIdx.x] += tile[threadIdx.x];
-  }
+  __shared__ PartitionScratch<PART_B> scratch;
+  partition_block(n, ntypes, types, order, spec_off, scratch);
 }
 
 // ----------------------------------------------------------------------
@@ -1059,7 +1018,7 @@ int ae_launch_partition(int natoms, int ntypes, const int* types0, int* scratch,
   }
   // one block while its tiles take less time than two more launches (about
   // 1 us a tile of 1,024 atoms after the first)
-  if (natoms <= 4 * PART_B) {
+  if (natoms <= AE_PART_ONE) {
     k_part_one<<<1, PART_B, 0, s>>>(natoms, ntypes, types0, order, spec_off);
     return (int)cudaGetLastError();
   }
