@@ -2984,9 +2984,9 @@ EXPORT int aenet_gpu_neighbor_list_energy_forces(int nlocal, int nall, const dou
     st = plan_eval(P, nullptr, nullptr, s, false, false, false);
     if (st) return st;
     if (cudaMemsetAsync(c.Facc, 0, 4 * tsz * (size_t)nall, s) ||
-        cudaMemsetAsync(P->virial, 0, 72, s))
+        (virial && cudaMemsetAsync(P->virial, 0, 72, s)))
       return AENET_ERR_CUDA;
-    DescBuffers d = desc_buffers(P, nullptr, true);
+    DescBuffers d = desc_buffers(P, nullptr, virial != nullptr);
     d.F = c.Facc;
     if (g.lpa_adjoint) d.lpa = g.lpa_adjoint;
     int e = (pd.sp[0].sftype == AE_SF_BEHLER) ? ae_launch_behler_adjoint(pd, d, P->fp64, s)

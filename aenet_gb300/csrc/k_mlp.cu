@@ -326,9 +326,9 @@ __device__ __forceinline__ double block_sum256(double s, double* ws) {
   __syncthreads();
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
   __syncthreads();
-  s = 0.0;
+  s = ws[threadIdx.x & 7];
 #pragma unroll
-  for (int w = 0; w < 8; ++w) s += ws[w];
+  for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
   return s;
 }
 // block c of nblocks
@@ -345,6 +345,13 @@ __device__ __forceinline__ void energy_block(int c, int nblocks, const EnergySum
       if (a < a1) s += e.E_atom[g.atom_off + a];
     }
     s = block_sum256(s, ws);
+    if (e.nchunks == 1 && e.nstruc == 1) {   // nothing to add it to
+      if (threadIdx.x == 0) {
+        e.E_struct[0] = s;
+        if (e.E_out) e.E_out[0] = s;
+      }
+      return;
+    }
     if (threadIdx.x == 0) e.part[c] = make_double2(s, 0.0);
   }
   if (threadIdx.x == 0) {
