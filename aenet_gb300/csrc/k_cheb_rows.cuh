@@ -725,6 +725,10 @@ __device__ __forceinline__ void add_force(float* F, int atom, float fx, float fy
   atomicAdd(reinterpret_cast<float4*>(F) + atom, make_float4(fx, fy, fz, 0.f));
 }
 
+// FP64 pair form, a warp per atom: the adjoint of an atom may be shared out
+template <typename T, int LPA, bool MOM>
+constexpr bool ADJ_PARTS = sizeof(T) == 8 && LPA == 32 && !MOM;
+
 template <typename T, int R, int A, int LPA, bool GUARD, int SPIN, bool MOM>
 __global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>())
     k_adjoint_rows(PotDevice pd, DescBuffers b) {
@@ -733,6 +737,9 @@ __global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>(
   constexpr int GPW = 32 / LPA;
   constexpr bool MULTI = SPIN != SPIN_NONE;
   constexpr int NC = classes<SPIN>();
+  // blocks per atom: each takes some of the radial rounds and pair steps
+  constexpr bool PARTS = ADJ_PARTS<T, LPA, MOM>;
+  const int part = PARTS ? blockIdx.y : 0, pmask = PARTS ? gridDim.y - 1 : 0;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ float s_spin[AE_MAXT * AE_MAXT];
   const int lane = threadIdx.x & 31, grp = lane / LPA, sl = lane % LPA;
@@ -816,7 +823,8 @@ __global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>(
     const T d = v.w;
     const float s = SPIN == SPIN_UNIT ? s_spin[ti * AE_MAXT + t] : 0.f;
     T c = T(0);   // (dE/dd) / d
-    if (d <= r_Rc && d > T(SFB_EPS)) {
+    const bool own = !PARTS || ((base / LPA) & pmask) == part;
+    if (own && d <= r_Rc && d > T(SFB_EPS)) {
       const T inv = recip(d);
       T fc, dfc;   // dfc: fc' / d
       cutoff<true, true>(d, r_Rc, r_a, inv, fc, dfc);
@@ -940,6 +948,7 @@ __global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>(
     PairWalk pw;
     pw.start(sl, na);
     for (int q0 = 0; q0 < steps; ++q0, pw.advance(na, stride)) {
+      if (PARTS && ((q0 + 1) & pmask) != part) continue;
       const bool live = sl < stride && pw.p < P;
       const int a = live ? pw.a : 0, k = live ? pw.partner(na) : 0;
       const T4 ua = w.su[a], uk = w.su[k];
@@ -1054,7 +1063,7 @@ template <typename T, bool MOM>
 constexpr bool HAS_ADJOINT = sizeof(T) == 8 || !MOM;
 
 template <typename T, int R, int A, int LPA, bool GUARD, int SPIN, bool MOM>
-int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int warps,
+int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int warps, int parts,
                  cudaStream_t s) {
   const int atoms = warps * (32 / LPA);
   const size_t smem = group_smem<T, R, A, SPIN, MOM>(pd, b, adjoint) * atoms;
@@ -1066,7 +1075,8 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
   }
   if (smem + AE_STATIC_SMEM > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kern<<<blocks, 32 * warps, smem, s>>>(pd, b);
+  const int split = adjoint && ADJ_PARTS<T, LPA, MOM> ? parts : 1;
+  kern<<<dim3(blocks, split), 32 * warps, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }
 
@@ -1087,10 +1097,16 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
   // four warps per block once they fill the SMs (FP32)
   const int warps = sizeof(T) == 4 && b.natoms >= 64 * nsm && 16 * one <= most ? 4 : 1;
   if (b.natoms >= 20 * nsm && 4 * one <= most)
-    return launch_lanes<T, R, A, 8, GUARD, SPIN, MOM>(pd, b, adjoint, warps, s);
+    return launch_lanes<T, R, A, 8, GUARD, SPIN, MOM>(pd, b, adjoint, warps, 1, s);
   if (b.natoms >= 8 * nsm && 2 * one <= most)
-    return launch_lanes<T, R, A, 16, GUARD, SPIN, MOM>(pd, b, adjoint, 1, s);
-  return launch_lanes<T, R, A, 32, GUARD, SPIN, MOM>(pd, b, adjoint, 1, s);
+    return launch_lanes<T, R, A, 16, GUARD, SPIN, MOM>(pd, b, adjoint, 1, 1, s);
+  // Blocks per atom in the FP64 pair adjoint: a scheduler starts one FP64
+  // instruction in 64 cycles, so that up to two atoms an SM leave it waiting
+  // on their chains.  Adjoint with 1, 2 and 4 (us): 108 atoms 35.8, 25.6 and
+  // 21.5, 256 36.9, 28.7 and 28.6, 400 36.9, 34.8 and 41.0, 500 36.9, 36.9
+  // and 45.0, 864 49.1, 57.3 and 75.8.
+  const int parts = b.natoms <= nsm ? 4 : 2 * b.natoms <= 5 * nsm ? 2 : 1;
+  return launch_lanes<T, R, A, 32, GUARD, SPIN, MOM>(pd, b, adjoint, 1, parts, s);
 }
 
 // (the forward takes any spins in its SPIN_UNIT instance)
