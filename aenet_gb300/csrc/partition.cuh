@@ -12,7 +12,7 @@ struct PartitionScratch {
 template <int B>
 __device__ __forceinline__ void partition_block(int n, int ntypes, const int* types, int* order,
                                                 int* spec_off, PartitionScratch<B>& s) {
-  static_assert(B / 32 >= AE_MAXT && B <= 1024, "a warp per species, a lane per warp");
+  static_assert(B >= 32 && B <= 1024, "a lane per warp");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < AE_MAXT) s.cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -40,16 +40,16 @@ __device__ __forceinline__ void partition_block(int n, int ntypes, const int* ty
     }
     __syncthreads();
     // a warp per species scans the warps' counts
-    if (warp < ntypes) {
-      const int c = lane < B / 32 ? s.wc[lane][warp] : 0;
+    for (int q = warp; q < ntypes; q += B / 32) {
+      const int c = lane < B / 32 ? s.wc[lane][q] : 0;
       int x = c;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, x, d);
         if (lane >= d) x += y;
       }
-      if (lane < B / 32) s.wc[lane][warp] = x - c;
-      if (lane == 31) s.tile[warp] = x;
+      if (lane < B / 32) s.wc[lane][q] = x - c;
+      if (lane == 31) s.tile[q] = x;
     }
     __syncthreads();
     if (t >= 0) order[s.cnt[t] + s.wc[warp][t] + __popc(mine & ((1u << lane) - 1u))] = i;
