@@ -1257,7 +1257,10 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
   const size_t smem = behler_smem_per_warp<T>(b.cap, pd.nsf_pad, adjoint);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   const int lists = pd.ntypes * (pd.ntypes + 1) / 2;
-  const bool split = split_lists<T>(b.natoms, lists), grid = pd.behler_grid_only;
+  // (a single row's neighbours get their forces in one addition each, the same
+  // bits every time)
+  const bool split = split_lists<T>(b.natoms, lists) && !(adjoint && b.natoms == 1);
+  const bool grid = pd.behler_grid_only;
   auto pick = [&](auto one, auto each) { return split ? each : one; };
   auto kern = adjoint ? (grid ? pick(k_behler_adjoint<T, true, false>, k_behler_adjoint<T, true, true>)
                               : pick(k_behler_adjoint<T, false, false>, k_behler_adjoint<T, false, true>))

@@ -1104,8 +1104,9 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
   // instruction in 64 cycles, so that up to two atoms an SM leave it waiting
   // on their chains.  Adjoint with 1, 2 and 4 (us): 108 atoms 35.8, 25.6 and
   // 21.5, 256 36.9, 28.7 and 28.6, 400 36.9, 34.8 and 41.0, 500 36.9, 36.9
-  // and 45.0, 864 49.1, 57.3 and 75.8.
-  const int parts = b.natoms <= nsm ? 4 : 2 * b.natoms <= 5 * nsm ? 2 : 1;
+  // and 45.0, 864 49.1, 57.3 and 75.8.  A single row keeps one block: its
+  // neighbours' forces are one addition each, the same bits every time.
+  const int parts = b.natoms == 1 ? 1 : b.natoms <= nsm ? 4 : 2 * b.natoms <= 5 * nsm ? 2 : 1;
   return launch_lanes<T, R, A, 32, GUARD, SPIN, MOM>(pd, b, adjoint, 1, parts, s);
 }
 
