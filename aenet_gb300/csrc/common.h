@@ -369,9 +369,9 @@ int ae_launch_mlp_tc(const PotDevice& pd, const DescBuffers& b, const int* order
 int ae_fma_peak(double* tflops, cudaStream_t s);
 int ae_launch_types(int natoms, const int* types1, int* types0, int ntypes,
                     unsigned* status, cudaStream_t s);
-// per-structure energies: FP64 sums over chunks of AE_ECHUNK atoms (one
-// warp each; chunk_struct[c] = structure of chunk c), then over each
-// structure's chunks, in pairwise order
+// per-structure energies: FP64 sums over chunks of AE_ECHUNK atoms
+// (chunk_struct[c] = structure of chunk c), then over each structure's chunks,
+// in pairwise order
 // one_chunk_each: every structure has 1 .. AE_ECHUNK atoms (a warp per
 // structure); otherwise a block per chunk, and the last block to finish adds
 // the chunks (ticket: a zeroed word, zero again afterwards).  E_out: optional

@@ -4,7 +4,9 @@
 // FP64: the FP64 pipe of this GPU takes two lanes per clock and SM, 64 times
 // fewer than FP32, and bounds these kernels (85 % busy); loads, shared memory
 // and integer work run beside it for free.  FP32: instruction issue bounds
-// them.  For both the work is arranged for few instructions, each with all its
+// them (83 % busy in the pair forward of 256,000 atoms), in the pair adjoint the
+// shared-memory pipe (82 %: coefficient tables, staged neighbours and their
+// sums).  For both the work is arranged for few instructions, each with all its
 // lanes in use:
 //   * FP64: the cut-off is a series in r^2 (no square root, sine or division:
 //     14 multiply-adds for fc, 13 more for fc'), reciprocals come by Newton

@@ -23,7 +23,7 @@
 //
 // Order-fixed reduction: atoms are partitioned by species with a stable
 // counting sort, every block owns a fixed range of them and writes its
-// partial gradient to its own row; a final kernel sums the rows in block
+// partial gradient to its own row; a final kernel sums the rows in a fixed
 // order in FP64.  No atomics touch the gradient (the forces and cell lists
 // upstream do use atomics, so reruns agree to rounding, not bit for bit).
 #include "common.h"
