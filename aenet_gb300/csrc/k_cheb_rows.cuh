@@ -36,6 +36,7 @@
 // us; 4,096 Li/Si/O cells (597,000 atoms, moments) forward 569 -> 460 us.
 #pragma once
 #include "common.h"
+#include "chain.cuh"
 #include "cutoff64.cuh"
 #include "k_cheb_mom.cuh"
 
@@ -508,6 +509,7 @@ __global__ void __launch_bounds__(max_threads<T>(), fwd_blocks<T, R, A, SPIN, MO
   constexpr bool MULTI = SPIN != SPIN_NONE;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ float s_spin[AE_MAXT * AE_MAXT];
+  wait_for_previous();
   const int lane = threadIdx.x & 31, grp = lane / LPA, sl = lane % LPA;
   if (MULTI) {
     for (int q = threadIdx.x; q < pd.ntypes * AE_MAXT; q += blockDim.x)
@@ -744,6 +746,7 @@ __global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>(
   const int part = PARTS ? blockIdx.y : 0, pmask = PARTS ? gridDim.y - 1 : 0;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   __shared__ float s_spin[AE_MAXT * AE_MAXT];
+  wait_for_previous();
   const int lane = threadIdx.x & 31, grp = lane / LPA, sl = lane % LPA;
   if (MULTI) {
     for (int q = threadIdx.x; q < pd.ntypes * AE_MAXT; q += blockDim.x)
@@ -1078,8 +1081,7 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
   if (smem + AE_STATIC_SMEM > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int split = adjoint && ADJ_PARTS<T, LPA, MOM> ? parts : 1;
-  kern<<<dim3(blocks, split), 32 * warps, smem, s>>>(pd, b);
-  return (int)cudaGetLastError();
+  return (int)launch_next(kern, dim3(blocks, split), 32 * warps, smem, s, pd, b);
 }
 
 // Lanes per atom: 8 use every lane best (a whole number of rounds over the

@@ -14,6 +14,7 @@
 // normalisation scale 1/s (sfsetup.f90:1010-1031): the adjoint kernels
 // contract it with the derivatives of the raw descriptor.
 #include "common.h"
+#include "chain.cuh"
 #include "activate.cuh"
 
 namespace {
@@ -132,6 +133,7 @@ struct Mlp64Shape {
 __global__ void __launch_bounds__(32 * MLP64_WARPS) k_mlp64(PotDevice pd, DescBuffers b, int wtotal,
                                                             Mlp64Shape sh) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  wait_for_previous();
   double* sW = reinterpret_cast<double*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int q = threadIdx.x; q < wtotal; q += blockDim.x) sW[q] = pd.w64[q];
@@ -413,6 +415,7 @@ __global__ void __launch_bounds__(256) k_results(int eblocks, int one_chunk_each
                                                  int natoms, const T* __restrict__ Facc,
                                                  double* __restrict__ F, double f,
                                                  double* __restrict__ E_atoms) {
+  wait_for_previous();
   if ((int)blockIdx.x < eblocks) {
     if (one_chunk_each) energy_warp((blockIdx.x * 256 + threadIdx.x) >> 5, e);
     else energy_block(blockIdx.x, eblocks, e);
@@ -532,7 +535,7 @@ int ae_launch_mlp(const PotDevice& pd, const DescBuffers& b, int fp64, cudaStrea
     const int nblk = min((tiles + MLP64_WARPS - 1) / MLP64_WARPS, nsm * 4);
     if (need + AE_STATIC_SMEM > 48 * 1024)
       cudaFuncSetAttribute(k_mlp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
-    k_mlp64<<<nblk, 32 * MLP64_WARPS, need, s>>>(pd, b, wtotal, sh);
+    launch_next(k_mlp64, nblk, 32 * MLP64_WARPS, need, s, pd, b, wtotal, sh);
   } else {
     if (smem + AE_STATIC_SMEM > 48 * 1024)
       cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -563,11 +566,11 @@ int ae_launch_results(const EnergySum& e, int one_chunk_each, int natoms, const 
   const int blocks = eblocks + (F || E_atoms ? (natoms + 255) / 256 : 0);
   if (blocks == 0) return 0;
   if (fp64)
-    k_results<double><<<blocks, 256, 0, s>>>(eblocks, warps, e, natoms, (const double*)Facc, F, sign,
-                                             E_atoms);
+    launch_next(k_results<double>, blocks, 256, 0, s, eblocks, (int)warps, e, natoms,
+                (const double*)Facc, F, sign, E_atoms);
   else
-    k_results<float><<<blocks, 256, 0, s>>>(eblocks, warps, e, natoms, (const float*)Facc, F, sign,
-                                            E_atoms);
+    launch_next(k_results<float>, blocks, 256, 0, s, eblocks, (int)warps, e, natoms,
+                (const float*)Facc, F, sign, E_atoms);
   return (int)cudaGetLastError();
 }
 

@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 
 #include "common.h"
+#include "chain.cuh"
 
 namespace {
 
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(128) k_mlp_tc(PotDevice pd, DescBuffers b,
                                                 const int* __restrict__ order,
                                                 const int* __restrict__ spec_off, int tiles_ub) {
   extern __shared__ __align__(1024) unsigned char sm[];
+  wait_for_previous();
   constexpr int KA = KIN > H ? KIN : H;
   const TcLayout L = tc_layout(KIN, H);
   unsigned char* img = sm;
@@ -443,8 +445,7 @@ int launch_tc(const PotDevice& pd, const DescBuffers& b, const int* order, const
   occ = max(1, min(occ, (int)(512 / TMEM_COLS)));
   const int tiles_ub = (b.natoms + TILE - 1) / TILE + pd.ntypes;
   const int grid = max(1, min(tiles_ub, nsm * occ));
-  kern<<<grid, TILE, smem, s>>>(pd, b, order, spec_off, tiles_ub);
-  return (int)cudaGetLastError();
+  return (int)launch_next(kern, grid, TILE, smem, s, pd, b, order, spec_off, tiles_ub);
 }
 
 }  // namespace

@@ -36,6 +36,7 @@
 //                  in shared memory, then the same per-atom search (the
 //                  global cell lists and the kernels above are skipped).
 #include "common.h"
+#include "chain.cuh"
 #include "partition.cuh"
 
 namespace {
@@ -258,6 +259,7 @@ constexpr int ONE_B = 1024;
 constexpr int ONE_PER = AE_ONE_ATOMS / ONE_B;
 __global__ void __launch_bounds__(ONE_B) k_cells_one(int natoms, NbBuffers nb) {
   extern __shared__ int sm_one[];
+  wait_for_previous();
   __shared__ int wt[33], sp_cnt[AE_MAXT], sp_off[AE_MAXT];
   const int nc = nb.ncells_total;
   int* start = sm_one;            // [nc + 1] counts, then offsets
@@ -673,6 +675,7 @@ __global__ void __launch_bounds__(256, 4) k_neighbors(int natoms, NbBuffers nb) 
   __shared__ int su_base[8][32 * NB_UPL];      // per warp: cell_atoms offset of each unit
   __shared__ float4 su_sh[8][32 * NB_UPL];     // image shift and packed image of each unit
   __shared__ int su_first[8][32];              // unit starting at each offset of a batch
+  wait_for_previous();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -828,6 +831,7 @@ template <typename T4>
 __global__ void __launch_bounds__(ALL_B) k_neighbors_all(int natoms, NbBuffers nb) {
   __shared__ int s_queue[ALL_B / 32][64];
   __shared__ PartitionScratch<ALL_B> s_part;
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   if (nb.order_out && blockIdx.x == gridDim.x - 1) {
     partition_block(natoms, nb.ntypes, nb.types0_out, nb.order_out, nb.spec_off_out, s_part);
@@ -1916,9 +1920,9 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
     if (nb.ev_search) cudaEventRecord(nb.ev_search, s);
     const int blocks = (natoms * 32 + ALL_B - 1) / ALL_B + (nb.order_out ? 1 : 0);
     if (fp64)
-      k_neighbors_all<double4_32a><<<blocks, ALL_B, 0, s>>>(natoms, nb);
+      launch_next(k_neighbors_all<double4_32a>, blocks, ALL_B, 0, s, natoms, nb);
     else
-      k_neighbors_all<float4><<<blocks, ALL_B, 0, s>>>(natoms, nb);
+      launch_next(k_neighbors_all<float4>, blocks, ALL_B, 0, s, natoms, nb);
     return (int)cudaGetLastError();
   }
   if (nb.cell_kernel == 5 && nb.struct_order) {
@@ -1963,7 +1967,7 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
     const size_t smem = sizeof(int) * ((size_t)nc + 1 + natoms);
     if (smem + AE_STATIC_SMEM > 48 * 1024)
       cudaFuncSetAttribute(k_cells_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_cells_one<<<1, ONE_B, smem, s>>>(natoms, nb);
+    launch_next(k_cells_one, 1, ONE_B, smem, s, natoms, nb);
   } else {
     e = cudaMemsetAsync(nb.cell_count, 0, sizeof(int) * (size_t)nc, s);
     if (e != cudaSuccess) return (int)e;
@@ -2005,8 +2009,8 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
   }
   const int blocks = (natoms + 7) / 8;
   if (fp64)
-    k_neighbors<double4_32a><<<blocks, 256, 0, s>>>(natoms, nb);
+    launch_next(k_neighbors<double4_32a>, blocks, 256, 0, s, natoms, nb);
   else
-    k_neighbors<float4><<<blocks, 256, 0, s>>>(natoms, nb);
+    launch_next(k_neighbors<float4>, blocks, 256, 0, s, natoms, nb);
   return (int)cudaGetLastError();
 }
