@@ -32,6 +32,16 @@
 // static shared memory a kernel may add to its dynamic allocation; the
 // launchers opt in to large dynamic shared memory once the sum passes 48 KB
 #define AE_STATIC_SMEM 1024
+#define AE_SMEM_MAX (227 * 1024 - AE_STATIC_SMEM)
+// Allows `kern` a dynamic allocation of `smem` bytes.  The limit belongs to
+// the kernel and is shared by all host threads, so it is always set to `most`,
+// the largest that the kernel's launcher takes, and never lowered to one
+// launch's need: a thread with a smaller plan would make another's launch fail.
+template <typename Kernel>
+inline cudaError_t allow_smem(Kernel kern, size_t smem, size_t most) {
+  if (smem + AE_STATIC_SMEM <= 48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 
 // status bits written by kernels into a device word
 #define AE_ST_NB_OVERFLOW 1u

@@ -1266,8 +1266,7 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
                               : pick(k_behler_adjoint<T, false, false>, k_behler_adjoint<T, false, true>))
                       : (grid ? pick(k_behler_forward<T, true, false>, k_behler_forward<T, true, true>)
                               : pick(k_behler_forward<T, false, false>, k_behler_forward<T, false, true>));
-  if (smem + AE_STATIC_SMEM > 48 * 1024)
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(kern, smem, 200 * 1024);
   kern<<<dim3(b.natoms, split ? lists : 1), 32, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }
@@ -1410,8 +1409,7 @@ int ae_launch_behler_jacobian(const PotDevice& pd, const DescBuffers& b, int ato
   const int warps = 4;
   const size_t smem = behler_smem_per_warp<double>(b.cap, pd.nsf_pad, false) * warps;
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  if (smem + AE_STATIC_SMEM > 48 * 1024)
-    cudaFuncSetAttribute(k_behler_jacobian, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_behler_jacobian, smem, 200 * 1024);
   k_behler_jacobian<<<(count + warps - 1) / warps, warps * 32, smem, s>>>(pd, b, atom0, count,
                                                                          nsf_max, Ji, Jj, nbl, nnb);
   return (int)cudaGetLastError();

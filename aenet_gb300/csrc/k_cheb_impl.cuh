@@ -388,8 +388,7 @@ int launch_adjoint_mom(const PotDevice& pd, const DescBuffers& b, cudaStream_t s
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   const int blocks = (b.natoms + groups - 1) / groups;
   auto kern = k_adjoint_mom<R, A, LPA>;
-  if (smem + AE_STATIC_SMEM > 48 * 1024)
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(kern, smem, 200 * 1024);
   kern<<<blocks, warps * 32, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }

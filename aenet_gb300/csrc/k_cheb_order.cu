@@ -122,12 +122,12 @@ int ae_launch_stale_order(int natoms, const StructGeom* geom, const int* atom_st
   const int blocks = (natoms + warps - 1) / warps;
   if (fp64) {
     auto kern = k_stale_order<double4_32a>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem, 200 * 1024);
     kern<<<blocks, warps * 32, smem, s>>>(natoms, geom, atom_struct, r_wrap, pd, b, caller_order,
                                           rank, seff);
   } else {
     auto kern = k_stale_order<float4>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem, 200 * 1024);
     kern<<<blocks, warps * 32, smem, s>>>(natoms, geom, atom_struct, r_wrap, pd, b, caller_order,
                                           rank, seff);
   }

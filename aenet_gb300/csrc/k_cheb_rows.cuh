@@ -1060,7 +1060,7 @@ size_t group_smem(const PotDevice& pd, const DescBuffers& b, bool adjoint) {
   return (size_t)layout<T>(b.cap_a, pd.nsf_pad, nt, R, classes<SPIN>(), A, adjoint, MOM).bytes;
 }
 
-constexpr size_t SMEM_MAX = 226 * 1024;
+constexpr size_t SMEM_MAX = AE_SMEM_MAX;
 // the FP32 adjoint in moment form is k_cheb_impl.cuh's, which keeps its
 // coefficients in registers: 576 us for 4,096 Li/Si/O cells against 625 us
 // with the tables of this file's and 620 us with registers in it
@@ -1078,10 +1078,10 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
   if constexpr (HAS_ADJOINT<T, MOM>) {
     if (adjoint) kern = k_adjoint_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
   }
-  if (smem + AE_STATIC_SMEM > 48 * 1024)
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(kern, smem, SMEM_MAX);
   const int split = adjoint && ADJ_PARTS<T, LPA, MOM> ? parts : 1;
-  return (int)launch_next(kern, dim3(blocks, split), 32 * warps, smem, s, pd, b);
+  launch_next(kern, dim3(blocks, split), 32 * warps, smem, s, pd, b);
+  return (int)cudaGetLastError();
 }
 
 // Lanes per atom: 8 use every lane best (a whole number of rounds over the

@@ -533,12 +533,10 @@ int ae_launch_mlp(const PotDevice& pd, const DescBuffers& b, int fp64, cudaStrea
     const size_t need = bytes(sh.tile);
     const int tiles = (b.natoms + sh.tile - 1) / sh.tile;
     const int nblk = min((tiles + MLP64_WARPS - 1) / MLP64_WARPS, nsm * 4);
-    if (need + AE_STATIC_SMEM > 48 * 1024)
-      cudaFuncSetAttribute(k_mlp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    allow_smem(k_mlp64, need, AE_SMEM_MAX);
     launch_next(k_mlp64, nblk, 32 * MLP64_WARPS, need, s, pd, b, wtotal, sh);
   } else {
-    if (smem + AE_STATIC_SMEM > 48 * 1024)
-      cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_mlp, smem, AE_SMEM_MAX);
     k_mlp<<<blocks, warps * 32, smem, s>>>(pd, b, pd.w32, wtotal);
   }
   return (int)cudaGetLastError();

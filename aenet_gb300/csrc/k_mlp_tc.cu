@@ -445,7 +445,8 @@ int launch_tc(const PotDevice& pd, const DescBuffers& b, const int* order, const
   occ = max(1, min(occ, (int)(512 / TMEM_COLS)));
   const int tiles_ub = (b.natoms + TILE - 1) / TILE + pd.ntypes;
   const int grid = max(1, min(tiles_ub, nsm * occ));
-  return (int)launch_next(kern, grid, TILE, smem, s, pd, b, order, spec_off, tiles_ub);
+  launch_next(kern, grid, TILE, smem, s, pd, b, order, spec_off, tiles_ub);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace

@@ -1965,9 +1965,12 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
   if (ae_cells_one(natoms, nc)) {
     k_wrap_bin<<<wrap_blocks, WRAP_B, 0, s>>>(natoms, pos, types, nb, 1);
     const size_t smem = sizeof(int) * ((size_t)nc + 1 + natoms);
-    if (smem + AE_STATIC_SMEM > 48 * 1024)
-      cudaFuncSetAttribute(k_cells_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_next(k_cells_one, 1, ONE_B, smem, s, natoms, nb);
+    e = allow_smem(k_cells_one, smem, sizeof(int) * (AE_ONE_CELLS + 1 + AE_ONE_ATOMS));
+    if (e == cudaSuccess) e = launch_next(k_cells_one, 1, ONE_B, smem, s, natoms, nb);
+    if (e != cudaSuccess) {   // the search must not read another pass's lists
+      cudaGetLastError();
+      return (int)e;
+    }
   } else {
     e = cudaMemsetAsync(nb.cell_count, 0, sizeof(int) * (size_t)nc, s);
     if (e != cudaSuccess) return (int)e;

@@ -1092,8 +1092,7 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
   }
   if (tneed + AE_STATIC_SMEM <= 200 * 1024) {
     auto go_tile = [&](auto kern) {
-      if (tneed + AE_STATIC_SMEM > 48 * 1024)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tneed);
+      allow_smem(kern, tneed, 200 * 1024);
       kern<<<rows, WT_THREADS, tneed, s>>>(pd, A);
     };
     if (fp64) {
@@ -1121,7 +1120,7 @@ int ae_launch_mlp_wgrad(const PotDevice& pd, const int* order, const int* spec_o
   if (tile < 4) return (int)cudaErrorInvalidValue;
   A.tile = tile;
   auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    allow_smem(kern, need, 200 * 1024);
     kern<<<rows, warps * 32, need, s>>>(pd, A);
   };
   if (fp64) {
