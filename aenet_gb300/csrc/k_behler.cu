@@ -1279,6 +1279,10 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
 // (G4/G5 carry the factor 2 of symmfunc.f90:724); the central atom's row is
 // minus the sum over the neighbours.
 // ----------------------------------------------------------------------
+// shared memory of one warp: the staged neighbours and their table slots
+__host__ __device__ inline size_t jacobian_smem_per_warp(int cap) {
+  return ((sizeof(double4_32a) + sizeof(int)) * (size_t)cap + 31) & ~size_t(31);
+}
 __global__ void __launch_bounds__(128) k_behler_jacobian(PotDevice pd, DescBuffers b, int atom0,
                                                          int count, int nsf_max,
                                                          double* __restrict__ Ji,
@@ -1293,9 +1297,9 @@ __global__ void __launch_bounds__(128) k_behler_jacobian(PotDevice pd, DescBuffe
   const int r = blockIdx.x * (blockDim.x >> 5) + warp;
   if (r >= count) return;
   const int i = atom0 + r;
-  unsigned char* base = smem_raw + behler_smem_per_warp<T>(b.cap, pd.nsf_pad, false) * warp;
+  unsigned char* base = smem_raw + jacobian_smem_per_warp(b.cap) * warp;
   T4* sR = reinterpret_cast<T4*>(base);
-  int* sslot = reinterpret_cast<int*>(sR + 2 * b.cap);
+  int* sslot = reinterpret_cast<int*>(sR + b.cap);
   const int ti = b.types[i];
   const BehlerTable* tab = table_of<T>(pd, ti);
   const int nt = pd.ntypes;
@@ -1407,7 +1411,7 @@ int ae_launch_behler_jacobian(const PotDevice& pd, const DescBuffers& b, int ato
                               cudaStream_t s) {
   if (count <= 0) return 0;
   const int warps = 4;
-  const size_t smem = behler_smem_per_warp<double>(b.cap, pd.nsf_pad, false) * warps;
+  const size_t smem = jacobian_smem_per_warp(b.cap) * warps;
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   allow_smem(k_behler_jacobian, smem, 200 * 1024);
   k_behler_jacobian<<<(count + warps - 1) / warps, warps * 32, smem, s>>>(pd, b, atom0, count,
