@@ -715,8 +715,9 @@ __device__ __forceinline__ float nearest(float dx, float L, int& T) {
 }
 
 // One accepted pair per lane into the row: vector e (to image img of atom j)
-// and its squared length dd2; FP64 decides near the cut-off.
-template <typename T4>
+// and its squared length dd2; FP64 decides near the cut-off.  OWN: j may be an
+// image of i itself, whose vector the predicate forms from the lattice alone.
+template <typename T4, bool OWN>
 __device__ __forceinline__ void push_pair(bool in, int i, int j, float4 rj, float ex, float ey,
                                           float ez, float dd2, int t0, int t1, int t2,
                                           const NbBuffers& nb, const StructGeom* g, size_t row,
@@ -724,7 +725,7 @@ __device__ __forceinline__ void push_pair(bool in, int i, int j, float4 rj, floa
   bool accept = in;
   const int img = (t0 & 1023) | ((t1 & 1023) << 10) | ((t2 & 1023) << 20);
   if (accept && !(dd2 < g->rc2_lo))
-    accept = dd2 <= g->rc2_hi && band_fp64(nb, g, g->pbc, false, img, i, j, g->rc2);
+    accept = dd2 <= g->rc2_hi && band_fp64(nb, g, g->pbc, OWN && i == j, img, i, j, g->rc2);
   const unsigned mask = __ballot_sync(0xffffffffu, accept);
   const int k = cnt + __popc(mask & lt);
   if (accept && k < nb.cap) {
@@ -777,7 +778,7 @@ __device__ __forceinline__ void search_all(int i, const NbBuffers& nb, const Str
       const float ex = nearest(rq.x - ri.x, L0, t0), ey = nearest(rq.y - ri.y, L1, t1),
                   ez = nearest(rq.z - ri.z, L2, t2);
       const float dd2 = ex * ex + ey * ey + ez * ez;
-      push_pair<T4>(lane < c, i, a0 + e, rq, ex, ey, ez, dd2, t0, t1, t2, nb, g, row, cnt, lt);
+      push_pair<T4, false>(lane < c, i, a0 + e, rq, ex, ey, ez, dd2, t0, t1, t2, nb, g, row, cnt, lt);
       __syncwarp();
     }
   }
@@ -812,8 +813,8 @@ __device__ __noinline__ void search_images(int i, const NbBuffers& nb, const Str
           const float dd2 = ex * ex + ey * ey + ez * ez;
           const bool in = jb + lane < n && dd2 <= g->rc2_hi && (j != i || t0 || t1 || t2);
           if (__any_sync(0xffffffffu, in))
-            push_pair<T4>(in, i, j, rj, ex, ey, ez, dd2, t0, t1, t2, nb, g, row, cnt,
-                          (1u << lane) - 1u);
+            push_pair<T4, true>(in, i, j, rj, ex, ey, ez, dd2, t0, t1, t2, nb, g, row, cnt,
+                                (1u << lane) - 1u);
         }
       }
   if (lane == 0) {
