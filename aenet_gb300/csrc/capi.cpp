@@ -965,10 +965,10 @@ struct aenet_gpu_plan {
   double* E_struct = nullptr;
   double* virial = nullptr;
   unsigned* status = nullptr;
-  unsigned* ticket = nullptr;   // of the energy reduction's last block
+  unsigned* ticket = nullptr;   // of the loss's last block
+  unsigned* e_ticket = nullptr; // [nstruc] of the structures' energy sums
   int nchunks = 0;            // energy-reduction chunks over all structures
-  int one_chunk_each = 0;     // every structure has 1 .. AE_ECHUNK atoms
-  double2* e_part = nullptr;
+  double* e_part = nullptr;
   int* chunk_struct = nullptr;  // [nchunks] structure of each energy chunk
   int* order = nullptr;       // atoms grouped by species (tensor-core networks, training)
   int* spec_off = nullptr;    // [AE_MAXT + 1]
@@ -1161,6 +1161,12 @@ bool stale_spin_wanted() {
   return false;
 }
 
+// chunks of a structure's energy sum
+int energy_chunks(const aenet_gpu_plan* P, int s) {
+  const int n = P->natoms_h[s];
+  return P->nstruc == 1 || n > AE_ECHUNK ? (n + AE_ECHUNK - 1) / AE_ECHUNK : 0;
+}
+
 int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices) {
   const double rc = P->rc;
   int cell_off = 0, atom_off = 0, nchunks = 0;
@@ -1176,7 +1182,7 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
     G.cell_off = cell_off;
     G.atom_off = atom_off;
     G.chunk_off = nchunks;
-    nchunks += (P->natoms_h[s] + AE_ECHUNK - 1) / AE_ECHUNK;
+    nchunks += energy_chunks(P, s);
     cell_off += nc;
     atom_off += P->natoms_h[s];
     natoms += P->natoms_h[s];
@@ -1198,9 +1204,6 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   P->natoms = (int)natoms;
   P->ncells = cell_off;
   P->nchunks = nchunks;
-  P->one_chunk_each = 1;
-  for (int s = 0; s < P->nstruc; ++s)
-    if (P->natoms_h[s] < 1 || P->natoms_h[s] > AE_ECHUNK) P->one_chunk_each = 0;
   if (P->cap <= 0) {
     int cap = (int)std::ceil(1.5 * dens_max + 32.0);
     P->cap = (cap + 31) & ~31;
@@ -1262,7 +1265,8 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   size_t o_Es = take(8 * (size_t)P->nstruc);
   size_t o_V = take(72 * (size_t)P->nstruc);
   size_t o_st = take(16);
-  size_t o_ep = take(16 * (size_t)(P->nchunks + 1));
+  size_t o_ep = take(8 * (size_t)(P->nchunks + 1));
+  size_t o_et = take(4 * (size_t)P->nstruc);
   size_t o_chs = take(4 * (size_t)(P->nchunks + 1));
   size_t o_ord = take(4 * (size_t)N);
   size_t o_spo = take(4 * (AE_MAXT + 1));
@@ -1316,7 +1320,8 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   P->virial = (double*)(b + o_V);
   P->status = (unsigned*)(b + o_st);
   P->ticket = P->status + 2;
-  P->e_part = (double2*)(b + o_ep);
+  P->e_part = (double*)(b + o_ep);
+  P->e_ticket = (unsigned*)(b + o_et);
   P->chunk_struct = (int*)(b + o_chs);
   P->order = (int*)(b + o_ord);
   P->spec_off = (int*)(b + o_spo);
@@ -1339,9 +1344,10 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   std::vector<int> cs;
   cs.reserve(P->nchunks);
   for (int s = 0; s < P->nstruc; ++s)
-    for (int c = 0; c < (P->natoms_h[s] + AE_ECHUNK - 1) / AE_ECHUNK; ++c) cs.push_back(s);
+    cs.insert(cs.end(), energy_chunks(P, s), s);
   if (!cs.empty())
     cudaMemcpy(P->chunk_struct, cs.data(), 4 * cs.size(), cudaMemcpyHostToDevice);
+  cudaMemset(P->e_ticket, 0, 4 * (size_t)P->nstruc);
   cudaMemset(P->status, 0, 16);
   if (cudaDeviceSynchronize() != cudaSuccess) return AENET_ERR_CUDA;
   return 0;
@@ -1464,7 +1470,7 @@ NbBuffers search_buffers(aenet_gpu_plan* P, bool* grouped) {
 
 EnergySum energy_sum(const aenet_gpu_plan* P, double* d_E) {
   return EnergySum{P->nstruc, P->nchunks, P->geom_d,   P->chunk_struct, P->E_atom,
-                   P->e_part, P->E_struct, d_E, P->ticket};
+                   P->e_part, P->E_struct, d_E, P->e_ticket};
 }
 
 // what a pass hands its caller beside the forces, when one launch at its end
@@ -1526,7 +1532,7 @@ int plan_eval(aenet_gpu_plan* P, double* d_E, double* d_E_atoms, cudaStream_t s,
   if (ck(e)) return AENET_ERR_CUDA;
   if (plan_networks(P, d, s, grouped)) return AENET_ERR_CUDA;
   if (!energies) return 0;
-  if (ck(ae_launch_energy_reduce_chunked(energy_sum(P, d_E), P->one_chunk_each, s)))
+  if (ck(ae_launch_energy_reduce_chunked(energy_sum(P, d_E), s)))
     return AENET_ERR_CUDA;
   if (d_E_atoms &&
       cudaMemcpyAsync(d_E_atoms, P->E_atom, 8 * (size_t)P->natoms, cudaMemcpyDeviceToDevice, s))
@@ -1547,7 +1553,7 @@ int plan_adjoint(aenet_gpu_plan* P, const double* grad_scale, double* d_out, dou
                                              : ae_launch_chebyshev_adjoint(pd, d, P->fp64, s);
   if (ck(e)) return AENET_ERR_CUDA;
   if (results) {
-    if (ck(ae_launch_results(energy_sum(P, results->E), P->one_chunk_each, P->natoms, P->Facc, P->fp64,
+    if (ck(ae_launch_results(energy_sum(P, results->E), P->natoms, P->Facc, P->fp64,
                              d_out, out_sign, results->E_atoms, s)))
       return AENET_ERR_CUDA;
   } else if (d_out && ck(ae_launch_forces_out(P->natoms, P->Facc, P->fp64, d_out, out_sign, s))) {
@@ -2992,7 +2998,7 @@ EXPORT int aenet_gpu_neighbor_list_energy_forces(int nlocal, int nall, const dou
     int e = (pd.sp[0].sftype == AE_SF_BEHLER) ? ae_launch_behler_adjoint(pd, d, P->fp64, s)
                                                : ae_launch_chebyshev_adjoint(pd, d, P->fp64, s);
     // (the atoms' energies go to the host from the plan's own array)
-    if (ck(e) || ck(ae_launch_results(energy_sum(P, c.E), P->one_chunk_each, nall, c.Facc, P->fp64, c.F,
+    if (ck(e) || ck(ae_launch_results(energy_sum(P, c.E), nall, c.Facc, P->fp64, c.F,
                                       1.0, nullptr, s)))
       return AENET_ERR_CUDA;
     unsigned status = 0;
@@ -3079,7 +3085,7 @@ EXPORT int aenet_gpu_plan_descriptor_loss_gradient(aenet_gpu_plan* P, const int*
   if (ck(ae_launch_types(P->natoms, d_types, P->types0, pd.ntypes, P->status, s))) return AENET_ERR_CUDA;
   DescBuffers d = desc_buffers(P, nullptr, false);
   if (plan_networks(P, d, s)) return AENET_ERR_CUDA;
-  if (ck(ae_launch_energy_reduce_chunked(energy_sum(P, d_E), P->one_chunk_each, s)))
+  if (ck(ae_launch_energy_reduce_chunked(energy_sum(P, d_E), s)))
     return AENET_ERR_CUDA;
   if (ck(ae_launch_loss(P->nstruc, P->natoms, P->geom_d, P->E_struct, d_E_target, P->Facc, nullptr, 0, 1.0, 0.0,
                         pd.sp[0].E_scale, P->cE, P->U, P->loss_part, d_loss, P->ticket, P->fp64, s)) ||
@@ -3190,7 +3196,7 @@ EXPORT int aenet_gpu_plan_profile(aenet_gpu_plan* P, const double* d_coords, con
   cudaEventRecord(ev[3], s);
   e |= plan_networks(P, d, s, grouped);
   cudaEventRecord(ev[4], s);
-  e |= ae_launch_energy_reduce_chunked(energy_sum(P, d_E), P->one_chunk_each, s);
+  e |= ae_launch_energy_reduce_chunked(energy_sum(P, d_E), s);
   cudaEventRecord(ev[5], s);
   const size_t tsz = P->fp64 ? 8 : 4;
   cudaMemsetAsync(P->Facc, 0, 4 * tsz * (size_t)P->natoms, s);

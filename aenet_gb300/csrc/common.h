@@ -222,7 +222,7 @@ struct StructGeom {
   int kr[3];          // stencil half width per axis
   int cell_off;       // first cell of this structure in the global grid
   int atom_off, natoms;
-  int chunk_off;      // first energy-reduction chunk (AE_ECHUNK atoms each)
+  int chunk_off;      // first energy-reduction chunk, where the structure has any
 };
 
 #define AE_ECHUNK 2048      // atoms per chunk of the per-structure energy sum
@@ -379,28 +379,27 @@ int ae_launch_mlp_tc(const PotDevice& pd, const DescBuffers& b, const int* order
 int ae_fma_peak(double* tflops, cudaStream_t s);
 int ae_launch_types(int natoms, const int* types1, int* types0, int ntypes,
                     unsigned* status, cudaStream_t s);
-// per-structure energies: FP64 sums over chunks of AE_ECHUNK atoms
-// (chunk_struct[c] = structure of chunk c), then over each structure's chunks,
-// in pairwise order
-// one_chunk_each: every structure has 1 .. AE_ECHUNK atoms (a warp per
-// structure); otherwise a block per chunk, and the last block to finish adds
-// the chunks (ticket: a zeroed word, zero again afterwards).  E_out: optional
-// second copy of the totals.
+// per-structure energies: FP64 sums in pairwise order, over the atoms of a
+// structure (a warp each) or, beyond AE_ECHUNK atoms and where the plan holds
+// one structure, over chunks of AE_ECHUNK atoms (a block each; chunk_struct[c] =
+// structure of chunk c) and then over the chunks, by the structure's last block
+// to finish (ticket: a zeroed word per structure, zero again afterwards).
+// E_out: optional second copy of the totals.
 struct EnergySum {
   int nstruc, nchunks;
   const StructGeom* geom;
   const int* chunk_struct;
   const double* E_atom;
-  double2* part;
+  double* part;
   double* E_struct;
   double* E_out;
   unsigned* ticket;
 };
-int ae_launch_energy_reduce_chunked(const EnergySum& e, int one_chunk_each, cudaStream_t s);
+int ae_launch_energy_reduce_chunked(const EnergySum& e, cudaStream_t s);
 // the same with the force output (F = sign Facc, optional) and a copy of the
 // atoms' energies (optional) in one launch
-int ae_launch_results(const EnergySum& e, int one_chunk_each, int natoms, const void* Facc, int fp64,
-                      double* F, double sign, double* E_atoms, cudaStream_t s);
+int ae_launch_results(const EnergySum& e, int natoms, const void* Facc, int fp64, double* F,
+                      double sign, double* E_atoms, cudaStream_t s);
 int ae_launch_energy_reduce(int nstruc, const StructGeom* geom,
                             const double* E_atom, double* E_struct,
                             cudaStream_t s);

@@ -289,13 +289,14 @@ __global__ void k_energy_reduce(int nstruc, const StructGeom* geom, const double
   if (lane == 0) E_struct[sidx] = s + c;
 }
 
-// structures of one chunk: a warp each.  Pairwise order (a lane's run, then a
-// tree over the lanes): the rounding error stays within (AE_ECHUNK/32 + 5) ulp
-// of sum |E_i|
+// Structures that have no chunks (at most AE_ECHUNK atoms): a warp each.
+// Pairwise order (a lane's run, then a tree over the lanes): the rounding error
+// stays within (AE_ECHUNK/32 + 5) ulp of sum |E_i|
 __device__ __forceinline__ void energy_warp(int sidx, const EnergySum& e) {
   const int lane = threadIdx.x & 31;
   if (sidx >= e.nstruc) return;
   const int n = e.geom[sidx].natoms;
+  if (n > AE_ECHUNK) return;
   const double* E = e.E_atom + e.geom[sidx].atom_off;
   double s = 0.0;
   for (int a = lane; a < n; a += 256) {
@@ -317,11 +318,13 @@ __global__ void k_energy_warp(EnergySum e) {
   energy_warp((blockIdx.x * blockDim.x + threadIdx.x) >> 5, e);
 }
 
-// a block of 256 threads per chunk of AE_ECHUNK atoms (eight atoms a thread,
-// then a tree), and the last block to finish adds each structure's chunks in
-// the same way: one launch, the same order every time.  (One warp per chunk
-// and a second kernel took 13 us at 4,000 atoms, a chain of 64 loads and FP64
-// additions.)
+// the others: a block of 256 threads per chunk of AE_ECHUNK atoms (eight atoms a thread,
+// then a tree); of a structure with several chunks the last block to finish
+// adds them in the same way: one launch, the same order every time.  (One warp
+// per chunk and a second kernel took 13 us at 4,000 atoms, a chain of 64 loads
+// and FP64 additions.  4,095 structures of 145 atoms and one of 4,096, the energy
+// stage: 496 us with one last block that added the chunks of every structure,
+// 39 with a block for each structure, 12 like this.)
 __device__ __forceinline__ double block_sum256(double s, double* ws) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
@@ -333,66 +336,47 @@ __device__ __forceinline__ double block_sum256(double s, double* ws) {
   for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
   return s;
 }
-// block c of nblocks
-__device__ __forceinline__ void energy_block(int c, int nblocks, const EnergySum& e) {
+__device__ __forceinline__ void energy_chunk(int c, const EnergySum& e) {
   __shared__ double ws[8];
   __shared__ bool s_last;
-  if (c < e.nchunks) {
-    const StructGeom& g = e.geom[e.chunk_struct[c]];
-    const int a0 = (c - g.chunk_off) * AE_ECHUNK, a1 = min(g.natoms, a0 + AE_ECHUNK);
-    double s = 0.0;
+  const int sidx = e.chunk_struct[c];
+  const StructGeom& g = e.geom[sidx];
+  const int c0 = g.chunk_off, count = (g.natoms + AE_ECHUNK - 1) / AE_ECHUNK;
+  const int a0 = (c - c0) * AE_ECHUNK, a1 = min(g.natoms, a0 + AE_ECHUNK);
+  double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < AE_ECHUNK / 256; ++q) {
-      const int a = a0 + q * 256 + threadIdx.x;
-      if (a < a1) s += e.E_atom[g.atom_off + a];
+  for (int q = 0; q < AE_ECHUNK / 256; ++q) {
+    const int a = a0 + q * 256 + threadIdx.x;
+    if (a < a1) s += e.E_atom[g.atom_off + a];
+  }
+  s = block_sum256(s, ws);
+  if (count > 1) {
+    if (threadIdx.x == 0) {
+      e.part[c] = s;
+      __threadfence();
+      s_last = atomicAdd(e.ticket + sidx, 1u) == (unsigned)count - 1;
     }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const volatile double* vp = e.part + c0;
+    s = 0.0;
+    for (int k = threadIdx.x; k < count; k += 256) s += vp[k];
     s = block_sum256(s, ws);
-    if (e.nchunks == 1 && e.nstruc == 1) {   // nothing to add it to
-      if (threadIdx.x == 0) {
-        e.E_struct[0] = s;
-        if (e.E_out) e.E_out[0] = s;
-      }
-      return;
-    }
-    if (threadIdx.x == 0) e.part[c] = make_double2(s, 0.0);
+    if (threadIdx.x == 0) e.ticket[sidx] = 0u;
   }
   if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(e.ticket, 1u) == (unsigned)nblocks - 1;
+    e.E_struct[sidx] = s;
+    if (e.E_out) e.E_out[sidx] = s;
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const volatile double2* vp = e.part;
-  // a warp per structure for many, the whole block for one
-  if (e.nstruc == 1) {
-    double s = 0.0;
-    for (int k = threadIdx.x; k < e.nchunks; k += 256) s += vp[k].x;
-    s = block_sum256(s, ws);
-    if (threadIdx.x == 0) {
-      e.E_struct[0] = s;
-      if (e.E_out) e.E_out[0] = s;
-    }
-  } else {
-    const int lane = threadIdx.x & 31;
-    for (int sidx = threadIdx.x >> 5; sidx < e.nstruc; sidx += 8) {
-      const int c0 = e.geom[sidx].chunk_off;
-      const int c1 = sidx + 1 < e.nstruc ? e.geom[sidx + 1].chunk_off : e.nchunks;
-      double s = 0.0;
-      for (int k = c0 + lane; k < c1; k += 32) s += vp[k].x;
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-      if (lane == 0) {
-        e.E_struct[sidx] = s;
-        if (e.E_out) e.E_out[sidx] = s;
-      }
-    }
-  }
-  if (threadIdx.x == 0) *e.ticket = 0u;
 }
-__global__ void __launch_bounds__(256) k_energy_blocks(EnergySum e) {
-  energy_block(blockIdx.x, gridDim.x, e);
+// block b of a launch of energy_blocks(e) blocks of 256 threads: the chunks
+// first, as they take longest
+__device__ __forceinline__ void energy_block(int b, const EnergySum& e) {
+  if (b < e.nchunks) energy_chunk(b, e);
+  else energy_warp(((b - e.nchunks) * 256 + threadIdx.x) >> 5, e);
 }
+__global__ void __launch_bounds__(256) k_energy_blocks(EnergySum e) { energy_block(blockIdx.x, e); }
 
 template <typename T>
 __global__ void k_forces_out(int natoms, const T* __restrict__ Facc, double* __restrict__ F,
@@ -405,20 +389,18 @@ __global__ void k_forces_out(int natoms, const T* __restrict__ Facc, double* __r
 }
 
 // The results of a pass in one launch: the first `eblocks` blocks sum the
-// energies (energy_warp or energy_block), the others write the forces and
+// energies (energy_block), the others write the forces and
 // copy the atoms' energies.  The sums are a chain of loads and FP64 additions
 // of a few blocks, as long as a launch of its own at any size; here it runs
 // beside the forces (one pass of 256 Cu atoms 62 -> 53 us, with the grouping by
 // species inside the search).
 template <typename T>
-__global__ void __launch_bounds__(256) k_results(int eblocks, int one_chunk_each, EnergySum e,
-                                                 int natoms, const T* __restrict__ Facc,
+__global__ void __launch_bounds__(256) k_results(int eblocks, EnergySum e, int natoms, const T* __restrict__ Facc,
                                                  double* __restrict__ F, double f,
                                                  double* __restrict__ E_atoms) {
   wait_for_previous();
   if ((int)blockIdx.x < eblocks) {
-    if (one_chunk_each) energy_warp((blockIdx.x * 256 + threadIdx.x) >> 5, e);
-    else energy_block(blockIdx.x, eblocks, e);
+    energy_block(blockIdx.x, e);
     return;
   }
   const int i = (blockIdx.x - eblocks) * 256 + threadIdx.x;
@@ -543,32 +525,32 @@ int ae_launch_mlp(const PotDevice& pd, const DescBuffers& b, int fp64, cudaStrea
 }
 
 namespace {
-// one structure takes the blocks at any size (a block sums 256 atoms at a
-// time, a warp 32)
-bool energy_by_warps(const EnergySum& e, int one_chunk_each) { return one_chunk_each && e.nstruc > 1; }
+// (a single structure has chunks at any size)
+int energy_blocks(const EnergySum& e) {
+  return e.nchunks + (e.nstruc > 1 || e.nchunks == 0 ? (e.nstruc + 7) / 8 : 0);
+}
 }  // namespace
 
-int ae_launch_energy_reduce_chunked(const EnergySum& e, int one_chunk_each, cudaStream_t s) {
+int ae_launch_energy_reduce_chunked(const EnergySum& e, cudaStream_t s) {
   if (e.nstruc <= 0) return 0;
-  if (energy_by_warps(e, one_chunk_each))
+  if (e.nchunks == 0)   // (two warps a block spread better)
     k_energy_warp<<<(e.nstruc + 1) / 2, 64, 0, s>>>(e);
   else
-    k_energy_blocks<<<e.nchunks > 0 ? e.nchunks : 1, 256, 0, s>>>(e);
+    k_energy_blocks<<<energy_blocks(e), 256, 0, s>>>(e);
   return (int)cudaGetLastError();
 }
 
-int ae_launch_results(const EnergySum& e, int one_chunk_each, int natoms, const void* Facc, int fp64,
-                      double* F, double sign, double* E_atoms, cudaStream_t s) {
-  const bool warps = energy_by_warps(e, one_chunk_each);
-  const int eblocks = e.nstruc <= 0 ? 0 : warps ? (e.nstruc + 7) / 8 : e.nchunks > 0 ? e.nchunks : 1;
+int ae_launch_results(const EnergySum& e, int natoms, const void* Facc, int fp64, double* F,
+                      double sign, double* E_atoms, cudaStream_t s) {
+  const int eblocks = e.nstruc > 0 ? energy_blocks(e) : 0;
   const int blocks = eblocks + (F || E_atoms ? (natoms + 255) / 256 : 0);
   if (blocks == 0) return 0;
   if (fp64)
-    launch_next(k_results<double>, blocks, 256, 0, s, eblocks, (int)warps, e, natoms,
-                (const double*)Facc, F, sign, E_atoms);
+    launch_next(k_results<double>, blocks, 256, 0, s, eblocks, e, natoms, (const double*)Facc, F,
+                sign, E_atoms);
   else
-    launch_next(k_results<float>, blocks, 256, 0, s, eblocks, (int)warps, e, natoms,
-                (const float*)Facc, F, sign, E_atoms);
+    launch_next(k_results<float>, blocks, 256, 0, s, eblocks, e, natoms, (const float*)Facc, F, sign,
+                E_atoms);
   return (int)cudaGetLastError();
 }
 
