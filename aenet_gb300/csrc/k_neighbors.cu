@@ -251,7 +251,8 @@ __global__ void k_scatter(int natoms, NbBuffers nb) {
 
 // Cell offsets, the atoms in cell order (ascending index inside a cell, so
 // that rows come out the same every time) and, when asked, the atoms grouped
-// by species, for small plans in one block: one launch instead of a memset,
+// by species (ascending index as well: the weight gradients' sums go by it),
+// for small plans in one block: one launch instead of a memset,
 // three scans, a scatter and the three kernels of the general partition, none
 // of which does more than launch at these sizes (whole pass, with the energy
 // sum in one launch: 256 copper atoms 112 -> 79 us, 4,000 Au/Cu 152 -> 109).
@@ -261,14 +262,18 @@ __global__ void __launch_bounds__(ONE_B) k_cells_one(int natoms, NbBuffers nb) {
   extern __shared__ int sm_one[];
   wait_for_previous();
   __shared__ int wt[33], sp_cnt[AE_MAXT], sp_off[AE_MAXT];
+  __shared__ int sp_before[AE_MAXT][ONE_PER * (ONE_B / 32)];   // by species and 32 atoms
   const int nc = nb.ncells_total;
   int* start = sm_one;            // [nc + 1] counts, then offsets
   int* list = sm_one + nc + 1;    // [natoms] atoms by cell, unordered
   for (int c = threadIdx.x; c < nc; c += ONE_B) start[c] = 0;
-  if (threadIdx.x < AE_MAXT) sp_cnt[threadIdx.x] = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tiles = (natoms + ONE_B - 1) / ONE_B;
+  if (nb.order_out)
+    for (int t = 0; t < nb.ntypes; ++t)
+      if (threadIdx.x < tiles * (ONE_B / 32)) sp_before[t][threadIdx.x] = 0;
   __syncthreads();
   int cell[ONE_PER], rank[ONE_PER], spec[ONE_PER], srank[ONE_PER];
-  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < ONE_PER; ++q) {
     const int i = q * ONE_B + threadIdx.x;
@@ -281,13 +286,25 @@ __global__ void __launch_bounds__(ONE_B) k_cells_one(int natoms, NbBuffers nb) {
     }
     if (nb.order_out && __any_sync(0xffffffffu, i < natoms)) {
       const unsigned m = __match_any_sync(0xffffffffu, spec[q]);
-      const int lead = __ffs(m) - 1;
-      int b = 0;
-      if (lane == lead && spec[q] >= 0) b = atomicAdd(&sp_cnt[spec[q]], __popc(m));
-      srank[q] = __shfl_sync(0xffffffffu, b, lead) + __popc(m & ((1u << lane) - 1u));
+      srank[q] = __popc(m & ((1u << lane) - 1u));
+      if (srank[q] == 0 && spec[q] >= 0) sp_before[spec[q]][q * (ONE_B / 32) + warp] = __popc(m);
     }
   }
   __syncthreads();
+  // species: a warp each turns the counts into those of the atoms before
+  if (nb.order_out && warp < nb.ntypes) {
+    int* w = sp_before[warp] + lane * tiles;   // a run of `tiles` entries per lane
+    int sum = 0;
+    for (int k = 0; k < tiles; ++k) sum += w[k];
+    const int incl = warp_incl_scan(sum, lane);
+    if (lane == 31) sp_cnt[warp] = incl;
+    int run = incl - sum;
+    for (int k = 0; k < tiles; ++k) {
+      const int v = w[k];
+      w[k] = run;
+      run += v;
+    }
+  }
   // offsets: a run of cells per thread
   const int per = (nc + ONE_B - 1) / ONE_B, c0 = threadIdx.x * per;
   int sum = 0;
@@ -302,13 +319,15 @@ __global__ void __launch_bounds__(ONE_B) k_cells_one(int natoms, NbBuffers nb) {
   if (threadIdx.x == 0) {
     start[nc] = total;
     nb.cell_start[nc] = total;
-    int o = 0;
-    for (int t = 0; t < nb.ntypes; ++t) {
-      sp_off[t] = o;
-      if (nb.order_out) nb.spec_off_out[t] = o;
-      o += sp_cnt[t];
+    if (nb.order_out) {
+      int o = 0;
+      for (int t = 0; t < nb.ntypes; ++t) {
+        sp_off[t] = o;
+        nb.spec_off_out[t] = o;
+        o += sp_cnt[t];
+      }
+      nb.spec_off_out[nb.ntypes] = o;
     }
-    if (nb.order_out) nb.spec_off_out[nb.ntypes] = o;
   }
   __syncthreads();
 #pragma unroll
@@ -324,7 +343,8 @@ __global__ void __launch_bounds__(ONE_B) k_cells_one(int natoms, NbBuffers nb) {
       for (int k = b; k < e; ++k) p += list[k] < i;
       nb.cell_atoms[p] = i;
       nb.cell_pos[p] = nb.r_f32[i];
-      if (nb.order_out) nb.order_out[sp_off[spec[q]] + srank[q]] = i;
+      if (nb.order_out)
+        nb.order_out[sp_off[spec[q]] + sp_before[spec[q]][q * (ONE_B / 32) + warp] + srank[q]] = i;
     }
 }
 
@@ -1966,7 +1986,9 @@ int ae_launch_neighbors(int natoms, const double* pos, const int* types, const N
   if (ae_cells_one(natoms, nc)) {
     k_wrap_bin<<<wrap_blocks, WRAP_B, 0, s>>>(natoms, pos, types, nb, 1);
     const size_t smem = sizeof(int) * ((size_t)nc + 1 + natoms);
-    e = allow_smem(k_cells_one, smem, sizeof(int) * (AE_ONE_CELLS + 1 + AE_ONE_ATOMS));
+    // (beside its static arrays, most of them the counts by species)
+    e = allow_smem(k_cells_one, smem + sizeof(int) * AE_MAXT * ONE_PER * (ONE_B / 32),
+                   sizeof(int) * (AE_ONE_CELLS + 1 + AE_ONE_ATOMS));
     if (e == cudaSuccess) e = launch_next(k_cells_one, 1, ONE_B, smem, s, natoms, nb);
     if (e != cudaSuccess) {   // the search must not read another pass's lists
       cudaGetLastError();
