@@ -749,6 +749,7 @@ bool angular_grid(const std::vector<BehlerFn>& fns, int f0, int f1, BehlerGrid& 
     gr.out[l * AE_BG_NE + e] = b.out;
   }
   gr.fRc = (float)gr.Rc;
+  gr.steep = 1;
   for (int l = 0; l < gr.nl; ++l) {
     gr.lam[l] = lz[l].first;
     gr.zeta[l] = lz[l].second;
@@ -756,6 +757,7 @@ bool angular_grid(const std::vector<BehlerFn>& fns, int f0, int f1, BehlerGrid& 
     gr.fzeta[l] = (float)gr.zeta[l];
     const double z = gr.zeta[l];
     gr.izeta[l] = (z >= 1.0 && z <= 64.0 && z == std::floor(z)) ? (int)z : 0;
+    gr.steep = gr.steep && z >= 1.0;
   }
   for (int e = 0; e < gr.ne; ++e) {
     gr.eta[e] = et[e];

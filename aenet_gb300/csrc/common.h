@@ -99,6 +99,7 @@ struct BehlerGrid {
   // squarings, slot[s][i] is its entry.  general: each sign's entries in
   // order, ngeneral of the longer sign (grids without a chain).
   int chain, ngeneral;
+  int steep;                          // every zeta is one or more
   int sq[AE_BG_NZ];
   int slot[2][AE_BG_NZ];
   int general[2][AE_BG_NL + AE_BG_NZ];

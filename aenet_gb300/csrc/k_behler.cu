@@ -344,11 +344,6 @@ __device__ __forceinline__ float rsq_approx(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // exp in FP64 for kernels that the FP64 pipe bounds: x = k ln 2 / 32 + r, |r| <
 // ln 2 / 64, exp x = 2^(k / 32) (1 + r + r^2 (1/2 + ... + r^4 / 720)); the powers
 // of 2^(1/32) from a table (load pipe), each with what its rounding left off;
@@ -438,11 +433,26 @@ __device__ __forceinline__ void cut_x(double x, double Rc2, double a2, double, d
 }
 template <bool DERIV>
 __device__ __forceinline__ void cut_x(float x, float Rc2, float, float a, float& fc, float& dfc) {
-  const float ri = rsq_approx(fmaxf(x, 1e-16f));
+  // the root and its reciprocal to their last rounding: one Newton step each
+  // from the approximate reciprocal root
+  x = fminf(fmaxf(x, 1e-16f), Rc2);
+  const float y = rsq_approx(x), g = x * y, e = fmaf(-g, y, 1.f);
   float s, c;
-  __sincosf(a * (fminf(x, Rc2) * ri), &s, &c);
+  __sincosf(a * fmaf(0.5f * g, e, g), &s, &c);
   fc = fmaf(0.5f, c, 0.5f);
-  if (DERIV) dfc = -0.25f * a * s * ri;
+  if (DERIV) dfc = -0.25f * a * s * fmaf(0.5f * y, e, y);
+}
+// the same of a staged neighbour at r, d fc / dr
+__device__ __forceinline__ void cut_r(double r, double Rc2, double a2, double, double& fc,
+                                      double& dfc) {
+  cut_x<true>(r * r, Rc2, a2, 0.0, fc, dfc);
+  dfc *= 2.0 * r;
+}
+__device__ __forceinline__ void cut_r(float r, float, float, float a, float& fc, float& dfc) {
+  float s, c;
+  __sincosf(a * r, &s, &c);
+  fc = fmaf(0.5f, c, 0.5f);
+  dfc = -0.5f * a * s;
 }
 
 // Per-neighbour factors of a grid block: h_e = exp(-eta_e r^2) fc(r), 1/r
@@ -464,13 +474,13 @@ __device__ __forceinline__ void fill_factors(const typename V4<T>::type* sR, T R
   for (int j = j0 + lane; j < j1; j += 32) {
     const T r = sR[j].w, x = r * r;
     T fc, dfc;
-    cut_x<true>(x, Rc * Rc, a2, a, fc, dfc);
+    cut_r(r, Rc * Rc, a2, a, fc, dfc);
     fc = fc_floor(fc);
     T4 h;
-    h.x = exp_t(-eta[0] * x) * fc;
-    h.y = exp_t(-eta[1] * x) * fc;
+    h.x = exp(-eta[0] * x) * fc;
+    h.y = exp(-eta[1] * x) * fc;
     h.z = T(1) / r;
-    h.w = T(2) * r * dfc / fc;
+    h.w = dfc / fc;
     if (!(x < Rc * Rc)) h.x = h.y = T(0);
     sH[j] = h;
   }
@@ -517,7 +527,8 @@ __device__ __forceinline__ T reduce16(T (&v)[16], int lane) {
 // s (0: lambda = +1, 1: -1) and the i-th zeta.  CHAIN: the zetas of the grid
 // are z_0 = 2^s_0, z_i = z_{i-1} 2^{s_i} (BehlerGrid::chain), so that a
 // sign's powers are a run of squarings; otherwise up to four entries of any
-// zeta per pass, in list order.
+// zeta per pass, in list order (always in FP32, where CHAIN instances are those
+// for zetas of one at least).
 constexpr int NZ = AE_BG_NZ;
 
 // ----------------------------------------------------------------------
@@ -685,28 +696,39 @@ __device__ __forceinline__ void power_sums(double u, const GridBlock<double>& B,
       }
     }
 }
-// FP32: D = zeta F / u (zero at u = 0, where the gradient of the cosine that
-// it multiplies vanishes)
+// FP32: D = zeta P with P = u^(zeta - 1), F = P u: exact at zeta = 1, and at u =
+// 0 too (of two neighbours in line u rounds to zero before the gradient of
+// the cosine that D multiplies does).  Zetas below one have no D there and
+// take zero (CHAIN: there are none).
 template <bool CHAIN>
 __device__ __forceinline__ void power_sums(float u, const GridBlock<float>& B, int s, int nz,
                                            const float* g, float (&A)[BE], float (&d)[BE]) {
-  float F[NZ];
-  powers<CHAIN>(u, B, s, nz, F);
+  float F[NZ], z[NZ];
+  const float l = lg2_approx(CHAIN ? fmaxf(u, 1.2e-38f) : u);
+  const float inv = CHAIN || !(u > 0.f) ? 0.f : __frcp_rn(u);
+#pragma unroll
+  for (int i = 0; i < NZ; ++i) {
+    const float zeta = B.zeta[s][i];
+    if (CHAIN) {
+      const float P = ex2_approx(fmaf(zeta, l, -l));
+      F[i] = P * u;
+      z[i] = P * zeta;
+    } else {
+      F[i] = ex2_approx(zeta * l);
+      z[i] = zeta == 1.f ? 1.f : zeta * (F[i] * inv);
+    }
+  }
 #pragma unroll
   for (int e = 0; e < BE; ++e) d[e] = 0.f;
   const float4* g4 = reinterpret_cast<const float4*>(g + s * NZ * BE);
 #pragma unroll
   for (int i = 0; i < NZ; i += 2) {
     const float4 q = g4[i / 2];
-    const float z0 = B.zeta[s][i] * F[i], z1 = B.zeta[s][i + 1] * F[i + 1];
     A[0] = fmaf(q.z, F[i + 1], fmaf(q.x, F[i], A[0]));
     A[1] = fmaf(q.w, F[i + 1], fmaf(q.y, F[i], A[1]));
-    d[0] = fmaf(q.z, z1, fmaf(q.x, z0, d[0]));
-    d[1] = fmaf(q.w, z1, fmaf(q.y, z0, d[1]));
+    d[0] = fmaf(q.z, z[i + 1], fmaf(q.x, z[i], d[0]));
+    d[1] = fmaf(q.w, z[i + 1], fmaf(q.y, z[i], d[1]));
   }
-  const float inv = rcp_approx(fmaxf(u, 1e-30f));   // F is zero at u = 0
-#pragma unroll
-  for (int e = 0; e < BE; ++e) d[e] *= inv;
 }
 
 template <bool CHAIN>
@@ -1067,15 +1089,16 @@ __device__ void adjoint_grid(const BehlerGrid* gr, const PairList& L, const Warp
   const bool g4 = gr->kind == 4;
   const T Rc = gval<T>(&gr->Rc, &gr->fRc, 0);
   const T a = T(SF_PI) / Rc, a2 = a * a, Rc2 = Rc * Rc;
-  const int npass = CHAIN ? 1 : (gr->ngeneral + NZ - 1) / NZ;
+  constexpr bool ORDER = CHAIN && sizeof(T) == 8;   // the entries in the chain's order
+  const int npass = ORDER ? 1 : (gr->ngeneral + NZ - 1) / NZ;
   for (int e0 = 0; e0 < gr->ne; e0 += BE)
     for (int pass = 0; pass < npass; ++pass) {
       GridBlock<T> B;
-      B.load(gr, CHAIN, NZ * pass, e0);
-      const int nz = CHAIN ? gr->chain : min(NZ, gr->ngeneral - NZ * pass);
+      B.load(gr, ORDER, NZ * pass, e0);
+      const int nz = ORDER ? gr->chain : min(NZ, gr->ngeneral - NZ * pass);
       __syncwarp();
       if (lane < 2 * NZ * BE) {
-        const int f = GridBlock<T>::feature(gr, CHAIN, NZ * pass, e0, lane / (NZ * BE),
+        const int f = GridBlock<T>::feature(gr, ORDER, NZ * pass, e0, lane / (NZ * BE),
                                             lane / BE % NZ, lane % BE);
         w.sB[lane] = f >= 0 ? T(2) * w.sg[f] : T(0);
       }
@@ -1231,8 +1254,8 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_beh
       const int gi = tab->grid_of[a * nt + c];
       if (GRID || gi >= 0) {
         const BehlerGrid* gr = grids + gi;
-        if (sizeof(T) == 8 && gr->chain)
-          adjoint_grid<T, sizeof(T) == 8>(gr, L, w, key, lane);
+        if (sizeof(T) == 8 ? gr->chain > 0 : gr->steep)
+          adjoint_grid<T, true>(gr, L, w, key, lane);
         else
           adjoint_grid<T, false>(gr, L, w, key, lane);
       } else {
