@@ -1249,12 +1249,12 @@ int plan_alloc(aenet_gpu_plan* P, const double* coords0, const double* lattices)
   size_t o_jt = take(4 * npairs);
   size_t o_vec = take((P->fp64 ? 32 : 16) * npairs);
   size_t o_img = P->keep_images ? take(4 * npairs) : 0;
-  // moment buffer: both blocks' moments per atom
+  // moment buffer, for potentials that have a moment form: both blocks'
+  // moments per atom
   P->mom_pad = 0;
-  if (P->pd && P->pd->qleg) {
-    int aN = 0;
-    for (int t = 0; t < P->pd->ntypes; ++t) aN = std::max(aN, P->pd->sp[t].cheb.a_N);
-    if (aN <= (P->fp64 ? AE_MOMA64 : AE_MOMA)) P->mom_pad = (2 * aN * aN + 3) & ~3;
+  if (P->pd && ae_cheb_moments(*P->pd, P->fp64)) {
+    const int aN = P->pd->sp[0].cheb.a_N;
+    P->mom_pad = (2 * aN * aN + 3) & ~3;
   }
   size_t o_M = P->mom_pad ? take(tsz * (size_t)P->mom_pad * N) : 0;
   const bool stale = stale_spin_wanted();

@@ -28,7 +28,6 @@
 #define AE_MAXG4 64          // Behler angular functions per triple type
 #define AE_MAXG2 64          // Behler radial functions per pair type
 #define AE_MOMA 7            // angular functions (order + 1) of the moment form
-#define AE_MOMA64 5          // the same of the FP64 kernels (registers)
 // static shared memory a kernel may add to its dynamic allocation; the
 // launchers opt in to large dynamic shared memory once the sum passes 48 KB
 #define AE_STATIC_SMEM 1024
@@ -327,6 +326,8 @@ int ae_launch_stale_order(int natoms, const StructGeom* geom, const int* atom_st
                           const double* r_wrap, const PotDevice& pd, const DescBuffers& b,
                           int fp64, int caller_order, int* rank, float* seff, cudaStream_t s);
 
+// whether the potentials' passes keep moments (DescBuffers::M, M64)
+bool ae_cheb_moments(const PotDevice& pd, int fp64);
 int ae_launch_chebyshev_forward(const PotDevice& pd, const DescBuffers& b,
                                 int fp64, cudaStream_t s);
 // One FP64 Chebyshev atom per launch (the per-atom entry points): one

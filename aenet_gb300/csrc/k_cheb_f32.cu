@@ -5,6 +5,7 @@
 #include "k_cheb_rows.cuh"
 
 int ae_cheb_f64(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s);
+bool ae_cheb_moments_f64(const PotDevice& pd);
 
 namespace {
 int cheb_f32(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
@@ -13,6 +14,10 @@ int cheb_f32(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream
   return chebr::dispatch_rows<float>(pd, b, adjoint, s);
 }
 }  // namespace
+
+bool ae_cheb_moments(const PotDevice& pd, int fp64) {
+  return fp64 ? ae_cheb_moments_f64(pd) : chebr::moment_sizes<float>(chebr::sizes(pd));
+}
 
 int ae_launch_chebyshev_forward(const PotDevice& pd, const DescBuffers& b, int fp64,
                                 cudaStream_t s) {

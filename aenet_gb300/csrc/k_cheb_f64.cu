@@ -5,3 +5,7 @@
 int ae_cheb_f64(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
   return chebr::dispatch_rows<double>(pd, b, adjoint, s);
 }
+
+bool ae_cheb_moments_f64(const PotDevice& pd) {
+  return chebr::moment_sizes<double>(chebr::sizes(pd));
+}

@@ -1147,16 +1147,21 @@ inline Sizes sizes(const PotDevice& pd) {
 inline bool exact(const Sizes& z, const DescBuffers& b) {
   return z.same && !b.nb_rank;
 }
-// whether the angular terms take the moment form: a moment buffer, an
-// instantiated size, and in FP64 spins that the adjoint's tables cover
+// whether the potentials have a moment form: an instantiated size, and in
+// FP64 spins that the adjoint's tables cover
+template <typename T>
+bool moment_sizes(const Sizes& z) {
+  if (!z.same || (sizeof(T) == 8 && z.spin == SPIN_ANY)) return false;
+  return (z.rN == 11 && z.aN == 5) || (z.rN == 17 && z.aN == 5) ||
+         (sizeof(T) == 4 && z.rN == 13 && z.aN == 7);
+}
+// whether the angular terms of a pass take it: there is a moment buffer, and
+// every neighbour carries its own spin
 template <typename T>
 bool moment_form(const PotDevice& pd, const DescBuffers& b) {
   const Sizes z = sizes(pd);
-  if (!exact(z, b) || !MomRows<T>::rows(b) || !MomRows<T>::q(pd) ||
-      b.mom_pad < 2 * z.aN * z.aN || (sizeof(T) == 8 && z.spin == SPIN_ANY))
-    return false;
-  return (z.rN == 11 && z.aN == 5) || (z.rN == 17 && z.aN == 5) ||
-         (sizeof(T) == 4 && z.rN == 13 && z.aN == 7);
+  return moment_sizes<T>(z) && !b.nb_rank && MomRows<T>::rows(b) && MomRows<T>::q(pd) &&
+         b.mom_pad >= 2 * z.aN * z.aN;
 }
 
 // The instances for a set of potentials: exact ones for the common (radial,

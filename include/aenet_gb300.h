@@ -70,9 +70,11 @@ extern "C" {
  *       hidden layers and widths up to 64) or on FP32 SIMT.
  *   "angular_terms" = "moments" | "pairs"   angular Chebyshev terms from
  *       per-atom moments of real spherical harmonics (the pair sum rewritten
- *       by the addition theorem; cost linear in the angular neighbours;
- *       angular orders up to 6 on the mixed path, up to 4 in FP64) or from
- *       the pair sum itself.  Same values up to rounding.
+ *       by the addition theorem; cost linear in the angular neighbours) or
+ *       from the pair sum itself.  Bases of radial order 10 or 16 and angular
+ *       order 4 have the moment form, on the mixed path also those of orders
+ *       12 and 6, the same for every species; all others sum pairs.  Same
+ *       values up to rounding.
  *   "angular_spin" = "own" | "stale"   spin weights of the Chebyshev
  *       angular pairs (species-weighted bases).  own: s_j s_k.  stale: as
  *       sfb_eval forms them (src/ext/sfbasis.f90:514, 556), where s_j is
