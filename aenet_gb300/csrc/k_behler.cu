@@ -54,12 +54,7 @@ constexpr int FCH = 16;                      // functions per register chunk
 // resident one-warp blocks per SM asked of the register allocator (FP32);
 // 9,000 rutile atoms: forward 243 us at 24, 270 at 20, 251 at 28; adjoint
 // 431 us at 16, 464 at 20, 440 at 24
-#ifndef BEH_FWD_BLOCKS
-#define BEH_FWD_BLOCKS 24
-#endif
-#ifndef BEH_ADJ_BLOCKS
-#define BEH_ADJ_BLOCKS 16
-#endif
+constexpr int FWD_BLOCKS = 24, ADJ_BLOCKS = 16;
 
 template <typename T>
 struct V4;
@@ -900,7 +895,7 @@ bool split_lists(int natoms, int lists) {
 // which frees its registers).  One warp per block: the warps of a block
 // share nothing, and small blocks spread a few hundred atoms evenly.
 template <typename T, bool GRID, bool SPLIT>
-__global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_FWD_BLOCKS : 1) k_behler_forward(PotDevice pd, DescBuffers b) {
+__global__ void __launch_bounds__(32, sizeof(T) == 4 ? FWD_BLOCKS : 1) k_behler_forward(PotDevice pd, DescBuffers b) {
   using T4 = typename V4<T>::type;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   const int lane = threadIdx.x;
@@ -1191,7 +1186,7 @@ __device__ void adjoint_generic(const BehlerTable* tab, int f0, int f1e, const P
 // sum over its neighbours (the energy depends on R_j - R_i only), and the
 // atom's virial contribution is -sum_j R_ij (x) dE_i/dR_j.
 template <typename T, bool GRID, bool SPLIT>
-__global__ void __launch_bounds__(32, sizeof(T) == 4 ? BEH_ADJ_BLOCKS : 1) k_behler_adjoint(PotDevice pd, DescBuffers b) {
+__global__ void __launch_bounds__(32, sizeof(T) == 4 ? ADJ_BLOCKS : 1) k_behler_adjoint(PotDevice pd, DescBuffers b) {
   using T4 = typename V4<T>::type;
   extern __shared__ __align__(32) unsigned char smem_raw[];
   const int lane = threadIdx.x;

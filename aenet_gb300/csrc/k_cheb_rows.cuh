@@ -479,22 +479,13 @@ template <typename T>
 constexpr int max_threads() {
   return sizeof(T) == 8 ? 32 : 128;
 }
-#ifndef AE_ROWS_FWD
-#define AE_ROWS_FWD 7
-#endif
-#ifndef AE_ROWS_ADJ
-#define AE_ROWS_ADJ 6
-#endif
-#ifndef AE_MROWS_FWD
-#define AE_MROWS_FWD 7
-#endif
 template <typename T, int R, int A, int SPIN, bool MOM>
 constexpr int fwd_blocks() {
-  return sizeof(T) == 8 ? 1 : MOM ? (A <= 5 ? AE_MROWS_FWD : 3) : R <= 17 ? AE_ROWS_FWD : 4;
+  return sizeof(T) == 8 ? 1 : MOM ? (A <= 5 ? 7 : 3) : R <= 17 ? 7 : 4;
 }
-template <typename T, int A, int SPIN, bool MOM>
+template <typename T>
 constexpr int adj_blocks() {
-  return sizeof(T) == 8 ? 1 : AE_ROWS_ADJ;
+  return sizeof(T) == 8 ? 1 : 6;
 }
 
 // ----------------------------------------------------------------------
@@ -734,7 +725,7 @@ template <typename T, int LPA, bool MOM>
 constexpr bool ADJ_PARTS = sizeof(T) == 8 && LPA == 32 && !MOM;
 
 template <typename T, int R, int A, int LPA, bool GUARD, int SPIN, bool MOM>
-__global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T, A, SPIN, MOM>())
+__global__ void __launch_bounds__(max_threads<T>(), adj_blocks<T>())
     k_adjoint_rows(PotDevice pd, DescBuffers b) {
   using T4 = typename Num<T>::v4;
   using T2 = typename Num<T>::v2;
@@ -1066,6 +1057,9 @@ constexpr size_t SMEM_MAX = AE_SMEM_MAX;
 // with the tables of this file's and 620 us with registers in it
 template <typename T, bool MOM>
 constexpr bool HAS_ADJOINT = sizeof(T) == 8 || !MOM;
+// the unguarded forward of SPIN_UNIT takes any spins (launch_spin)
+template <bool GUARD, int SPIN>
+constexpr bool HAS_FORWARD = GUARD || SPIN != SPIN_ANY;
 
 template <typename T, int R, int A, int LPA, bool GUARD, int SPIN, bool MOM>
 int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int warps, int parts,
@@ -1074,10 +1068,14 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
   const size_t smem = group_smem<T, R, A, SPIN, MOM>(pd, b, adjoint) * atoms;
   if (smem > SMEM_MAX) return (int)cudaErrorInvalidValue;
   const int blocks = (b.natoms + atoms - 1) / atoms;
-  void (*kern)(PotDevice, DescBuffers) = k_forward_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
+  void (*kern)(PotDevice, DescBuffers) = nullptr;
+  if constexpr (HAS_FORWARD<GUARD, SPIN>) {
+    if (!adjoint) kern = k_forward_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
+  }
   if constexpr (HAS_ADJOINT<T, MOM>) {
     if (adjoint) kern = k_adjoint_rows<T, R, A, LPA, GUARD, SPIN, MOM>;
   }
+  if (!kern) return (int)cudaErrorInvalidValue;
   allow_smem(kern, smem, SMEM_MAX);
   const int split = adjoint && ADJ_PARTS<T, LPA, MOM> ? parts : 1;
   launch_next(kern, dim3(blocks, split), 32 * warps, smem, s, pd, b);
