@@ -4,13 +4,14 @@ Four knobs decide most of the run time of a batch: the neighbour-search
 kernel (one warp per atom over the full or the half stencil, or per home
 cell with a lane per home atom or a lane per candidate), the number of neighbour-search cells per cut-off
 length (1, 2 or 3), their refinement along the third axis (1, 2 or 4) and
-the number of lanes that cooperate on one atom in the descriptor and
-adjoint kernels (8, 16 or 32).  The first three only change the neighbour
-search and the last only the descriptor kernels, so :func:`tune` times a
-full energy-and-force pass of the caller's batch (CUDA events on the
-current stream) over the kernel and cell size at a fixed lane count, then
-the refinement, then the lane counts of the forward and of the adjoint;
-results are cached per workload key in a JSON file.
+the number of lanes that cooperate on one atom in the Chebyshev descriptor
+and adjoint kernels (8, 32, or by the number of atoms: 16).  The first three
+only change the neighbour search and the last only the descriptor kernels,
+so :func:`tune` times a full energy-and-force pass of the caller's batch
+(CUDA events on the current stream) over the kernel and cell size at the
+default lanes, then the refinement, then the lanes of the forward and of the
+adjoint, which leave the default where they gain a hundredth or more; results
+are cached per workload key in a JSON file.
 """
 import json
 import os
@@ -20,7 +21,8 @@ import torch
 from . import core
 from .plan import Plan
 
-LANES = (8, 16, 32)
+LANES = (16, 8, 32)
+GAIN = 0.99      # what other lanes than the first have to bring
 CELL_DIVS = (1, 2, 3)
 Z_REFINES = (1, 2, 4)
 NB_KERNELS = ("cell", "atom", "stream", "half", "struct", "struct_half")
@@ -62,6 +64,7 @@ def tune(natoms, cells, pbc, positions, types, precision=core.MIXED, key=None, r
         results = []
         lp0 = lanes[0]
         core.set_option("lanes_per_atom", lp0)
+        core.set_option("adjoint_lanes_per_atom", 0)
         core.set_option("z_refine", 1)
         for cd in cell_divs:
             core.set_option("cell_div", cd)
@@ -85,23 +88,30 @@ def tune(natoms, cells, pbc, positions, types, precision=core.MIXED, key=None, r
         zr = min(zres)[1]
         core.set_option("z_refine", zr)
         plan = Plan(natoms, cells, pbc, precision=precision, coords0=positions)
-        for lp in lanes[1:]:
-            core.set_option("lanes_per_atom", lp)
-            results.append((_time(plan, p, t, reps), lp, cd, nk))
+        ms, lp = _time(plan, p, t, reps), lp0
+        first = ms
+        for q in lanes[1:]:
+            core.set_option("lanes_per_atom", q)
+            results.append((_time(plan, p, t, reps), q, cd, nk))
+            if results[-1][0] < min(ms, GAIN * first):
+                ms, lp = results[-1][0], q
         plan.close()
-        ms, lp, cd, nk = min(results)
         # the adjoint's lanes per atom, at the chosen forward shape
         core.set_option("lanes_per_atom", lp)
         plan = Plan(natoms, cells, pbc, precision=precision, coords0=positions)
         adj = [(ms, 0)]
         for la in lanes:
-            if la == lp:
+            if la == lp != 16:
                 continue
             core.set_option("adjoint_lanes_per_atom", la)
             adj.append((_time(plan, p, t, reps), la))
         core.set_option("adjoint_lanes_per_atom", 0)
         plan.close()
-        ms, la = min(adj)
+        best_ms, la = min(adj)
+        if best_ms < GAIN * ms:
+            ms = best_ms
+        else:
+            la = 0
         best = {"neighbour_kernel": nk, "cell_div": cd, "z_refine": zr, "lanes_per_atom": lp,
                 "adjoint_lanes_per_atom": la, "ms": ms,
                 "all": [[r[3], r[2], r[1], r[0]] for r in results] +

@@ -267,7 +267,7 @@ struct State {
   int angular_legacy = 0;
   int cell_div = 2;
   int z_refine = 1;          // search cells along the third axis per cell_div cell
-  int lpa_default = 16;
+  int lpa_default = 16;       // lanes per atom (16: by the number of atoms)
   int lpa_adjoint = 0;        // lanes per atom of the adjoint (0: as the forward)
   int networks_tc = 1;       // tensor-core networks on the mixed path when eligible
   int nb_cell = 0;           // neighbour search: warp per atom (0), per home cell with a lane
@@ -946,7 +946,6 @@ struct aenet_gpu_plan {
   int ncells = 0;
   int cap = 0;
   int cap_a = 0;      // staged angular neighbours per atom
-  int lpa = 0;        // lanes per atom in the descriptor kernels (0 = default)
   int* nb_cnt = nullptr;
   int* nb_jt = nullptr;
   void* nb_vec = nullptr;
@@ -1396,7 +1395,7 @@ DescBuffers desc_buffers(aenet_gpu_plan* P, const double* grad_scale, bool viria
   d.nb_vec = P->nb_vec;
   d.cap = P->cap;
   d.cap_a = P->cap_a;
-  d.lpa = P->lpa ? P->lpa : g.lpa_default;
+  d.lpa = ae_lanes_per_atom();
   d.G = P->G;
   d.dEdG = P->dEdG;
   d.E_atom = P->E_atom;
@@ -3260,7 +3259,7 @@ int ae_device_tables(PotDevice* out, double* rc, int* cell_div) {
   return 0;
 }
 
-int ae_lanes_per_atom() { return g.lpa_default; }
+int ae_lanes_per_atom() { return g.lpa_default == 16 ? 0 : g.lpa_default; }
 
 // Geometry of one periodic structure (host arithmetic only).
 int ae_periodic_geom(StructGeom* G, const double* lattice, int natoms, double rc, int cell_div) {

@@ -292,7 +292,7 @@ struct DescBuffers {
   const void* nb_vec;
   int cap;
   int cap_a;                   // staged angular neighbours per atom
-  int lpa;                     // lanes per atom of the descriptor kernels
+  int lpa;                     // lanes per atom of the Chebyshev kernels (0: by the number of atoms)
   void* G;                     // [N][nsf_pad] (T)
   void* dEdG;                  // [N][nsf_pad] (T)
   double* E_atom;              // [N]
@@ -328,6 +328,7 @@ int ae_launch_stale_order(int natoms, const StructGeom* geom, const int* atom_st
 
 // whether the potentials' passes keep moments (DescBuffers::M, M64)
 bool ae_cheb_moments(const PotDevice& pd, int fp64);
+int ae_lanes_per_atom();
 int ae_launch_chebyshev_forward(const PotDevice& pd, const DescBuffers& b,
                                 int fp64, cudaStream_t s);
 // One FP64 Chebyshev atom per launch (the per-atom entry points): one

@@ -392,7 +392,7 @@ int launch_adjoint_mom(const PotDevice& pd, const DescBuffers& b, cudaStream_t s
   kern<<<blocks, warps * 32, smem, s>>>(pd, b);
   return (int)cudaGetLastError();
 }
-// Lanes per atom: as asked (8 or 32), else 8 from 20 atoms per SM on and 16
+// Lanes per atom: as asked, else 8 from 20 atoms per SM on and 16
 // below.  Whole mixed passes with 8, 16 and 32 lanes: 864 Au/Cu atoms 74, 72
 // and 72 us, 4,000 90, 94 and 97, 32,000 246, 261 and 290; 512 Li/Si/O cells
 // (72,513 atoms) 359, 380 and 418 us.  More lanes where a block's rows would
@@ -402,7 +402,7 @@ int adjoint_mom(const PotDevice& pd, const DescBuffers& b, cudaStream_t s) {
   int dev = 0, nsm = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  int lanes = b.lpa == 8 || b.lpa == 32 ? b.lpa : b.natoms >= 20 * nsm ? 8 : 16;
+  int lanes = b.lpa ? b.lpa : b.natoms >= 20 * nsm ? 8 : 16;
   while (lanes < 32 &&
          adjoint_mom_smem(b.cap_a, pd.nsf_pad) * (size_t)(4 * 32 / lanes) > 200 * 1024)
     lanes *= 2;

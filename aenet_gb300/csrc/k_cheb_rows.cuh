@@ -1082,26 +1082,27 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
   return (int)cudaGetLastError();
 }
 
-// Lanes per atom: 8 use every lane best (a whole number of rounds over the
-// neighbours, cheap group sums), 32 spread few atoms over more SMs (one warp
-// each) and take rows too long for several groups' shared memory.  Whole FP64
-// passes with 32, 16 and 8 lanes: 864 Au/Cu atoms 148, 158 and 217 us; 1,176
-// 168, 165 and 224; 1,792 239, 222 and 253; 2,772 361, 331 and 337; 4,840
-// Cu/Au atoms 541, 464 and 442.  Hence below 8 atoms per SM 32, below 20 16
-// (the FP32 kernels follow the same line).
+// Lanes per atom, as asked or by the number of atoms: 8 use every lane best (a
+// whole number of rounds over the neighbours, cheap group sums), 32 spread few
+// atoms over more SMs (one warp each) and take rows too long for several
+// groups' shared memory.  Whole FP64 passes with 32, 16 and 8 lanes: 864 Au/Cu
+// atoms 148, 158 and 217 us; 1,176 168, 165 and 224; 1,792 239, 222 and 253;
+// 2,772 361, 331 and 337; 4,840 Cu/Au atoms 541, 464 and 442.  Hence below 8
+// atoms per SM 32, below 20 16 (the FP32 kernels follow the same line).
 template <typename T, int R, int A, bool GUARD, int SPIN, bool MOM>
 int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
   int dev = 0, nsm = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // several groups share a block while three blocks still fit an SM
-  const size_t most = SMEM_MAX / 3, one = group_smem<T, R, A, SPIN, MOM>(pd, b, true);
+  // several groups share a block while three blocks still fit an SM (as asked:
+  // while they fit at all)
+  const size_t three = SMEM_MAX / 3, one = group_smem<T, R, A, SPIN, MOM>(pd, b, true);
+  int lanes = b.lpa ? b.lpa : b.natoms >= 20 * nsm ? 8 : b.natoms >= 8 * nsm ? 16 : 32;
+  while (lanes < 32 && 32 / lanes * one > (b.lpa ? SMEM_MAX : three)) lanes *= 2;
   // four warps per block once they fill the SMs (FP32)
-  const int warps = sizeof(T) == 4 && b.natoms >= 64 * nsm && 16 * one <= most ? 4 : 1;
-  if (b.natoms >= 20 * nsm && 4 * one <= most)
-    return launch_lanes<T, R, A, 8, GUARD, SPIN, MOM>(pd, b, adjoint, warps, 1, s);
-  if (b.natoms >= 8 * nsm && 2 * one <= most)
-    return launch_lanes<T, R, A, 16, GUARD, SPIN, MOM>(pd, b, adjoint, 1, 1, s);
+  const int warps = sizeof(T) == 4 && b.natoms >= 64 * nsm && 16 * one <= three ? 4 : 1;
+  if (lanes == 8) return launch_lanes<T, R, A, 8, GUARD, SPIN, MOM>(pd, b, adjoint, warps, 1, s);
+  if (lanes == 16) return launch_lanes<T, R, A, 16, GUARD, SPIN, MOM>(pd, b, adjoint, 1, 1, s);
   // Blocks per atom in the FP64 pair adjoint: a scheduler starts one FP64
   // instruction in 64 cycles, so that up to two atoms an SM leave it waiting
   // on their chains.  Adjoint with 1, 2 and 4 (us): 108 atoms 35.8, 25.6 and

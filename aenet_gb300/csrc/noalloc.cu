@@ -22,8 +22,8 @@
 // results differ from aenet_gpu_structure_energy_forces by FP32 rounding
 // only.  The staged angular neighbours per atom follow the structure's
 // density (as the plans do, at most the neighbour limit) and the lanes per
-// atom of the descriptor kernels are raised when their shared memory would
-// not fit.
+// atom of the descriptor kernels are raised, by their launchers, when their
+// shared memory would not fit.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -32,7 +32,6 @@
 #include "common.h"
 
 int ae_device_tables(PotDevice* out, double* rc, int* cell_div);
-int ae_lanes_per_atom();
 int ae_periodic_geom(StructGeom* G, const double* lattice, int natoms, double rc, int cell_div);
 
 namespace {
@@ -179,14 +178,7 @@ extern "C" __attribute__((visibility("default"))) int aenet_gpu_structure_energy
     ca = (ca + 7) & ~7;
     d.cap_a = std::min(std::max(ca, 8), (int)NA_NB);
   }
-  // lanes per atom: as set, raised while the descriptor kernels' shared
-  // memory per block (4 warps of 32 / lpa atoms) would exceed 200 KB
   d.lpa = ae_lanes_per_atom();
-  {
-    const size_t t4 = fp64 ? 32 : 16;
-    const size_t group = (2 * t4 + 3 * tsz) * (size_t)d.cap_a + tsz * (size_t)pd.nsf_pad + 32;
-    while (d.lpa < 32 && group * (size_t)(4 * 32 / d.lpa) > 200 * 1024) d.lpa *= 2;
-  }
   d.G = b + O_G;
   d.dEdG = b + O_DG;
   d.E_atom = (double*)(b + O_EA);

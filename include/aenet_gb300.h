@@ -44,11 +44,12 @@ extern "C" {
  *   "z_refine" = "1" .. "4"   the search cells are that many times narrower
  *       along the third lattice axis: the same stencil rows, each cut more
  *       finely to the cut-off sphere (performance only).
- *   "lanes_per_atom" = "8" | "16" | "32"   lanes per atom of the mixed path's
- *       moment-form adjoint; 16 (the default) leaves it to the number of atoms
- *       (performance only; the other descriptor kernels always choose so).
- *   "adjoint_lanes_per_atom" = "0" | "8" | "16" | "32"   the same, taking
- *       precedence; 0 follows lanes_per_atom (performance only).
+ *   "lanes_per_atom" = "8" | "16" | "32"   lanes per atom of the Chebyshev
+ *       descriptor and adjoint kernels; 16 (the default) leaves them to the
+ *       number of atoms, and all are raised where a block's rows would not fit
+ *       its shared memory (performance only).
+ *   "adjoint_lanes_per_atom" = "0" | "8" | "16" | "32"   those of the adjoint
+ *       kernels, as given; 0 follows lanes_per_atom (performance only).
  *   "neighbour_kernel" = "atom" | "cell" | "stream" | "half" | "struct" |
  *       "struct_half"   neighbour
  *       search with one warp per atom (pruned per atom), one warp per home
