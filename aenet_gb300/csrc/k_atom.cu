@@ -48,6 +48,7 @@
 #include "common.h"
 #include "activate.cuh"
 #include "cutoff64.cuh"
+#include "exp64.cuh"
 #include "k_cheb_impl.cuh"
 
 namespace cg = cooperative_groups;

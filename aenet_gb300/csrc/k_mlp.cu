@@ -16,6 +16,7 @@
 #include "common.h"
 #include "chain.cuh"
 #include "activate.cuh"
+#include "exp64.cuh"
 
 namespace {
 
@@ -120,9 +121,10 @@ __global__ void __launch_bounds__(256) k_mlp(PotDevice pd, DescBuffers b,
 // a warp takes `tile` atoms at once and spreads their (atom, node) pairs over
 // its lanes: 20 or 25 nodes fill as many lanes as 32 (a warp per atom leaves
 // lanes idle in every layer that is not a multiple of 32 wide), and tanh is
-// evaluated without branches.  A warp per atom before, this now: 72,513
-// atoms 32-32-32-1 974 -> 900 us (85 % of the pipe, of which the products are
-// two thirds), 2,765 atoms 40-25-25-1 60 -> 53 us.  The activations of a tile live in shared memory beside the weights.
+// evaluated without branches.  A warp per atom before, this now: 72,513 atoms
+// 32-32-32-1 974 -> 942 us (of which the products are two thirds), 2,765 atoms
+// 40-25-25-1 60 -> 55 us.  The activations of a tile live in shared memory
+// beside the weights.
 constexpr int MLP64_WARPS = 4;
 struct Mlp64Shape {
   int tile;       // atoms per warp
