@@ -27,14 +27,25 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+constexpr int MLP_WARPS = 8;
 __host__ __device__ constexpr int mlp_warp_elems() {
   return 2 * (AE_MAXNSF + 1) + 2 * AE_MAXLAYERS * (AE_MAXNODES + 1) + 1;
 }
 
-// FP32 networks (shapes that the tensor-core kernel does not take)
-__global__ void __launch_bounds__(256) k_mlp(PotDevice pd, DescBuffers b,
-                                             const float* __restrict__ W, int wtotal) {
-  using T = float;
+// 1/s of a feature (the FP32 kernels' copy)
+template <typename T>
+__device__ __forceinline__ T nscale(const PotDevice& pd, size_t k);
+template <>
+__device__ __forceinline__ float nscale<float>(const PotDevice& pd, size_t k) { return pd.scale32[k]; }
+template <>
+__device__ __forceinline__ double nscale<double>(const PotDevice& pd, size_t k) { return pd.scale[k]; }
+
+// a warp per atom: FP32 networks that the tensor-core kernel does not take,
+// and FP64 networks (networks_in_tiles)
+template <typename T>
+__global__ void __launch_bounds__(256) k_mlp(PotDevice pd, DescBuffers b, const T* __restrict__ W,
+                                             int wtotal) {
+  wait_for_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sW = reinterpret_cast<T*>(smem_raw);
   const int warps = blockDim.x >> 5;
@@ -111,20 +122,17 @@ __global__ void __launch_bounds__(256) k_mlp(PotDevice pd, DescBuffers b,
     T* out = reinterpret_cast<T*>(b.dEdG) + (size_t)i * pd.nsf_pad;
     const T es = T(sp.E_scale);
     for (int k = lane; k < nsf; k += 32)
-      out[k] = es * delta_cur[k] * pd.scale32[(size_t)ti * pd.nsf_pad + k];
+      out[k] = es * delta_cur[k] * nscale<T>(pd, (size_t)ti * pd.nsf_pad + k);
     if (lane == 0) b.E_atom[i] = sp.E_scale * (double)y + sp.E_shift + sp.E_atom;
     __syncwarp();
   }
 }
 
-// FP64 networks.  The FP64 pipe (two lanes per clock and SM) bounds them, so
-// a warp takes `tile` atoms at once and spreads their (atom, node) pairs over
-// its lanes: 20 or 25 nodes fill as many lanes as 32 (a warp per atom leaves
-// lanes idle in every layer that is not a multiple of 32 wide), and tanh is
-// evaluated without branches.  A warp per atom before, this now: 72,513 atoms
-// 32-32-32-1 974 -> 942 us (of which the products are two thirds), 2,765 atoms
-// 40-25-25-1 60 -> 55 us.  The activations of a tile live in shared memory
-// beside the weights.
+// FP64 networks by tiles (networks_in_tiles).  The FP64 pipe (two lanes per
+// clock and SM) bounds them, so a warp takes `tile` atoms at once and spreads
+// their (atom, node) pairs over its lanes: 20 or 25 nodes fill as many lanes as
+// 32, and tanh is evaluated without branches.  The activations of a tile live
+// in shared memory beside the weights.
 constexpr int MLP64_WARPS = 4;
 struct Mlp64Shape {
   int tile;       // atoms per warp
@@ -483,47 +491,87 @@ int ae_launch_types(int natoms, const int* types1, int* types0, int ntypes, unsi
   return (int)cudaGetLastError();
 }
 
+namespace {
+template <typename T>
+size_t mlp_smem(int wtotal) {
+  return sizeof(T) * ((((size_t)wtotal + 1) & ~(size_t)1) + (size_t)MLP_WARPS * mlp_warp_elems());
+}
+
+template <typename T>
+int launch_mlp(const PotDevice& pd, const DescBuffers& b, const T* W, int wtotal, int nsm,
+               cudaStream_t s) {
+  const size_t smem = mlp_smem<T>(wtotal);
+  allow_smem(k_mlp<T>, smem, AE_SMEM_MAX);
+  const int blocks = min((b.natoms + MLP_WARPS - 1) / MLP_WARPS, nsm * 4);
+  launch_next(k_mlp<T>, blocks, 32 * MLP_WARPS, smem, s, pd, b, W, wtotal);
+  return (int)cudaGetLastError();
+}
+
+// Whether the FP64 networks go by tiles of atoms (k_mlp64): where their layers
+// leave lanes of a warp per atom idle, and the atoms fill the SMs.  The
+// measure is the FP64 instructions of an atom's layers, a warp each and
+// flattened, with tanh at 45 (the library's two branches) and 32.  A warp per
+// atom and tiles (us): 26-20-20-1 2,304 atoms 31 and 33, 2,916 55 and 45, 32,000
+// 348 and 252; 40-25-25-1 two species 2,916 74 and 55, 10,976 170 and 158; but
+// 32-32-32-1 three species 8,255 125 and 165, 72,519 967 and 942, rutile's 9,000
+// 170 and 207; eight species 32-32-32-1 of 1,000 atoms 31 and 74 (four warps
+// wait for 200 KB of weights).  Few atoms of one small network: 256 atoms
+// 26-20-20-1 20 and 17, 864 21 and 23.
+bool networks_in_tiles(const PotDevice& pd, const DescBuffers& b, int wtotal, int nsm) {
+  if (mlp_smem<double>(wtotal) > AE_SMEM_MAX) return true;
+  const bool many = b.natoms >= 16 * nsm;
+  const bool few = b.natoms >= 32 && b.natoms <= 4 * nsm && wtotal <= 2048;
+  if (!many && !few) return false;
+  long long warp = 0, flat = 0;   // 32 lanes each
+  for (int t = 0; t < pd.ntypes; ++t) {
+    const NetTable& net = pd.sp[t].net;
+    for (int l = 0; l + 1 < net.nlayers - 1; ++l) {
+      const int in = net.nnodes[l], out = net.nnodes[l + 1];
+      warp += 32 * ((out + 31) / 32 * (in + 45) + (in + 31) / 32 * out);
+      flat += out * (in + 32) + in * out;
+    }
+  }
+  return 10 * warp >= 14 * flat;
+}
+
+int launch_mlp64(const PotDevice& pd, const DescBuffers& b, int wtotal, int nsm, cudaStream_t s) {
+  Mlp64Shape sh{};
+  int hidden = 0;
+  for (int t = 0; t < pd.ntypes; ++t) {
+    const NetTable& net = pd.sp[t].net;
+    hidden = max(hidden, net.nlayers - 2);
+    for (int l = 1; l < net.nlayers - 1; ++l) sh.hmax = max(sh.hmax, net.nnodes[l]);
+  }
+  sh.hmax |= 1;
+  sh.in = pd.nsf_pad | 1;
+  sh.per = (sh.in + 2 * hidden * sh.hmax) | 1;
+  // eight atoms per warp where that leaves two warps per SM or more, fewer
+  // for few atoms or long rows
+  auto bytes = [&](int tile) {
+    return sizeof(double) * ((size_t)wtotal + (size_t)MLP64_WARPS * tile * sh.per);
+  };
+  sh.tile = 8;
+  while (sh.tile > 1 && (b.natoms < 2 * nsm * MLP64_WARPS * sh.tile || bytes(sh.tile) > 110 * 1024))
+    sh.tile /= 2;
+  const size_t need = bytes(sh.tile);
+  allow_smem(k_mlp64, need, AE_SMEM_MAX);
+  const int tiles = (b.natoms + sh.tile - 1) / sh.tile;
+  const int blocks = min((tiles + MLP64_WARPS - 1) / MLP64_WARPS, nsm * 4);
+  launch_next(k_mlp64, blocks, 32 * MLP64_WARPS, need, s, pd, b, wtotal, sh);
+  return (int)cudaGetLastError();
+}
+}  // namespace
+
 int ae_launch_mlp(const PotDevice& pd, const DescBuffers& b, int fp64, cudaStream_t s) {
   if (b.natoms <= 0) return 0;
   int wtotal = 0;
   for (int t = 0; t < pd.ntypes; ++t) wtotal = max(wtotal, pd.sp[t].net.wtotal);
-  const int warps = 8;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = sizeof(float) * ((((size_t)wtotal + 1) & ~(size_t)1) + (size_t)warps * mlp_warp_elems());
-  int blocks = (b.natoms + warps - 1) / warps;
-  int maxb = nsm * 4;
-  if (blocks > maxb) blocks = maxb;
-  if (fp64) {
-    Mlp64Shape sh{};
-    int hidden = 0;
-    for (int t = 0; t < pd.ntypes; ++t) {
-      const NetTable& net = pd.sp[t].net;
-      hidden = max(hidden, net.nlayers - 2);
-      for (int l = 1; l < net.nlayers - 1; ++l) sh.hmax = max(sh.hmax, net.nnodes[l]);
-    }
-    sh.hmax |= 1;
-    sh.in = pd.nsf_pad | 1;
-    sh.per = (sh.in + 2 * hidden * sh.hmax) | 1;
-    // eight atoms per warp where that leaves two warps per SM or more, fewer
-    // for few atoms or long rows
-    auto bytes = [&](int tile) {
-      return sizeof(double) * ((size_t)wtotal + (size_t)MLP64_WARPS * tile * sh.per);
-    };
-    sh.tile = 8;
-    while (sh.tile > 1 && (b.natoms < 2 * nsm * MLP64_WARPS * sh.tile || bytes(sh.tile) > 110 * 1024))
-      sh.tile /= 2;
-    const size_t need = bytes(sh.tile);
-    const int tiles = (b.natoms + sh.tile - 1) / sh.tile;
-    const int nblk = min((tiles + MLP64_WARPS - 1) / MLP64_WARPS, nsm * 4);
-    allow_smem(k_mlp64, need, AE_SMEM_MAX);
-    launch_next(k_mlp64, nblk, 32 * MLP64_WARPS, need, s, pd, b, wtotal, sh);
-  } else {
-    allow_smem(k_mlp, smem, AE_SMEM_MAX);
-    k_mlp<<<blocks, warps * 32, smem, s>>>(pd, b, pd.w32, wtotal);
-  }
-  return (int)cudaGetLastError();
+  if (!fp64) return launch_mlp<float>(pd, b, pd.w32, wtotal, nsm, s);
+  return networks_in_tiles(pd, b, wtotal, nsm) ? launch_mlp64(pd, b, wtotal, nsm, s)
+                                               : launch_mlp<double>(pd, b, pd.w64, wtotal, nsm, s);
 }
 
 namespace {
