@@ -1088,7 +1088,12 @@ int launch_lanes(const PotDevice& pd, const DescBuffers& b, bool adjoint, int wa
 // groups' shared memory.  Whole FP64 passes with 32, 16 and 8 lanes: 864 Au/Cu
 // atoms 148, 158 and 217 us; 1,176 168, 165 and 224; 1,792 239, 222 and 253;
 // 2,772 361, 331 and 337; 4,840 Cu/Au atoms 541, 464 and 442.  Hence below 8
-// atoms per SM 32, below 20 16 (the FP32 kernels follow the same line).
+// atoms per SM 32, below 20 16.  The moment form in FP32 follows the same line
+// (864 Au/Cu atoms 56, 59 and 65 us; 2,304 71, 64 and 69; 4,000 84, 81 and 73);
+// its pair sums, whose warps wait for the longest of their rows, gain from more
+// lanes for longer: 2,048 Cu/Au atoms 58, 59 and 66 us, 2,304 Cu atoms 55, 56 and
+// 62, 3,240 69, 67 and 74, 5,324 86, 80 and 84, 6,336 81, 77 and 79, 7,488 100, 96
+// and 94, hence 32 below 16 atoms per SM and 16 below 42.
 template <typename T, int R, int A, bool GUARD, int SPIN, bool MOM>
 int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t s) {
   int dev = 0, nsm = 152;
@@ -1097,7 +1102,9 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
   // several groups share a block while three blocks still fit an SM (as asked:
   // while they fit at all)
   const size_t three = SMEM_MAX / 3, one = group_smem<T, R, A, SPIN, MOM>(pd, b, true);
-  int lanes = b.lpa ? b.lpa : b.natoms >= 20 * nsm ? 8 : b.natoms >= 8 * nsm ? 16 : 32;
+  constexpr bool PAIRS32 = sizeof(T) == 4 && !MOM;
+  constexpr int LINE16 = PAIRS32 ? 16 : 8, LINE8 = PAIRS32 ? 42 : 20;   // atoms per SM
+  int lanes = b.lpa ? b.lpa : b.natoms >= LINE8 * nsm ? 8 : b.natoms >= LINE16 * nsm ? 16 : 32;
   while (lanes < 32 && 32 / lanes * one > (b.lpa ? SMEM_MAX : three)) lanes *= 2;
   // four warps per block once they fill the SMs (FP32)
   const int warps = sizeof(T) == 4 && b.natoms >= 64 * nsm && 16 * one <= three ? 4 : 1;
