@@ -885,6 +885,13 @@ int build_behler(std::vector<std::vector<unsigned char>>& out, std::vector<doubl
     hdr.ang_off[nt * nt] = (int)fns.size();
     hdr.nfn = (int)fns.size();
     hdr.rc_max = rcm;
+    std::fill(hdr.list_of, hdr.list_of + AE_MAXNSF, (short)-1);
+    for (int gj = 0, u = 0; gj < nt; ++gj)
+      for (int gk = gj; gk < nt; ++gk, ++u)
+        for (int q = hdr.ang_off[gj * nt + gk]; q < hdr.ang_off[gj * nt + gk + 1]; ++q) {
+          const int k = fns[q].out;
+          if (k >= 0 && k < AE_MAXNSF && hdr.list_of[k] < 0) hdr.list_of[k] = (short)u;
+        }
     // product grids of the angular lists (evaluation order only; the
     // functions and their feature indices are the ones listed above)
     std::vector<BehlerGrid> grids;

@@ -114,6 +114,8 @@ struct BehlerTable {
   int grid_of[AE_MAXT * AE_MAXT];     // index of the pair's BehlerGrid, or -1
   int grid_off;                       // byte offset of the BehlerGrid array
   int nfn;
+  short list_of[AE_MAXNSF];           // the pair (tj <= tk, counted row by row) that feeds a
+                                      // feature, or -1
   BehlerFn fn[1];                     // variable length (allocated larger)
 };
 

@@ -138,11 +138,11 @@ __device__ __forceinline__ T ipow(T a, int n) {
 }
 
 // radial value and d/dr (sf_G1_ij, sf_G2_ij, sf_G3_ij)
-// A: the staged (1/r, fc, dfc), used when the function's cut-off is theirs
+// A: the staged (dfc, fc, 1/r), used when the function's cut-off is theirs
 template <typename T>
 __device__ __forceinline__ void radial_fn(const Fn<T>& f, T r, bool cached,
                                           const typename V4<T>::type& A, T& v, T& dv) {
-  T fc = A.y, dfc = A.z;
+  T fc = A.y, dfc = A.x;
   if (!cached) cutfn(r, f.Rc, fc, dfc);
   if (f.kind == 2) {
     const T a = r - f.p1;
@@ -193,7 +193,7 @@ __device__ __forceinline__ float normalise(float g, const PotDevice& pd, size_t 
 
 // Stage the neighbours inside rc into shared memory grouped by species.
 // bstart[s] .. bstart[s+1] is bucket s; returns the number staged.  sA
-// (optional) receives 1/r, fc(r) and dfc(r) for the cut-off rc.
+// (optional) receives dfc(r), fc(r) (cut-off rc) and 1/r.
 template <typename T>
 __device__ int stage_buckets(const typename V4<T>::type* __restrict__ vec,
                              const int* __restrict__ jt, int n, int nt, T rc,
@@ -218,8 +218,8 @@ __device__ int stage_buckets(const typename V4<T>::type* __restrict__ vec,
         sslot[k] = j;
         if (sA) {
           T4 a;
-          a.x = T(1) / v.w;
-          cutfn(v.w, rc, a.y, a.z);
+          a.z = T(1) / v.w;
+          cutfn(v.w, rc, a.y, a.x);
           a.w = T(0);
           sA[k] = a;
         }
@@ -380,16 +380,18 @@ __device__ __forceinline__ void cut_x(float x, float Rc2, float, float a, float&
   if (DERIV) dfc = -0.25f * a * s * fmaf(0.5f * y, e, y);
 }
 // the same of a staged neighbour at r, d fc / dr
+template <bool DERIV>
 __device__ __forceinline__ void cut_r(double r, double Rc2, double a2, double, double& fc,
                                       double& dfc) {
-  cut_x<true>(r * r, Rc2, a2, 0.0, fc, dfc);
-  dfc *= 2.0 * r;
+  cut_x<DERIV>(r * r, Rc2, a2, 0.0, fc, dfc);
+  if (DERIV) dfc *= 2.0 * r;
 }
+template <bool DERIV>
 __device__ __forceinline__ void cut_r(float r, float, float, float a, float& fc, float& dfc) {
   float s, c;
   __sincosf(a * r, &s, &c);
   fc = fmaf(0.5f, c, 0.5f);
-  dfc = -0.5f * a * s;
+  if (DERIV) dfc = -0.5f * a * s;
 }
 
 // Per-neighbour factors of a grid block: h_e = exp(-eta_e r^2) fc(r), 1/r
@@ -403,41 +405,54 @@ struct FactorKey {
 };
 __device__ __forceinline__ double fc_floor(double fc) { return fmax(fc, 1e-30); }
 __device__ __forceinline__ float fc_floor(float fc) { return fmaxf(fc, 1e-12f); }
-template <typename T>
-__device__ __forceinline__ void fill_factors(const typename V4<T>::type* sR, T Rc, T a, T a2,
-                                             const T (&eta)[BE], int j0, int j1,
-                                             typename V4<T>::type* sH, int lane) {
-  using T4 = typename V4<T>::type;
-  for (int j = j0 + lane; j < j1; j += 32) {
-    const T r = sR[j].w, x = r * r;
-    T fc, dfc;
-    cut_r(r, Rc * Rc, a2, a, fc, dfc);
-    fc = fc_floor(fc);
-    T4 h;
-    h.x = exp(-eta[0] * x) * fc;
-    h.y = exp(-eta[1] * x) * fc;
-    h.z = T(1) / r;
-    h.w = dfc / fc;
-    if (!(x < Rc * Rc)) h.x = h.y = T(0);
-    sH[j] = h;
-  }
+// a / b with b > 0 normal in FP32: FP64 by Newton's iteration for 1/b from an
+// FP32 seed and one correction of the quotient
+__device__ __forceinline__ float quotient(float a, float b) { return a / b; }
+__device__ __forceinline__ double quotient(double a, double b) {
+  float f;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)b));
+  double y = (double)f;
+  y = fma(y, fma(-b, y, 1.0), y);
+  const double q = a * y;
+  return fma(fma(-q, b, a), y, q);
 }
-// the factors of a list's two buckets
-template <typename T>
+__device__ __forceinline__ float exp_fill(float x) { return expf(x); }
+__device__ __forceinline__ double exp_fill(double x) { return exp_table(x); }
+
+// The factors of a list's two buckets, filled together: lists of a few
+// neighbours are many where there are many species, and each round costs a
+// warp's FP64 instructions whatever lanes it uses.  (Calls of one row, five species
+// whose lists have etas of their own: 6 neighbours 333 -> 248 us, 27 neighbours
+// 483 -> 387 us.)
+// DERIV: fc'/fc too (the adjoint).  sH comes with 1/r in place (stage_buckets).
+template <typename T, bool DERIV>
 __device__ __forceinline__ void need_factors(FactorKey<T>& key, const PairList& L,
                                              const typename V4<T>::type* sR, T Rc, T a, T a2,
                                              const T (&eta)[BE], typename V4<T>::type* sH,
                                              int lane) {
+  using T4 = typename V4<T>::type;
   if (key.eta0 != eta[0] || key.eta1 != eta[1] || key.Rc != Rc) {
     key.eta0 = eta[0];
     key.eta1 = eta[1];
     key.Rc = Rc;
     key.filled = 0u;
   }
+  const int nr = key.filled >> L.rs & 1u ? 0 : L.mr;
+  const int n = nr + (L.tri || (key.filled >> L.cs & 1u) ? 0 : L.mc);
   __syncwarp();   // the previous list's readers are done
-  if (!(key.filled >> L.rs & 1u)) fill_factors<T>(sR, Rc, a, a2, eta, L.r0, L.r0 + L.mr, sH, lane);
-  if (!L.tri && !(key.filled >> L.cs & 1u))
-    fill_factors<T>(sR, Rc, a, a2, eta, L.c0, L.c0 + L.mc, sH, lane);
+  for (int q = lane; q < n; q += 32) {
+    const int j = q < nr ? L.r0 + q : L.c0 + q - nr;
+    const T r = sR[j].w, x = r * r;
+    T fc, dfc;
+    cut_r<DERIV>(r, Rc * Rc, a2, a, fc, dfc);
+    fc = fc_floor(fc);
+    T4 h = sH[j];
+    h.x = exp_fill(-eta[0] * x) * fc;
+    h.y = exp_fill(-eta[1] * x) * fc;
+    if (DERIV) h.w = quotient(dfc, fc);
+    if (!(x < Rc * Rc)) h.x = h.y = T(0);
+    sH[j] = h;
+  }
   key.filled |= (1u << L.rs) | (1u << L.cs);
   __syncwarp();
 }
@@ -482,7 +497,7 @@ struct WarpMem {
 };
 
 // Shared memory of one warp: the staged neighbours (x, y, z, r), their
-// factors (first 1/r, fc, dfc at the table's largest Rc for the radial
+// factors (first dfc, fc, 1/r at the table's largest Rc for the radial
 // functions, then those of the grids), FP32 positions for the pair test (FP64
 // kernels), in the adjoint the accumulators and the scaled dE/dG row, the
 // table slot of each staged neighbour and the pair queue.
@@ -688,7 +703,7 @@ __device__ void forward_grid(const BehlerGrid* gr, const PairList& L, const Warp
       GridBlock<T> B;
       B.load(gr, CHAIN, NZ * pass, e0);
       const int nz = CHAIN ? gr->chain : min(NZ, gr->ngeneral - NZ * pass);
-      need_factors<T>(key, L, w.sR, Rc, a, a2, B.eta, w.sH, lane);
+      need_factors<T, false>(key, L, w.sR, Rc, a, a2, B.eta, w.sH, lane);
       T acc[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) acc[q] = T(0);
@@ -794,13 +809,10 @@ struct ListOf {
   __device__ __forceinline__ bool first() const { return !SPLIT || blockIdx.y == 0; }
   __device__ __forceinline__ bool list(int x, int y) const { return !SPLIT || (x == a && y == c); }
   // whether this block sets feature k
-  __device__ __forceinline__ bool mine(const BehlerTable* tab, int nt, int k) const {
+  __device__ __forceinline__ bool mine(const BehlerTable* tab, int k) const {
     if (!SPLIT) return true;
-    for (int x = 0; x < nt; ++x)
-      for (int y = x; y < nt; ++y)
-        for (int q = tab->ang_off[x * nt + y]; q < tab->ang_off[x * nt + y + 1]; ++q)
-          if (tab->fn[q].out == k) return list(x, y);
-    return first();
+    const int u = tab->list_of[k];
+    return u < 0 ? first() : u == (int)blockIdx.y;
   }
   // whether staged neighbour j can have a force from this block
   __device__ __forceinline__ bool touches(const int* bstart, int j) const {
@@ -865,7 +877,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? FWD_BLOCKS : 1) k_behler_
   // features that no function feeds are normalised zeros (symmfunc.f90:367);
   // a block with one list of its own leaves the other lists' alone
   for (int k = lane; k < nsf; k += 32)
-    if (of.mine(tab, nt, k)) G[k] = normalise(T(0), pd, nrow + k);
+    if (of.mine(tab, k)) G[k] = normalise(T(0), pd, nrow + k);
   __syncwarp();
 
   // ---- radial lists: function by function, lanes over the bucket's
@@ -1039,7 +1051,7 @@ __device__ void adjoint_grid(const BehlerGrid* gr, const PairList& L, const Warp
                                             lane / BE % NZ, lane % BE);
         w.sB[lane] = f >= 0 ? T(2) * w.sg[f] : T(0);
       }
-      need_factors<T>(key, L, w.sR, Rc, a, a2, B.eta, w.sH, lane);
+      need_factors<T, true>(key, L, w.sR, Rc, a, a2, B.eta, w.sH, lane);
       run_pairs(L, w.sP, g4, filter_rc2(Rc), w.queue, lane, [&](bool live, int j, int k, int step) {
         const T4 Rj = w.sR[j], Rk = w.sR[k], Hj = w.sH[j], Hk = w.sH[k];
         const T invj = Hj.z, invk = Hk.z;
@@ -1169,7 +1181,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? ADJ_BLOCKS : 1) k_behler_
     }
     // FP64 sums coefficients of R_j, FP32 the vector
     T4 acc = w.sR[j];
-    c *= A.x;
+    c *= A.z;
     const T cv = sizeof(T) == 8 ? T(0) : c;
     acc.x *= cv;
     acc.y *= cv;
