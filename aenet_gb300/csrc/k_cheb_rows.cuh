@@ -1099,15 +1099,19 @@ int launch(const PotDevice& pd, const DescBuffers& b, bool adjoint, cudaStream_t
   int dev = 0, nsm = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // several groups share a block while three blocks still fit an SM (as asked:
-  // while they fit at all)
-  const size_t three = SMEM_MAX / 3, one = group_smem<T, R, A, SPIN, MOM>(pd, b, true);
+  // long rows leave room for few warps on an SM, and few warps wait for each
+  // other's latencies: groups share a warp while 16 warps (FP64 8) still fit (as
+  // asked: while one does).  21,658 atoms of 64 neighbours, nearly all angular,
+  // mixed, descriptor and adjoint with 8, 16 and 32 lanes (24, 12 and 6 KB a
+  // warp): 619 + 725, - + 449 and 404 + 377 us
+  const size_t one = group_smem<T, R, A, SPIN, MOM>(pd, b, true);
+  const size_t room = b.lpa ? SMEM_MAX : SMEM_MAX / (sizeof(T) == 4 ? 16 : 8);
   constexpr bool PAIRS32 = sizeof(T) == 4 && !MOM;
   constexpr int LINE16 = PAIRS32 ? 16 : 8, LINE8 = PAIRS32 ? 42 : 20;   // atoms per SM
   int lanes = b.lpa ? b.lpa : b.natoms >= LINE8 * nsm ? 8 : b.natoms >= LINE16 * nsm ? 16 : 32;
-  while (lanes < 32 && 32 / lanes * one > (b.lpa ? SMEM_MAX : three)) lanes *= 2;
+  while (lanes < 32 && 32 / lanes * one > room) lanes *= 2;
   // four warps per block once they fill the SMs (FP32)
-  const int warps = sizeof(T) == 4 && b.natoms >= 64 * nsm && 16 * one <= three ? 4 : 1;
+  const int warps = sizeof(T) == 4 && b.natoms >= 64 * nsm && 16 * one <= SMEM_MAX / 3 ? 4 : 1;
   if (lanes == 8) return launch_lanes<T, R, A, 8, GUARD, SPIN, MOM>(pd, b, adjoint, warps, 1, s);
   if (lanes == 16) return launch_lanes<T, R, A, 16, GUARD, SPIN, MOM>(pd, b, adjoint, 1, 1, s);
   // Blocks per atom in the FP64 pair adjoint: a scheduler starts one FP64
