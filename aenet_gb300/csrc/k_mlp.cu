@@ -492,6 +492,7 @@ int ae_launch_types(int natoms, const int* types1, int* types0, int ntypes, unsi
 }
 
 namespace {
+constexpr size_t MLP_SMEM_MAX = 227 * 1024;   // (no static shared memory beside it)
 template <typename T>
 size_t mlp_smem(int wtotal) {
   return sizeof(T) * ((((size_t)wtotal + 1) & ~(size_t)1) + (size_t)MLP_WARPS * mlp_warp_elems());
@@ -501,37 +502,42 @@ template <typename T>
 int launch_mlp(const PotDevice& pd, const DescBuffers& b, const T* W, int wtotal, int nsm,
                cudaStream_t s) {
   const size_t smem = mlp_smem<T>(wtotal);
-  allow_smem(k_mlp<T>, smem, AE_SMEM_MAX);
+  allow_smem(k_mlp<T>, smem, MLP_SMEM_MAX);
   const int blocks = min((b.natoms + MLP_WARPS - 1) / MLP_WARPS, nsm * 4);
   launch_next(k_mlp<T>, blocks, 32 * MLP_WARPS, smem, s, pd, b, W, wtotal);
   return (int)cudaGetLastError();
 }
 
-// Whether the FP64 networks go by tiles of atoms (k_mlp64): where their layers
-// leave lanes of a warp per atom idle, and the atoms fill the SMs.  The
-// measure is the FP64 instructions of an atom's layers, a warp each and
-// flattened, with tanh at 45 (the library's two branches) and 32.  A warp per
-// atom and tiles (us): 26-20-20-1 2,304 atoms 31 and 33, 2,916 55 and 45, 32,000
-// 348 and 252; 40-25-25-1 two species 2,916 74 and 55, 10,976 170 and 158; but
-// 32-32-32-1 three species 8,255 125 and 165, 72,519 967 and 942, rutile's 9,000
-// 170 and 207; eight species 32-32-32-1 of 1,000 atoms 31 and 74 (four warps
-// wait for 200 KB of weights).  Few atoms of one small network: 256 atoms
-// 26-20-20-1 20 and 17, 864 21 and 23.
+// Whether the FP64 networks go by tiles of atoms (k_mlp64): where their layers,
+// of up to 32 nodes, leave a third of the lanes of a warp per atom idle, the
+// weights leave room for several blocks on an SM, and the atoms fill the SMs
+// (or, for one small network, are few).  The measure is the FP64 instructions
+// of an atom's layers, a warp each and flattened, with tanh at 45 (the
+// library's two branches) and 32.  A warp per atom and tiles (us): 26-20-20-1
+// 2,304 atoms 31 and 33, 2,916 55 and 45, 32,000 348 and 252, 256 20 and 17, 864
+// 21 and 23; 40-25-25-1 two species 2,916 74 and 55, 10,976 170 and 158; but
+// 32-32-32-1 three species 8,255 125 and 165, 72,519 967 and 942; rutile's 9,000
+// 170 and 207; 32-50-50-1 1.0 to 1.2 times as long by tiles; five species
+// 57-20-20-1 (63 KB of weights) of 4,496 72 and 119, eight species 32-32-32-1 of
+// 1,000 31 and 74.
 bool networks_in_tiles(const PotDevice& pd, const DescBuffers& b, int wtotal, int nsm) {
-  if (mlp_smem<double>(wtotal) > AE_SMEM_MAX) return true;
+  if (mlp_smem<double>(wtotal) > MLP_SMEM_MAX) return true;
+  if (wtotal > 4096) return false;
   const bool many = b.natoms >= 16 * nsm;
   const bool few = b.natoms >= 32 && b.natoms <= 4 * nsm && wtotal <= 2048;
   if (!many && !few) return false;
   long long warp = 0, flat = 0;   // 32 lanes each
+  int widest = 0;
   for (int t = 0; t < pd.ntypes; ++t) {
     const NetTable& net = pd.sp[t].net;
     for (int l = 0; l + 1 < net.nlayers - 1; ++l) {
       const int in = net.nnodes[l], out = net.nnodes[l + 1];
+      widest = max(widest, out);
       warp += 32 * ((out + 31) / 32 * (in + 45) + (in + 31) / 32 * out);
       flat += out * (in + 32) + in * out;
     }
   }
-  return 10 * warp >= 14 * flat;
+  return widest <= 32 && 10 * warp >= 15 * flat;
 }
 
 int launch_mlp64(const PotDevice& pd, const DescBuffers& b, int wtotal, int nsm, cudaStream_t s) {
