@@ -72,8 +72,10 @@ constexpr int AT_LPF = 8;                     // lanes per feature sum
 constexpr int AT_LPA = 4;                     // lanes per angular neighbour's gradient
 constexpr int AT_NSTRIDE = AE_MAXNODES + 1;
 constexpr int AC_CTAS = 8;                    // blocks of the cluster form
-constexpr int AT_WMAX = 4096;                 // network weights staged in shared memory
-                                              // (doubles; larger networks read L2)
+constexpr int AT_WMAX = 8192;                 // network weights staged in shared memory
+                                              // (doubles; larger networks read L2: calls
+                                              // of 12 neighbours, 32-40-56-51-1 and eight
+                                              // species, 62 us from there and 53 staged)
 
 template <int RB, int AB>
 __host__ __device__ constexpr size_t at_red_elems() {
