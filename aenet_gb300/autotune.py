@@ -5,7 +5,8 @@ kernel (one warp per atom over the full or the half stencil, or per home
 cell with a lane per home atom or a lane per candidate), the number of neighbour-search cells per cut-off
 length (1, 2 or 3), their refinement along the third axis (1, 2 or 4) and
 the number of lanes that cooperate on one atom in the Chebyshev descriptor
-and adjoint kernels (8, 32, or by the number of atoms: 16).  The first three
+and adjoint kernels (8, from 20 atoms per SM on, 32, or by the number of
+atoms: 16).  The first three
 only change the neighbour search and the last only the descriptor kernels,
 so :func:`tune` times a full energy-and-force pass of the caller's batch
 (CUDA events on the current stream) over the kernel and cell size at the
@@ -90,7 +91,10 @@ def tune(natoms, cells, pbc, positions, types, precision=core.MIXED, key=None, r
         plan = Plan(natoms, cells, pbc, precision=precision, coords0=positions)
         ms, lp = _time(plan, p, t, reps), lp0
         first = ms
+        nsm = torch.cuda.get_device_properties(p.device).multi_processor_count
         for q in lanes[1:]:
+            if q == 8 and lp0 == 16 and len(t) < 20 * nsm:
+                continue                     # (the same launches)
             core.set_option("lanes_per_atom", q)
             results.append((_time(plan, p, t, reps), q, cd, nk))
             if results[-1][0] < min(ms, GAIN * first):

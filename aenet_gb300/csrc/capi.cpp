@@ -1402,7 +1402,7 @@ DescBuffers desc_buffers(aenet_gpu_plan* P, const double* grad_scale, bool viria
   d.nb_vec = P->nb_vec;
   d.cap = P->cap;
   d.cap_a = P->cap_a;
-  d.lpa = ae_lanes_per_atom();
+  d.lpa = ae_lanes_per_atom(P->natoms);
   d.G = P->G;
   d.dEdG = P->dEdG;
   d.E_atom = P->E_atom;
@@ -3266,7 +3266,16 @@ int ae_device_tables(PotDevice* out, double* rc, int* cell_div) {
   return 0;
 }
 
-int ae_lanes_per_atom() { return g.lpa_default == 16 ? 0 : g.lpa_default; }
+// The lanes asked for the descriptor kernels, or 0: by the number of atoms.  8
+// leave fewer than two warps a scheduler below 20 atoms per SM: a shape chosen for
+// a large batch took 164 us instead of 98 for 446 atoms (Li/Si/O, FP64).
+int ae_lanes_per_atom(int natoms) {
+  if (g.lpa_default != 8) return g.lpa_default == 16 ? 0 : g.lpa_default;
+  int dev = 0, nsm = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return natoms >= 20 * nsm ? 8 : 0;
+}
 
 // Geometry of one periodic structure (host arithmetic only).
 int ae_periodic_geom(StructGeom* G, const double* lattice, int natoms, double rc, int cell_div) {

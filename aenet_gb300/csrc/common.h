@@ -330,7 +330,7 @@ int ae_launch_stale_order(int natoms, const StructGeom* geom, const int* atom_st
 
 // whether the potentials' passes keep moments (DescBuffers::M, M64)
 bool ae_cheb_moments(const PotDevice& pd, int fp64);
-int ae_lanes_per_atom();
+int ae_lanes_per_atom(int natoms);
 int ae_launch_chebyshev_forward(const PotDevice& pd, const DescBuffers& b,
                                 int fp64, cudaStream_t s);
 // One FP64 Chebyshev atom per launch (the per-atom entry points): one

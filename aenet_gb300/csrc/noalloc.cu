@@ -178,7 +178,7 @@ extern "C" __attribute__((visibility("default"))) int aenet_gpu_structure_energy
     ca = (ca + 7) & ~7;
     d.cap_a = std::min(std::max(ca, 8), (int)NA_NB);
   }
-  d.lpa = ae_lanes_per_atom();
+  d.lpa = ae_lanes_per_atom(natoms);
   d.G = b + O_G;
   d.dEdG = b + O_DG;
   d.E_atom = (double*)(b + O_EA);

@@ -46,8 +46,9 @@ extern "C" {
  *       finely to the cut-off sphere (performance only).
  *   "lanes_per_atom" = "8" | "16" | "32"   lanes per atom of the Chebyshev
  *       descriptor and adjoint kernels; 16 (the default) leaves them to the
- *       number of atoms, and all are raised where a block's rows would not fit
- *       its shared memory (performance only).
+ *       number of atoms, as 8 does below 20 atoms per multiprocessor, and all
+ *       are raised where a block's rows would not fit its shared memory
+ *       (performance only).
  *   "adjoint_lanes_per_atom" = "0" | "8" | "16" | "32"   those of the adjoint
  *       kernels, as given; 0 follows lanes_per_atom (performance only).
  *   "neighbour_kernel" = "atom" | "cell" | "stream" | "half" | "struct" |
