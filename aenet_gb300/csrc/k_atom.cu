@@ -29,7 +29,7 @@
 // (cutoff64.cuh), constants divided on the host, spin sums only where there
 // are spins, derivatives as sums over q U_(q-1) with the order multiplied
 // into the coefficients once, tanh without branches and pair gradients from
-// sums of scalars instead of two vectors a pair: the kernel 41 -> 30 us, the
+// sums of scalars instead of two vectors a pair: the kernel 41 -> 31 us, the
 // phases before 7,600, 8,900, 19,000, 27,500 and 2,300 cycles.
 //
 // In the cluster each block stages a contiguous slice of the rows and takes

@@ -22,8 +22,8 @@
 // per clock and SM, 75-80 % busy) in FP64; the neighbour rows fit L2.
 // Measured on rutile Ti/O with 64 functions, before (an exponential of the
 // whole sum per eta and pair, sin/cos of r_jk, shared-memory atomics in the
-// adjoint) and now: 9,000 atoms mixed, forward 324 -> 243 us, adjoint 717 ->
-// 431 us; 763 atoms FP64, forward 1160 -> 515 us, adjoint 1733 -> 897 us.
+// adjoint) and now: 9,000 atoms mixed, forward 324 -> 238 us, adjoint 717 ->
+// 429 us; 763 atoms FP64, forward 1160 -> 487 us, adjoint 1733 -> 889 us.
 // The tables come from build_behler (capi.cpp): they already encode the
 // reference's indexing (functions registered under the global species
 // index, evaluated with the central atom's local one) and the feature

@@ -5,7 +5,8 @@
 //
 // Weights of every species are staged once per block in shared memory;
 // blocks are persistent (grid-stride over atoms), one warp per atom, lane o
-// computing node o of a layer.  Rows of a layer's weight matrix are stored
+// computing node o of a layer, or (FP64, networks_in_tiles) a warp per eight
+// atoms.  Rows of a layer's weight matrix are stored
 // W[o][k] with the bias in column n_in and an odd row pitch, so that both
 // the forward pass (lanes over rows) and the backward pass (lanes over
 // columns) read shared memory without bank conflicts.
